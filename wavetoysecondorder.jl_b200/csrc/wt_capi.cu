@@ -442,6 +442,17 @@ int ensure_mu(wt_ws* ws) {
   return 0;
 }
 
+// dstP += koT sum_d D_d^6 fP and dstQ += koT sum_d D_d^6 fQ, both fields in each launch.
+int ko_add2(wt_ctx* ctx, const wt::DevMesh& m, void* dstP, const void* fP, void* dstQ, const void* fQ, double koT,
+            void* scratch) {
+  void* dst[2] = {dstP, dstQ};
+  const void* f[2] = {fP, fQ};
+  int launched = 0;
+  const int rc = lrc(ctx, wt::launch_ko_add(m, 2, dst, f, koT, ctx->stream, scratch, &launched), "Kreiss-Oliger");
+  ctx->launches += launched;
+  return rc;
+}
+
 // One RHS evaluation of the conservative system (non-fused).
 int rhs_curved_impl(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, const void* Phi, const void* Pi, void* Phid,
                     void* Pid, double eps_ko, const wt::ConsBC& bc, int use_metric) {
@@ -454,11 +465,8 @@ int rhs_curved_impl(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, const void* Phi
              "rhs K2"));
   ctx->launches += 2;
   if (eps_ko != 0.0) {
-    const double koT = eps_ko * ws->inv_mu5;
     // the flux scratch is free once K2 has run
-    WT_TRY(lrc(ctx, wt::launch_ko_add(m, Phid, Phi, koT, ctx->stream, ws->F), "Kreiss-Oliger"));
-    WT_TRY(lrc(ctx, wt::launch_ko_add(m, Pid, Pi, koT, ctx->stream, ws->F), "Kreiss-Oliger"));
-    ctx->launches += 6;
+    WT_TRY(ko_add2(ctx, m, Phid, Phi, Pid, Pi, eps_ko * ws->inv_mu5, ws->F));
   }
   return 0;
 }
@@ -1304,9 +1312,11 @@ int wt_ko_add(wt_ctx* ctx, wt_ws* ws, void* dst, const void* field, double eps_k
   if (!dst || !field) return fail(ctx, WT_EINVAL, "wt_ko_add: NULL argument");
   WT_TRY(ensure_mu(ws));
   WT_TRY(ws_buffers(ws));
-  ctx->launches += 3;
-  return lrc(ctx, wt::launch_ko_add(ws->mesh->m, dst, field, eps_ko * ws->inv_mu5, ctx->stream, ws->F),
-             "Kreiss-Oliger");
+  int launched = 0;
+  const int rc = lrc(ctx, wt::launch_ko_add(ws->mesh->m, 1, &dst, &field, eps_ko * ws->inv_mu5, ctx->stream, ws->F,
+                                            &launched), "Kreiss-Oliger");
+  ctx->launches += launched;
+  return rc;
 }
 
 int wt_gradient3d(wt_ctx* ctx, wt_ws* ws, const void* u, void* g1, void* g2, void* g3) {
@@ -2102,10 +2112,7 @@ static int step_sipg_once(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, 
     WT_TRY(wt_rhs_sipg(ctx, ws, inU, inV, ws->kQ, bv, tau, R));
     cudaMemcpyAsync(ws->kP, inV, nb, cudaMemcpyDeviceToDevice, s);
     if (eps_ko != 0.0) {
-      const double koT = eps_ko * ws->inv_mu5;
-      WT_TRY(lrc(ctx, wt::launch_ko_add(m, ws->kP, inU, koT, s, ws->F), "Kreiss-Oliger"));
-      WT_TRY(lrc(ctx, wt::launch_ko_add(m, ws->kQ, inV, koT, s, ws->F), "Kreiss-Oliger"));
-      ctx->launches += 6;
+      WT_TRY(ko_add2(ctx, m, ws->kP, inU, ws->kQ, inV, eps_ko * ws->inv_mu5, ws->F));
     }
     WT_TRY(lrc(ctx, wt::launch_rk_update(m.nn, m.precision, st, dt, u, ws->accP, ws->S0, ws->kP, s), "rk4"));
     WT_TRY(lrc(ctx, wt::launch_rk_update(m.nn, m.precision, st, dt, ut, ws->accQ, ws->SQ, ws->kQ, s), "rk4"));
@@ -2873,11 +2880,8 @@ int wt_rhs_curved_noalloc(wt_ctx* ctx, const wt_coef* coef, const void* Phi, con
   WT_TRY(lrc(ctx, wt::launch_cons_k2(m, F, Pidot, bbuf, use_metric, b, rk, nullptr, ctx->stream, n8), "rhs K2"));
   ctx->launches += 2;
   if (eps_ko != 0.0) {
-    const double koT = eps_ko * std::pow(1.0 / mu, 5);
     // the flux scratch is free once K2 has run
-    WT_TRY(lrc(ctx, wt::launch_ko_add(m, Phidot, Phi, koT, ctx->stream, F), "Kreiss-Oliger"));
-    WT_TRY(lrc(ctx, wt::launch_ko_add(m, Pidot, Pi, koT, ctx->stream, F), "Kreiss-Oliger"));
-    ctx->launches += 6;
+    WT_TRY(ko_add2(ctx, m, Phidot, Phi, Pidot, Pi, eps_ko * std::pow(1.0 / mu, 5), F));
   }
   return 0;
 }

@@ -369,9 +369,17 @@ size_t cons_gen_param_size(int precision, int which);
 void cons_gen_fill_params(int which, const SolveStage& ss, unsigned* flag, void* dst);
 int launch_cons_gen_batch(int which, int N, int precision, int epb_variant, int cp, const void* plist, const int2* tiles,
                           long long ntiles, cudaStream_t s);
-// dst += koT * sum_d D_d^6 field; scratch (2 nn words, may be NULL when every
-// axis has straight element lines) serves meshes without them
-int launch_ko_add(const DevMesh& m, void* dst, const void* field, double koT, cudaStream_t s, void* scratch);
+// Kreiss-Oliger (wt_ko.cu): dst[q] += koT * sum_d D_d^6 field[q] for nf <= 2 fields;
+// scratch (2 nn words, may be NULL when every axis has straight element lines)
+// serves meshes without them.  *launches grows by the kernels launched.
+int launch_ko_add(const DevMesh& m, int nf, void* const* dst, const void* const* field, double koT, cudaStream_t s,
+                  void* scratch, int* launches);
+// out[q] = koT * sum_d D_d^6 field[q], on meshes whose every axis has straight
+// lines (ko_all_lines).  split = 1: the three axes in one launch, axis d's part
+// in out[q] + d nn; split = 0: three launches, the sum in out[q].
+bool ko_all_lines(const DevMesh& m);
+int launch_ko_fields(const DevMesh& m, int nf, void* const* out, const void* const* field, double koT, int split,
+                     cudaStream_t s, int* launches);
 int launch_div3d(const DevMesh& m, const void* F, void* out, cudaStream_t s);
 
 // second-order forms (wt_second.cu)

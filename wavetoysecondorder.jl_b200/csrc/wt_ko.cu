@@ -1,0 +1,294 @@
+// wt_ko.cu -- Kreiss-Oliger dissipation eps mu^-5 sum_d D_d^6 of up to two
+// fields (src/wave3d_curved.jl:182-192) along whole grid lines.
+//
+// D_d (apply_D!) couples only the nodes of one axis-d grid line
+// (METHODS.md:151-155), so a thread keeps one pencil of one element (N values)
+// in registers and the threads of a CTA hold whole element lines: applying D_d
+// six times needs, per pass, only the two end values of the pencils next to it.
+//
+// What bounds it: per axis and field 3 words of DRAM traffic per node (the
+// field in, the destination in and out) against 6 N multiply-adds, which FP64
+// at N = 8 would make the longer of the two.  The derivative matrix is
+// antisymmetric about its centre (G[N-1-i][N-1-p] = -G[i][p]), so in the basis
+// of sums and differences of mirrored values a pass is two half-size products,
+// N^2/2 multiply-adds per pencil, and the six passes stay in that basis.  The
+// half-size matrices are kernel parameters (constant bank: no shared-memory
+// operand loads).  Only the end values go through shared memory, double
+// buffered, one barrier per pass.  Axis 0 pencils are contiguous in memory:
+// each warp transposes its 32 pencils through a padded shared buffer of its
+// own; along axes 1 and 2 consecutive threads hold consecutive nodes and load
+// directly.
+//
+// Measured (FP64, one axis of two fields, B200): 24^3 elements of n = 8, 86 us
+// (3.9 TB/s; the whole pencils through shared memory on every pass, two
+// barriers each and the matrix read from shared memory: 212 us); 40^3 of n = 6,
+// 177 us (before: 450 us).
+#include "wt_common.cuh"
+
+#include <algorithm>
+#include <vector>
+
+namespace wt {
+
+template <int N, typename real>
+struct KoP {
+  static constexpr int M = (N + 1) / 2, HH = N / 2;
+  real A[M * HH];  // even part of D v from the differences: A[i][p] = G[i][p] - G[i][N-1-p]; centre row G[c][p]
+  real B[HH * M];  // odd part of D v from the sums: G[i][p] + G[i][N-1-p]; centre column 2 G[i][c]
+  const real* f[2];
+  real* out[2];
+  long long ostride;  // words between the outputs of consecutive axes (0: one output)
+  int rmw;            // 1: out += koT D^6 f, 0: out = koT D^6 f
+  real koT, cH;       // cH = 1 / (2 H_end)
+  const real* sdiag;
+  int nax;
+  struct Axis {
+    int d, len, closed, pb;  // axis, elements per line, periodic, pencils per CTA
+    unsigned b0;             // first CTA of the axis
+    const int32_t* lines;
+  } ax[3];
+};
+
+// CTA: pb pencils of one element line, thread (pencil, element) with the pencil fastest.
+template <int N, typename real, int TMAX>
+__global__ void __launch_bounds__(TMAX) k_ko(const __grid_constant__ KoP<N, real> P) {
+  constexpr int N2 = N * N, N3 = N * N * N, M = KoP<N, real>::M, HH = KoP<N, real>::HH;
+  constexpr int NP = N | 1;  // odd pitch of a staged pencil: no bank conflicts
+  extern __shared__ __align__(16) unsigned char smraw[];
+  real* ends = reinterpret_cast<real*>(smraw);  // [2 buffers][low, high end][thread]
+  const int T = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31;
+  real* stage = ends + 4 * T + (tid >> 5) * 32 * NP;  // this warp's staged pencils (axis 0)
+  int d = P.ax[0].d, len = P.ax[0].len, closed = P.ax[0].closed, PB = P.ax[0].pb, a = 0;
+  unsigned b0 = P.ax[0].b0;
+  const int32_t* lines = P.ax[0].lines;
+#pragma unroll
+  for (int q = 1; q < 3; ++q)
+    if (q < P.nax && blockIdx.x >= P.ax[q].b0) {
+      d = P.ax[q].d; len = P.ax[q].len; closed = P.ax[q].closed; PB = P.ax[q].pb; b0 = P.ax[q].b0;
+      lines = P.ax[q].lines; a = q;
+    }
+  const real* __restrict__ f = blockIdx.y ? P.f[1] : P.f[0];
+  real* __restrict__ out = (blockIdx.y ? P.out[1] : P.out[0]) + a * P.ostride;
+  const int parts = N2 / PB;
+  const unsigned blk = blockIdx.x - b0;
+  const int line = blk / parts, part = blk - line * parts;
+  const int pb = tid % PB, sg = tid / PB;
+  const bool act = sg < len;
+  long long base = -1;
+  int stride = 1;
+  real s = 0;
+  if (act) {
+    const int e = lines[(long long)line * len + sg];
+    s = P.sdiag[3 * (long long)e + d];
+    const int pp = part * PB + pb;  // the pencil, its first tangential index fastest
+    if (d == 0) { base = (long long)e * N3 + N * pp; }
+    else if (d == 1) { base = (long long)e * N3 + pp % N + N2 * (pp / N); stride = N; }
+    else { base = (long long)e * N3 + pp; stride = N2; }
+  }
+  real v[N];
+  if (d == 0) {
+#pragma unroll
+    for (int it = 0; it < N; ++it) {
+      const int q = it * 32 + lane, pr = q / N;
+      const long long bs = __shfl_sync(0xffffffffu, base, pr);
+      stage[pr * NP + q % N] = bs >= 0 ? f[bs + q % N] : (real)0;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int l = 0; l < N; ++l) v[l] = stage[lane * NP + l];
+    __syncwarp();
+  } else {
+#pragma unroll
+    for (int l = 0; l < N; ++l) v[l] = act ? f[base + l * stride] : (real)0;
+  }
+  real ev[M], od[HH];
+#pragma unroll
+  for (int i = 0; i < HH; ++i) {
+    ev[i] = v[i] + v[N - 1 - i];
+    od[i] = v[i] - v[N - 1 - i];
+  }
+  if (N & 1) ev[M - 1] = v[HH];
+  const bool has_prev = act && (closed || sg > 0), has_next = act && (closed || sg < len - 1);
+  const int tp = pb + PB * (sg == 0 ? len - 1 : sg - 1), tn = pb + PB * (sg == len - 1 ? 0 : sg + 1);
+#pragma unroll 1
+  for (int it = 0; it < 6; ++it) {
+    real* eb = ends + (it & 1) * 2 * T;
+    const real vl = (real)0.5 * (ev[0] + od[0]), vh = (real)0.5 * (ev[0] - od[0]);
+    eb[tid] = vl;
+    eb[T + tid] = vh;
+    __syncthreads();
+    // the centred-flux SAT of the two end nodes, in the sum / difference basis
+    const real lo = has_prev ? P.cH * (vl - eb[T + tp]) : (real)0;
+    const real hi = has_next ? P.cH * (eb[tn] - vh) : (real)0;
+    real ne[M], no[HH];
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+      real acc = i == 0 ? lo + hi : (real)0;
+#pragma unroll
+      for (int p = 0; p < HH; ++p) acc += P.A[i * HH + p] * od[p];
+      ne[i] = s * acc;
+    }
+#pragma unroll
+    for (int i = 0; i < HH; ++i) {
+      real acc = i == 0 ? lo - hi : (real)0;
+#pragma unroll
+      for (int p = 0; p < M; ++p) acc += P.B[i * M + p] * ev[p];
+      no[i] = s * acc;
+    }
+#pragma unroll
+    for (int i = 0; i < M; ++i) ev[i] = ne[i];
+#pragma unroll
+    for (int i = 0; i < HH; ++i) od[i] = no[i];
+  }
+#pragma unroll
+  for (int i = 0; i < HH; ++i) {
+    v[i] = P.koT * ((real)0.5 * (ev[i] + od[i]));
+    v[N - 1 - i] = P.koT * ((real)0.5 * (ev[i] - od[i]));
+  }
+  if (N & 1) v[HH] = P.koT * ev[M - 1];
+  if (d == 0) {
+#pragma unroll
+    for (int l = 0; l < N; ++l) stage[lane * NP + l] = v[l];
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < N; ++it) {
+      const int q = it * 32 + lane, pr = q / N;
+      const long long bs = __shfl_sync(0xffffffffu, base, pr);
+      if (bs >= 0) {
+        const long long n = bs + q % N;
+        out[n] = P.rmw ? out[n] + stage[pr * NP + q % N] : stage[pr * NP + q % N];
+      }
+    }
+  } else if (act) {
+    if (P.rmw) {
+#pragma unroll
+      for (int l = 0; l < N; ++l) v[l] += out[base + l * stride];
+    }
+#pragma unroll
+    for (int l = 0; l < N; ++l) out[base + l * stride] = v[l];
+  }
+}
+
+template <int N, typename real, int TMAX>
+static int ko_run(const KoP<N, real>& P, unsigned blocks, int nf, int threads, cudaStream_t s) {
+  const size_t smem = (size_t)threads * (4 + (N | 1)) * sizeof(real);
+  if (smem > 48 * 1024) {
+    // set on every launch that needs it: the attribute belongs to the current device
+    if (cudaFuncSetAttribute(k_ko<N, real, TMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return -2;
+  }
+  k_ko<N, real, TMAX><<<dim3(blocks, nf), threads, smem, s>>>(P);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <int N, typename real>
+static int ko_lines_n(const DevMesh& m, const int* axes, int nax, int nf, void* const* out, long long ostride, int rmw,
+                      const void* const* f, double koT, cudaStream_t s) {
+  KoP<N, real> P;
+  constexpr int M = KoP<N, real>::M, HH = KoP<N, real>::HH;
+  const std::vector<double>& G = m.ops.G;
+  for (int i = 0; i < M; ++i)
+    for (int p = 0; p < HH; ++p)
+      P.A[i * HH + p] = (real)((N & 1) && i == M - 1 ? G[i * N + p] : G[i * N + p] - G[i * N + N - 1 - p]);
+  for (int i = 0; i < HH; ++i)
+    for (int p = 0; p < M; ++p)
+      P.B[i * M + p] = (real)((N & 1) && p == M - 1 ? 2.0 * G[i * N + p] : G[i * N + p] + G[i * N + N - 1 - p]);
+  for (int q = 0; q < 2; ++q) {
+    P.f[q] = (const real*)f[q < nf ? q : 0];
+    P.out[q] = (real*)out[q < nf ? q : 0];
+  }
+  P.ostride = ostride;
+  P.rmw = rmw;
+  P.koT = (real)koT;
+  P.cH = (real)(1.0 / (2.0 * m.ops.H[0]));
+  P.sdiag = (const real*)m.sdiag;
+  P.nax = nax;
+  unsigned blocks = 0;
+  int threads = 32;
+  for (int q = 0; q < nax; ++q) {
+    const int d = axes[q], len = m.line_len[d];
+    // pencils per CTA: the most (a divisor of N times N) that keeps a CTA at
+    // 512 threads or fewer, so that along axis 2 a load covers whole sectors and
+    // short lines still fill a CTA; very long lines keep the N pencils of one plane
+    int g = N;
+    while (g > 1 && (N % g != 0 || len * N * g > 512)) --g;
+    auto& A = P.ax[q];
+    A.d = d; A.len = len; A.closed = m.line_closed[d]; A.pb = N * g; A.b0 = blocks; A.lines = m.lines[d];
+    blocks += (unsigned)m.nlines[d] * (unsigned)(N / g);
+    threads = std::max(threads, (len * N * g + 31) / 32 * 32);
+  }
+  for (int q = nax; q < 3; ++q) P.ax[q] = P.ax[0];
+  if (blocks == 0 || nf == 0) return 0;
+  return threads <= 512 ? ko_run<N, real, 512>(P, blocks, nf, threads, s)
+                        : ko_run<N, real, 1024>(P, blocks, nf, threads, s);
+}
+
+static int ko_lines(const DevMesh& m, const int* axes, int nax, int nf, void* const* out, long long ostride, int rmw,
+                    const void* const* f, double koT, cudaStream_t s) {
+#define WT_KO_CASE(NN)                                                                                    \
+  case NN:                                                                                                \
+    return m.precision == 0 ? ko_lines_n<NN, double>(m, axes, nax, nf, out, ostride, rmw, f, koT, s)      \
+                            : ko_lines_n<NN, float>(m, axes, nax, nf, out, ostride, rmw, f, koT, s);
+  switch (m.N) {
+    WT_KO_CASE(2) WT_KO_CASE(3) WT_KO_CASE(4) WT_KO_CASE(5) WT_KO_CASE(6) WT_KO_CASE(7) WT_KO_CASE(8)
+    default: return -4;
+  }
+#undef WT_KO_CASE
+}
+
+// Axes whose elements form straight lines short enough for one CTA run line-
+// locally; the others (multi-patch meshes, whose axis-d neighbours may meet at
+// another face or orientation) as the reference's _ko_axis3! does it
+// (src/wave3d_curved.jl:182-192): six apply_D! calls ping-ponging through scratch
+// (2 nn words), then dst += koT * result.
+static bool ko_axis_lines(const DevMesh& m, int d) { return m.line_ok[d] && m.line_len[d] * m.N <= 1024; }
+
+bool ko_all_lines(const DevMesh& m) { return ko_axis_lines(m, 0) && ko_axis_lines(m, 1) && ko_axis_lines(m, 2); }
+
+int launch_ko_add(const DevMesh& m, int nf, void* const* dst, const void* const* field, double koT, cudaStream_t s,
+                  void* scratch, int* launches) {
+  for (int d = 0; d < 3; ++d) {
+    if (ko_axis_lines(m, d)) {
+      const int rc = ko_lines(m, &d, 1, nf, dst, 0, 1, field, koT, s);
+      if (rc) return rc;
+      *launches += 1;
+      continue;
+    }
+    if (!scratch) return -4;
+    char* buf = static_cast<char*>(scratch);
+    const size_t nb = (size_t)m.nn * (m.precision == 0 ? sizeof(double) : sizeof(float));
+    for (int q = 0; q < nf; ++q) {
+      const void* src = field[q];
+      for (int r = 0; r < 6; ++r) {
+        void* to = buf + (r & 1) * nb;
+        const int rc = launch_apply_D(m, src, to, d, s);
+        if (rc) return rc;
+        src = to;
+      }
+      const int rc = launch_axpy(m.nn, m.precision, dst[q], koT, src, s);
+      if (rc) return rc;
+      *launches += 7;
+    }
+  }
+  return 0;
+}
+
+int launch_ko_fields(const DevMesh& m, int nf, void* const* out, const void* const* field, double koT, int split,
+                     cudaStream_t s, int* launches) {
+  const int axes[3] = {0, 1, 2};
+  if (!ko_all_lines(m)) return -4;
+  if (split) {
+    *launches += 1;
+    return ko_lines(m, axes, 3, nf, out, m.nn, 0, field, koT, s);
+  }
+  for (int d = 0; d < 3; ++d) {
+    const int rc = ko_lines(m, axes + d, 1, nf, out, 0, d > 0, field, koT, s);
+    if (rc) return rc;
+  }
+  *launches += 3;
+  return 0;
+}
+
+}  // namespace wt
