@@ -87,6 +87,8 @@ struct wt_ws {
   void* accP = nullptr;
   void* accQ = nullptr;
   void* trace = nullptr;  // 6 N^2 Ne
+  void* trace2 = nullptr; // the same (SIPG stages ping-pong between them)
+  void* ko = nullptr;     // dissipation increments of both fields, 3 axes each (small meshes; else kP, kQ)
   void* zero = nullptr;   // nn zeros
   void* Lu = nullptr;     // nn
   // FP32 state: the low parts the FP32 state arrays lost (the state is
@@ -453,6 +455,48 @@ int ko_add2(wt_ctx* ctx, const wt::DevMesh& m, void* dstP, const void* fP, void*
   return rc;
 }
 
+// Where the dissipation increments of a fused RK4 stage go.  Split: one launch
+// writes the three axes' parts of both fields (6 nn words, added where they are
+// consumed); otherwise three launches sum them into kP, kQ.  Both move 9 words per
+// node and field.  Split up to kKoSplitNodes nodes, where two launches a stage
+// count and the extra 4 nn words of memory do not: ten SIPG steps on 4^3 elements,
+// n = 6, 623 us against 815 us; one step on 40^3 (13.8M nodes) 4.04 ms split
+// against 3.69 ms summed, the destination then staying in L2 from axis to axis.
+constexpr long long kKoSplitNodes = 4 << 20;
+bool ko_split(const wt::DevMesh& m) { return wt::ko_all_lines(m) && m.nn <= kKoSplitNodes; }
+
+int ko_buffers(wt_ws* ws) {
+  const wt::DevMesh& m = ws->mesh->m;
+  const size_t nb = (size_t)m.nn * rsize(m.precision);
+  if (ko_split(m)) return ensure(ws, &ws->ko, 6 * nb);
+  WT_TRY(ws_buffers(ws));  // F: the scratch of meshes without straight lines
+  return ws_k_buffers(ws);
+}
+
+// The increments eps mu^-5 sum_d D_d^6 of (P, Q) for a fused stage: nko fields each, nn words apart.
+int ko_increments(wt_ctx* ctx, wt_ws* ws, const void* P, const void* Q, double eps_ko, const void** koP,
+                  const void** koQ, int* nko) {
+  const wt::DevMesh& m = ws->mesh->m;
+  const size_t nb = (size_t)m.nn * rsize(m.precision);
+  const double koT = eps_ko * ws->inv_mu5;
+  const bool split = ko_split(m);
+  void* out[2] = {split ? ws->ko : ws->kP, split ? (void*)((char*)ws->ko + 3 * nb) : ws->kQ};
+  const void* f[2] = {P, Q};
+  *koP = out[0];
+  *koQ = out[1];
+  *nko = split ? 3 : 1;
+  if (!wt::ko_all_lines(m)) {
+    cudaMemsetAsync(out[0], 0, nb, ctx->stream);
+    cudaMemsetAsync(out[1], 0, nb, ctx->stream);
+    return ko_add2(ctx, m, out[0], P, out[1], Q, koT, ws->F);
+  }
+  int launched = 0;
+  const int rc = lrc(ctx, wt::launch_ko_fields(m, 2, out, f, koT, split ? 1 : 0, ctx->stream, &launched),
+                     "Kreiss-Oliger");
+  ctx->launches += launched;
+  return rc;
+}
+
 // One RHS evaluation of the conservative system (non-fused).
 int rhs_curved_impl(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, const void* Phi, const void* Pi, void* Phid,
                     void* Pid, double eps_ko, const wt::ConsBC& bc, int use_metric) {
@@ -595,7 +639,8 @@ int wt_ctx_bounds_status(wt_ctx* ctx, unsigned int* word) {
   if (!ctx || !word) return WT_EINVAL;
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "wt_ctx_bounds_status");
-  *word = wt::bounds_take_cons() | wt::bounds_take_n8() | wt::bounds_take_second() | wt::bounds_take_geom();
+  *word = wt::bounds_take_cons() | wt::bounds_take_n8() | wt::bounds_take_second() |
+          wt::bounds_take_sipg() | wt::bounds_take_geom();
   return 0;
 }
 
@@ -1175,7 +1220,7 @@ int wt_workspace_destroy(wt_ws* ws) {
   if (!ws) return WT_EINVAL;
   cudaStreamSynchronize(ws->ctx->stream);
   void* bufs[] = {ws->F, ws->F2, ws->bbuf, ws->grad, ws->kP, ws->kQ, ws->S0, ws->S1, ws->SQ, ws->accP, ws->accQ,
-                  ws->trace, ws->zero, ws->Lu, ws->compP, ws->compQ, ws->erk, ws->evo[0], ws->evo[1],
+                  ws->trace, ws->trace2, ws->ko, ws->zero, ws->Lu, ws->compP, ws->compQ, ws->erk, ws->evo[0], ws->evo[1],
                   ws->evo[2], ws->evo[3], ws->evoE};
   for (void* p : bufs) dfree(ws->ctx, p);
   delete ws;
@@ -1358,8 +1403,14 @@ int wt_rhs_sipg(wt_ctx* ctx, wt_ws* ws, const void* u, const void* ut, void* utt
   if (!m.affine) return fail(ctx, WT_ENOTSUP, "wt_rhs_sipg: this build supports axis-aligned affine meshes only");
   WT_TRY(ensure(ws, &ws->trace, (size_t)6 * m.N * m.N * m.Ne * rsize(m.precision)));
   const double inv_R = (std::isfinite(sommerfeld_R) && sommerfeld_R > 0) ? 1.0 / sommerfeld_R : 0.0;
+  wt::SipgStage S;
+  S.u = u; S.ut = ut; S.utt = utt;
+  S.trace = S.trace_out = ws->trace;
+  for (int f = 0; f < 6; ++f) S.bvals[f] = bdry_values[f];
+  S.tau = tau; S.inv_R = inv_R;
   ctx->launches += 2;
-  return lrc(ctx, wt::launch_sipg(m, u, ut, utt, ws->trace, bdry_values, tau, inv_R, ctx->stream), "rhs_sipg");
+  WT_TRY(lrc(ctx, wt::launch_sipg(m, S, true, ctx->stream), "rhs_sipg"));
+  return lrc(ctx, wt::launch_sipg(m, S, false, ctx->stream), "rhs_sipg");
 }
 
 int wt_rhs_strong(wt_ctx* ctx, wt_ws* ws, const void* u, const void* ut, void* utt, double tau,
@@ -2101,22 +2152,33 @@ int wt_erk_tableau(int method, int* stages, double* c, double* A, double* b) {
   return 0;
 }
 
+// One RK4 step of (u, ut); the traces of u are in ws->trace on entry and, of the new
+// u, on return (the stages ping-pong between the two trace buffers).
 static int step_sipg_once(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, const double bv[6], double tau,
                           double R, double eps_ko) {
   const wt::DevMesh& m = ws->mesh->m;
   cudaStream_t s = ctx->stream;
-  const size_t nb = (size_t)m.nn * rsize(m.precision);
+  void* SP[2] = {ws->S0, ws->S1};
+  void* T[2] = {ws->trace, ws->trace2};
   for (int st = 0; st < 4; ++st) {
-    const void* inU = st == 0 ? u : ws->S0;
-    const void* inV = st == 0 ? ut : ws->SQ;
-    WT_TRY(wt_rhs_sipg(ctx, ws, inU, inV, ws->kQ, bv, tau, R));
-    cudaMemcpyAsync(ws->kP, inV, nb, cudaMemcpyDeviceToDevice, s);
-    if (eps_ko != 0.0) {
-      WT_TRY(ko_add2(ctx, m, ws->kP, inU, ws->kQ, inV, eps_ko * ws->inv_mu5, ws->F));
-    }
-    WT_TRY(lrc(ctx, wt::launch_rk_update(m.nn, m.precision, st, dt, u, ws->accP, ws->S0, ws->kP, s), "rk4"));
-    WT_TRY(lrc(ctx, wt::launch_rk_update(m.nn, m.precision, st, dt, ut, ws->accQ, ws->SQ, ws->kQ, s), "rk4"));
-    ctx->launches += 2;
+    wt::SipgStage S;
+    S.u = st == 0 ? u : SP[(st - 1) % 2];
+    S.ut = st == 0 ? ut : ws->SQ;
+    S.trace = T[st % 2];
+    S.trace_out = T[(st + 1) % 2];
+    for (int f = 0; f < 6; ++f) S.bvals[f] = bv[f];
+    S.tau = tau;
+    S.inv_R = (std::isfinite(R) && R > 0) ? 1.0 / R : 0.0;
+    if (eps_ko != 0.0)
+      WT_TRY(ko_increments(ctx, ws, S.u, S.ut, eps_ko, &S.koU, &S.koV, &S.nko));
+    S.rkU.on = S.rkV.on = 1;
+    S.rkU.stage = S.rkV.stage = st;
+    S.rkU.dt = S.rkV.dt = dt;
+    S.rkU.y = u; S.rkU.acc = ws->accP; S.rkU.out = SP[st % 2]; S.rkU.comp = ws->compP;
+    S.rkV.y = ut; S.rkV.acc = ws->accQ; S.rkV.out = ws->SQ; S.rkV.comp = ws->compQ;
+    wt::NvtxRange nv("rk4 sipg stage");
+    WT_TRY(lrc(ctx, wt::launch_sipg(m, S, false, s), "rk4 sipg"));
+    ctx->launches += 1;
   }
   return 0;
 }
@@ -2129,11 +2191,23 @@ int wt_step_rk4_sipg(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, int n
   if (nsteps < 0 || !(dt > 0)) return fail(ctx, WT_EINVAL, "bad nsteps/dt");
   if (!ws->mesh->m.affine) return fail(ctx, WT_ENOTSUP, "SIPG stepping supports affine meshes only");
   WT_TRY(ws_step_buffers(ws));
-  WT_TRY(ws_k_buffers(ws));
-  WT_TRY(ws_buffers(ws));  // Kreiss-Oliger scratch (allocated before any graph capture)
-  if (eps_ko != 0.0) WT_TRY(ensure_mu(ws));
+  comp_track(ws, u, ut);
+  if (eps_ko != 0.0) {  // buffers and mu before any graph capture
+    WT_TRY(ko_buffers(ws));
+    WT_TRY(ensure_mu(ws));
+  }
   const wt::DevMesh& m = ws->mesh->m;
-  WT_TRY(ensure(ws, &ws->trace, (size_t)6 * m.N * m.N * m.Ne * rsize(m.precision)));
+  const size_t tb = (size_t)6 * m.N * m.N * m.Ne * rsize(m.precision);
+  WT_TRY(ensure(ws, &ws->trace, tb));
+  WT_TRY(ensure(ws, &ws->trace2, tb));
+  if (nsteps == 0) return 0;
+  {
+    wt::SipgStage S;
+    S.u = u;
+    S.trace_out = ws->trace;
+    WT_TRY(lrc(ctx, wt::launch_sipg(m, S, true, ctx->stream), "rk4 sipg traces"));
+    ctx->launches += 1;
+  }
   if (nsteps <= 2) {
     for (int i = 0; i < nsteps; ++i) WT_TRY(step_sipg_once(ctx, ws, u, ut, dt, bdry_values, tau, sommerfeld_R, eps_ko));
     return 0;

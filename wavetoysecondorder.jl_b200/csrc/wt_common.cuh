@@ -91,10 +91,12 @@ __device__ __forceinline__ int bc_slot(int v, int) { return v; }
 #define WT_BOUNDS_TAKE(fn) \
   unsigned int fn() { return 0; }
 #endif
-// the bounds words of the kernel translation units (wt_cons.cu, wt_cons_n8.cu, wt_second.cu, wt_geom.cu)
+// the bounds words of the kernel translation units (wt_cons.cu, wt_cons_n8.cu, wt_second.cu, wt_sipg.cu,
+// wt_geom.cu)
 unsigned int bounds_take_cons();
 unsigned int bounds_take_n8();
 unsigned int bounds_take_second();
+unsigned int bounds_take_sipg();
 unsigned int bounds_take_geom();
 
 // ---- host-side GLL operators (product code, independent of the oracle) -----
@@ -382,9 +384,27 @@ int launch_ko_fields(const DevMesh& m, int nf, void* const* out, const void* con
                      cudaStream_t s, int* launches);
 int launch_div3d(const DevMesh& m, const void* F, void* out, cudaStream_t s);
 
-// second-order forms (wt_second.cu)
-int launch_sipg(const DevMesh& m, const void* u, const void* ut, void* utt, void* trace, const double bvals[6],
-                double tau, double inv_R, cudaStream_t s);
+// SIPG right-hand side and fused RK4 stage (wt_sipg.cu).  trace: the normal
+// derivatives of u at the face nodes (6 N^2 Ne words); trace_only writes them
+// to trace_out.  With rkU.on the RK4 stage of (u, ut) is applied instead of
+// writing utt, and trace_out gets the traces of the u it wrote; koU, koV: nko
+// (0, 1, 3) dissipation increments per field, nn words apart.
+struct SipgStage {
+  const void* u = nullptr;
+  const void* ut = nullptr;
+  void* utt = nullptr;
+  const void* trace = nullptr;
+  void* trace_out = nullptr;
+  double bvals[6] = {0, 0, 0, 0, 0, 0};
+  double tau = 0.0, inv_R = 0.0;
+  RKStage rkU, rkV;
+  int nko = 0;
+  const void* koU = nullptr;
+  const void* koV = nullptr;
+};
+int launch_sipg(const DevMesh& m, const SipgStage& S, bool trace_only, cudaStream_t s);
+
+// other second-order forms (wt_second.cu)
 int launch_strong(const DevMesh& m, const void* u, const void* ut, void* utt, double tau, double inv_R,
                   cudaStream_t s);
 int launch_lap_strong_cons(const DevMesh& m, const void* u, void* Lu, double h, double tau, cudaStream_t s);

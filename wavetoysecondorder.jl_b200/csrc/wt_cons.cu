@@ -20,6 +20,8 @@
 // conflict-free.  Streamed coefficients: a, beta (3), K (6) and, curvilinear,
 // Ja (9) and 1/J.
 #include "wt_common.cuh"
+#include "wt_async.cuh"
+#include "wt_rk.cuh"
 
 #include <initializer_list>
 #include <type_traits>
@@ -81,162 +83,6 @@ struct K1P {
   const double* Ja0;
   real* hcopy;
 };
-
-// Low-storage classic RK4 stage update.  Without compensation acc holds
-// y + partial increments.  With compensation (FP32 state) acc holds the
-// increment of the step alone and the final y + increment is a Kahan sum; comp
-// holds the low part the FP32 y lost (the state is y + comp), so that small
-// increments are not lost to the rounding of y over many steps.
-template <typename real>
-__device__ __forceinline__ void rk_epilogue(int stage, double dt, real k, real yin, real* y, real* acc, real* out,
-                                            real* comp, long long n, unsigned int* nonfinite) {
-  if (comp) {
-    if (stage == 0) {
-      out[n] = yin + (real)(0.5 * dt) * k;
-      acc[n] = (real)(dt / 6.0) * k;
-    } else if (stage == 1) {
-      out[n] = y[n] + (real)(0.5 * dt) * k;
-      acc[n] = acc[n] + (real)(dt / 3.0) * k;
-    } else if (stage == 2) {
-      out[n] = y[n] + (real)dt * k;
-      acc[n] = acc[n] + (real)(dt / 3.0) * k;
-    } else {
-      const real inc = acc[n] + (real)(dt / 6.0) * k;
-      const real yv = y[n];
-      const real t = inc + comp[n];
-      const real v = yv + t;
-      comp[n] = t - (v - yv);
-      y[n] = v;
-      if (nonfinite && !isfinite((double)v)) atomicOr(nonfinite, 1u);
-    }
-    return;
-  }
-  if (stage == 0) {
-    out[n] = yin + (real)(0.5 * dt) * k;
-    acc[n] = yin + (real)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = y[n] + (real)(0.5 * dt) * k;
-    acc[n] = acc[n] + (real)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = y[n] + (real)dt * k;
-    acc[n] = acc[n] + (real)(dt / 3.0) * k;
-  } else {
-    real v = acc[n] + (real)(dt / 6.0) * k;
-    y[n] = v;
-    if (nonfinite && !isfinite((double)v)) atomicOr(nonfinite, 1u);
-  }
-}
-
-// RK4 stage update of the compensated FP32 form (the Phi side, K1): the state
-// is (y, comp) = (high, low part) and the stage the next K1 reads is its high
-// part plus out = low part + c dt k; the step's final sum is formed in FP64 and
-// split again.  hi: this node's high part of the state (the K1 input).
-__device__ __forceinline__ void rk_epilogue_cp(int stage, double dt, float k, float hi, float* y, float* acc,
-                                               float* out, float* comp, float* hcopy, long long n,
-                                               unsigned int* nonfinite) {
-  const float lo = comp[n];
-  if (stage == 0) {
-    out[n] = lo + (float)(0.5 * dt) * k;
-    acc[n] = (float)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = lo + (float)(0.5 * dt) * k;
-    acc[n] = acc[n] + (float)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = lo + (float)dt * k;
-    acc[n] = acc[n] + (float)(dt / 3.0) * k;
-    hcopy[n] = hi;
-  } else {
-    const float inc = acc[n] + (float)(dt / 6.0) * k;
-    const double v = (double)hi + ((double)lo + (double)inc);
-    const float h = (float)v;
-    y[n] = h;
-    comp[n] = (float)(v - (double)h);
-    if (nonfinite && !isfinite(h)) atomicOr(nonfinite, 1u);
-  }
-}
-
-// Per-thread asynchronous copy of one word (4 or 8 bytes) global -> shared,
-// and the wait for all of this thread's copies.  The generic kernels copy the
-// words their node pass reads at their own node (coefficients, Pi, RK state)
-// at kernel start, so that those loads run under the contraction; each thread
-// reads back only its own words, so the wait needs no CTA barrier.
-template <typename T>
-__device__ __forceinline__ void cp_async_word(T* dst, const T* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_own() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// The RK4 stage updates above with the words they read at node n passed in
-// (yv = y[n], accv = acc[n], compv = comp[n]; only those the stage reads need
-// to be valid): the same arithmetic in the same order.
-template <typename real>
-__device__ __forceinline__ void rk_epilogue_v(int stage, double dt, real k, real yin, real yv, real accv, real compv,
-                                              real* y, real* acc, real* out, real* comp, long long n,
-                                              unsigned int* nonfinite) {
-  if (comp) {
-    if (stage == 0) {
-      out[n] = yin + (real)(0.5 * dt) * k;
-      acc[n] = (real)(dt / 6.0) * k;
-    } else if (stage == 1) {
-      out[n] = yv + (real)(0.5 * dt) * k;
-      acc[n] = accv + (real)(dt / 3.0) * k;
-    } else if (stage == 2) {
-      out[n] = yv + (real)dt * k;
-      acc[n] = accv + (real)(dt / 3.0) * k;
-    } else {
-      const real inc = accv + (real)(dt / 6.0) * k;
-      const real t = inc + compv;
-      const real v = yv + t;
-      comp[n] = t - (v - yv);
-      y[n] = v;
-      if (nonfinite && !isfinite((double)v)) atomicOr(nonfinite, 1u);
-    }
-    return;
-  }
-  if (stage == 0) {
-    out[n] = yin + (real)(0.5 * dt) * k;
-    acc[n] = yin + (real)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = yv + (real)(0.5 * dt) * k;
-    acc[n] = accv + (real)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = yv + (real)dt * k;
-    acc[n] = accv + (real)(dt / 3.0) * k;
-  } else {
-    real v = accv + (real)(dt / 6.0) * k;
-    y[n] = v;
-    if (nonfinite && !isfinite((double)v)) atomicOr(nonfinite, 1u);
-  }
-}
-
-// rk_epilogue_cp with lov = comp[n] and accv = acc[n] passed in
-__device__ __forceinline__ void rk_epilogue_cp_v(int stage, double dt, float k, float hi, float lov, float accv,
-                                                 float* y, float* acc, float* out, float* comp, float* hcopy,
-                                                 long long n, unsigned int* nonfinite) {
-  const float lo = lov;
-  if (stage == 0) {
-    out[n] = lo + (float)(0.5 * dt) * k;
-    acc[n] = (float)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = lo + (float)(0.5 * dt) * k;
-    acc[n] = accv + (float)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = lo + (float)dt * k;
-    acc[n] = accv + (float)(dt / 3.0) * k;
-    hcopy[n] = hi;
-  } else {
-    const float inc = accv + (float)(dt / 6.0) * k;
-    const double v = (double)hi + ((double)lo + (double)inc);
-    const float h = (float)v;
-    y[n] = h;
-    comp[n] = (float)(v - (double)h);
-    if (nonfinite && !isfinite(h)) atomicOr(nonfinite, 1u);
-  }
-}
 
 // contraction along axis d of a smem field f (N^3) with transposed G (GT[p*N+i] = G[i][p])
 template <int N, typename real>
@@ -595,16 +441,6 @@ struct PipeK1 {
   static constexpr int OCC = OCC_SM < 1024 / T ? OCC_SM : 1024 / T;
   static_assert(!CP || ((NW * N3 + NF * N2) * sizeof(real)) % 8 == 0, "Ja0 must be 8-byte aligned in a block");
 };
-
-// 4- or 8-byte cp.async, zero-filled (src not read) when !valid
-template <typename T>
-__device__ __forceinline__ void cp_async_word_z(T* dst, const T* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
-}
 
 template <int N, typename real, bool CP>
 __global__ void __launch_bounds__(PipeK1<N, real, CP>::T, PipeK1<N, real, CP>::OCC)

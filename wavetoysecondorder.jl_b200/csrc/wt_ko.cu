@@ -19,13 +19,14 @@
 // own; along axes 1 and 2 consecutive threads hold consecutive nodes and load
 // directly.
 //
-// Measured (FP64, one axis of two fields, B200): 24^3 elements of n = 8, 86 us
-// (3.9 TB/s; the whole pencils through shared memory on every pass, two
+// Measured (FP64, one axis of two fields, B200): 24^3 elements of n = 8, 66 us
+// (5.2 TB/s; the whole pencils through shared memory on every pass, two
 // barriers each and the matrix read from shared memory: 212 us); 40^3 of n = 6,
-// 177 us (before: 450 us).
+// 150 us (before: 450 us).
 #include "wt_common.cuh"
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 namespace wt {
@@ -44,14 +45,19 @@ struct KoP {
   int nax;
   struct Axis {
     int d, len, closed, pb;  // axis, elements per line, periodic, pencils per CTA
+    int parts;               // CTAs per line, N^2 / pb
+    unsigned pb_magic;       // floor(2^32 / pb) + 1: __umulhi(t, magic) = t / pb for t < 1024
     unsigned b0;             // first CTA of the axis
     const int32_t* lines;
   } ax[3];
 };
 
-// CTA: pb pencils of one element line, thread (pencil, element) with the pencil fastest.
+// CTA: pb pencils of one element line of field blockIdx.y, thread (pencil, element)
+// with the pencil fastest.  (Both fields in one thread shared indices, scales and
+// barriers, 28 % fewer instructions, but the registers halved the resident warps:
+// 3 % slower at 40^3 n = 6, 13 % on a 4^3 step.)
 template <int N, typename real, int TMAX>
-__global__ void __launch_bounds__(TMAX) k_ko(const __grid_constant__ KoP<N, real> P) {
+__global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant__ KoP<N, real> P) {
   constexpr int N2 = N * N, N3 = N * N * N, M = KoP<N, real>::M, HH = KoP<N, real>::HH;
   constexpr int NP = N | 1;  // odd pitch of a staged pencil: no bank conflicts
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -59,59 +65,72 @@ __global__ void __launch_bounds__(TMAX) k_ko(const __grid_constant__ KoP<N, real
   const int T = blockDim.x;
   const int tid = threadIdx.x, lane = tid & 31;
   real* stage = ends + 4 * T + (tid >> 5) * 32 * NP;  // this warp's staged pencils (axis 0)
-  int d = P.ax[0].d, len = P.ax[0].len, closed = P.ax[0].closed, PB = P.ax[0].pb, a = 0;
-  unsigned b0 = P.ax[0].b0;
+  int d = P.ax[0].d, len = P.ax[0].len, closed = P.ax[0].closed, PB = P.ax[0].pb, parts = P.ax[0].parts, a = 0;
+  unsigned b0 = P.ax[0].b0, pbm = P.ax[0].pb_magic;
   const int32_t* lines = P.ax[0].lines;
 #pragma unroll
   for (int q = 1; q < 3; ++q)
     if (q < P.nax && blockIdx.x >= P.ax[q].b0) {
-      d = P.ax[q].d; len = P.ax[q].len; closed = P.ax[q].closed; PB = P.ax[q].pb; b0 = P.ax[q].b0;
-      lines = P.ax[q].lines; a = q;
+      d = P.ax[q].d; len = P.ax[q].len; closed = P.ax[q].closed; PB = P.ax[q].pb; parts = P.ax[q].parts;
+      b0 = P.ax[q].b0; pbm = P.ax[q].pb_magic; lines = P.ax[q].lines; a = q;
     }
-  const real* __restrict__ f = blockIdx.y ? P.f[1] : P.f[0];
-  real* __restrict__ out = (blockIdx.y ? P.out[1] : P.out[0]) + a * P.ostride;
-  const int parts = N2 / PB;
   const unsigned blk = blockIdx.x - b0;
   const int line = blk / parts, part = blk - line * parts;
-  const int pb = tid % PB, sg = tid / PB;
+  const int sg = __umulhi(tid, pbm), pb = tid - sg * PB;  // tid / PB, tid % PB
   const bool act = sg < len;
   long long base = -1;
-  int stride = 1;
   real s = 0;
   if (act) {
     const int e = lines[(long long)line * len + sg];
     s = P.sdiag[3 * (long long)e + d];
     const int pp = part * PB + pb;  // the pencil, its first tangential index fastest
-    if (d == 0) { base = (long long)e * N3 + N * pp; }
-    else if (d == 1) { base = (long long)e * N3 + pp % N + N2 * (pp / N); stride = N; }
-    else { base = (long long)e * N3 + pp; stride = N2; }
+    base = (long long)e * N3 + (d == 0 ? N * pp : d == 1 ? pp % N + N2 * (pp / N) : pp);
   }
-  real v[N];
+  const real* const fp = blockIdx.y ? P.f[1] : P.f[0];
+  real* const op = (blockIdx.y ? P.out[1] : P.out[0]) + a * P.ostride;
+  real ev[M], od[HH];
+  auto fold = [&](const real v[N]) {
+#pragma unroll
+    for (int i = 0; i < HH; ++i) {
+      ev[i] = v[i] + v[N - 1 - i];
+      od[i] = v[i] - v[N - 1 - i];
+    }
+    if (N & 1) ev[M - 1] = v[HH];
+  };
+  auto load = [&](auto st) {
+    constexpr int stride = decltype(st)::value;
+    const real* __restrict__ f = fp + (act ? base : 0);
+    real v[N];
+#pragma unroll
+    for (int l = 0; l < N; ++l) v[l] = act ? f[l * stride] : (real)0;
+    fold(v);
+  };
   if (d == 0) {
+    real v[N];
 #pragma unroll
     for (int it = 0; it < N; ++it) {
-      const int q = it * 32 + lane, pr = q / N;
+      const int w = it * 32 + lane, pr = w / N;
       const long long bs = __shfl_sync(0xffffffffu, base, pr);
-      stage[pr * NP + q % N] = bs >= 0 ? f[bs + q % N] : (real)0;
+      v[it] = bs >= 0 ? fp[bs + w % N] : (real)0;
+    }
+#pragma unroll
+    for (int it = 0; it < N; ++it) {
+      const int w = it * 32 + lane, pr = w / N;
+      stage[pr * NP + w % N] = v[it];
     }
     __syncwarp();
 #pragma unroll
     for (int l = 0; l < N; ++l) v[l] = stage[lane * NP + l];
     __syncwarp();
+    fold(v);
+  } else if (d == 1) {
+    load(std::integral_constant<int, N>());
   } else {
-#pragma unroll
-    for (int l = 0; l < N; ++l) v[l] = act ? f[base + l * stride] : (real)0;
+    load(std::integral_constant<int, N2>());
   }
-  real ev[M], od[HH];
-#pragma unroll
-  for (int i = 0; i < HH; ++i) {
-    ev[i] = v[i] + v[N - 1 - i];
-    od[i] = v[i] - v[N - 1 - i];
-  }
-  if (N & 1) ev[M - 1] = v[HH];
   const bool has_prev = act && (closed || sg > 0), has_next = act && (closed || sg < len - 1);
   const int tp = pb + PB * (sg == 0 ? len - 1 : sg - 1), tn = pb + PB * (sg == len - 1 ? 0 : sg + 1);
-#pragma unroll 1
+#pragma unroll 2
   for (int it = 0; it < 6; ++it) {
     real* eb = ends + (it & 1) * 2 * T;
     const real vl = (real)0.5 * (ev[0] + od[0]), vh = (real)0.5 * (ev[0] - od[0]);
@@ -141,32 +160,50 @@ __global__ void __launch_bounds__(TMAX) k_ko(const __grid_constant__ KoP<N, real
 #pragma unroll
     for (int i = 0; i < HH; ++i) od[i] = no[i];
   }
+  auto unfold = [&](real v[N]) {
 #pragma unroll
-  for (int i = 0; i < HH; ++i) {
-    v[i] = P.koT * ((real)0.5 * (ev[i] + od[i]));
-    v[N - 1 - i] = P.koT * ((real)0.5 * (ev[i] - od[i]));
-  }
-  if (N & 1) v[HH] = P.koT * ev[M - 1];
+    for (int i = 0; i < HH; ++i) {
+      v[i] = P.koT * ((real)0.5 * (ev[i] + od[i]));
+      v[N - 1 - i] = P.koT * ((real)0.5 * (ev[i] - od[i]));
+    }
+    if (N & 1) v[HH] = P.koT * ev[M - 1];
+  };
+  auto store = [&](auto st) {
+    constexpr int stride = decltype(st)::value;
+    if (!act) return;
+    real* o = op + base;
+    real v[N];
+    unfold(v);
+    if (P.rmw) {
+#pragma unroll
+      for (int l = 0; l < N; ++l) v[l] += o[l * stride];
+    }
+#pragma unroll
+    for (int l = 0; l < N; ++l) o[l * stride] = v[l];
+  };
   if (d == 0) {
+    real v[N];
+    unfold(v);
 #pragma unroll
     for (int l = 0; l < N; ++l) stage[lane * NP + l] = v[l];
     __syncwarp();
+    long long at[N];
 #pragma unroll
     for (int it = 0; it < N; ++it) {
-      const int q = it * 32 + lane, pr = q / N;
+      const int w = it * 32 + lane, pr = w / N;
       const long long bs = __shfl_sync(0xffffffffu, base, pr);
-      if (bs >= 0) {
-        const long long n = bs + q % N;
-        out[n] = P.rmw ? out[n] + stage[pr * NP + q % N] : stage[pr * NP + q % N];
-      }
-    }
-  } else if (act) {
-    if (P.rmw) {
-#pragma unroll
-      for (int l = 0; l < N; ++l) v[l] += out[base + l * stride];
+      at[it] = bs >= 0 ? bs + w % N : -1;
+      v[it] = stage[pr * NP + w % N];
+      if (P.rmw && at[it] >= 0) v[it] += op[at[it]];
     }
 #pragma unroll
-    for (int l = 0; l < N; ++l) out[base + l * stride] = v[l];
+    for (int it = 0; it < N; ++it)
+      if (at[it] >= 0) op[at[it]] = v[it];
+    __syncwarp();
+  } else if (d == 1) {
+    store(std::integral_constant<int, N>());
+  } else {
+    store(std::integral_constant<int, N2>());
   }
 }
 
@@ -210,19 +247,21 @@ static int ko_lines_n(const DevMesh& m, const int* axes, int nax, int nf, void* 
   for (int q = 0; q < nax; ++q) {
     const int d = axes[q], len = m.line_len[d];
     // pencils per CTA: the most (a divisor of N times N) that keeps a CTA at
-    // 512 threads or fewer, so that along axis 2 a load covers whole sectors and
-    // short lines still fill a CTA; very long lines keep the N pencils of one plane
+    // 256 threads or fewer (512: 3 % slower at 40^3 n = 6); longer lines keep the N
+    // pencils of one plane
     int g = N;
-    while (g > 1 && (N % g != 0 || len * N * g > 512)) --g;
+    while (g > 1 && (N % g != 0 || len * N * g > 256)) --g;
     auto& A = P.ax[q];
-    A.d = d; A.len = len; A.closed = m.line_closed[d]; A.pb = N * g; A.b0 = blocks; A.lines = m.lines[d];
+    A.d = d; A.len = len; A.closed = m.line_closed[d]; A.pb = N * g; A.parts = N / g;
+    A.pb_magic = (unsigned)(0x100000000ull / (unsigned)A.pb) + 1u; A.b0 = blocks; A.lines = m.lines[d];
     blocks += (unsigned)m.nlines[d] * (unsigned)(N / g);
     threads = std::max(threads, (len * N * g + 31) / 32 * 32);
   }
   for (int q = nax; q < 3; ++q) P.ax[q] = P.ax[0];
   if (blocks == 0 || nf == 0) return 0;
-  return threads <= 512 ? ko_run<N, real, 512>(P, blocks, nf, threads, s)
-                        : ko_run<N, real, 1024>(P, blocks, nf, threads, s);
+  return threads <= 256   ? ko_run<N, real, 256>(P, blocks, nf, threads, s)
+         : threads <= 512 ? ko_run<N, real, 512>(P, blocks, nf, threads, s)
+                          : ko_run<N, real, 1024>(P, blocks, nf, threads, s);
 }
 
 static int ko_lines(const DevMesh& m, const int* axes, int nax, int nf, void* const* out, long long ostride, int rmw,

@@ -1,11 +1,5 @@
-// wt_second.cu -- second-order-in-space forms u_tt = L u on the device:
-//   * rhs_wave3d! (src/wave.jl:573-611): the SIPG Laplacian of HexSBPSAT's
-//     apply_laplacian! (restated from README.md:57-80) on axis-aligned affine
-//     meshes, plus the tag-7 Sommerfeld pass (src/wave.jl:453-542).  Two
-//     passes: a face-trace kernel (each element's physical normal derivative
-//     at its six faces) and the volume + SAT kernel that reads the
-//     neighbour's trace (the reference's pass-1/pass-2 structure,
-//     src/wave.jl:594-597).
+// wt_second.cu -- second-order-in-space forms u_tt = L u on the device
+// (the SIPG form: wt_sipg.cu):
 //   * wave_strong_rhs_mesh! (src/wave_strong_rhs.jl:95-341): chain-rule
 //     curvilinear Laplacian with Mattsson-Nordstrom SAT and BGT Sommerfeld.
 //   * wave_lap_strong_conservative_mesh! (src/wave_lap_strong.jl:183-308).
@@ -37,147 +31,6 @@ __device__ __forceinline__ real ctr(const real* __restrict__ f, const real* __re
     for (int p = 0; p < N; ++p) s += GT[p * N + k] * f[i + N * (j + N * p)];
   }
   return s;
-}
-
-// pass 1: trace[(6e + f) N^2 + pq] = s_ax * (G_ax u)(face node)
-template <int N, typename real>
-__global__ void __launch_bounds__(Sp<N>::T) k_sipg_trace(long long Ne, const real* __restrict__ u,
-                                                        real* __restrict__ trace, const real* __restrict__ sdiag,
-                                                        const double* __restrict__ G) {
-  constexpr int N3 = Sp<N>::N3, N2 = Sp<N>::N2, EPB = Sp<N>::EPB;
-  __shared__ real GT[N2];
-  __shared__ real su[EPB][N3];
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const long long e = (long long)blockIdx.x * EPB + le;
-  const bool valid = e < Ne;
-  const long long ec = valid ? e : 0;
-  if (tid < N2) GT[(tid % N) * N + tid / N] = (real)G[tid];
-  su[le][t] = valid ? u[ec * N3 + t] : (real)0;
-  __syncthreads();
-  if (!valid) return;
-  for (int idx = t; idx < 6 * N2; idx += N3) {
-    const int f = idx / N2, pq = idx - f * N2;
-    const int ax = f >> 1, r = frow(f, N), p = pq % N, q = pq / N;
-    const int fnode = face_node(ax, r, p, q, N);
-    const int i = fnode % N, j = (fnode / N) % N, k = fnode / N2;
-    trace[(6 * ec + f) * N2 + pq] = sdiag[3 * ec + ax] * ctr<N>(su[le], GT, i, j, k, ax);
-  }
-}
-
-template <typename real>
-struct SipgP {
-  long long Ne;
-  const real* u;
-  const real* ut;
-  real* utt;
-  const real* trace;
-  const real* sdiag;
-  const int32_t* nbr;
-  const int32_t* nbrf;
-  const int32_t* bdry;
-  const int32_t* bslot;
-  int nbf;
-  const real* bnorm;
-  const double* G;
-  const double* H;
-  real bv[6];
-  real tau, inv_R;
-};
-
-template <int N, typename real>
-__global__ void __launch_bounds__(Sp<N>::T) k_sipg_rhs(const SipgP<real> P) {
-  constexpr int N3 = Sp<N>::N3, N2 = Sp<N>::N2, EPB = Sp<N>::EPB;
-  __shared__ real GT[N2];
-  __shared__ real Hs[N];
-  __shared__ real su[EPB][N3];
-  __shared__ real sD[EPB][3][N3];
-  __shared__ real sdu[EPB][6][N2];
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const int i = t % N, j = (t / N) % N, k = t / N2;
-  const long long e = (long long)blockIdx.x * EPB + le;
-  const bool valid = e < P.Ne;
-  const long long ec = valid ? e : 0;
-  const long long n = ec * N3 + t;
-  if (tid < N2) GT[(tid % N) * N + tid / N] = (real)P.G[tid];
-  if (tid < N) Hs[tid] = (real)P.H[tid];
-  const real uv = valid ? P.u[n] : (real)0;
-  su[le][t] = uv;
-  real sd[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) sd[d] = P.sdiag[3 * ec + d];
-  __syncthreads();
-  real D[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    D[d] = sd[d] * ctr<N>(su[le], GT, i, j, k, d);
-    sD[le][d][t] = D[d];
-  }
-  // face jumps du (0 on inactive faces)
-  for (int idx = t; idx < 6 * N2; idx += N3) {
-    const int f = idx / N2, pq = idx - f * N2;
-    real du = 0;
-    if (valid) {
-      const int tag = P.bdry[f + 6 * ec];
-      const int en = ::wt::bc_elem(P.nbr[f + 6 * ec], P.Ne);
-      const int ax = f >> 1;
-      const int fl = face_node(ax, frow(f, N), pq % N, pq / N, N);
-      if (tag == 0 && en >= 0) {
-        const int fs = P.nbrf[f + 6 * ec];  // fn | ori << 3
-        du = su[le][fl] - P.u[(long long)en * N3 + nbr_face_node(fs, pq % N, pq / N, N)];
-      } else if (tag >= 1 && tag <= 6) {
-        du = su[le][fl] - P.bv[tag - 1];
-      }
-    }
-    sdu[le][f][pq] = du;
-  }
-  __syncthreads();
-  if (!valid) return;
-  real acc = 0;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) acc += sd[d] * ctr<N>(sD[le][d], GT, i, j, k, d);
-  const int idx3[3] = {i, j, k};
-  for (int f = 0; f < 6; ++f) {
-    const int tag = P.bdry[f + 6 * ec];
-    const int en = ::wt::bc_elem(P.nbr[f + 6 * ec], P.Ne);
-    const bool interior = tag == 0 && en >= 0;
-    const bool dir = tag >= 1 && tag <= 6;
-    if (!interior && !dir) continue;
-    const int ax = f >> 1, r = frow(f, N);
-    const real nh = (f & 1) ? (real)1 : (real)-1;
-    const real s = sd[ax];
-    const real al = interior ? (real)0.5 : (real)1;
-    const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-    const real du = sdu[le][f][p + N * q];
-    const int l = idx3[ax];
-    // alpha G^T B du, lifted
-    acc += al * nh * s * s * GT[l * N + r] / Hs[l] * du;
-    if (l == r) {
-      real dGu = 0;
-      if (interior) {
-        const int fs = P.nbrf[f + 6 * ec];  // fn | ori << 3
-        int pn, qn;
-        face_perm((fs >> 3) & 7, p, q, N, pn, qn);
-        dGu = D[ax] - P.trace[((long long)6 * en + (fs & 7)) * N2 + pn + N * qn];
-      }
-      acc += -P.tau * s * s / Hs[r] * du;
-      acc += (real)-0.5 * nh * s / Hs[r] * dGu;
-    }
-  }
-  // Sommerfeld pass on tag-7 outer faces
-  for (int f = 0; f < 6; ++f) {
-    if (P.nbr[f + 6 * ec] >= 0 || P.bdry[f + 6 * ec] != 7) continue;
-    const int ax = f >> 1;
-    if (idx3[ax] != frow(f, N)) continue;
-    const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-    const long long nb = (long long)P.nbf * N2;
-    const long long bi = (long long)::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf) * N2 + p + N * q;
-    const real nx = P.bnorm[bi], ny = P.bnorm[nb + bi], nz = P.bnorm[2 * nb + bi], wFH = P.bnorm[4 * nb + bi];
-    const real Gn = nx * D[0] + ny * D[1] + nz * D[2];
-    acc -= wFH * (P.ut[n] + Gn + P.inv_R * uv);
-  }
-  P.utt[n] = acc;
 }
 
 // ---------------------------------------------------------------------------
@@ -489,30 +342,6 @@ __global__ void k_curved4_bg(long long nn, const double* __restrict__ coords, in
     case 8: { constexpr int NN = 8; return CALL; } \
     default: return -4;           \
   }
-
-template <int N, typename real>
-static int sipg_dispatch(const DevMesh& m, const void* u, const void* ut, void* utt, void* trace,
-                         const double bvals[6], double tau, double inv_R, cudaStream_t s) {
-  const unsigned blocks = (unsigned)((m.Ne + Sp<N>::EPB - 1) / Sp<N>::EPB);
-  k_sipg_trace<N, real><<<blocks, Sp<N>::T, 0, s>>>(m.Ne, (const real*)u, (real*)trace, (const real*)m.sdiag, m.G);
-  SipgP<real> P;
-  P.Ne = m.Ne; P.u = (const real*)u; P.ut = (const real*)ut; P.utt = (real*)utt; P.trace = (const real*)trace;
-  P.sdiag = (const real*)m.sdiag; P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot;
-  P.nbf = m.nbf; P.bnorm = (const real*)m.bnorm; P.G = m.G; P.H = m.H;
-  for (int f = 0; f < 6; ++f) P.bv[f] = (real)bvals[f];
-  P.tau = (real)tau; P.inv_R = (real)inv_R;
-  k_sipg_rhs<N, real><<<blocks, Sp<N>::T, 0, s>>>(P);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-
-int launch_sipg(const DevMesh& m, const void* u, const void* ut, void* utt, void* trace, const double bvals[6],
-                double tau, double inv_R, cudaStream_t s) {
-  if (m.precision == 0) {
-    WT_DISPATCH_N2(m.N, (sipg_dispatch<NN, double>(m, u, ut, utt, trace, bvals, tau, inv_R, s)));
-  } else {
-    WT_DISPATCH_N2(m.N, (sipg_dispatch<NN, float>(m, u, ut, utt, trace, bvals, tau, inv_R, s)));
-  }
-}
 
 template <int N, typename real>
 static int strong_dispatch(const DevMesh& m, const void* u, const void* ut, void* utt, double tau, double inv_R,
