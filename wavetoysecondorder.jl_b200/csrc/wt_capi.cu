@@ -1420,9 +1420,9 @@ int wt_rhs_strong(wt_ctx* ctx, wt_ws* ws, const void* u, const void* ut, void* u
   if (!u || !ut || !utt) return fail(ctx, WT_EINVAL, "wt_rhs_strong: NULL argument");
   WT_TRY(need_setup_geometry(ws->mesh, "wt_rhs_strong"));
   wt::DevMesh& m = ws->mesh->m;
-  if (!m.dinvjac) {
-    WT_TRY(dalloc(ctx, &m.dinvjac, 27 * (size_t)m.nn * sizeof(double), &ws->mesh->owned));
-    WT_TRY(lrc(ctx, wt::launch_dinvjac(m, ctx->stream), "make_metric_derivs"));
+  if (!m.strong_c) {
+    WT_TRY(dalloc(ctx, &m.strong_c, 9 * (size_t)m.nn * sizeof(double), &ws->mesh->owned));
+    WT_TRY(lrc(ctx, wt::launch_strong_coef(m, ctx->stream), "make_metric_derivs"));
     ctx->launches += 1;
   }
   const double inv_R = (std::isfinite(sommerfeld_R) && sommerfeld_R > 0) ? 1.0 / sommerfeld_R : 0.0;

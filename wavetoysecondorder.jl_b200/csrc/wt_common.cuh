@@ -135,7 +135,7 @@ struct DevMesh {
   double* Ja = nullptr;      // 9 fields, field-major
   double* invdetJ = nullptr;
   double* Hd = nullptr;
-  double* dinvjac = nullptr; // lazily: [a + 3c + 9d + 27n]
+  double* strong_c = nullptr; // lazily: the strong form's nine node coefficients, field-major (k_strong_coef)
   // streamed copies in the state precision
   void* Ja_r = nullptr;      // 9 fields
   void* invdetJ_r = nullptr;
@@ -252,7 +252,7 @@ struct Status {
 int launch_geom_analytic(DevMesh& m, double x0, double x1, double A, cudaStream_t s, int z0 = 0, int Mz = 0);
 int launch_geom_derived(DevMesh& m, cudaStream_t s);
 int launch_metric(DevMesh& m, cudaStream_t s);
-int launch_dinvjac(DevMesh& m, cudaStream_t s);
+int launch_strong_coef(DevMesh& m, cudaStream_t s);
 int launch_boundary_normals(DevMesh& m, cudaStream_t s);
 int launch_streamed_geometry(DevMesh& m, cudaStream_t s);
 // kinds 4, 5 (spacetime-metric backgrounds) are sampled at time *d_t + toff

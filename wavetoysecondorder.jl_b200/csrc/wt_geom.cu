@@ -246,23 +246,35 @@ __global__ void k_metric(int N, long long Ne, const double* __restrict__ Gg, con
   Hd[n] = Hq[i] * Hq[j] * Hq[k] * fabs(detjac[n]);
 }
 
-// dinvjac[a,c,d] = Dhat_d invjac[a,c] (make_metric_derivs).
-__global__ void k_dinvjac(int N, long long Ne, const double* __restrict__ Gg, const double* __restrict__ invjac,
-                          double* __restrict__ dinvjac) {
+// The strong form's node coefficients (make_metric_derivs, src/wave_strong_rhs.jl:376-391,
+// contracted as wave_strong_rhs_element! uses them): with I = invjac,
+//   G^{ab} = sum_i I[a,i] I[b,i] and W_b = sum_{a,i} I[a,i] Dhat_a I[b,i],
+// nine fields (G00, 2 G01, 2 G02, G11, 2 G12, G22, W0, W1, W2), each in node order.
+__global__ void k_strong_coef(int N, long long Ne, const double* __restrict__ Gg, const double* __restrict__ invjac,
+                              double* __restrict__ sc) {
   extern __shared__ double sm[];
   const int N3 = N * N * N;
-  double* f = sm;
-  double* G = f + N3;
-  const long long e = blockIdx.x;
+  double* f = sm;  // the nine entries of invjac
+  double* G = f + 9 * N3;
+  const long long e = blockIdx.x, nn = Ne * N3;
   const int t = threadIdx.x;
   const int i = t % N, j = (t / N) % N, k = t / (N * N);
   if (t < N * N) G[t] = Gg[t];
   const long long n = e * N3 + t;
-  for (int ac = 0; ac < 9; ++ac) {
-    __syncthreads();
-    f[t] = invjac[ac + 9 * n];
-    __syncthreads();
-    for (int d = 0; d < 3; ++d) dinvjac[ac + 9 * d + 27 * n] = sm_deriv(f, G, N, i, j, k, d);
+  double I[9];
+  for (int c = 0; c < 9; ++c) f[c * N3 + t] = I[c] = invjac[c + 9 * n];
+  __syncthreads();
+  int o = 0;
+  for (int a = 0; a < 3; ++a)
+    for (int b = a; b < 3; ++b) {
+      const double g = I[a] * I[b] + I[a + 3] * I[b + 3] + I[a + 6] * I[b + 6];
+      sc[(o++) * nn + n] = a == b ? g : 2.0 * g;
+    }
+  for (int b = 0; b < 3; ++b) {
+    double W = 0.0;
+    for (int a = 0; a < 3; ++a)
+      for (int c = 0; c < 3; ++c) W += I[a + 3 * c] * sm_deriv(f + (b + 3 * c) * N3, G, N, i, j, k, a);
+    sc[(o++) * nn + n] = W;
   }
 }
 
@@ -431,10 +443,10 @@ int launch_metric(DevMesh& m, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int launch_dinvjac(DevMesh& m, cudaStream_t s) {
+int launch_strong_coef(DevMesh& m, cudaStream_t s) {
   const int N3 = m.N * m.N * m.N;
-  size_t smem = ((size_t)N3 + m.N * m.N) * sizeof(double);
-  k_dinvjac<<<(unsigned)m.Ne, N3, smem, s>>>(m.N, m.Ne, m.G, m.invjac, m.dinvjac);
+  const size_t smem = (9 * N3 + m.N * m.N) * sizeof(double);  // at most 37 KB
+  k_strong_coef<<<(unsigned)m.Ne, N3, smem, s>>>(m.N, m.Ne, m.G, m.invjac, m.strong_c);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -34,121 +34,162 @@ __device__ __forceinline__ real ctr(const real* __restrict__ f, const real* __re
 }
 
 // ---------------------------------------------------------------------------
-// wave_strong_rhs_element! restated on the device (orientation 0).
-template <typename real>
+// wave_strong_rhs_element! restated on the device.  With G^{ab}, W_b of
+// k_strong_coef, d_a = Dhat_a u and dd_ab = Dhat_b d_a (a <= b):
+//   u_tt = sum_ab G^{ab} dd_ab + sum_b W_b d_b
+// and on an axis-a face (sign s, row r): the physical normal derivative is
+// s sum_b G^{ab} d_b / |n|, |n|^2 = G^{aa}, so the interior / Dirichlet SAT is
+//   -(s sum_b G^{ab} d_b + tau |n| (u - u_nbr)) / H_r.
+//
+// Bound by memory latency and bandwidth: 11 words a node (u, nine coefficients,
+// the result; the 9 inverse-Jacobian entries and their 27 derivatives, node-major,
+// were 36).  3 N^2 threads per element, one per (axis, pencil), operator in the
+// constant bank: first d_a and dd_aa along the own axis, then one mixed
+// derivative each (dd_01 along y, dd_02 and dd_12 along z) and the boundary terms
+// of the pencil's two ends (in the node pass, where most warps hold nodes of all
+// faces, they took a third of the instructions), then a node pass in node order.  Measured (FP64, n = 5, 28^3 elements, B200): 80 us
+// (3.0 TB/s), before 255 us.
+template <int N, typename real>
 struct StrongP {
-  long long Ne;
+  double G[N * N];
+  double H[N];
+  double invH;  // 1 / H_end
+  long long Ne, nn;
   const real* u;
   const real* ut;
   real* utt;
-  const double* invjac;
-  const double* dinvjac;
+  const double* sc;
   const double* detjac;
   const double* Hphys;
   const int32_t* nbr;
   const int32_t* nbrf;
   const int32_t* bdry;
-  const double* G;
-  const double* H;
   double tau, inv_R;
 };
 
+// elements per CTA: about 200 threads
+template <int N>
+struct Pen {
+  static constexpr int EPB = 3 * N * N >= 128 ? 1 : 224 / (3 * N * N);
+  static constexpr int T = 3 * N * N * EPB;
+};
+
 template <int N, typename real>
-__global__ void __launch_bounds__(Sp<N>::T) k_strong(const StrongP<real> P) {
-  constexpr int N3 = Sp<N>::N3, N2 = Sp<N>::N2, EPB = Sp<N>::EPB;
-  __shared__ double GT[N2];
-  __shared__ double Hs[N];
-  __shared__ double su[EPB][N3];
-  __shared__ double sdu[EPB][3][N3];
-  __shared__ double suf[EPB][6][N2];
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const int i = t % N, j = (t / N) % N, k = t / N2;
+__global__ void __launch_bounds__(Pen<N>::T, (N >= 7 ? 588 : 1024) / Pen<N>::T) k_strong(const __grid_constant__ StrongP<N, real> P) {
+  constexpr int N2 = N * N, N3 = N * N * N, TE = 3 * N2, EPB = Pen<N>::EPB;
+  constexpr int P1 = N | 1;       // odd row pitch: x pencils without bank conflicts
+  constexpr int NS = N * N * P1;  // words of one field of an element
+  constexpr int NI = (N3 + TE - 1) / TE;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  const int tid = threadIdx.x, le = tid / TE, t = tid - le * TE, ax = t / N2, pq = t - ax * N2, p = pq % N, q = pq / N;
+  double* su = reinterpret_cast<double*>(smraw) + (size_t)le * (10 * NS + 6 * N2);
+  double* sd = su + NS;       // d_0, d_1, d_2
+  double* sdd = su + 4 * NS;  // dd_00, dd_11, dd_22, dd_01, dd_02, dd_12
+  double* suf = su + 10 * NS; // the face nodes' boundary terms
   const long long e = (long long)blockIdx.x * EPB + le;
   const bool valid = e < P.Ne;
   const long long ec = valid ? e : 0;
-  const long long n = ec * N3 + t;
-  if (tid < N2) GT[(tid % N) * N + tid / N] = P.G[tid];
-  if (tid < N) Hs[tid] = P.H[tid];
-  const double uv = valid ? (double)P.u[n] : 0.0;
-  su[le][t] = uv;
-  for (int idx = t; idx < 6 * N2; idx += N3) {
-    const int f = idx / N2, pq = idx - f * N2;
-    double v = 0.0;
-    if (valid) {
-      const int en = ::wt::bc_elem(P.nbr[f + 6 * ec], P.Ne);
-      if (en >= 0) {
-        const int fs = P.nbrf[f + 6 * ec];  // fn | ori << 3
-        v = (double)P.u[(long long)en * N3 + nbr_face_node(fs, pq % N, pq / N, N)];
-      }
-    }
-    suf[le][f][pq] = v;
+  auto place = [](int w) { return w + (P1 - N) * (w / N); };
+#pragma unroll
+  for (int it = 0; it < NI; ++it) {
+    const int w = t + it * TE;
+    if (w < N3) su[place(w)] = valid ? (double)P.u[ec * N3 + w] : 0.0;
+  }
+  double uf[2];  // the neighbours' values at the ends of this thread's pencil (0 without one)
+  int tag[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int f = 2 * ax + h;
+    const int en = valid ? ::wt::bc_elem(P.nbr[f + 6 * ec], P.Ne) : -1;
+    tag[h] = valid ? P.bdry[f + 6 * ec] : 8;
+    uf[h] = en >= 0 ? (double)P.u[(long long)en * N3 + nbr_face_node(P.nbrf[f + 6 * ec], p, q, N)] : 0.0;
   }
   __syncthreads();
-  double du[3];
+  {
+    const int pb = ax == 0 ? P1 * (p + N * q) : ax == 1 ? p + P1 * N * q : p + P1 * q;
+    const int ps = ax == 0 ? 1 : ax == 1 ? P1 : P1 * N;
+    double v[N], d[N];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    du[c] = ctr<N>(su[le], GT, i, j, k, c);
-    sdu[le][c][t] = du[c];
+    for (int l = 0; l < N; ++l) v[l] = su[pb + ps * l];
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      double s = 0;
+#pragma unroll
+      for (int m = 0; m < N; ++m) s += P.G[l * N + m] * v[m];
+      d[l] = s;
+      sd[ax * NS + pb + ps * l] = s;
+    }
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      double s = 0;
+#pragma unroll
+      for (int m = 0; m < N; ++m) s += P.G[l * N + m] * d[m];
+      sdd[ax * NS + pb + ps * l] = s;
+    }
+  }
+  __syncthreads();
+  {
+    // dd_01: d_0 along y; dd_02: d_0 along z; dd_12: d_1 along z
+    const int pb = ax == 0 ? p + P1 * N * q : p + P1 * q, ps = ax == 0 ? P1 : P1 * N;
+    const double* src = sd + (ax == 2 ? NS : 0);
+    double v[N];
+#pragma unroll
+    for (int l = 0; l < N; ++l) v[l] = src[pb + ps * l];
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      double s = 0;
+#pragma unroll
+      for (int m = 0; m < N; ++m) s += P.G[l * N + m] * v[m];
+      sdd[(3 + ax) * NS + pb + ps * l] = s;
+    }
+  }
+  {
+    const int c0 = ax, c1 = ax == 0 ? 1 : ax == 1 ? 3 : 4, c2 = ax == 0 ? 2 : ax == 1 ? 4 : 5;  // G^{ax,0..2}
+    const double f0 = ax == 0 ? 1.0 : 0.5, f1 = ax == 1 ? 1.0 : 0.5, f2 = ax == 2 ? 1.0 : 0.5;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      double b = 0.0;
+      if (tag[h] != 8 && tag[h] >= 0 && tag[h] <= 7) {
+        const int w = face_node(ax, h ? N - 1 : 0, p, q, N), at = place(w);
+        const long long n = ec * N3 + w;
+        const double g0 = f0 * P.sc[c0 * P.nn + n], g1 = f1 * P.sc[c1 * P.nn + n], g2 = f2 * P.sc[c2 * P.nn + n];
+        const double gd = (h ? 1.0 : -1.0) * (g0 * sd[at] + g1 * sd[NS + at] + g2 * sd[2 * NS + at]);  // |n| d_n u
+        const double nrm = sqrt(ax == 0 ? g0 : ax == 1 ? g1 : g2), uv = su[at];
+        if (tag[h] != 7) {
+          b = -gd * P.invH - P.tau * (nrm * P.invH) * (uv - uf[h]);
+        } else {
+          const double hpq = P.detjac[n] * P.H[p] * P.H[q];
+          b = -(hpq * nrm * ((double)P.ut[n] + P.inv_R * uv) + hpq * gd) / P.Hphys[n];
+        }
+      }
+      suf[(2 * ax + h) * N2 + pq] = b;
+    }
   }
   __syncthreads();
   if (!valid) return;
-  double dd[3][3];
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+  for (int it = 0; it < NI; ++it) {
+    const int w = t + it * TE;
+    if (N3 % TE != 0 && w >= N3) break;
+    const int at = place(w);
+    const long long n = ec * N3 + w;
+    double c[9];
 #pragma unroll
-    for (int d = c; d < 3; ++d) dd[c][d] = ctr<N>(sdu[le][c], GT, i, j, k, d);
-  const double* ij = P.invjac + 9 * n;
-  const double* dij = P.dinvjac + 27 * n;
-  double I[9];
-#pragma unroll
-  for (int c = 0; c < 9; ++c) I[c] = ij[c];
-  double dphys[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) dphys[a] = I[0 + 3 * a] * du[0] + I[1 + 3 * a] * du[1] + I[2 + 3 * a] * du[2];
-  double s = 0.0;
-#pragma unroll
-  for (int al = 0; al < 3; ++al) {
-    double Gaa = I[al] * I[al] + I[al + 3] * I[al + 3] + I[al + 6] * I[al + 6];
-    s += Gaa * dd[al][al];
-#pragma unroll
-    for (int be = al + 1; be < 3; ++be) {
-      double Gab = I[al] * I[be] + I[al + 3] * I[be + 3] + I[al + 6] * I[be + 6];
-      s += 2.0 * Gab * dd[al][be];
-    }
+    for (int o = 0; o < 9; ++o) c[o] = P.sc[o * P.nn + n];
+    double s = c[0] * sdd[at] + c[1] * sdd[3 * NS + at] + c[2] * sdd[4 * NS + at] + c[3] * sdd[NS + at] +
+               c[4] * sdd[5 * NS + at] + c[5] * sdd[2 * NS + at];
+    s += c[6] * sd[at];
+    s += c[7] * sd[NS + at];
+    s += c[8] * sd[2 * NS + at];
+    const int i = w % N, j = (w / N) % N, k = w / N2;
+    if (i == 0) s += suf[j + N * k];
+    if (i == N - 1) s += suf[N2 + j + N * k];
+    if (j == 0) s += suf[2 * N2 + i + N * k];
+    if (j == N - 1) s += suf[3 * N2 + i + N * k];
+    if (k == 0) s += suf[4 * N2 + i + N * j];
+    if (k == N - 1) s += suf[5 * N2 + i + N * j];
+    P.utt[n] = (real)s;
   }
-#pragma unroll
-  for (int be = 0; be < 3; ++be) {
-    double Wb = 0.0;
-#pragma unroll
-    for (int al = 0; al < 3; ++al)
-#pragma unroll
-      for (int ii = 0; ii < 3; ++ii) Wb += I[al + 3 * ii] * dij[be + 3 * ii + 9 * al];
-    s += Wb * du[be];
-  }
-  const int idx3[3] = {i, j, k};
-  for (int f = 0; f < 6; ++f) {
-    const int al = f >> 1, fr = frow(f, N);
-    if (idx3[al] != fr) continue;
-    const int tag = P.bdry[f + 6 * ec];
-    if (tag == 8) continue;
-    const bool somm = tag == 7;
-    const bool intdir = tag == 0 || (tag >= 1 && tag <= 6);
-    const int p = al == 0 ? j : i, q = al == 2 ? j : k;
-    const double fs = (f & 1) ? 1.0 : -1.0;
-    const double nux = I[al], nuy = I[al + 3], nuz = I[al + 6];
-    const double nrm = sqrt(nux * nux + nuy * nuy + nuz * nuz);
-    const double dnu = (fs * nux / nrm) * dphys[0] + (fs * nuy / nrm) * dphys[1] + (fs * nuz / nrm) * dphys[2];
-    if (intdir) {
-      const double w = nrm / Hs[fr];
-      s += -w * dnu;
-      s += -P.tau * w * (uv - suf[le][f][p + N * q]);
-    } else if (somm) {
-      const double wF = nrm * P.detjac[n] * Hs[p] * Hs[q];
-      s -= wF * ((double)P.ut[n] + dnu + P.inv_R * uv) / P.Hphys[n];
-    }
-  }
-  P.utt[n] = (real)s;
 }
 
 // wave_lap_strong_conservative_element! on every element (uniform h).
@@ -346,12 +387,20 @@ __global__ void k_curved4_bg(long long nn, const double* __restrict__ coords, in
 template <int N, typename real>
 static int strong_dispatch(const DevMesh& m, const void* u, const void* ut, void* utt, double tau, double inv_R,
                            cudaStream_t s) {
-  StrongP<real> P;
-  P.Ne = m.Ne; P.u = (const real*)u; P.ut = (const real*)ut; P.utt = (real*)utt;
-  P.invjac = m.invjac; P.dinvjac = m.dinvjac; P.detjac = m.detjac; P.Hphys = m.Hphys;
-  P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.G = m.G; P.H = m.H; P.tau = tau; P.inv_R = inv_R;
-  const unsigned blocks = (unsigned)((m.Ne + Sp<N>::EPB - 1) / Sp<N>::EPB);
-  k_strong<N, real><<<blocks, Sp<N>::T, 0, s>>>(P);
+  StrongP<N, real> P;
+  for (int q = 0; q < N * N; ++q) P.G[q] = m.ops.G[q];
+  for (int q = 0; q < N; ++q) P.H[q] = m.ops.H[q];
+  P.invH = 1.0 / m.ops.H[0];
+  P.Ne = m.Ne; P.nn = m.nn; P.u = (const real*)u; P.ut = (const real*)ut; P.utt = (real*)utt;
+  P.sc = m.strong_c; P.detjac = m.detjac; P.Hphys = m.Hphys;
+  P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.tau = tau; P.inv_R = inv_R;
+  constexpr int EPB = Pen<N>::EPB;
+  const unsigned blocks = (unsigned)((m.Ne + EPB - 1) / EPB);
+  const size_t smem = (size_t)EPB * (10 * N * N * (N | 1) + 6 * N * N) * sizeof(double);
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(k_strong<N, real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return -2;
+  k_strong<N, real><<<blocks, Pen<N>::T, smem, s>>>(P);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
