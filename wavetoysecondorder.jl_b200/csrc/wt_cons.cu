@@ -14,11 +14,9 @@
 //   K2  per element: F -> smem, neighbour F face traces -> smem; split-form
 //       divergence with centred-flux SAT; adds the boundary increments; writes
 //       Pidot or the fused RK4 stage update of Pi.
-// One CTA owns EPB elements with one thread per node; every element block is a
-// contiguous N^3 run, so all global loads are fully coalesced; the reference
-// derivative matrix is held transposed in smem so the N-term contractions read
-// conflict-free.  Streamed coefficients: a, beta (3), K (6) and, curvilinear,
-// Ja (9) and 1/J.
+// Every element block is a contiguous N^3 run, so all global loads are fully
+// coalesced.  Streamed coefficients: a, beta (3), K (6) and, curvilinear, Ja (9)
+// and 1/J.
 #include "wt_common.cuh"
 #include "wt_async.cuh"
 #include "wt_rk.cuh"
@@ -102,23 +100,15 @@ __device__ __forceinline__ real contract(const real* __restrict__ f, const real*
   return s;
 }
 
-// resident CTAs per SM the generic kernels are compiled for: about 1024 threads
-template <int T>
-struct GenOcc {
-  static constexpr int value = T >= 1024 ? 1 : 1024 / T;
-};
-
 // The node pass of K1 at node n (element ec, node (i, j, k)): flux, Phidot,
 // boundary terms (into bbuf) and the RK4 stage update or Phidot.  g: the
 // gradient; u: the stage input (CP: its high part), ug: the value the gradient
 // differentiated; sd: the affine axis scales; a, b, K, Pi: the node's
-// coefficients and Pi.  PRE: the RK words the update reads (yv, accv, compv)
-// were loaded by the caller; otherwise the update reads them itself.
-template <int N, typename real, bool CP, bool PRE, typename gt>
+// coefficients and Pi.
+template <int N, typename real, bool CP, typename gt>
 __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long ec, long long n, int i, int j, int k,
                                           int emask, const real g[3], real u, gt ug, const real sd[3], real Hend,
-                                          real a, const real b[3], const real K[6], real Pi, real yv, real accv,
-                                          real compv) {
+                                          real a, const real b[3], const real K[6], real Pi, real yv, real accv, real compv) {
   constexpr int N2 = Ep<N>::N2;
   const long long nn = P.nn;
   // flux and Phidot
@@ -192,437 +182,283 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long ec, long
   P.F[n] = F0;
   P.F[nn + n] = F1;
   P.F[2 * nn + n] = F2;
-  if constexpr (PRE) {
-    if constexpr (CP) {
-      if (P.epi)
-        rk_epilogue_cp_v(P.stage, P.dt, phid, u, compv, accv, P.y, P.acc, P.out, P.comp, P.hcopy, n, P.nonfinite);
-      else
-        P.Phidot[n] = phid;
-    } else {
-      if (P.epi)
-        rk_epilogue_v<real>(P.stage, P.dt, phid, u, yv, accv, compv, P.y, P.acc, P.out, P.comp, n, P.nonfinite);
-      else
-        P.Phidot[n] = phid;
-    }
-  } else if constexpr (CP) {
+  if constexpr (CP) {
     if (P.epi)
-      rk_epilogue_cp(P.stage, P.dt, phid, u, P.y, P.acc, P.out, P.comp, P.hcopy, n, P.nonfinite);
+      rk_epilogue_cp_v(P.stage, P.dt, phid, u, compv, accv, P.y, P.acc, P.out, P.comp, P.hcopy, n, P.nonfinite);
     else
       P.Phidot[n] = phid;
   } else {
     if (P.epi)
-      rk_epilogue<real>(P.stage, P.dt, phid, u, P.y, P.acc, P.out, P.comp, n, P.nonfinite);
+      rk_epilogue_v<real>(P.stage, P.dt, phid, u, yv, accv, compv, P.y, P.acc, P.out, P.comp, n, P.nonfinite);
     else
       P.Phidot[n] = phid;
   }
-}
-
-// BATCH: the CTA's elements come from a work list of (solve, element) tiles
-// and each tile reads the parameter block of its solve (plist); otherwise
-// element blockIdx.x * EPB + le of the single solve P0.  EPB_: elements per CTA.
-// CP (real = float): the compensated form -- the Phi the stage reads (high
-// plus small part) and the split-form gradient of it in FP64.
-template <int N, typename real, bool CURV, bool BATCH, int EPB_, bool CP = false>
-__global__ void __launch_bounds__(Ep<N>::N3 * EPB_, GenOcc<Ep<N>::N3 * EPB_>::value) k_cons_k1(const K1P<real> P0, const K1P<real>* __restrict__ plist,
-                                                            const int2* __restrict__ tiles, long long ntiles) {
-  constexpr int N3 = Ep<N>::N3, N2 = Ep<N>::N2, EPB = EPB_;
-  // CP: u = Phi + Phit and its derivative D u in FP64; with Ja = Ja0 + dJa
-  // (Ja0 element-constant, FP64) the split form is
-  //   0.5 D(Ja u) + 0.5 Ja D u = (Ja0 + 0.5 dJa) D u + 0.5 D(dJa u),
-  // and only the last contraction, of the small dJa u, runs in FP32
-  using gt = typename std::conditional<CP, double, real>::type;  // precision of u and D u
-  __shared__ gt GT[N2];
-  __shared__ real GTr[CP ? N2 : 1];  // CP: the operator in FP32 for D(dJa u)
-  __shared__ gt su[EPB][N3];
-  __shared__ gt sun[EPB][6][N2];
-  __shared__ real sw[CURV ? EPB : 1][CURV ? 9 : 1][CURV ? N3 : 1];
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const int i = t % N, j = (t / N) % N, k = t / N2;
-  long long e = (BATCH ? 0 : P0.e0) + (long long)blockIdx.x * EPB + le;
-  int sid = 0;
-  bool valid;
-  if constexpr (BATCH) {
-    valid = e < ntiles;
-    if (valid) {
-      const int2 tl = tiles[e];
-      sid = tl.x;
-      e = tl.y;
-    }
-  } else {
-    valid = e < P0.e1;
-  }
-  const K1P<real>& P = BATCH ? plist[sid] : P0;
-  const long long ec = valid ? e : 0;  // clamp for address arithmetic
-  const long long n = ec * N3 + t;
-  const long long nn = P.nn;
-  if (tid < N2) GT[(tid % N) * N + tid / N] = (gt)P.G[tid];
-  if constexpr (CP) {
-    if (tid < N2) GTr[(tid % N) * N + tid / N] = (real)P.G[tid];
-  }
-  // the node pass's own-node words, copied now (cp.async) so that their loads run
-  // under the contraction: c10 [0..9], Pi [10], RK state y [11], acc [12],
-  // comp [13] (only the words this stage's update reads)
-  constexpr bool PF = 14 * N3 * EPB * sizeof(real) <= 24576;
-  __shared__ real spf[PF ? EPB : 1][PF ? 14 : 1][PF ? N3 : 1];
-  const bool grad_only = P.c10 == nullptr;
-  const bool pf_y = P.epi && (P.stage == 1 || P.stage == 2 || (!CP && P.comp && P.stage == 3));
-  const bool pf_acc = P.epi && P.stage >= 1;
-  const bool pf_comp = P.epi && (CP || (P.comp && P.stage == 3));
-  if constexpr (PF) {
-    if (valid && !grad_only) {
-#pragma unroll
-      for (int c = 0; c < 10; ++c) cp_async_word(&spf[le][c][t], P.c10 + c * nn + n);
-      cp_async_word(&spf[le][10][t], P.Pi + n);
-      if (pf_y) cp_async_word(&spf[le][11][t], P.y + n);
-      if (pf_acc) cp_async_word(&spf[le][12][t], P.acc + n);
-      if (pf_comp) cp_async_word(&spf[le][13][t], P.comp + n);
-    }
-  }
-  const real u = valid ? P.Phi[n] : (real)0;  // CP: the high part
-  gt ug = u;                                   // the value the gradient differentiates
-  if constexpr (CP) {
-    if (valid && P.Phit) ug += (gt)P.Phit[n];
-  }
-  su[le][t] = ug;
-  // element tables: SAT mask / outer-face flag, and the neighbour face sources
-  const int emask = valid ? P.emask[ec] : 0;
-  // neighbour Phi face traces (fsrc is -1 exactly where the SAT mask bit is 0,
-  // so the trace loads need not wait for the mask)
-  for (int idx = t; idx < 6 * N2; idx += N3) {
-    const int f = idx / N2, pq = idx - f * N2;
-    gt v = 0;
-    const int src = valid ? ::wt::bc_src(P.fsrc[f + 6 * ec], P.Ne) : -1;
-    if (src >= 0) {
-      const long long nb = (long long)(src >> 6) * N3 + nbr_face_node(src, pq % N, pq / N, N);
-      v = P.Phi[nb];
-      if constexpr (CP) {
-        if (P.Phit) v += (gt)P.Phit[nb];
-      }
-    }
-    sun[le][f][pq] = v;
-  }
-  real m[CURV ? 9 : 1];   // Ja (CP: its deviation dJa)
-  real m0[CP && CURV ? 9 : 1];  // CP: the element-constant part Ja0
-  real invJ = 0, sd[3];
-  if (CURV) {
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-      if constexpr (CP) {
-        m[c] = valid ? P.dJa[c * nn + n] : (real)0;
-        m0[c] = valid ? (real)P.Ja0[9 * ec + c] : (real)0;
-      } else {
-        m[c] = valid ? P.Ja[c * nn + n] : (real)0;
-      }
-    }
-    invJ = valid ? P.invdetJ[n] : (real)0;
-  } else {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) sd[d] = P.sdiag[3 * ec + d];
-  }
-  const real Hend = (real)P.H[0];
-  if (CURV) {
-#pragma unroll
-    for (int c = 0; c < 9; ++c) sw[le][c][t] = m[c] * (real)ug;  // CP: dJa u
-  }
-  __syncthreads();
-  real du[3];  // D u (CP: formed in FP64, then a gradient-sized value)
-#pragma unroll
-  for (int d = 0; d < 3; ++d) du[d] = (real)contract<N>(su[le], GT, i, j, k, d);
-  real g[3];
-  if (CURV) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      real acc = 0;
-#pragma unroll
-      for (int al = 0; al < 3; ++al) {
-        if constexpr (CP)
-          acc += (real)0.5 * contract<N>(sw[le][al * 3 + c], GTr, i, j, k, al) +
-                 (m0[al * 3 + c] + (real)0.5 * m[al * 3 + c]) * du[al];
-        else
-          acc += (real)0.5 * contract<N>(sw[le][al * 3 + c], GT, i, j, k, al) + (real)0.5 * m[al * 3 + c] * du[al];
-      }
-      g[c] = acc;
-    }
-  } else {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) g[d] = sd[d] * du[d];
-  }
-  // centred-flux SAT on interior faces through this node (CP: the jump formed in FP64)
-  if (valid) {
-    const int idx3[3] = {i, j, k};
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      const int ax = f >> 1;
-      if (idx3[ax] != frow(f, N)) continue;
-      if (!((emask >> f) & 1)) continue;
-      const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-      const real jump = (real)(sun[le][f][p + N * q] - ug);
-      const real nh = (f & 1) ? (real)1 : (real)-1;
-      if (CURV) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          real mc = m[ax * 3 + c];
-          if constexpr (CP) mc += m0[ax * 3 + c];
-          g[c] += nh * mc * jump / ((real)2 * Hend);
-        }
-      } else {
-        g[ax] += nh * sd[ax] / ((real)2 * Hend) * jump;
-      }
-    }
-  }
-  if (CURV) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) g[c] *= invJ;
-  }
-  if (!valid) return;
-  // the node's coefficients and Pi: from the words copied at kernel start, or
-  // (no room for them) loaded only now -- held in registers across the
-  // contraction they would cost the registers that keep more CTAs resident
-  real a = 0, b[3] = {0, 0, 0}, K[6] = {0, 0, 0, 0, 0, 0}, Pi = 0;
-  if (!grad_only) {
-    if constexpr (PF) {
-      cp_async_wait_own();
-      a = spf[le][0][t];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) b[c] = spf[le][1 + c][t];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) K[c] = spf[le][4 + c][t];
-      Pi = spf[le][10][t];
-    } else {
-      a = P.c10[n];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) b[c] = P.c10[(1 + c) * nn + n];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) K[c] = P.c10[(4 + c) * nn + n];
-      Pi = P.Pi[n];
-    }
-  }
-  if (P.grad_out) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) P.grad_out[c * nn + n] = g[c];
-  }
-  if (grad_only) return;
-  k1_finish<N, real, CP, PF>(P, ec, n, i, j, k, emask, g, u, ug, sd, Hend, a, b, K, Pi,
-                             PF && pf_y ? spf[le][11][t] : (real)0, PF && pf_acc ? spf[le][12][t] : (real)0,
-                             PF && pf_comp ? spf[le][13][t] : (real)0);
 }
 
 // ---------------------------------------------------------------------------
-// Persistent, cp.async-pipelined K1 for work lists of n < 8 solves (the batch's
-// and the server's n = 4 and n = 6 groups).  The generic K1 above loads its
-// inputs when its one element starts (the face traces behind two dependent
-// loads), so it waits on global memory: about 0.2 of DRAM throughput, long-
-// scoreboard stalls.  Here a CTA loops over groups of EPB tiles and copies
-// everything group g + 1 reads at its own nodes -- Phi (and Phit), the metric
-// terms, 1/J, the ten coefficients, Pi, the RK words, the neighbour face
-// traces (sources loaded one group earlier) and Ja0 -- into the second of two
-// shared buffers while it computes group g.  The arithmetic is the generic
-// K1's (same contractions, same order, k1_finish for the node pass), so both
-// give the same bits.
-template <int N, typename real, bool CP>
-struct PipeK1 {
-  static constexpr int N3 = Ep<N>::N3, N2 = Ep<N>::N2, EPB = Ep<N>::EPB, T = N3 * EPB;
-  // own-node word planes of an element block in a buffer
-  static constexpr int PHI = 0, PHIT = 1, JA = CP ? 2 : 1, INVJ = JA + 9, C10 = INVJ + 1, PI = C10 + 10,
-                       Y = PI + 1, ACC = Y + 1, COMP = ACC + 1, NW = COMP + 1;
-  static constexpr int NF = CP ? 12 : 6;               // face-trace planes: Phi [+ Phit] on the 6 faces
-  static constexpr int NFR = (6 * N2 + N3 - 1) / N3;  // face entries per thread
-  // words of one element block (padded to 16 bytes) and of one buffer
-  static constexpr size_t EW = ((NW * N3 + NF * N2) * sizeof(real) + (CP ? 9 * sizeof(double) : 0) + 15) / 16 * 16;
-  static constexpr size_t BUF = EPB * EW;
-  using gt = typename std::conditional<CP, double, real>::type;
-  static constexpr size_t SU = ((size_t)EPB * N3 * sizeof(gt) + 15) / 16 * 16;
-  static constexpr size_t SW = ((size_t)EPB * 9 * N3 * sizeof(real) + 15) / 16 * 16;
-  static constexpr size_t SMEM = 2 * BUF + SU + SW + N2 * sizeof(gt) + N2 * sizeof(real) + 16;
-  // resident CTAs per SM the registers are sized for: as many as the shared memory
-  // allows, up to 1024 threads
-  static constexpr int OCC_SM = (int)(220000 / SMEM) > 0 ? (int)(220000 / SMEM) : 1;
-  static constexpr int OCC = OCC_SM < 1024 / T ? OCC_SM : 1024 / T;
-  static_assert(!CP || ((NW * N3 + NF * N2) * sizeof(real)) % 8 == 0, "Ja0 must be 8-byte aligned in a block");
+// The kernels of any order.  3 N^2 threads per element, one per (axis, pencil):
+// a thread takes its pencil's N values into registers and applies the operator,
+// kernel parameters in the constant bank, so that a multiply-add costs no operand
+// load from shared memory (with a thread per node both operands came from there,
+// 24 N words a node).  What bounds the kernels now is the latency of their global
+// loads at the occupancy the pencils' registers leave: N = 6 FP64, 24^3 elements,
+// K1 reaches 4.7 TB/s (26 words a node), K2 3.1 TB/s (14 words).  Measured, one RK4
+// step (B200, FP64 / compensated FP32): N = 4, 36^3 elements 1184 -> 1026 / 876 ->
+// 687 us; N = 5, 28^3 1280 -> 845 / 765 -> 611; N = 6, 24^3 1336 -> 971 / 942 ->
+// 601; N = 7, 20^3 1581 -> 1003 / 1118 -> 579.  Fields that are read along pencils (Phi and the metric terms in
+// K1, F and the metric terms in K2) arrive by cp.async in a padded layout; axis
+// al's results replace its own metric terms there, pencil by pencil, and after one
+// barrier a node pass sums the three axes, in node order.
+//
+// BATCH: the CTA's elements come from a work list of (solve, element) tiles
+// and each tile reads the parameter block of its solve (plist); otherwise
+// element e0 + blockIdx.x * epb + le of the single solve P0.  epb: elements per CTA.
+template <int N>
+struct Pen {
+  static constexpr int N2 = N * N, N3 = N * N * N, TE = 3 * N2;
+  static constexpr int EPB = TE >= 96 ? 1 : 160 / TE;  // the most elements a CTA holds
+  static constexpr int T = TE * EPB;
+  static constexpr int P1 = N | 1;       // odd row pitch: x pencils without bank conflicts
+  static constexpr int NS = N * N * P1;  // words of one padded field of an element
+  static constexpr int NI = (N3 + TE - 1) / TE;  // nodes per thread of the node pass
+  // Threads per SM the registers are sized for.  FP64 up to N = 5: 768 (72
+  // registers, a few spills; 576 without spills took 15-30 % longer), N = 6: 640
+  // with the node pass's words prefetched (pf1), N = 7: 600, N = 8: 448 (at 768 the pencils
+  // spill: N = 7 33 % slower); FP32: 1024.
+  template <typename real>
+  static constexpr int occ() { return (sizeof(real) == 4 ? 1024 : N == 8 ? 448 : N == 7 ? 600 : N == 6 ? 640 : 768) / T; }
+  // Whether K1 copies the node pass's words (coefficients, Pi, 1/J, RK words) to
+  // shared memory at kernel start: it hides their latency and costs resident
+  // CTAs.  24^3 elements, one step (B200): N = 6 FP64 971 us with, 1044 without;
+  // N = 4, 5, 7 FP64 7-18 % slower with, FP32 0-14 %.  K2's three words always.
+  template <typename real>
+  static constexpr bool pf1() { return sizeof(real) == 8 && N == 6; }
+  static __device__ __forceinline__ int place(int w) { return w + (P1 - N) * (w / N); }
 };
 
-template <int N, typename real, bool CP>
-__global__ void __launch_bounds__(PipeK1<N, real, CP>::T, PipeK1<N, real, CP>::OCC)
-    k_cons_k1_pipe(const K1P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles) {
-  using L = PipeK1<N, real, CP>;
-  using gt = typename L::gt;
-  constexpr int N3 = L::N3, N2 = L::N2, EPB = L::EPB, NFR = L::NFR;
+// the operator: G in FP64 (CP's gradient of Phi) and in the state's type, 1 / (2 H_end)
+template <int N, typename real>
+struct OpP {
+  real G[N * N];
+  double Gd[N * N];
+  real c2H;
+};
+
+// where a tile's element is: false if there is none
+template <bool BATCH, typename KP>
+__device__ __forceinline__ bool tile_element(const KP& P0, const int2* __restrict__ tiles, long long ntiles, int epb,
+                                             int le, int& sid, long long& e) {
+  e = (BATCH ? 0 : P0.e0) + (long long)blockIdx.x * epb + le;
+  sid = 0;
+  if constexpr (BATCH) {
+    if (e >= ntiles) return false;
+    const int2 tl = tiles[e];
+    sid = tl.x;
+    e = tl.y;
+    return true;
+  } else {
+    return e < P0.e1;
+  }
+}
+
+// shared words of one element in K1: Phi (CP: and its small part), the nine metric
+// terms / axis results (affine: three results)
+template <int N, typename real, bool CURV, bool CP>
+constexpr int k1_words() {
+  return Pen<N>::NS * ((CP ? 2 : 1) + (CURV ? 9 : 3)) + (Pen<N>::template pf1<real>() ? 15 * Pen<N>::N3 : 0);
+}
+
+// CP (real = float): the compensated form -- u = Phi + Phit and D u in FP64; with
+// Ja = Ja0 + dJa (Ja0 element-constant, FP64) the split form is
+//   0.5 D(Ja u) + 0.5 Ja D u = (Ja0 + 0.5 dJa) D u + 0.5 D(dJa u),
+// and only the last contraction, of the small dJa u, runs in FP32.
+template <int N, typename real, bool CURV, bool BATCH, bool CP>
+__global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
+    k_cons_k1(const __grid_constant__ K1P<real> P0, const __grid_constant__ OpP<N, real> O,
+              const K1P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles, int epb) {
+  using L = Pen<N>;
+  using gt = typename std::conditional<CP, double, real>::type;  // precision of u and D u
+  constexpr int N2 = L::N2, N3 = L::N3, TE = L::TE, NS = L::NS, P1 = L::P1;
   extern __shared__ __align__(16) unsigned char smraw[];
-  gt* su = reinterpret_cast<gt*>(smraw + 2 * L::BUF);                   // [EPB][N3]
-  real* sw = reinterpret_cast<real*>(smraw + 2 * L::BUF + L::SU);       // [EPB][9][N3]
-  gt* GT = reinterpret_cast<gt*>(smraw + 2 * L::BUF + L::SU + L::SW);   // transposed G
-  real* GTr = reinterpret_cast<real*>(GT + N2);                         // CP: G in FP32
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const int i = t % N, j = (t / N) % N, k = t / N2;
-  const long long ngroups = (ntiles + EPB - 1) / EPB;
-  const long long GS = gridDim.x;
-  auto blk = [&](int bb) -> real* { return reinterpret_cast<real*>(smraw + bb * L::BUF + le * L::EW); };
-  // this thread's tile in group gg (x = -1: none)
-  auto tile_of = [&](long long gg) -> int2 {
-    const long long ti = gg * EPB + le;
-    return (gg < ngroups && ti < ntiles) ? tiles[ti] : make_int2(-1, -1);
-  };
-  auto src_load = [&](int2 tl, int src[NFR]) {
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = t + r * N3;
-      src[r] = (tl.x >= 0 && idx < 6 * N2) ? ::wt::bc_src(plist[tl.x].fsrc[idx / N2 + 6 * tl.y], plist[tl.x].Ne) : -1;
-    }
-  };
-  // copy what tile tl reads at this thread's node, and this thread's face-trace
-  // entries, into buffer bb
-  auto issue = [&](int2 tl, const int src[NFR], int bb) {
-    if (tl.x < 0) return;
-    const K1P<real>& P = plist[tl.x];
-    const long long e = tl.y, n = e * N3 + t, nn = P.nn;
-    real* w = blk(bb);
-    cp_async_word(w + L::PHI * N3 + t, P.Phi + n);
-    if constexpr (CP) cp_async_word_z(w + L::PHIT * N3 + t, P.Phit ? P.Phit + n : P.Phi + n, P.Phit != nullptr);
+  const int tid = threadIdx.x, le = tid / TE, t = tid - le * TE, ax = t / N2, pq = t - ax * N2, p = pq % N, q = pq / N;
+  real* sphi = reinterpret_cast<real*>(smraw) + (size_t)le * k1_words<N, real, CURV, CP>();
+  real* sphit = sphi + NS;               // CP
+  real* sr = sphi + (CP ? 2 : 1) * NS;   // metric terms, then the axes' results
+  constexpr bool PF = L::template pf1<real>();
+  real* sw = sr + (CURV ? 9 : 3) * NS;   // the node pass's own words (PF)
+  int sid;
+  long long e;
+  const bool valid = tile_element<BATCH>(P0, tiles, ntiles, epb, le, sid, e);
+  const K1P<real>& P = BATCH ? plist[sid] : P0;
+  const long long ec = valid ? e : 0, nn = P.nn;
+  const bool pf_y = P.epi && (P.stage == 1 || P.stage == 2 || (!CP && P.comp && P.stage == 3));
+  const bool pf_acc = P.epi && P.stage >= 1;
+  const bool pf_comp = P.epi && P.comp && (CP || P.stage == 3);
+  real jh[2] = {0, 0};  // n jump / (2 H) at the two ends
+  gt un[2] = {0, 0};
+  int src[2] = {-1, -1};
+  real m0[3] = {0, 0, 0}, sd = 0;
+  if (valid) {
     const real* ja = CP ? P.dJa : P.Ja;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) cp_async_word(w + (L::JA + c) * N3 + t, ja + c * nn + n);
-    cp_async_word(w + L::INVJ * N3 + t, P.invdetJ + n);
-    if (P.c10) {
+    for (int it = 0; it < L::NI; ++it) {
+      const int w = t + it * TE;
+      if (N3 % TE != 0 && w >= N3) break;
+      const long long n = ec * N3 + w;
+      const int at = L::place(w);
+      cp_async_word(sphi + at, P.Phi + n);
+      if constexpr (CP) {
+        if (P.Phit) cp_async_word(sphit + at, P.Phit + n);
+      }
+      if constexpr (CURV) {
 #pragma unroll
-      for (int c = 0; c < 10; ++c) cp_async_word(w + (L::C10 + c) * N3 + t, P.c10 + c * nn + n);
-      cp_async_word(w + L::PI * N3 + t, P.Pi + n);
-    }
-    if (P.epi && (P.stage == 1 || P.stage == 2 || (!CP && P.comp && P.stage == 3)))
-      cp_async_word(w + L::Y * N3 + t, P.y + n);
-    if (P.epi && P.stage >= 1) cp_async_word(w + L::ACC * N3 + t, P.acc + n);
-    if (P.epi && (CP || (P.comp && P.stage == 3))) cp_async_word(w + L::COMP * N3 + t, P.comp + n);
-    real* fc = w + L::NW * N3;
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = t + r * N3;
-      if (idx < 6 * N2) {
-        const int f = idx / N2, pq = idx - f * N2, sr = src[r];
-        const long long nb = sr >= 0 ? (long long)(sr >> 6) * N3 + nbr_face_node(sr, pq % N, pq / N, N) : 0;
-        cp_async_word_z(fc + f * N2 + pq, P.Phi + nb, sr >= 0);
-        if constexpr (CP) cp_async_word_z(fc + (6 + f) * N2 + pq, (P.Phit ? P.Phit : P.Phi) + nb, sr >= 0 && P.Phit);
+        for (int c = 0; c < 9; ++c) cp_async_word(sr + c * NS + at, ja + c * nn + n);
       }
     }
-    if constexpr (CP) {
-      if (t < 9) cp_async_word(reinterpret_cast<double*>(fc + L::NF * N2) + t, P.Ja0 + 9 * e + t);
+    cp_async_commit();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (src[h] >= 0) {
+        const long long nb = (long long)(src[h] >> 6) * N3 + nbr_face_node(src[h], p, q, N);
+        un[h] = P.Phi[nb];
+        if constexpr (CP) {
+          if (P.Phit) un[h] += (gt)P.Phit[nb];
+        }
+      }
+    if constexpr (CP && CURV) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) m0[c] = (real)P.Ja0[9 * ec + 3 * ax + c];
     }
-  };
-
-  if (tid < N2) {
-    GT[(tid % N) * N + tid / N] = (gt)plist[0].G[tid];  // every solve of a group has the same N, hence G
-    if constexpr (CP) GTr[(tid % N) * N + tid / N] = (real)plist[0].G[tid];
+    if constexpr (!CURV) sd = P.sdiag[3 * ec + ax];
+    if constexpr (PF) {
+#pragma unroll
+      for (int it = 0; it < L::NI; ++it) {
+        const int w = t + it * TE;
+        if (N3 % TE != 0 && w >= N3) break;
+        const long long n = ec * N3 + w;
+        if constexpr (CURV) cp_async_word(sw + w, P.invdetJ + n);
+        if (P.c10) {
+#pragma unroll
+          for (int c = 0; c < 10; ++c) cp_async_word(sw + (1 + c) * N3 + w, P.c10 + c * nn + n);
+          cp_async_word(sw + 11 * N3 + w, P.Pi + n);
+        }
+        if (pf_y) cp_async_word(sw + 12 * N3 + w, P.y + n);
+        if (pf_acc) cp_async_word(sw + 13 * N3 + w, P.acc + n);
+        if (pf_comp) cp_async_word(sw + 14 * N3 + w, P.comp + n);
+      }
+      cp_async_commit();
+    }
   }
-  long long g = blockIdx.x;
-  int2 tcur = tile_of(g), tnext = tile_of(g + GS);
-  int src[NFR];
-  src_load(tcur, src);
-  issue(tcur, src, 0);
-  src_load(tnext, src);
-  int emcur = tcur.x >= 0 ? plist[tcur.x].emask[tcur.y] : 0;
-  for (int it = 0; g < ngroups; g += GS, ++it) {
-    const int bb = it & 1;
-    const int2 tn2 = tile_of(g + 2 * GS);
-    const int emnext = tnext.x >= 0 ? plist[tnext.x].emask[tnext.y] : 0;
-    cp_async_wait_own();
-    // this group's words are visible to every thread, and every thread is done
-    // with the previous group: the other buffer, su and sw are free
-    __syncthreads();
-    issue(tnext, src, bb ^ 1);
-    src_load(tn2, src);
-    const bool valid = tcur.x >= 0;
-    const K1P<real>& P = plist[valid ? tcur.x : 0];
-    const long long ec = valid ? tcur.y : 0, n = ec * N3 + t;
-    const real* w = blk(bb);
-    const real* fc = w + L::NW * N3;
-    const int emask = emcur;
-    const real u = valid ? w[L::PHI * N3 + t] : (real)0;  // CP: the high part
+  cp_async_wait_group<PF ? 1 : 0>();
+  __syncthreads();
+  if (valid) {
+    const int pb = ax == 0 ? P1 * (p + N * q) : ax == 1 ? p + P1 * N * q : p + P1 * q;
+    const int ps = ax == 0 ? 1 : ax == 1 ? P1 : P1 * N;
+    gt u[N];
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      u[l] = sphi[pb + ps * l];
+      if constexpr (CP) {
+        if (P.Phit) u[l] += (gt)sphit[pb + ps * l];
+      }
+    }
+    if (src[0] >= 0) jh[0] = -((real)(un[0] - u[0]) * O.c2H);
+    if (src[1] >= 0) jh[1] = (real)(un[1] - u[N - 1]) * O.c2H;
+    real du[N];  // D u (CP: formed in FP64, then a gradient-sized value)
+#pragma unroll
+    for (int l = 0; l < N; ++l) {
+      gt s = 0;
+#pragma unroll
+      for (int m = 0; m < N; ++m) {
+        if constexpr (CP) s += O.Gd[l * N + m] * u[m];
+        else s += O.G[l * N + m] * u[m];
+      }
+      du[l] = (real)s;
+    }
+    if constexpr (CURV) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        real* f = sr + (3 * ax + c) * NS + pb;
+        real w[N];
+#pragma unroll
+        for (int l = 0; l < N; ++l) w[l] = f[ps * l] * (real)u[l];
+#pragma unroll
+        for (int l = 0; l < N; ++l) {
+          real s = 0;
+#pragma unroll
+          for (int k = 0; k < N; ++k) s += O.G[l * N + k] * w[k];
+          const real m = f[ps * l];  // read again: held, the pencil's terms would cost resident CTAs
+          real r = (real)0.5 * s + (CP ? m0[c] + (real)0.5 * m : (real)0.5 * m) * du[l];
+          if (l == 0) r += (CP ? m + m0[c] : m) * jh[0];
+          if (l == N - 1) r += (CP ? m + m0[c] : m) * jh[1];
+          f[ps * l] = r;
+        }
+      }
+    } else {
+      real* f = sr + ax * NS + pb;
+#pragma unroll
+      for (int l = 0; l < N; ++l) {
+        real r = sd * du[l];
+        if (l == 0) r += sd * jh[0];
+        if (l == N - 1) r += sd * jh[1];
+        f[ps * l] = r;
+      }
+    }
+  }
+  __syncthreads();
+  if (!valid) return;
+  cp_async_wait_own();
+  const bool grad_only = P.c10 == nullptr;
+  const int emask = P.emask[ec];
+  real sda[3] = {0, 0, 0};
+  if constexpr (!CURV) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) sda[d] = P.sdiag[3 * ec + d];
+  }
+  const real Hend = (real)P.H[0];
+#pragma unroll
+  for (int it = 0; it < L::NI; ++it) {
+    const int w = t + it * TE;
+    if (N3 % TE != 0 && w >= N3) break;
+    const long long n = ec * N3 + w;
+    const int at = L::place(w);
+    real a = 0, b[3] = {0, 0, 0}, K[6] = {0, 0, 0, 0, 0, 0}, Pi = 0;
+    if (!grad_only) {
+      const real* cw = PF ? sw + N3 + w : P.c10 + n;
+      const long long cs = PF ? N3 : nn;
+      a = cw[0];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) b[c] = cw[(1 + c) * cs];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) K[c] = cw[(4 + c) * cs];
+      Pi = PF ? sw[11 * N3 + w] : P.Pi[n];
+    }
+    const real yv = !pf_y ? (real)0 : PF ? sw[12 * N3 + w] : P.y[n];
+    const real accv = !pf_acc ? (real)0 : PF ? sw[13 * N3 + w] : P.acc[n];
+    const real compv = !pf_comp ? (real)0 : PF ? sw[14 * N3 + w] : P.comp[n];
+    real g[3];
+    if constexpr (CURV) {
+      const real invJ = PF ? sw[w] : P.invdetJ[n];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) g[c] = (sr[c * NS + at] + sr[(3 + c) * NS + at] + sr[(6 + c) * NS + at]) * invJ;
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) g[c] = sr[c * NS + at];
+    }
+    if (P.grad_out) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) P.grad_out[c * nn + n] = g[c];
+    }
+    if (grad_only) continue;
+    const real u = sphi[at];  // CP: the high part
     gt ug = u;
     if constexpr (CP) {
-      if (valid && P.Phit) ug += (gt)w[L::PHIT * N3 + t];
+      if (P.Phit) ug += (gt)sphit[at];
     }
-    su[le * N3 + t] = ug;
-    real m[9], m0[CP ? 9 : 1];
-    const double* ja0 = reinterpret_cast<const double*>(fc + L::NF * N2);
-#pragma unroll
-    for (int c = 0; c < 9; ++c) {
-      m[c] = valid ? w[(L::JA + c) * N3 + t] : (real)0;
-      if constexpr (CP) m0[c] = valid ? (real)ja0[c] : (real)0;
-    }
-    const real invJ = valid ? w[L::INVJ * N3 + t] : (real)0;
-    const real Hend = (real)P.H[0];
-#pragma unroll
-    for (int c = 0; c < 9; ++c) sw[(le * 9 + c) * N3 + t] = m[c] * (real)ug;
-    __syncthreads();
-    real du[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) du[d] = (real)contract<N>(su + le * N3, GT, i, j, k, d);
-    real g3[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      real acc = 0;
-#pragma unroll
-      for (int al = 0; al < 3; ++al) {
-        if constexpr (CP)
-          acc += (real)0.5 * contract<N>(sw + (le * 9 + al * 3 + c) * N3, GTr, i, j, k, al) +
-                 (m0[al * 3 + c] + (real)0.5 * m[al * 3 + c]) * du[al];
-        else
-          acc += (real)0.5 * contract<N>(sw + (le * 9 + al * 3 + c) * N3, GT, i, j, k, al) +
-                 (real)0.5 * m[al * 3 + c] * du[al];
-      }
-      g3[c] = acc;
-    }
-    if (valid) {
-      const int idx3[3] = {i, j, k};
-#pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        const int ax = f >> 1;
-        if (idx3[ax] != frow(f, N)) continue;
-        if (!((emask >> f) & 1)) continue;
-        const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-        gt sv = fc[f * N2 + p + N * q];
-        if constexpr (CP) {
-          if (P.Phit) sv += (gt)fc[(6 + f) * N2 + p + N * q];
-        }
-        const real jump = (real)(sv - ug);
-        const real nh = (f & 1) ? (real)1 : (real)-1;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          real mc = m[ax * 3 + c];
-          if constexpr (CP) mc += m0[ax * 3 + c];
-          g3[c] += nh * mc * jump / ((real)2 * Hend);
-        }
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) g3[c] *= invJ;
-    if (valid) {
-      if (P.grad_out) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) P.grad_out[c * P.nn + n] = g3[c];
-      }
-      if (P.c10) {
-        const real a = w[L::C10 * N3 + t];
-        real b[3], K[6];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) b[c] = w[(L::C10 + 1 + c) * N3 + t];
-#pragma unroll
-        for (int c = 0; c < 6; ++c) K[c] = w[(L::C10 + 4 + c) * N3 + t];
-        const real Pi = w[L::PI * N3 + t];
-        const bool pf_y = P.epi && (P.stage == 1 || P.stage == 2 || (!CP && P.comp && P.stage == 3));
-        const bool pf_acc = P.epi && P.stage >= 1;
-        const bool pf_comp = P.epi && (CP || (P.comp && P.stage == 3));
-        const real sd[3] = {0, 0, 0};
-        k1_finish<N, real, CP, true>(P, ec, n, i, j, k, emask, g3, u, ug, sd, Hend, a, b, K, Pi,
-                                     pf_y ? w[L::Y * N3 + t] : (real)0, pf_acc ? w[L::ACC * N3 + t] : (real)0,
-                                     pf_comp ? w[L::COMP * N3 + t] : (real)0);
-      }
-    }
-    tcur = tnext;
-    tnext = tn2;
-    emcur = emnext;
+    k1_finish<N, real, CP>(P, ec, n, w % N, (w / N) % N, w / N2, emask, g, u, ug, sda, Hend, a, b, K, Pi, yv, accv, compv);
   }
-  cp_async_wait_own();
 }
 
 template <typename real>
@@ -655,288 +491,164 @@ struct K2P {
   unsigned int* nonfinite;
 };
 
-template <int N, typename real, bool CURV, bool BATCH, int EPB_>
-__global__ void __launch_bounds__(Ep<N>::N3 * EPB_) k_cons_k2(const K2P<real> P0, const K2P<real>* __restrict__ plist,
-                                                            const int2* __restrict__ tiles, long long ntiles) {
-  constexpr int N3 = Ep<N>::N3, N2 = Ep<N>::N2, EPB = EPB_;
-  __shared__ real GT[N2];
-  __shared__ real sF[EPB][3][N3];
-  __shared__ real sFn[EPB][6][CURV ? 3 : 1][N2];
-  __shared__ real sw[CURV ? EPB : 1][CURV ? 3 : 1][CURV ? N3 : 1];
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const int i = t % N, j = (t / N) % N, k = t / N2;
-  long long e = (BATCH ? 0 : P0.e0) + (long long)blockIdx.x * EPB + le;
-  int sid = 0;
-  bool valid;
-  if constexpr (BATCH) {
-    valid = e < ntiles;
-    if (valid) {
-      const int2 tl = tiles[e];
-      sid = tl.x;
-      e = tl.y;
-    }
-  } else {
-    valid = e < P0.e1;
-  }
-  const K2P<real>& P = BATCH ? plist[sid] : P0;
-  const long long ec = valid ? e : 0;
-  const long long n = ec * N3 + t;
-  const long long nn = P.nn;
-  if (tid < N2) GT[(tid % N) * N + tid / N] = (real)P.G[tid];
-  // the RK state words the stage update reads at this node, copied now (see K1):
-  // y [0], acc [1], comp [2]
-  constexpr bool PF = 3 * N3 * EPB * sizeof(real) <= 12288;
-  __shared__ real spf[PF ? EPB : 1][PF ? 3 : 1][PF ? N3 : 1];
-  const bool pf_y = P.epi && (P.stage <= 2 || (P.comp && P.stage == 3));
-  const bool pf_acc = P.epi && P.stage >= 1;
-  const bool pf_comp = P.epi && P.comp && P.stage == 3;
-  if constexpr (PF) {
-    if (valid) {
-      if (pf_y) cp_async_word(&spf[le][0][t], P.y + n);
-      if (pf_acc) cp_async_word(&spf[le][1][t], P.acc + n);
-      if (pf_comp) cp_async_word(&spf[le][2][t], P.comp + n);
-    }
-  }
-  const real* Fp[3] = {P.F0, P.F1, P.F2};
-  real Fv[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    Fv[c] = valid ? Fp[c][n] : (real)0;
-    sF[le][c][t] = Fv[c];
-  }
-  const int emask = valid ? P.emask[ec] : 0;
-  for (int idx = t; idx < 6 * N2; idx += N3) {
-    const int f = idx / N2, pq = idx - f * N2;
-    long long src = -1;
-    const int fs = valid ? ::wt::bc_src(P.fsrc[f + 6 * ec], P.Ne) : -1;  // -1 exactly where the SAT mask bit is 0
-    if (fs >= 0) src = (long long)(fs >> 6) * N3 + nbr_face_node(fs, pq % N, pq / N, N);
-    if (CURV) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) sFn[le][f][c][pq] = src >= 0 ? Fp[c][src] : (real)0;
-    } else {
-      sFn[le][f][0][pq] = src >= 0 ? Fp[f >> 1][src] : (real)0;
-    }
-  }
-  real m[CURV ? 9 : 1];
-  real invJ = 0, sd[3];
-  if (CURV) {
-#pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = valid ? P.Ja[c * nn + n] : (real)0;
-    invJ = valid ? P.invdetJ[n] : (real)0;
-#pragma unroll
-    for (int al = 0; al < 3; ++al) sw[le][al][t] = m[al * 3] * Fv[0] + m[al * 3 + 1] * Fv[1] + m[al * 3 + 2] * Fv[2];
-  } else {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) sd[d] = P.sdiag[3 * ec + d];
-  }
-  const real Hend = (real)P.H[0];
-  __syncthreads();
-  real dv = 0;
-  if (CURV) {
-#pragma unroll
-    for (int al = 0; al < 3; ++al) {
-      dv += (real)0.5 * contract<N>(sw[le][al], GT, i, j, k, al);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) dv += (real)0.5 * m[al * 3 + c] * contract<N>(sF[le][c], GT, i, j, k, al);
-    }
-  } else {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) dv += sd[d] * contract<N>(sF[le][d], GT, i, j, k, d);
-  }
-  if (!valid) return;
-  const int idx3[3] = {i, j, k};
-#pragma unroll
-  for (int f = 0; f < 6; ++f) {
-    const int ax = f >> 1;
-    if (idx3[ax] != frow(f, N)) continue;
-    if (!((emask >> f) & 1)) continue;
-    const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-    const real nh = (f & 1) ? (real)1 : (real)-1;
-    if (CURV) {
-      real s = 0;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) s += m[ax * 3 + c] * (sFn[le][f][c][p + N * q] - Fv[c]);
-      dv += nh * s / ((real)2 * Hend);
-    } else {
-      dv += nh * sd[ax] / ((real)2 * Hend) * (sFn[le][f][0][p + N * q] - Fv[ax]);
-    }
-  }
-  if (CURV) dv *= invJ;
-  if (P.bc_on && (emask >> 6)) {
-    for (int f = 0; f < 6; ++f) {
-      if (P.bdry[f + 6 * ec] == 0) continue;
-      const int ax = f >> 1;
-      if (idx3[ax] != frow(f, N)) continue;
-      const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-      dv += P.bbuf[(long long)::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf) * N2 + p + N * q];
-    }
-  }
-  if (P.epi) {
-    if constexpr (PF) {
-      cp_async_wait_own();
-      const real yv = pf_y ? spf[le][0][t] : (real)0, accv = pf_acc ? spf[le][1][t] : (real)0,
-                 compv = pf_comp ? spf[le][2][t] : (real)0;
-      rk_epilogue_v<real>(P.stage, P.dt, dv, P.stage == 0 ? yv : (real)0, yv, accv, compv, P.y, P.acc, P.out, P.comp,
-                          n, P.nonfinite);
-    } else {
-      const real yin = P.stage == 0 ? P.y[n] : (real)0;
-      rk_epilogue<real>(P.stage, P.dt, dv, yin, P.y, P.acc, P.out, P.comp, n, P.nonfinite);
-    }
-  } else {
-    P.Pidot[n] = dv;
-  }
+// shared words of one element in K2: F and the nine metric terms / axis results
+template <int N, bool CURV>
+constexpr int k2_words() {
+  return Pen<N>::NS * (CURV ? 12 : 3) + 4 * Pen<N>::N3;
 }
 
-// Persistent, cp.async-pipelined K2 for work lists of n < 8 solves (see
-// k_cons_k1_pipe): group g + 1's F, metric terms, 1/J, RK words and neighbour
-// flux face traces are copied into the second shared buffer while group g is
-// computed with the generic K2's arithmetic.
-template <int N, typename real>
-struct PipeK2 {
-  static constexpr int N3 = Ep<N>::N3, N2 = Ep<N>::N2, EPB = Ep<N>::EPB, T = N3 * EPB;
-  static constexpr int F = 0, JA = 3, INVJ = 12, Y = 13, ACC = 14, COMP = 15, NW = 16;
-  static constexpr int NF = 18;                        // face-trace planes: F_c on the 6 faces
-  static constexpr int NFR = (6 * N2 + N3 - 1) / N3;  // face points per thread (3 components each)
-  static constexpr size_t EW = ((NW * N3 + NF * N2) * sizeof(real) + 15) / 16 * 16;
-  static constexpr size_t BUF = EPB * EW;
-  static constexpr size_t SW = ((size_t)EPB * 3 * N3 * sizeof(real) + 15) / 16 * 16;
-  static constexpr size_t SMEM = 2 * BUF + SW + N2 * sizeof(real) + 16;
-  static constexpr int OCC_SM = (int)(220000 / SMEM) > 0 ? (int)(220000 / SMEM) : 1;
-  static constexpr int OCC = OCC_SM < 1024 / T ? OCC_SM : 1024 / T;
-};
-
-template <int N, typename real>
-__global__ void __launch_bounds__(PipeK2<N, real>::T, PipeK2<N, real>::OCC)
-    k_cons_k2_pipe(const K2P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles) {
-  using L = PipeK2<N, real>;
-  constexpr int N3 = L::N3, N2 = L::N2, EPB = L::EPB, NFR = L::NFR;
+template <int N, typename real, bool CURV, bool BATCH>
+__global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
+    k_cons_k2(const __grid_constant__ K2P<real> P0, const __grid_constant__ OpP<N, real> O,
+              const K2P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles, int epb) {
+  using L = Pen<N>;
+  constexpr int N2 = L::N2, N3 = L::N3, TE = L::TE, NS = L::NS, P1 = L::P1;
   extern __shared__ __align__(16) unsigned char smraw[];
-  real* sw = reinterpret_cast<real*>(smraw + 2 * L::BUF);              // [EPB][3][N3]
-  real* GT = reinterpret_cast<real*>(smraw + 2 * L::BUF + L::SW);      // transposed G
-  const int tid = threadIdx.x;
-  const int le = tid / N3, t = tid - le * N3;
-  const int i = t % N, j = (t / N) % N, k = t / N2;
-  const long long ngroups = (ntiles + EPB - 1) / EPB;
-  const long long GS = gridDim.x;
-  auto blk = [&](int bb) -> real* { return reinterpret_cast<real*>(smraw + bb * L::BUF + le * L::EW); };
-  auto tile_of = [&](long long gg) -> int2 {
-    const long long ti = gg * EPB + le;
-    return (gg < ngroups && ti < ntiles) ? tiles[ti] : make_int2(-1, -1);
-  };
-  auto src_load = [&](int2 tl, int src[NFR]) {
+  const int tid = threadIdx.x, le = tid / TE, t = tid - le * TE, ax = t / N2, pq = t - ax * N2, p = pq % N, q = pq / N;
+  real* sF = reinterpret_cast<real*>(smraw) + (size_t)le * k2_words<N, CURV>();
+  real* sJ = sF + 3 * NS;  // metric terms; axis al's result replaces its first one (affine: F_al)
+  int sid;
+  long long e;
+  const bool valid = tile_element<BATCH>(P0, tiles, ntiles, epb, le, sid, e);
+  const K2P<real>& P = BATCH ? plist[sid] : P0;
+  const long long ec = valid ? e : 0, nn = P.nn;
+  const real* const Fp[3] = {P.F0, P.F1, P.F2};
+  real* sw = sF + (CURV ? 12 : 3) * NS;  // the node pass's own words
+  const bool pf_y = P.epi && (P.stage <= 2 || P.comp);
+  const bool pf_acc = P.epi && P.stage >= 1;
+  const bool pf_comp = P.epi && P.comp && P.stage == 3;
+  int src[2] = {-1, -1};
+  real fn[2][CURV ? 3 : 1] = {}, sd = 0;
+  if (valid) {
 #pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = t + r * N3;
-      src[r] = (tl.x >= 0 && idx < 6 * N2) ? ::wt::bc_src(plist[tl.x].fsrc[idx / N2 + 6 * tl.y], plist[tl.x].Ne) : -1;
-    }
-  };
-  auto issue = [&](int2 tl, const int src[NFR], int bb) {
-    if (tl.x < 0) return;
-    const K2P<real>& P = plist[tl.x];
-    const long long e = tl.y, n = e * N3 + t, nn = P.nn;
-    const real* Fp[3] = {P.F0, P.F1, P.F2};
-    real* w = blk(bb);
+    for (int it = 0; it < L::NI; ++it) {
+      const int w = t + it * TE;
+      if (N3 % TE != 0 && w >= N3) break;
+      const long long n = ec * N3 + w;
+      const int at = L::place(w);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) cp_async_word(w + (L::F + c) * N3 + t, Fp[c] + n);
+      for (int c = 0; c < 3; ++c) cp_async_word(sF + c * NS + at, Fp[c] + n);
+      if constexpr (CURV) {
 #pragma unroll
-    for (int c = 0; c < 9; ++c) cp_async_word(w + (L::JA + c) * N3 + t, P.Ja + c * nn + n);
-    cp_async_word(w + L::INVJ * N3 + t, P.invdetJ + n);
-    if (P.epi && (P.stage <= 2 || (P.comp && P.stage == 3))) cp_async_word(w + L::Y * N3 + t, P.y + n);
-    if (P.epi && P.stage >= 1) cp_async_word(w + L::ACC * N3 + t, P.acc + n);
-    if (P.epi && P.comp && P.stage == 3) cp_async_word(w + L::COMP * N3 + t, P.comp + n);
-    real* fc = w + L::NW * N3;
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = t + r * N3;
-      if (idx < 6 * N2) {
-        const int f = idx / N2, pq = idx - f * N2, sr = src[r];
-        const long long nb = sr >= 0 ? (long long)(sr >> 6) * N3 + nbr_face_node(sr, pq % N, pq / N, N) : 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) cp_async_word_z(fc + (f * 3 + c) * N2 + pq, Fp[c] + nb, sr >= 0);
+        for (int c = 0; c < 9; ++c) cp_async_word(sJ + c * NS + at, P.Ja + c * nn + n);
       }
     }
-  };
-  if (tid < N2) GT[(tid % N) * N + tid / N] = (real)plist[0].G[tid];
-  long long g = blockIdx.x;
-  int2 tcur = tile_of(g), tnext = tile_of(g + GS);
-  int src[NFR];
-  src_load(tcur, src);
-  issue(tcur, src, 0);
-  src_load(tnext, src);
-  int emcur = tcur.x >= 0 ? plist[tcur.x].emask[tcur.y] : 0;
-  for (int it = 0; g < ngroups; g += GS, ++it) {
-    const int bb = it & 1;
-    const int2 tn2 = tile_of(g + 2 * GS);
-    const int emnext = tnext.x >= 0 ? plist[tnext.x].emask[tnext.y] : 0;
-    cp_async_wait_own();
-    __syncthreads();  // see k_cons_k1_pipe
-    issue(tnext, src, bb ^ 1);
-    src_load(tn2, src);
-    const bool valid = tcur.x >= 0;
-    const K2P<real>& P = plist[valid ? tcur.x : 0];
-    const long long ec = valid ? tcur.y : 0, n = ec * N3 + t;
-    const real* w = blk(bb);
-    const real* fc = w + L::NW * N3;
-    const int emask = emcur;
-    real Fv[3], m[9];
+    cp_async_commit();
 #pragma unroll
-    for (int c = 0; c < 3; ++c) Fv[c] = valid ? w[(L::F + c) * N3 + t] : (real)0;
+    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
 #pragma unroll
-    for (int c = 0; c < 9; ++c) m[c] = valid ? w[(L::JA + c) * N3 + t] : (real)0;
-    const real invJ = valid ? w[L::INVJ * N3 + t] : (real)0;
+    for (int h = 0; h < 2; ++h)
+      if (src[h] >= 0) {
+        const long long nb = (long long)(src[h] >> 6) * N3 + nbr_face_node(src[h], p, q, N);
+        if constexpr (CURV) {
 #pragma unroll
-    for (int al = 0; al < 3; ++al)
-      sw[(le * 3 + al) * N3 + t] = m[al * 3] * Fv[0] + m[al * 3 + 1] * Fv[1] + m[al * 3 + 2] * Fv[2];
-    const real Hend = (real)P.H[0];
-    __syncthreads();
-    real dv = 0;
-#pragma unroll
-    for (int al = 0; al < 3; ++al) {
-      dv += (real)0.5 * contract<N>(sw + (le * 3 + al) * N3, GT, i, j, k, al);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) dv += (real)0.5 * m[al * 3 + c] * contract<N>(w + (L::F + c) * N3, GT, i, j, k, al);
-    }
-    if (valid) {
-      const int idx3[3] = {i, j, k};
-#pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        const int ax = f >> 1;
-        if (idx3[ax] != frow(f, N)) continue;
-        if (!((emask >> f) & 1)) continue;
-        const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-        const real nh = (f & 1) ? (real)1 : (real)-1;
-        real sacc = 0;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sacc += m[ax * 3 + c] * (fc[(f * 3 + c) * N2 + p + N * q] - Fv[c]);
-        dv += nh * sacc / ((real)2 * Hend);
-      }
-      dv *= invJ;
-      if (P.bc_on && (emask >> 6)) {
-        for (int f = 0; f < 6; ++f) {
-          if (P.bdry[f + 6 * ec] == 0) continue;
-          const int ax = f >> 1;
-          if (idx3[ax] != frow(f, N)) continue;
-          const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-          dv += P.bbuf[(long long)::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf) * N2 + p + N * q];
+          for (int c = 0; c < 3; ++c) fn[h][c] = Fp[c][nb];
+        } else {
+          fn[h][0] = (ax == 0 ? P.F0 : ax == 1 ? P.F1 : P.F2)[nb];
         }
       }
-      if (P.epi) {
-        const bool pf_y = P.stage <= 2 || (P.comp && P.stage == 3);
-        const real yv = pf_y ? w[L::Y * N3 + t] : (real)0;
-        const real accv = P.stage >= 1 ? w[L::ACC * N3 + t] : (real)0;
-        const real compv = P.comp && P.stage == 3 ? w[L::COMP * N3 + t] : (real)0;
-        rk_epilogue_v<real>(P.stage, P.dt, dv, P.stage == 0 ? yv : (real)0, yv, accv, compv, P.y, P.acc, P.out,
-                            P.comp, n, P.nonfinite);
-      } else {
-        P.Pidot[n] = dv;
+    if constexpr (!CURV) sd = P.sdiag[3 * ec + ax];
+#pragma unroll
+    for (int it = 0; it < L::NI; ++it) {
+      const int w = t + it * TE;
+      if (N3 % TE != 0 && w >= N3) break;
+      const long long n = ec * N3 + w;
+      if constexpr (CURV) cp_async_word(sw + w, P.invdetJ + n);
+      if (pf_y) cp_async_word(sw + N3 + w, P.y + n);
+      if (pf_acc) cp_async_word(sw + 2 * N3 + w, P.acc + n);
+      if (pf_comp) cp_async_word(sw + 3 * N3 + w, P.comp + n);
+    }
+    cp_async_commit();
+  }
+  cp_async_wait_group<1>();
+  __syncthreads();
+  if (valid) {
+    const int pb = ax == 0 ? P1 * (p + N * q) : ax == 1 ? p + P1 * N * q : p + P1 * q;
+    const int ps = ax == 0 ? 1 : ax == 1 ? P1 : P1 * N;
+    if constexpr (CURV) {
+      real w[N], r[N];
+      real s0 = 0, s1 = 0;  // sum_c Ja_c (F_c,nbr - F_c) at the ends
+#pragma unroll
+      for (int l = 0; l < N; ++l) w[l] = r[l] = 0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const real* Fc = sF + c * NS + pb;
+        const real* Jc = sJ + (3 * ax + c) * NS + pb;
+        real F[N], m[N];
+#pragma unroll
+        for (int l = 0; l < N; ++l) {
+          F[l] = Fc[ps * l];
+          m[l] = Jc[ps * l];
+          w[l] += m[l] * F[l];
+        }
+#pragma unroll
+        for (int l = 0; l < N; ++l) {
+          real s = 0;
+#pragma unroll
+          for (int k = 0; k < N; ++k) s += O.G[l * N + k] * F[k];
+          r[l] += (real)0.5 * m[l] * s;
+        }
+        s0 += m[0] * (fn[0][c] - F[0]);
+        s1 += m[N - 1] * (fn[1][c] - F[N - 1]);
+      }
+      if (src[0] >= 0) r[0] -= s0 * O.c2H;
+      if (src[1] >= 0) r[N - 1] += s1 * O.c2H;
+#pragma unroll
+      for (int l = 0; l < N; ++l) {
+        real s = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) s += O.G[l * N + k] * w[k];
+        sJ[3 * ax * NS + pb + ps * l] = r[l] + (real)0.5 * s;
+      }
+    } else {
+      real* Fd = sF + ax * NS + pb;
+      real F[N];
+#pragma unroll
+      for (int l = 0; l < N; ++l) F[l] = Fd[ps * l];
+#pragma unroll
+      for (int l = 0; l < N; ++l) {
+        real s = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) s += O.G[l * N + k] * F[k];
+        real r = sd * s;
+        if (l == 0 && src[0] >= 0) r -= sd * O.c2H * (fn[0][0] - F[0]);
+        if (l == N - 1 && src[1] >= 0) r += sd * O.c2H * (fn[1][0] - F[N - 1]);
+        Fd[ps * l] = r;
       }
     }
-    tcur = tnext;
-    tnext = tn2;
-    emcur = emnext;
   }
+  __syncthreads();
+  if (!valid) return;
   cp_async_wait_own();
+  const int emask = P.emask[ec];
+#pragma unroll
+  for (int it = 0; it < L::NI; ++it) {
+    const int w = t + it * TE;
+    if (N3 % TE != 0 && w >= N3) break;
+    const long long n = ec * N3 + w;
+    const int at = L::place(w);
+    real dv;
+    if constexpr (CURV) dv = (sJ[at] + sJ[3 * NS + at] + sJ[6 * NS + at]) * sw[w];
+    else dv = sF[at] + sF[NS + at] + sF[2 * NS + at];
+    if (P.bc_on && (emask >> 6)) {
+      const int idx3[3] = {w % N, (w / N) % N, w / N2};
+      for (int f = 0; f < 6; ++f) {
+        if (P.bdry[f + 6 * ec] == 0) continue;
+        const int fa = f >> 1;
+        if (idx3[fa] != frow(f, N)) continue;
+        const int fp = fa == 0 ? idx3[1] : idx3[0], fq = fa == 2 ? idx3[1] : idx3[2];
+        dv += P.bbuf[(long long)::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf) * N2 + fp + N * fq];
+      }
+    }
+    if (P.epi) {
+      const real yv = pf_y ? sw[N3 + w] : (real)0;
+      const real accv = pf_acc ? sw[2 * N3 + w] : (real)0;
+      const real compv = pf_comp ? sw[3 * N3 + w] : (real)0;
+      rk_epilogue_v<real>(P.stage, P.dt, dv, yv, yv, accv, compv, P.y, P.acc, P.out, P.comp, n, P.nonfinite);
+    } else {
+      P.Pidot[n] = dv;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1000,6 +712,7 @@ static K1P<real> k1p_params(const DevMesh& m, const DevCoef& c, const void* Phi,
   P.gDx = (const real*)bc.gDx; P.gDy = (const real*)bc.gDy; P.gDz = (const real*)bc.gDz;
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.nonfinite = rk.nonfinite;
+  if (!rk.on) P.y = P.acc = (real*)Phi;  // not read, but never a null address to form a load from
   P.Phit = (const real*)rk.phit; P.dJa = (const real*)m.dJa; P.Ja0 = m.Ja0; P.hcopy = (real*)rk.hcopy;
   return P;
 }
@@ -1026,7 +739,61 @@ static K2P<real> k2p_params(const DevMesh& m, const void* F, void* Pidot, const 
   P.Pidot = (real*)Pidot;
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.nonfinite = nonfinite;
+  if (!rk.on) P.y = P.acc = (real*)P.F0;  // not read (see k1p_params)
   return P;
+}
+
+template <int N, typename real>
+static OpP<N, real> op_params(const DevMesh* m) {
+  OpP<N, real> O;
+  const HostOps ops = m ? HostOps() : gll_operators(N);
+  const HostOps& o = m ? m->ops : ops;
+  for (int q = 0; q < N * N; ++q) {
+    O.G[q] = (real)o.G[q];
+    O.Gd[q] = o.G[q];
+  }
+  O.c2H = (real)(1.0 / (2.0 * o.H[0]));
+  return O;
+}
+
+// Elements per CTA.  Default (variant 0): Pen<N>::EPB, fewer where the work would
+// otherwise leave SMs without a CTA; variants 1 and 2 (batches): half and one.
+// (One CTA shape gives the same bits as another.)
+template <int N>
+static int elements_per_cta(long long ne, int variant) {
+  const int most = variant == 0 ? Pen<N>::EPB : variant == 1 ? (Pen<N>::EPB + 1) / 2 : 1;
+  const long long fill = ne / (2 * 148);
+  return (int)(fill < 1 ? 1 : fill < most ? fill : most);
+}
+
+template <typename K>
+static int gen_smem(K kernel, size_t smem) {
+  if (smem <= 48 * 1024) return 0;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess ? 0 : -2;
+}
+
+template <int N, typename real, bool CURV, bool BATCH, bool CP>
+static int k1_run(const K1P<real>& P, const OpP<N, real>& O, const void* plist, const int2* tiles, long long ne,
+                  int variant, cudaStream_t s) {
+  if (ne <= 0) return 0;
+  const int epb = elements_per_cta<N>(ne, variant);
+  const size_t smem = (size_t)epb * k1_words<N, real, CURV, CP>() * sizeof(real);
+  if (gen_smem(k_cons_k1<N, real, CURV, BATCH, CP>, smem)) return -2;
+  k_cons_k1<N, real, CURV, BATCH, CP><<<(unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s>>>(
+      P, O, (const K1P<real>*)plist, tiles, ne, epb);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <int N, typename real, bool CURV, bool BATCH>
+static int k2_run(const K2P<real>& P, const OpP<N, real>& O, const void* plist, const int2* tiles, long long ne,
+                  int variant, cudaStream_t s) {
+  if (ne <= 0) return 0;
+  const int epb = elements_per_cta<N>(ne, variant);
+  const size_t smem = (size_t)epb * k2_words<N, CURV>() * sizeof(real);
+  if (gen_smem(k_cons_k2<N, real, CURV, BATCH>, smem)) return -2;
+  k_cons_k2<N, real, CURV, BATCH><<<(unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s>>>(
+      P, O, (const K2P<real>*)plist, tiles, ne, epb);
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 template <int N, typename real>
@@ -1036,20 +803,14 @@ static int k1_dispatch(const DevMesh& m, const DevCoef& c, const void* Phi, cons
   K1P<real> P = k1p_params<real>(m, c, Phi, Pi, F, Phidot, bbuf, grad_out, bc, rk);
   P.e0 = e0;
   P.e1 = e1 < 0 ? m.Ne : e1;
-  const unsigned blocks = (unsigned)((P.e1 - P.e0 + Ep<N>::EPB - 1) / Ep<N>::EPB);
-  if (blocks == 0) return 0;
+  const long long ne = P.e1 - P.e0;
+  const OpP<N, real> O = op_params<N, real>(&m);
   constexpr bool F32 = std::is_same<real, float>::value;
-  if (F32 && gen_cp(m, grad_out)) {
-    if (use_metric)
-      k_cons_k1<N, real, true, false, Ep<N>::EPB, F32><<<blocks, Ep<N>::T, 0, s>>>(P, nullptr, nullptr, 0);
-    else
-      k_cons_k1<N, real, false, false, Ep<N>::EPB, F32><<<blocks, Ep<N>::T, 0, s>>>(P, nullptr, nullptr, 0);
-  } else if (use_metric) {
-    k_cons_k1<N, real, true, false, Ep<N>::EPB><<<blocks, Ep<N>::T, 0, s>>>(P, nullptr, nullptr, 0);
-  } else {
-    k_cons_k1<N, real, false, false, Ep<N>::EPB><<<blocks, Ep<N>::T, 0, s>>>(P, nullptr, nullptr, 0);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  if (F32 && gen_cp(m, grad_out))
+    return use_metric ? k1_run<N, real, true, false, F32>(P, O, nullptr, nullptr, ne, 0, s)
+                      : k1_run<N, real, false, false, F32>(P, O, nullptr, nullptr, ne, 0, s);
+  return use_metric ? k1_run<N, real, true, false, false>(P, O, nullptr, nullptr, ne, 0, s)
+                    : k1_run<N, real, false, false, false>(P, O, nullptr, nullptr, ne, 0, s);
 }
 
 template <int N, typename real>
@@ -1059,105 +820,25 @@ static int k2_dispatch(const DevMesh& m, const void* F, void* Pidot, const void*
   K2P<real> P = k2p_params<real>(m, F, Pidot, bbuf, bc, rk, nonfinite, F1, F2);
   P.e0 = e0;
   P.e1 = e1 < 0 ? m.Ne : e1;
-  const unsigned blocks = (unsigned)((P.e1 - P.e0 + Ep<N>::EPB - 1) / Ep<N>::EPB);
-  if (blocks == 0) return 0;
-  if (use_metric)
-    k_cons_k2<N, real, true, false, Ep<N>::EPB><<<blocks, Ep<N>::T, 0, s>>>(P, nullptr, nullptr, 0);
-  else
-    k_cons_k2<N, real, false, false, Ep<N>::EPB><<<blocks, Ep<N>::T, 0, s>>>(P, nullptr, nullptr, 0);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  const OpP<N, real> O = op_params<N, real>(&m);
+  return use_metric ? k2_run<N, real, true, false>(P, O, nullptr, nullptr, P.e1 - P.e0, 0, s)
+                    : k2_run<N, real, false, false>(P, O, nullptr, nullptr, P.e1 - P.e0, 0, s);
 }
 
-// elements per CTA of the work-list (batched) generic kernels: the default or twice it
-template <int N>
-struct EpAlt {
-  // the alternative must fit 1024 threads and the 48 KB of static shared memory
-  // of the curvilinear K1 (Phi, 6 face traces, 9 products per element, FP64)
-  static constexpr bool fits = Ep<N>::N3 * 2 * Ep<N>::EPB <= 1024 &&
-                               (10 * Ep<N>::N3 + 6 * Ep<N>::N2) * 2 * Ep<N>::EPB * 8 + 8 * Ep<N>::N2 <= 48 * 1024;
-  static constexpr int V1 = fits ? 2 * Ep<N>::EPB : Ep<N>::EPB;
-};
-
-template <int N, typename real, int EPB>
-static int gen_batch(int which, bool cp, const void* plist, const int2* tiles, long long ntiles, cudaStream_t s) {
-  const unsigned blocks = (unsigned)((ntiles + EPB - 1) / EPB);
-  if (blocks == 0) return 0;
+// one launch over a work list of (solve, element) tiles; variant: elements per CTA
+template <int N, typename real>
+static int gen_batch(int which, bool cp, int variant, const void* plist, const int2* tiles, long long ntiles,
+                     cudaStream_t s) {
+  static const OpP<N, real> O = op_params<N, real>(nullptr);
   constexpr bool F32 = std::is_same<real, float>::value;
-  if (which == 1 && F32 && cp)
-    k_cons_k1<N, real, true, true, EPB, F32><<<blocks, Ep<N>::N3 * EPB, 0, s>>>(K1P<real>(), (const K1P<real>*)plist,
-                                                                               tiles, ntiles);
-  else if (which == 1)
-    k_cons_k1<N, real, true, true, EPB><<<blocks, Ep<N>::N3 * EPB, 0, s>>>(K1P<real>(), (const K1P<real>*)plist, tiles,
-                                                                          ntiles);
-  else
-    k_cons_k2<N, real, true, true, EPB><<<blocks, Ep<N>::N3 * EPB, 0, s>>>(K2P<real>(), (const K2P<real>*)plist, tiles,
-                                                                          ntiles);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  if (which == 1)
+    return F32 && cp ? k1_run<N, real, true, true, F32>(K1P<real>(), O, plist, tiles, ntiles, variant, s)
+                     : k1_run<N, real, true, true, false>(K1P<real>(), O, plist, tiles, ntiles, variant, s);
+  return k2_run<N, real, true, true>(K2P<real>(), O, plist, tiles, ntiles, variant, s);
 }
 
-static int gen_sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
-// the pipelined kernels: a persistent grid of up to OCC CTAs per SM
-template <int N, typename real, bool CP>
-static int pipe_batch(int which, const void* plist, const int2* tiles, long long ntiles, cudaStream_t s) {
-  static bool attr1 = false, attr2 = false;
-  if (which == 1) {
-    using L = PipeK1<N, real, CP>;
-    if (!attr1) {
-      if (cudaFuncSetAttribute(k_cons_k1_pipe<N, real, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)L::SMEM) != cudaSuccess)
-        return -2;
-      attr1 = true;
-    }
-    const long long ng = (ntiles + L::EPB - 1) / L::EPB, cap = (long long)gen_sm_count() * L::OCC;
-    const long long grid = ng < cap ? ng : cap;
-    if (grid <= 0) return 0;
-    k_cons_k1_pipe<N, real, CP><<<(unsigned)grid, L::T, L::SMEM, s>>>((const K1P<real>*)plist, tiles, ntiles);
-  } else {
-    using L = PipeK2<N, real>;
-    if (!attr2) {
-      if (cudaFuncSetAttribute(k_cons_k2_pipe<N, real>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM) !=
-          cudaSuccess)
-        return -2;
-      attr2 = true;
-    }
-    const long long ng = (ntiles + L::EPB - 1) / L::EPB, cap = (long long)gen_sm_count() * L::OCC;
-    const long long grid = ng < cap ? ng : cap;
-    if (grid <= 0) return 0;
-    k_cons_k2_pipe<N, real><<<(unsigned)grid, L::T, L::SMEM, s>>>((const K2P<real>*)plist, tiles, ntiles);
-  }
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-
-// variant: 0 the generic kernels at Ep<N>::EPB elements per CTA, 1 at the
-// alternative EPB, 2 the pipelined kernels (n = 4 and 6; otherwise as 0)
-template <int N>
-static int gen_batch_n(int which, int precision, int variant, bool cp, const void* plist, const int2* tiles,
-                       long long ntiles, cudaStream_t s) {
-  if constexpr (N == 4 || N == 6) {
-    if (variant == 2) {
-      if (precision == 0) return pipe_batch<N, double, false>(which, plist, tiles, ntiles, s);
-      return cp ? pipe_batch<N, float, true>(which, plist, tiles, ntiles, s)
-                : pipe_batch<N, float, false>(which, plist, tiles, ntiles, s);
-    }
-  }
-  if (precision == 0)
-    return variant == 1 ? gen_batch<N, double, EpAlt<N>::V1>(which, false, plist, tiles, ntiles, s)
-                        : gen_batch<N, double, Ep<N>::EPB>(which, false, plist, tiles, ntiles, s);
-  return variant == 1 ? gen_batch<N, float, EpAlt<N>::V1>(which, cp, plist, tiles, ntiles, s)
-                      : gen_batch<N, float, Ep<N>::EPB>(which, cp, plist, tiles, ntiles, s);
-}
-
-bool cons_gen_pipe_available(int N) { return N == 4 || N == 6; }
+// orders with a third CTA shape (variant 2)
+bool cons_gen_third_variant(int N) { return N == 4 || N == 6; }
 
 size_t cons_gen_param_size(int precision, int which) {
   if (precision == 0) return which == 1 ? sizeof(K1P<double>) : sizeof(K2P<double>);
@@ -1265,7 +946,11 @@ int launch_apply_D(const DevMesh& m, const void* u, void* out, int d, cudaStream
 
 int launch_cons_gen_batch(int which, int N, int precision, int epb_variant, int cp, const void* plist, const int2* tiles,
                           long long ntiles, cudaStream_t s) {
-  WT_DISPATCH_N(N, (gen_batch_n<NN>(which, precision, epb_variant, cp != 0, plist, tiles, ntiles, s)));
+  if (precision == 0) {
+    WT_DISPATCH_N(N, (gen_batch<NN, double>(which, false, epb_variant, plist, tiles, ntiles, s)));
+  } else {
+    WT_DISPATCH_N(N, (gen_batch<NN, float>(which, cp != 0, epb_variant, plist, tiles, ntiles, s)));
+  }
 }
 
 // this file's bounds word (bounds-check build; 0 otherwise)

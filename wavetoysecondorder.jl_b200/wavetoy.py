@@ -601,8 +601,7 @@ class Batch(_Child):
     meshes of any order and size.  Solves of one (n, precision, path) group run
     as one work list of (solve, element) tiles per kernel launch, one RK4 step
     of all groups is a CUDA graph, and the launch variant of the generic
-    kernels (elements per CTA, or the pipelined kernels for n = 4, 6) is picked
-    by timing when the membership changes."""
+    kernels (elements per CTA) is picked by timing when the membership changes."""
 
     def __init__(self, ctx: Context, autotune: bool = True):
         self.ctx = ctx
@@ -626,9 +625,8 @@ class Batch(_Child):
         self._keep.pop(slot, None)
 
     def set_variant(self, k1: int = -1, k2: int = -1):
-        """Fix the launch variants of the generic groups' K1 and K2 (wt_batch_set_variant): 0 / 1 the
-        generic kernels at the default / alternative elements per CTA, 2 the pipelined kernels
-        (n = 4, 6); -1 leaves the choice to the autotuner."""
+        """Fix the launch variants of the generic groups' K1 and K2 (wt_batch_set_variant): 0 the default
+        elements per CTA, 1 half of it, 2 one (n = 4, 6); -1 leaves the choice to the autotuner."""
         self.ctx.check(library().wt_batch_set_variant(self.h, int(k1), int(k2)), "wt_batch_set_variant")
 
     def step(self, nsteps: int = 1):
