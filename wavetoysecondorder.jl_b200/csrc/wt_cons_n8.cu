@@ -192,6 +192,23 @@ __device__ __forceinline__ int opq(int al, int w, int b, int tig) {
   return al == 0 ? w + 8 * sl : sl + 8 * w;
 }
 
+// The partial sums of the contractions with their roundings written out, so that
+// the two-kernel stages and the fused stage kernel give the same bits however the
+// compiler would contract each: half_form = 0.5 d + 0.5 m e, half_pair = 0.5 m1 d1
+// + 0.5 m2 d2, dot3 = a0 b0 + a1 b1 + a2 b2, madd = r + a b.
+template <typename real>
+__device__ __forceinline__ real half_form(real d, real m, real e) { return fma((real)0.5 * m, e, (real)0.5 * d); }
+template <typename real>
+__device__ __forceinline__ real half_pair(real m1, real d1, real m2, real d2) {
+  return fma((real)0.5 * m2, d2, ((real)0.5 * m1) * d1);
+}
+template <typename real>
+__device__ __forceinline__ real dot3(real a0, real b0, real a1, real b1, real a2, real b2) {
+  return fma(a2, b2, fma(a1, b1, a0 * b0));
+}
+template <typename real>
+__device__ __forceinline__ real madd(real r, real a, real b) { return fma(a, b, r); }
+
 __device__ __forceinline__ bool wait_phase(uint64_t* bar, unsigned parity, unsigned* err) {
   for (long long it = 0; it < WAIT_LIMIT; ++it)
     if (mbar_try_wait(bar, parity)) return true;
@@ -687,8 +704,8 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
         for (int c = 0; c < 3; ++c)
           if ((comps >> c) & 1) {
             const real m = sJa[(al * 3 + c) * FS + no];
-            real r = (real)0.5 * cm[c][b] + (real)0.5 * m * cu[b];
-            if (sat) r += m * jump;
+            real r = half_form<real>(cm[c][b], m, cu[b]);
+            if (sat) r = madd(r, m, jump);
             sg[(al * 3 + c) * FS + no] = r;
           }
       }
@@ -1011,7 +1028,7 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
             if (half == 0) {
               // contravariant flux Ja^al . F and F_0
               const double f0 = sF[nd];
-              const double ft = m0[nd] * f0 + m1[nd] * sF[FS + nd] + m2[nd] * sF[2 * FS + nd];
+              const double ft = dot3<double>(m0[nd], f0, m1[nd], sF[FS + nd], m2[nd], sF[2 * FS + nd]);
               dmma(dx[0], dx[1], a, ft);
               dmma(dy[0], dy[1], a, f0);
             } else {
@@ -1051,16 +1068,16 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
           const int no = Lay<real>::at(onode(al, wt8, b, gq, tig));
           real r;
           if (half == 0) {
-            r = (real)0.5 * cx[b] + (real)0.5 * m0[no] * cy[b];
+            r = half_form<real>(cx[b], m0[no], cy[b]);
           } else {
-            r = (real)0.5 * m1[no] * cx[b] + (real)0.5 * m2[no] * cy[b];
+            r = half_pair<real>(m1[no], cx[b], m2[no], cy[b]);
           }
           if (sat) {
             const int pq = opq(al, wt8, b, tig);
-            const real sacc = m0[no] * (sfc[(sface_f * 3 + 0) * N2 + pq] - sF[no]) +
-                              m1[no] * (sfc[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no]) +
-                              m2[no] * (sfc[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
-            r += (gq ? inv2H : -inv2H) * sacc;
+            const real sacc = dot3<real>(m0[no], sfc[(sface_f * 3 + 0) * N2 + pq] - sF[no],
+                                         m1[no], sfc[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no],
+                                         m2[no], sfc[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
+            r = madd(r, gq ? inv2H : -inv2H, sacc);
           }
           if constexpr (NHALF == 2) rsum[b] = hh ? rsum[b] + r : r;
           else sdiv[(al * 2 + half) * FS + no] = r;
@@ -1140,40 +1157,34 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
 //     passes), so Pi_{s+1} is never stored;
 //   * the boundary buffer: each thread reads its node's slots in the K2 half
 //     before the K1 half rewrites them.
-// Only the node passes depend on each other, so the two contraction passes run
-// side by side: warps 0-7 contract the divergence (tile w, both halves of its
-// fields, as the 256-thread k_cons_k2_n8<double>), warps 8-15 the gradient
-// (tile w - 8, all nine components); one barrier later every thread does the
-// divergence node pass and then the gradient node pass of its node.  Two CTA
-// barriers per element, as in one of the two-kernel launches.  The metric terms
-// Ja staged for the divergence are read by the gradient too, and 1/J once.  Per
-// node and stage the fused kernel moves 33 words against 44 for the two
+// Per node and stage the fused kernel moves 33 words against 44 for the two
 // kernels (F 3 + Ja 9 + 1/J 1 + Pi RK 3 + Phi 1 + coefficients 10 + Phi RK 3 +
 // F_{s+1} 3).
-// CTA: 512 threads, one per SM (217 KB of shared memory); the flux and metric
-// terms (12 blocks) in a two-stage ring, issued one element ahead; the ten
-// coefficient blocks (read only by the node pass) single-buffered, issued once
-// the previous element's node pass is done; neighbour face traces of F_s and
-// Phi_{s+1} and Phi_{s+1} itself by per-thread cp.async one element ahead; 1/J
-// and the RK states prefetched into registers one element ahead.  Each partial
-// sum is formed by the instructions k_cons_k2_n8<double> and
-// k_cons_k1_n8<double> use and added in their order, so the fused step equals
-// the two-kernel step bit for bit.
-// Measured on the 64^3 x 8^3 solve: 262 DRAM bytes per node and launch (the two
-// kernels: 364); the RK4 step 1-7 % faster than the two-kernel step timed right
-// after it on the same GPU.  The kernels are bound by latency and issue (16
-// warps per SM, about 41 % issue active) rather than by DRAM bandwidth, so
-// the gain is smaller than the bytes saved.
+// CTA: one element, 256 threads, three CTAs per SM, so that one element's copies
+// in flight, another's contractions and a third's node pass share the SM (one
+// 512-thread CTA per SM with a two-stage ring spent its time waiting between its
+// own phases: 41 % of cycles issuing).  What lets three fit is the footprint,
+// 66 KB: warp w contracts tile w of both halves, so the metric terms of (axis,
+// tile) are read by that warp alone and its gradient partials replace them in
+// place; the divergence partials wait in registers until every warp is done with
+// F and then replace it; the node pass reads its coefficients and RK words
+// directly (asking L2 for them when the CTA starts gained nothing, and asking for
+// the element 222 or 444 CTAs ahead cost 5-20 %).  Each partial sum is formed by
+// the instructions k_cons_k2_n8<double> and k_cons_k1_n8<double> use and added in
+// their order, so the fused step equals the two-kernel step bit for bit.
+// Measured (B200, 40^3 elements): 1.90 ms a launch, 4.5 TB/s of its 33 words (70 %
+// of the measured copy rate), before 2.36 ms; 41 % -> 63 % of DRAM throughput at
+// 24^3 elements.  What is left: waits on global loads (a third of the stalls),
+// fixed-latency tensor and FP64 chains, and the shared-memory pipe (61 % busy).
 struct FKN8 {
   K2N8<double> a;  // stage s: F_s in (a.F0..F2), the Pi stage update
   K1N8<double> b;  // stage s + 1: Phi_{s+1} in (b.Phi), F_{s+1} out (b.F), the Phi stage update
 };
-constexpr int FK_NA = 12;  // ring stage: F (3) + Ja (9) blocks
-constexpr size_t fk_smem() {
-  return (2 * FK_NA * 512 + 10 * 512 + 12 * 512 + 2 * 6 * 3 * 64 + 2 * 6 * 64 + 2 * 512) * sizeof(double) +
-         64 * sizeof(double) + 64;
-}
-static_assert(fk_smem() + 64 + 1024 <= 233472, "the fused stage kernel's CTA must fit an SM");
+constexpr int FK_THREADS = 256;
+constexpr int FK_NA = 12;  // F (3) + Ja (9) blocks
+constexpr int FK_NFF = 6 * 3 * 64, FK_NFP = 6 * 64;  // flux / Phi face values
+constexpr size_t fk_smem() { return (FK_NA * 512 + 512 + FK_NFF + FK_NFP) * sizeof(double) + 16; }
+static_assert(3 * (fk_smem() + 64 + 1024) <= 233472, "three CTAs of the fused stage kernel must fit an SM");
 
 namespace n8 {
 // per-thread 8-byte asynchronous copy global -> shared, zero-filled when !valid
@@ -1209,335 +1220,188 @@ __device__ __forceinline__ double n8_rk_out(int stage, double dt, double k, doub
   return o;
 }
 
-__global__ void __launch_bounds__(n8::THREADS, 1) k_cons_fk_n8(const FKN8 P) {
+__global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_constant__ FKN8 P) {
   using namespace n8;
   using real = double;
   constexpr int FS = Lay<double>::FS;
-  constexpr int NFACE = 6 * 3 * N2;                     // flux face values
-  constexpr int NFR = (NFACE + THREADS - 1) / THREADS;  // per thread
-  constexpr int NPF = 6 * N2;                           // Phi face values
   const K2N8<double>& A = P.a;
   const K1N8<double>& B = P.b;
   extern __shared__ __align__(128) unsigned char smraw[];
-  double* sG = reinterpret_cast<double*>(smraw);  // 64
-  double* stg = sG + N2;                          // 2 x 12 blocks: F (3), Ja (9)
-  double* sC = stg + 2 * FK_NA * FS;              // 10 coefficient blocks (node order)
-  double* sdiv = sC + 10 * N3;                    // 3 partial divergences [al] (Lay)
-  double* sg = sdiv + 3 * FS;                     // 9 partial gradients [al * 3 + c] (Lay)
-  double* sfF = sg + 9 * FS;                      // 2 x 1152 flux face traces [f][c][pq]
-  double* sfP = sfF + 2 * NFACE;                  // 2 x 384 Phi face traces [f][pq]
-  double* sphi = sfP + 2 * NPF;                   // 2 x 512 Phi_{s+1} (Lay)
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sphi + 2 * N3);  // [0], [1] ring, [2] coefficients
+  double* sF = reinterpret_cast<double*>(smraw);  // 3 flux blocks, then the divergence partials [al] (Lay)
+  double* sJa = sF + 3 * FS;                      // 9 metric blocks, then the gradient partials [al * 3 + c] (Lay)
+  double* sphi = sJa + 9 * FS;                    // Phi_{s+1} (Lay)
+  double* sfF = sphi + N3;                        // flux face traces [f][c][pq]
+  double* sfP = sfF + FK_NFF;                     // Phi face traces [f][pq]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sfP + FK_NFP);
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int gq = lane >> 2, tig = lane & 3, wt8 = warp & 7;
-  const bool divw = warp < 8;  // divergence-contraction warp (else gradient)
+  const int gq = lane >> 2, tig = lane & 3;
   const real inv2H = (real)(1.0 / (2.0 * A.H[0]));
   const int sa = A.stage, sb = B.stage;  // sb = sa + 1
-  const bool needQy = sa <= 2, needQacc = sa >= 1;
-  const bool needPy = sb == 1 || sb == 2;
-  const unsigned txA = (unsigned)(FK_NA * FS * sizeof(real)), txC = (unsigned)(10 * N3 * sizeof(real));
-  const int ti = tid & 7, tj = (tid >> 3) & 7, tk = tid >> 6;
-  const int tpad = Lay<real>::at(tid);
-  const long long T = A.Ne, GS = gridDim.x;
+  const bool needQacc = sa >= 1, needPy = sb == 1 || sb == 2;
+  const long long e = blockIdx.x;
 
-  if (tid < N2) sG[tid] = A.G[tid];
-  if (tid == 0) {
-    abort_flag = 0;
-    for (int k = 0; k < 3; ++k) mbar_init(&bar[k], 1);
-    fence_barrier_init();
-  }
-  __syncthreads();
-
-  // warp 0: F_s and Ja of element e into ring stage s
-  auto issueA = [&](long long e, int s) {
+  if (warp == 0) {  // F_s and Ja of the element
     if (lane == 0) {
+      abort_flag = 0;
+      mbar_init(bar, 1);
+      fence_barrier_init();
       fence_proxy_async();
-      mbar_expect_tx(&bar[s], txA);
+      mbar_expect_tx(bar, (unsigned)(FK_NA * FS * sizeof(real)));
     }
     __syncwarp();
-    real* d = stg + s * FK_NA * FS;
     if (lane < FK_NA) {
       const real* src = lane < 3 ? (lane == 0 ? A.F0 : lane == 1 ? A.F1 : A.F2) + e * FS
                                  : A.Ja + ((long long)(lane - 3) * A.Ne + e) * FS;
-      bulk_g2s(d + lane * FS, src, FS * (unsigned)sizeof(real), &bar[s]);
-    }
-  };
-  // warp 0: the ten coefficient blocks of element e
-  auto issueC = [&](long long e) {
-    if (lane == 0) {
-      fence_proxy_async();
-      mbar_expect_tx(&bar[2], txC);
-    }
-    __syncwarp();
-    if (lane < 10) bulk_g2s(sC + lane * N3, B.c10 + lane * B.nn + e * N3, N3 * (unsigned)sizeof(real), &bar[2]);
-  };
-  // face sources of element e (-1: none or past the end), loaded one iteration
-  // before the traces they address
-  auto srcF_load = [&](long long e, int src[NFR]) {
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = tid + r * THREADS;
-      src[r] = (e < T && idx < NFACE) ? ::wt::bc_src(A.fsrc[idx / (3 * N2) + 6 * e], A.Ne) : -1;
-    }
-  };
-  auto srcP_load = [&](long long e) -> int { return (e < T && tid < NPF) ? ::wt::bc_src(B.fsrc[(tid >> 6) + 6 * e], B.Ne) : -1; };
-  auto faceF_load = [&](const int src[NFR], real fv[NFR]) {
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = tid + r * THREADS;
-      real v = 0;
-      if (src[r] >= 0) {
-        const int rem = idx % (3 * N2), c = rem >> 6, pq = rem & 63;
-        const real* Fc = c == 0 ? A.F0 : c == 1 ? A.F1 : A.F2;
-        v = Fc[(long long)(src[r] >> 6) * FS + Lay<real>::at(nbr_face_node(src[r], pq & 7, pq >> 3, N))];
-      }
-      fv[r] = v;
-    }
-  };
-  auto faceP_load = [&](int src) -> real {
-    if (src < 0) return (real)0;
-    const int pq = tid & 63;
-    return B.Phi[(long long)(src >> 6) * N3 + nbr_face_node(src, pq & 7, pq >> 3, N)];
-  };
-  struct PW {
-    real invJ, Qy, Qacc, Py, Pacc;
-  };
-  auto pw_load = [&](long long e, PW& w) {
-    const long long n = e * N3 + tid;
-    w.invJ = A.invdetJ[n];
-    w.Qy = needQy ? A.y[n] : (real)0;
-    w.Qacc = needQacc ? A.acc[n] : (real)0;
-    w.Py = needPy ? B.y[n] : (real)0;
-    w.Pacc = B.acc[n];  // stage s + 1 >= 1 reads the accumulator
-  };
-
-  PW cur;
-  int emcur = 0, srcF1[NFR], srcP1 = -1;
-#pragma unroll
-  for (int r = 0; r < NFR; ++r) srcF1[r] = -1;
-  {
-    const long long t0 = blockIdx.x;
-    if (t0 < T) {
-      if (warp == 0) issueA(t0, 0);
-      emcur = A.emask[t0];
-      int s0[NFR];
-      srcF_load(t0, s0);
-      real fv[NFR];
-      faceF_load(s0, fv);
-#pragma unroll
-      for (int r = 0; r < NFR; ++r)
-        if (tid + r * THREADS < NFACE) sfF[tid + r * THREADS] = fv[r];
-      const real pv = faceP_load(srcP_load(t0));
-      if (tid < NPF) sfP[tid] = pv;
-      pw_load(t0, cur);
-      sphi[tpad] = B.Phi[t0 * N3 + tid];
-      srcF_load(t0 + GS, srcF1);
-      srcP1 = srcP_load(t0 + GS);
+      bulk_g2s(sF + lane * FS, src, FS * (unsigned)sizeof(real), bar);
     }
   }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int w = tid + r * FK_THREADS;
+    cp_async8z(sphi + Lay<real>::at(w), B.Phi + e * N3 + w, true);
+  }
+  // neighbour face traces (zero-filled where a face has no neighbour); one thread
+  // per face node, so the four fields share one address
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int idx = tid + r * FK_THREADS;
+    if (idx < FK_NFP) {
+      const int f = idx >> 6, pq = idx & 63, src = ::wt::bc_src(A.fsrc[f + 6 * e], A.Ne);
+      const int nd = src >= 0 ? nbr_face_node(src, pq & 7, pq >> 3, N) : 0;
+      const long long b = src >= 0 ? (long long)(src >> 6) * N3 : 0;
+      const long long at = b + Lay<real>::at(nd);
+      double* d = sfF + f * 3 * N2 + pq;
+      cp_async8z(d, A.F0 + at, src >= 0);
+      cp_async8z(d + N2, A.F1 + at, src >= 0);
+      cp_async8z(d + 2 * N2, A.F2 + at, src >= 0);
+      cp_async8z(sfP + idx, B.Phi + b + nd, src >= 0);
+    }
+  }
+  const int em = A.emask[e], mask = em & 63, bnd = em >> 6;
+  const double aG0 = A.G[gq * 8 + tig], aG1 = A.G[gq * 8 + 4 + tig];
+  cp_async_wait_all();
+  if (tid == 0 && !wait_phase(bar, 0, A.flag)) abort_flag = 1;
   __syncthreads();
-  const double aG0 = sG[gq * 8 + tig], aG1 = sG[gq * 8 + 4 + tig];
+  if (abort_flag) {  // wait (bounded) for the copies in flight, then leave
+    if (tid == 0) wait_phase(bar, 0, nullptr);
+    return;
+  }
 
-  int it = 0;
-  for (long long t = blockIdx.x; t < T; t += GS, ++it) {
-    const int s = it & 1, fb = it & 1;
-    const unsigned parity = (it >> 1) & 1;
-    const long long t1 = t + GS;
-    const bool has_next = t1 < T;
-    const int emnext = has_next ? A.emask[t1] : 0;
-    int srcF2[NFR];
-    srcF_load(t + 2 * GS, srcF2);
-    const int srcP2 = srcP_load(t + 2 * GS);
-    // the next element's neighbour face traces and its Phi_{s+1} go straight into
-    // the buffers fb ^ 1 by per-thread asynchronous copies (zero-filled where a
-    // face has no neighbour; srcF1, srcP1 are -1 past the end); the previous
-    // group -- this element's -- is complete after the wait, and visible to
-    // every thread after the barrier below
+  // ---- contractions of tile `warp`: per axis the divergence of F_s (K2 half,
+  // kept in rs) and the split-form gradient of Phi_{s+1} (K1 half, in place) ----
+  real rs[3][2];
+#pragma unroll
+  for (int al = 0; al < 3; ++al) {
+    real* m0 = sJa + (al * 3 + 0) * FS;
+    real* m1 = sJa + (al * 3 + 1) * FS;
+    real* m2 = sJa + (al * 3 + 2) * FS;
+    double dt[2] = {0, 0}, d0[2] = {0, 0}, d1[2] = {0, 0}, d2[2] = {0, 0};
+    double du[2] = {0, 0}, dm[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+#pragma unroll
+    for (int kc = 0; kc < 2; ++kc) {
+      const int nd = Lay<real>::at(bnode(al, warp, kc, gq, tig));
+      const double a = kc ? aG1 : aG0;
+      const double j0 = m0[nd], j1 = m1[nd], j2 = m2[nd];
+      const double f0 = sF[nd], f1 = sF[FS + nd], f2 = sF[2 * FS + nd], u = sphi[nd];
+      const double ft = dot3(j0, f0, j1, f1, j2, f2);
+      dmma(dt[0], dt[1], a, ft);
+      dmma(d0[0], d0[1], a, f0);
+      dmma(d1[0], d1[1], a, f1);
+      dmma(d2[0], d2[1], a, f2);
+      dmma(du[0], du[1], a, u);
+      dmma(dm[0][0], dm[0][1], a, j0 * u);
+      dmma(dm[1][0], dm[1][1], a, j1 * u);
+      dmma(dm[2][0], dm[2][1], a, j2 * u);
+    }
+    const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
+    const bool sat = sface_f >= 0 && ((mask >> sface_f) & 1);
+    real gr[3][2];
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int no = Lay<real>::at(onode(al, warp, b, gq, tig));
+      const real j0 = m0[no], j1 = m1[no], j2 = m2[no];
+      const real r0 = half_form(dt[b], j0, d0[b]);
+      real r1 = half_pair(j1, d1[b], j2, d2[b]);
+      real g0 = half_form(dm[0][b], j0, du[b]);
+      real g1 = half_form(dm[1][b], j1, du[b]);
+      real g2 = half_form(dm[2][b], j2, du[b]);
+      if (sat) {
+        const int pq = opq(al, warp, b, tig);
+        const real sacc = dot3(j0, sfF[(sface_f * 3 + 0) * N2 + pq] - sF[no],
+                               j1, sfF[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no],
+                               j2, sfF[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
+        r1 = madd(r1, gq ? inv2H : -inv2H, sacc);
+        const real jump = (gq ? inv2H : -inv2H) * (sfP[sface_f * N2 + pq] - sphi[no]);
+        g0 = madd(g0, j0, jump);
+        g1 = madd(g1, j1, jump);
+        g2 = madd(g2, j2, jump);
+      }
+      rs[al][b] = r0 + r1;
+      gr[0][b] = g0;
+      gr[1][b] = g1;
+      gr[2][b] = g2;
+    }
+    __syncwarp();  // every lane has read this (axis, tile)'s metric terms
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int no = Lay<real>::at(onode(al, warp, b, gq, tig));
+      m0[no] = gr[0][b];
+      m1[no] = gr[1][b];
+      m2[no] = gr[2][b];
+    }
+  }
+  __syncthreads();  // every warp is done with F
+#pragma unroll
+  for (int al = 0; al < 3; ++al)
+#pragma unroll
+    for (int b = 0; b < 2; ++b) sF[al * FS + Lay<real>::at(onode(al, warp, b, gq, tig))] = rs[al][b];
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int w = tid + r * FK_THREADS, tp = Lay<real>::at(w);
+    const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
+    const long long n = e * N3 + w;
+    real cc[10];
+#pragma unroll
+    for (int c = 0; c < 10; ++c) cc[c] = B.c10[c * B.nn + n];
+    const real invJ = A.invdetJ[n], Qy = A.y[n], Qacc = needQacc ? A.acc[n] : (real)0;
+    const real Py = needPy ? B.y[n] : (real)0, Pacc = B.acc[n];  // stage s + 1 >= 1 reads the accumulator
+    // ---- divergence node pass: boundary terms, Pi stage update (K2 half) ----
+    real dv = (sF[tp] + sF[FS + tp]) + sF[2 * FS + tp];
+    dv *= invJ;
+    if (bnd && A.bc_on) {
+      const int idx3[3] = {ti, tj, tk};
+      for (int f = 0; f < 6; ++f) {
+        if (A.bdry[f + 6 * e] == 0) continue;
+        const int ax = f >> 1;
+        if (idx3[ax] != ((f & 1) ? 7 : 0)) continue;
+        const int p = ax == 0 ? tj : ti, q = ax == 2 ? tj : tk;
+        dv += A.bbuf[(long long)::wt::bc_slot(A.bslot[f + 6 * e], A.nbf) * N2 + p + 8 * q];
+      }
+    }
+    const real Pi = n8_rk_out(sa, A.dt, dv, Qy, Qacc, n, A.acc, A.out);  // Pi_{s+1}
+    // ---- gradient node pass: flux F_{s+1}, Phidot, boundary terms, Phi stage update (K1 half) ----
+    const real u = sphi[tp];
+    real g0 = (sJa[tp] + sJa[3 * FS + tp]) + sJa[6 * FS + tp];
+    real g1 = (sJa[FS + tp] + sJa[4 * FS + tp]) + sJa[7 * FS + tp];
+    real g2 = (sJa[2 * FS + tp] + sJa[5 * FS + tp]) + sJa[8 * FS + tp];
+    g0 *= invJ; g1 *= invJ; g2 *= invJ;
+    const real a = cc[0];
+    const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
+    const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
+    const real F0 = b0 * Pi + (K0 * g0 + K1v * g1 + K2 * g2);
+    const real F1 = b1 * Pi + (K1v * g0 + K3 * g1 + K4 * g2);
+    const real F2 = b2 * Pi + (K2 * g0 + K4 * g1 + K5 * g2);
+    real phid = b0 * g0 + b1 * g1 + b2 * g2 + a * Pi;
+    if (bnd && B.bc_on) k1_boundary<real>(B, e, ti, tj, tk, n, u, Pi, g0, g1, g2, cc, phid);
     {
-      double* dF = sfF + (fb ^ 1) * NFACE;
-#pragma unroll
-      for (int r = 0; r < NFR; ++r) {
-        const int idx = tid + r * THREADS;
-        if (idx < NFACE) {
-          const real* g = A.F0;
-          if (srcF1[r] >= 0) {
-            const int rem = idx % (3 * N2), c = rem >> 6, pq = rem & 63;
-            const real* Fc = c == 0 ? A.F0 : c == 1 ? A.F1 : A.F2;
-            g = Fc + (long long)(srcF1[r] >> 6) * FS + Lay<real>::at(nbr_face_node(srcF1[r], pq & 7, pq >> 3, N));
-          }
-          cp_async8z(dF + idx, g, srcF1[r] >= 0);
-        }
-      }
-      if (tid < NPF) {
-        const real* g = B.Phi;
-        if (srcP1 >= 0) {
-          const int pq = tid & 63;
-          g = B.Phi + (long long)(srcP1 >> 6) * N3 + nbr_face_node(srcP1, pq & 7, pq >> 3, N);
-        }
-        cp_async8z(sfP + (fb ^ 1) * NPF + tid, g, srcP1 >= 0);
-      }
-      cp_async8z(sphi + (fb ^ 1) * N3 + tpad, B.Phi + (has_next ? t1 : t) * N3 + tid, has_next);
-      cp_async_commit();
-      cp_async_wait_prior();
+      const long long fo = e * FS + tp, fstr = B.Ne * FS;
+      B.F[fo] = F0;
+      B.F[fstr + fo] = F1;
+      B.F[2 * fstr + fo] = F2;
     }
-    PW nxt;
-    if (has_next) pw_load(t1, nxt);
-    if (tid == 0 && !wait_phase(&bar[s], parity, A.flag)) abort_flag = 1;
-    // every thread has finished the previous element: ring stage s ^ 1, the
-    // coefficient buffer and the face / Phi buffers fb ^ 1 are free
-    __syncthreads();
-    if (abort_flag) {  // no bulk copy of this CTA is in flight (the coefficient copy was waited for)
-      cp_async_wait_all();
-      return;
-    }
-    if (warp == 0) {
-      issueC(t);
-      if (has_next) issueA(t1, s ^ 1);
-    }
-    const long long e = t;
-    const real* d = stg + s * FK_NA * FS;
-    const real* sF = d;
-    const real* sJa = d + 3 * FS;
-    const int mask = emcur & 63, bnd = emcur >> 6;
-
-    if (divw) {
-      // ---- divergence of F_s (K2 half), tile wt8: per axis the two halves of its
-      // fields, added in registers into sdiv[al] ----
-      const real* sfc = sfF + fb * NFACE;
-#pragma unroll
-      for (int al = 0; al < 3; ++al) {
-        const real* m0 = sJa + (al * 3 + 0) * FS;
-        const real* m1 = sJa + (al * 3 + 1) * FS;
-        const real* m2 = sJa + (al * 3 + 2) * FS;
-        real rsum[2] = {0, 0};
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          double dx[2] = {0, 0}, dy[2] = {0, 0};
-#pragma unroll
-          for (int kc = 0; kc < 2; ++kc) {
-            const int nd = Lay<real>::at(bnode(al, wt8, kc, gq, tig));
-            const double a = kc ? aG1 : aG0;
-            if (hh == 0) {
-              const double f0 = sF[nd];
-              const double ft = m0[nd] * f0 + m1[nd] * sF[FS + nd] + m2[nd] * sF[2 * FS + nd];
-              dmma(dx[0], dx[1], a, ft);
-              dmma(dy[0], dy[1], a, f0);
-            } else {
-              dmma(dx[0], dx[1], a, sF[FS + nd]);
-              dmma(dy[0], dy[1], a, sF[2 * FS + nd]);
-            }
-          }
-          const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
-          const bool sat = hh == 1 && sface_f >= 0 && ((mask >> sface_f) & 1);
-#pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            const int no = Lay<real>::at(onode(al, wt8, b, gq, tig));
-            real r;
-            if (hh == 0) {
-              r = (real)0.5 * dx[b] + (real)0.5 * m0[no] * dy[b];
-            } else {
-              r = (real)0.5 * m1[no] * dx[b] + (real)0.5 * m2[no] * dy[b];
-            }
-            if (sat) {
-              const int pq = opq(al, wt8, b, tig);
-              const real sacc = m0[no] * (sfc[(sface_f * 3 + 0) * N2 + pq] - sF[no]) +
-                                m1[no] * (sfc[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no]) +
-                                m2[no] * (sfc[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
-              r += (gq ? inv2H : -inv2H) * sacc;
-            }
-            rsum[b] = hh ? rsum[b] + r : r;
-          }
-        }
-#pragma unroll
-        for (int b = 0; b < 2; ++b) sdiv[al * FS + Lay<real>::at(onode(al, wt8, b, gq, tig))] = rsum[b];
-      }
-    } else {
-      // ---- split-form gradient of Phi_{s+1} (K1 half), tile wt8: all nine partials ----
-      const real* sPhi = sphi + fb * N3;
-      const real* sfc = sfP + fb * NPF;
-#pragma unroll
-      for (int al = 0; al < 3; ++al) {
-        double du[2] = {0, 0}, dm[3][2] = {{0, 0}, {0, 0}, {0, 0}};
-#pragma unroll
-        for (int kc = 0; kc < 2; ++kc) {
-          const int nd = Lay<real>::at(bnode(al, wt8, kc, gq, tig));
-          const double u = sPhi[nd];
-          const double a = kc ? aG1 : aG0;
-          dmma(du[0], du[1], a, u);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) dmma(dm[c][0], dm[c][1], a, sJa[(al * 3 + c) * FS + nd] * u);
-        }
-        const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
-        const bool sat = sface_f >= 0 && ((mask >> sface_f) & 1);
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int no = Lay<real>::at(onode(al, wt8, b, gq, tig));
-          real jump = 0;
-          if (sat) jump = (gq ? inv2H : -inv2H) * (sfc[sface_f * N2 + opq(al, wt8, b, tig)] - sPhi[no]);
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const real m = sJa[(al * 3 + c) * FS + no];
-            real r = (real)0.5 * dm[c][b] + (real)0.5 * m * du[b];
-            if (sat) r += m * jump;
-            sg[(al * 3 + c) * FS + no] = r;
-          }
-        }
-      }
-    }
-    if (tid == 0 && !wait_phase(&bar[2], (unsigned)(it & 1), A.flag)) abort_flag = 1;
-    __syncthreads();
-    if (abort_flag) {  // wait (bounded) for the next element's ring copy, then leave
-      if (tid == 0 && has_next) wait_phase(&bar[s ^ 1], ((it + 1) >> 1) & 1, nullptr);
-      cp_async_wait_all();
-      return;
-    }
-    {
-      const long long n = e * N3 + tid;
-      // ---- divergence node pass: boundary terms, Pi stage update (K2 half) ----
-      real dv = (sdiv[tpad] + sdiv[FS + tpad]) + sdiv[2 * FS + tpad];
-      dv *= cur.invJ;
-      if (bnd && A.bc_on) {
-        const int idx3[3] = {ti, tj, tk};
-        for (int f = 0; f < 6; ++f) {
-          if (A.bdry[f + 6 * e] == 0) continue;
-          const int ax = f >> 1;
-          if (idx3[ax] != ((f & 1) ? 7 : 0)) continue;
-          const int p = ax == 0 ? tj : ti, q = ax == 2 ? tj : tk;
-          dv += A.bbuf[(long long)::wt::bc_slot(A.bslot[f + 6 * e], A.nbf) * N2 + p + 8 * q];
-        }
-      }
-      const real Pi = n8_rk_out(sa, A.dt, dv, cur.Qy, cur.Qacc, n, A.acc, A.out);  // Pi_{s+1}
-      // ---- gradient node pass: flux F_{s+1}, Phidot, boundary terms, Phi stage update (K1 half) ----
-      const real u = sphi[fb * N3 + tpad];
-      real g0 = (sg[tpad] + sg[3 * FS + tpad]) + sg[6 * FS + tpad];
-      real g1 = (sg[FS + tpad] + sg[4 * FS + tpad]) + sg[7 * FS + tpad];
-      real g2 = (sg[2 * FS + tpad] + sg[5 * FS + tpad]) + sg[8 * FS + tpad];
-      g0 *= cur.invJ; g1 *= cur.invJ; g2 *= cur.invJ;
-      real cc[10];
-#pragma unroll
-      for (int c = 0; c < 10; ++c) cc[c] = sC[c * N3 + tid];
-      const real a = cc[0];
-      const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
-      const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
-      const real F0 = b0 * Pi + (K0 * g0 + K1v * g1 + K2 * g2);
-      const real F1 = b1 * Pi + (K1v * g0 + K3 * g1 + K4 * g2);
-      const real F2 = b2 * Pi + (K2 * g0 + K4 * g1 + K5 * g2);
-      real phid = b0 * g0 + b1 * g1 + b2 * g2 + a * Pi;
-      if (bnd && B.bc_on) k1_boundary<real>(B, e, ti, tj, tk, n, u, Pi, g0, g1, g2, cc, phid);
-      {
-        const long long fo = e * FS + tpad, fstr = B.Ne * FS;
-        B.F[fo] = F0;
-        B.F[fstr + fo] = F1;
-        B.F[2 * fstr + fo] = F2;
-      }
-      n8_rk<real>(sb, B.dt, phid, u, cur.Py, cur.Pacc, (real)0, n, B.y, B.acc, B.out, nullptr, B.flag);
-    }
-    cur = nxt;
-    emcur = emnext;
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) srcF1[r] = srcF2[r];
-    srcP1 = srcP2;
+    n8_rk<real>(sb, B.dt, phid, u, Py, Pacc, (real)0, n, B.y, B.acc, B.out, nullptr, B.flag);
   }
 }
 
@@ -2442,9 +2306,8 @@ int launch_cons_fk_n8(const DevMesh& m, const DevCoef& c, const void* Fin, void*
       return -2;
     attr = true;
   }
-  const long long cap = sm_count(), grid = m.Ne < cap ? m.Ne : cap;
-  if (grid <= 0) return 0;
-  k_cons_fk_n8<<<(unsigned)grid, n8::THREADS, fk_smem(), s>>>(P);
+  if (m.Ne <= 0) return 0;
+  k_cons_fk_n8<<<(unsigned)m.Ne, FK_THREADS, fk_smem(), s>>>(P);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
