@@ -24,6 +24,7 @@
 // barriers each and the matrix read from shared memory: 212 us); 40^3 of n = 6,
 // 150 us (before: 450 us).
 #include "wt_common.cuh"
+#include "wt_launch.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
     const int pp = part * PB + pb;  // the pencil, its first tangential index fastest
     base = (long long)e * N3 + (d == 0 ? N * pp : d == 1 ? pp % N + N2 * (pp / N) : pp);
   }
+  dep_wait();
   const real* const fp = blockIdx.y ? P.f[1] : P.f[0];
   real* const op = (blockIdx.y ? P.out[1] : P.out[0]) + a * P.ostride;
   real ev[M], od[HH];
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
   };
   auto load = [&](auto st) {
     constexpr int stride = decltype(st)::value;
-    const real* __restrict__ f = fp + (act ? base : 0);
+    const real* f = fp + (act ? base : 0);
     real v[N];
 #pragma unroll
     for (int l = 0; l < N; ++l) v[l] = act ? f[l * stride] : (real)0;
@@ -216,8 +218,7 @@ static int ko_run(const KoP<N, real>& P, unsigned blocks, int nf, int threads, c
         cudaSuccess)
       return -2;
   }
-  k_ko<N, real, TMAX><<<dim3(blocks, nf), threads, smem, s>>>(P);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_dep(k_ko<N, real, TMAX>, dim3(blocks, nf), threads, smem, s, P);
 }
 
 template <int N, typename real>

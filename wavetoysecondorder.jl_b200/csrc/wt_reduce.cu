@@ -3,6 +3,7 @@
 // Reductions write one partial sum per block; the host adds the partials in
 // a fixed order, so results are deterministic run to run.
 #include "wt_common.cuh"
+#include "wt_launch.cuh"
 
 #include <algorithm>
 
@@ -94,7 +95,8 @@ struct ErkSum {
   int nk;
 };
 template <typename real>
-__global__ void k_erk_combine(long long n, double dt, const real* __restrict__ y, real* __restrict__ out, ErkSum S) {
+__global__ void k_erk_combine(long long n, double dt, const real* y, real* out, ErkSum S) {
+  dep_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     real acc = 0;
     for (int j = 0; j < S.nk; ++j) acc += (real)S.a[j] * ((const real*)S.k[j])[i];
@@ -113,10 +115,8 @@ int launch_erk_combine(long long n, int precision, double dt, const void* y, voi
   }
   const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 4096);
   if (precision == 0)
-    k_erk_combine<double><<<grid, 256, 0, s>>>(n, dt, (const double*)y, (double*)out, S);
-  else
-    k_erk_combine<float><<<grid, 256, 0, s>>>(n, dt, (const float*)y, (float*)out, S);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    return launch_dep(k_erk_combine<double>, grid, 256, 0, s, n, dt, (const double*)y, (double*)out, S);
+  return launch_dep(k_erk_combine<float>, grid, 256, 0, s, n, dt, (const float*)y, (float*)out, S);
 }
 
 template <typename real>

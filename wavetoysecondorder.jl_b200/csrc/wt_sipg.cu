@@ -27,6 +27,7 @@
 // graph, two launches a stage instead of eleven.
 #include "wt_common.cuh"
 #include "wt_async.cuh"
+#include "wt_launch.cuh"
 #include "wt_rk.cuh"
 
 #include <algorithm>
@@ -86,6 +87,33 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
   // nodes t, t + TE, ... of the node pass; their place in the padded element
   constexpr int NI = (N3 + TE - 1) / TE;
   auto place = [](int w) { return w + (P1 - N) * (w / N); };
+  const real s = P.sdiag[3 * ec + ax];
+  // the two end faces: mode 0 none, 1 interior, 2 Dirichlet, 3 Sommerfeld; the outer value and trace
+  int mode[2];
+  real uo[2], to[2];
+  long long nu[2], nt[2];  // where the neighbour's value and trace are
+  if constexpr (!TRACE) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long long fi = 2 * ax + h + 6 * ec;
+      const int tag = valid ? P.bdry[fi] : 8;
+      const int nb = P.nbr[fi];
+      const int en = ::wt::bc_elem(nb, P.Ne);
+      const int fs = P.nbrf[fi];  // fn | ori << 3
+      mode[h] = tag == 0 && en >= 0 ? 1 : tag >= 1 && tag <= 6 ? 2 : tag == 7 && nb < 0 ? 3 : 0;
+      uo[h] = mode[h] == 2 ? P.bv[tag - 1] : (real)0;
+      to[h] = 0;
+      nu[h] = nt[h] = 0;
+      if (mode[h] == 1) {
+        int pn, qn;
+        face_perm((fs >> 3) & 7, p, q, N, pn, qn);
+        const int fn = fs & 7;
+        nu[h] = (long long)en * N3 + face_node(faxis(fn), frow(fn, N), pn, qn, N);
+        nt[h] = ((long long)6 * en + fn) * N2 + pn + N * qn;
+      }
+    }
+  }
+  dep_wait();
 #pragma unroll
   for (int it = 0; it < NI; ++it) {
     const int w = t + it * TE;
@@ -120,29 +148,13 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
     }
   }
   cp_async_commit();
-  const real s = P.sdiag[3 * ec + ax];
-  // the two end faces: mode 0 none, 1 interior, 2 Dirichlet, 3 Sommerfeld; the outer value and trace
-  int mode[2];
-  real uo[2], to[2];
   if constexpr (!TRACE) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const long long fi = 2 * ax + h + 6 * ec;
-      const int tag = valid ? P.bdry[fi] : 8;
-      const int nb = P.nbr[fi];
-      const int en = ::wt::bc_elem(nb, P.Ne);
-      const int fs = P.nbrf[fi];  // fn | ori << 3
-      mode[h] = tag == 0 && en >= 0 ? 1 : tag >= 1 && tag <= 6 ? 2 : tag == 7 && nb < 0 ? 3 : 0;
-      uo[h] = mode[h] == 2 ? P.bv[tag - 1] : (real)0;
-      to[h] = 0;
+    for (int h = 0; h < 2; ++h)
       if (mode[h] == 1) {
-        int pn, qn;
-        face_perm((fs >> 3) & 7, p, q, N, pn, qn);
-        const int fn = fs & 7;
-        uo[h] = P.u[(long long)en * N3 + face_node(faxis(fn), frow(fn, N), pn, qn, N)];
-        to[h] = P.trace[((long long)6 * en + fn) * N2 + pn + N * qn];
+        uo[h] = P.u[nu[h]];
+        to[h] = P.trace[nt[h]];
       }
-    }
   }
   cp_async_wait_group<1>();  // u
   __syncthreads();
@@ -273,9 +285,8 @@ static int sipg_run(const DevMesh& m, const SipgStage& S, bool trace_only, cudaS
       cudaFuncSetAttribute(k_sipg<N, real, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
           cudaSuccess)
     return -2;
-  if (trace_only) k_sipg<N, real, true><<<blocks, 3 * N * N * epb, smem, s>>>(P, epb);
-  else k_sipg<N, real, false><<<blocks, 3 * N * N * epb, smem, s>>>(P, epb);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_dep(trace_only ? k_sipg<N, real, true> : k_sipg<N, real, false>, blocks, 3 * N * N * epb, smem, s, P,
+                    epb);
 }
 
 int launch_sipg(const DevMesh& m, const SipgStage& S, bool trace_only, cudaStream_t s) {
