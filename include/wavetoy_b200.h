@@ -464,7 +464,7 @@ int wt_rk4_stage_curved(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, 
  * layers, so such a partition keeps six ghost layers beyond each cut and
  * refreshes them once per stage.  wt_rk4_stage_curved_ko runs one whole RK4
  * stage of wt_step_rk4_curved with eps_ko != 0 (the RHS with dissipation, then
- * both stage updates: the same kernels as that path).  wt_halo_state_copy then
+ * both stage updates; equal to that path up to rounding).  wt_halo_state_copy then
  * copies `count` element layers from `layer` of the state the next stage reads
  * (the stage outputs; the caller's Phi and Pi after stage 3) into buf (pack = 1,
  * Phi's layers then Pi's) or back (pack = 0), asynchronously on the context

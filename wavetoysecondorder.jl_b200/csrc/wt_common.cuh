@@ -296,6 +296,10 @@ struct RKStage {
   // after it), and the copy of the state's high part stage 2 writes for stage 3
   const void* phit = nullptr;
   void* hcopy = nullptr;
+  // FP64: nko dissipation increments added to the right-hand side before the
+  // stage update (fields of nn words, nn apart; wt_ko.cu)
+  const void* ko = nullptr;
+  int nko = 0;
 };
 // K1: gradient, flux F, Phidot (+ affine/curv BC increments), optional RK epilogue for Phi.
 // e0, e1: the elements [e0, e1) the launch covers (e1 < 0: to the last element)

@@ -19,6 +19,7 @@
 // and 1/J.
 #include "wt_common.cuh"
 #include "wt_async.cuh"
+#include "wt_launch.cuh"
 #include "wt_rk.cuh"
 
 #include <initializer_list>
@@ -80,6 +81,9 @@ struct K1P {
   const real* dJa;
   const double* Ja0;
   real* hcopy;
+  // dissipation increments of Phidot: nko fields, nn words apart
+  const real* ko;
+  int nko;
 };
 
 // contraction along axis d of a smem field f (N^3) with transposed G (GT[p*N+i] = G[i][p])
@@ -179,6 +183,7 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long ec, long
       P.bbuf[(long long)slot * N2 + p + N * q] = dP;
     }
   }
+  for (int c = 0; c < P.nko; ++c) phid += P.ko[c * nn + n];
   P.F[n] = F0;
   P.F[nn + n] = F1;
   P.F[2 * nn + n] = F2;
@@ -298,26 +303,33 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
   gt un[2] = {0, 0};
   int src[2] = {-1, -1};
   real m0[3] = {0, 0, 0}, sd = 0;
+  if (valid) {  // what no launch of a step writes: metric terms and tables
+    if constexpr (CURV) {
+      const real* ja = CP ? P.dJa : P.Ja;
+#pragma unroll
+      for (int it = 0; it < L::NI; ++it) {
+        const int w = t + it * TE;
+        if (N3 % TE != 0 && w >= N3) break;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) cp_async_word(sr + c * NS + L::place(w), ja + c * nn + ec * N3 + w);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+  }
+  dep_wait();
   if (valid) {
-    const real* ja = CP ? P.dJa : P.Ja;
 #pragma unroll
     for (int it = 0; it < L::NI; ++it) {
       const int w = t + it * TE;
       if (N3 % TE != 0 && w >= N3) break;
       const long long n = ec * N3 + w;
-      const int at = L::place(w);
-      cp_async_word(sphi + at, P.Phi + n);
+      cp_async_word(sphi + L::place(w), P.Phi + n);
       if constexpr (CP) {
-        if (P.Phit) cp_async_word(sphit + at, P.Phit + n);
-      }
-      if constexpr (CURV) {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) cp_async_word(sr + c * NS + at, ja + c * nn + n);
+        if (P.Phit) cp_async_word(sphit + L::place(w), P.Phit + n);
       }
     }
     cp_async_commit();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
 #pragma unroll
     for (int h = 0; h < 2; ++h)
       if (src[h] >= 0) {
@@ -489,6 +501,8 @@ struct K2P {
   real* out;
   real* comp;
   unsigned int* nonfinite;
+  const real* ko;  // dissipation increments of Pidot (see K1P)
+  int nko;
 };
 
 // shared words of one element in K2: F and the nine metric terms / axis results
@@ -519,23 +533,29 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
   const bool pf_comp = P.epi && P.comp && P.stage == 3;
   int src[2] = {-1, -1};
   real fn[2][CURV ? 3 : 1] = {}, sd = 0;
+  if (valid) {  // what no launch of a step writes: metric terms and tables
+    if constexpr (CURV) {
+#pragma unroll
+      for (int it = 0; it < L::NI; ++it) {
+        const int w = t + it * TE;
+        if (N3 % TE != 0 && w >= N3) break;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) cp_async_word(sJ + c * NS + L::place(w), P.Ja + c * nn + ec * N3 + w);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+  }
+  dep_wait();
   if (valid) {
 #pragma unroll
     for (int it = 0; it < L::NI; ++it) {
       const int w = t + it * TE;
       if (N3 % TE != 0 && w >= N3) break;
-      const long long n = ec * N3 + w;
-      const int at = L::place(w);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) cp_async_word(sF + c * NS + at, Fp[c] + n);
-      if constexpr (CURV) {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) cp_async_word(sJ + c * NS + at, P.Ja + c * nn + n);
-      }
+      for (int c = 0; c < 3; ++c) cp_async_word(sF + c * NS + L::place(w), Fp[c] + ec * N3 + w);
     }
     cp_async_commit();
-#pragma unroll
-    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
 #pragma unroll
     for (int h = 0; h < 2; ++h)
       if (src[h] >= 0) {
@@ -640,6 +660,7 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
         dv += P.bbuf[(long long)::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf) * N2 + fp + N * fq];
       }
     }
+    for (int c = 0; c < P.nko; ++c) dv += P.ko[c * nn + n];
     if (P.epi) {
       const real yv = pf_y ? sw[N3 + w] : (real)0;
       const real accv = pf_acc ? sw[2 * N3 + w] : (real)0;
@@ -714,6 +735,7 @@ static K1P<real> k1p_params(const DevMesh& m, const DevCoef& c, const void* Phi,
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.nonfinite = rk.nonfinite;
   if (!rk.on) P.y = P.acc = (real*)Phi;  // not read, but never a null address to form a load from
   P.Phit = (const real*)rk.phit; P.dJa = (const real*)m.dJa; P.Ja0 = m.Ja0; P.hcopy = (real*)rk.hcopy;
+  P.ko = (const real*)rk.ko; P.nko = rk.nko;
   return P;
 }
 
@@ -740,6 +762,7 @@ static K2P<real> k2p_params(const DevMesh& m, const void* F, void* Pidot, const 
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.nonfinite = nonfinite;
   if (!rk.on) P.y = P.acc = (real*)P.F0;  // not read (see k1p_params)
+  P.ko = (const real*)rk.ko; P.nko = rk.nko;
   return P;
 }
 
@@ -779,9 +802,8 @@ static int k1_run(const K1P<real>& P, const OpP<N, real>& O, const void* plist, 
   const int epb = elements_per_cta<N>(ne, variant);
   const size_t smem = (size_t)epb * k1_words<N, real, CURV, CP>() * sizeof(real);
   if (gen_smem(k_cons_k1<N, real, CURV, BATCH, CP>, smem)) return -2;
-  k_cons_k1<N, real, CURV, BATCH, CP><<<(unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s>>>(
-      P, O, (const K1P<real>*)plist, tiles, ne, epb);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_dep(k_cons_k1<N, real, CURV, BATCH, CP>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P,
+                    O, (const K1P<real>*)plist, tiles, ne, epb);
 }
 
 template <int N, typename real, bool CURV, bool BATCH>
@@ -791,9 +813,8 @@ static int k2_run(const K2P<real>& P, const OpP<N, real>& O, const void* plist, 
   const int epb = elements_per_cta<N>(ne, variant);
   const size_t smem = (size_t)epb * k2_words<N, CURV>() * sizeof(real);
   if (gen_smem(k_cons_k2<N, real, CURV, BATCH>, smem)) return -2;
-  k_cons_k2<N, real, CURV, BATCH><<<(unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s>>>(
-      P, O, (const K2P<real>*)plist, tiles, ne, epb);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_dep(k_cons_k2<N, real, CURV, BATCH>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P, O,
+                    (const K2P<real>*)plist, tiles, ne, epb);
 }
 
 template <int N, typename real>

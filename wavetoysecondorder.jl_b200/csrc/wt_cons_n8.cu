@@ -50,6 +50,7 @@
 //     one element before the neighbour traces they address, so no load in
 //     the loop waits on another load.
 #include "wt_common.cuh"
+#include "wt_launch.cuh"
 #include "../../include/wavetoy_b200.h"
 
 #include <cuda_bf16.h>
@@ -380,6 +381,9 @@ struct K1N8 {
   const double* Ja0;
   real* hcopy;
   double Gd[64];  // 0.5 G in FP64
+  // dissipation increments of Phidot (FP64): nko fields, nn words apart
+  const real* ko;
+  int nko;
 };
 
 // Boundary terms of K1 at a node on an outer face (the curvilinear boundary
@@ -751,6 +755,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
         Q.F[fstr + fo] = F1;
         Q.F[2 * fstr + fo] = F2;
       }
+      for (int c = 0; c < Q.nko; ++c) phid += Q.ko[c * Q.nn + n];
       if (P.epi)
         n8_rk<real>(P.stage, Q.dt, phid, u, cur.y, cur.acc, cur.comp, n, Q.y, Q.acc, Q.out, comp_on ? Q.comp : nullptr,
                     P.flag);
@@ -800,6 +805,8 @@ struct K2N8 {
   real* out;
   real* comp;
   unsigned* flag;
+  const real* ko;  // dissipation increments of Pidot (see K1N8)
+  int nko;
   float Gh[64];
 };
 
@@ -1116,6 +1123,7 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
           dv += Q.bbuf[(long long)::wt::bc_slot(Q.bslot[f + 6 * e], Q.nbf) * N2 + p + 8 * q];
         }
       }
+      for (int c = 0; c < Q.nko; ++c) dv += Q.ko[c * Q.nn + n];
       if (P.epi)
         n8_rk<real>(P.stage, Q.dt, dv, cur[r].y, cur[r].y, cur[r].acc, cur[r].comp, n, Q.y, Q.acc, Q.out,
                     comp_on ? Q.comp : nullptr, P.flag);
@@ -1250,12 +1258,20 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
       mbar_expect_tx(bar, (unsigned)(FK_NA * FS * sizeof(real)));
     }
     __syncwarp();
-    if (lane < FK_NA) {
-      const real* src = lane < 3 ? (lane == 0 ? A.F0 : lane == 1 ? A.F1 : A.F2) + e * FS
-                                 : A.Ja + ((long long)(lane - 3) * A.Ne + e) * FS;
-      bulk_g2s(sF + lane * FS, src, FS * (unsigned)sizeof(real), bar);
-    }
+    if (lane >= 3 && lane < FK_NA)
+      bulk_g2s(sF + lane * FS, A.Ja + ((long long)(lane - 3) * A.Ne + e) * FS, FS * (unsigned)sizeof(real), bar);
   }
+  int fsrc[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int idx = tid + r * FK_THREADS;
+    fsrc[r] = idx < FK_NFP ? ::wt::bc_src(A.fsrc[(idx >> 6) + 6 * e], A.Ne) : -1;
+  }
+  const int em = A.emask[e], mask = em & 63, bnd = em >> 6;
+  const double aG0 = A.G[gq * 8 + tig], aG1 = A.G[gq * 8 + 4 + tig];
+  dep_wait();  // above: mesh tables and metric terms, which no launch of a step writes
+  if (warp == 0 && lane < 3)
+    bulk_g2s(sF + lane * FS, (lane == 0 ? A.F0 : lane == 1 ? A.F1 : A.F2) + e * FS, FS * (unsigned)sizeof(real), bar);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int w = tid + r * FK_THREADS;
@@ -1267,7 +1283,7 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
   for (int r = 0; r < 2; ++r) {
     const int idx = tid + r * FK_THREADS;
     if (idx < FK_NFP) {
-      const int f = idx >> 6, pq = idx & 63, src = ::wt::bc_src(A.fsrc[f + 6 * e], A.Ne);
+      const int f = idx >> 6, pq = idx & 63, src = fsrc[r];
       const int nd = src >= 0 ? nbr_face_node(src, pq & 7, pq >> 3, N) : 0;
       const long long b = src >= 0 ? (long long)(src >> 6) * N3 : 0;
       const long long at = b + Lay<real>::at(nd);
@@ -1278,8 +1294,6 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
       cp_async8z(sfP + idx, B.Phi + b + nd, src >= 0);
     }
   }
-  const int em = A.emask[e], mask = em & 63, bnd = em >> 6;
-  const double aG0 = A.G[gq * 8 + tig], aG1 = A.G[gq * 8 + 4 + tig];
   cp_async_wait_all();
   if (tid == 0 && !wait_phase(bar, 0, A.flag)) abort_flag = 1;
   __syncthreads();
@@ -1380,6 +1394,7 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
         dv += A.bbuf[(long long)::wt::bc_slot(A.bslot[f + 6 * e], A.nbf) * N2 + p + 8 * q];
       }
     }
+    for (int c = 0; c < A.nko; ++c) dv += A.ko[c * A.nn + n];
     const real Pi = n8_rk_out(sa, A.dt, dv, Qy, Qacc, n, A.acc, A.out);  // Pi_{s+1}
     // ---- gradient node pass: flux F_{s+1}, Phidot, boundary terms, Phi stage update (K1 half) ----
     const real u = sphi[tp];
@@ -1401,6 +1416,7 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
       B.F[fstr + fo] = F1;
       B.F[2 * fstr + fo] = F2;
     }
+    for (int c = 0; c < B.nko; ++c) phid += B.ko[c * B.nn + n];
     n8_rk<real>(sb, B.dt, phid, u, Py, Pacc, (real)0, n, B.y, B.acc, B.out, nullptr, B.flag);
   }
 }
@@ -2178,6 +2194,8 @@ static K1N8<real> k1n8_params(const DevMesh& m, const DevCoef& c, const void* Ph
   P.Ja0 = m.Ja0;
   P.hcopy = (real*)rk.hcopy;
   for (int i = 0; i < 64; ++i) P.Gd[i] = 0.5 * m.ops.G[i];
+  P.ko = (const real*)rk.ko;
+  P.nko = rk.nko;
   return P;
 }
 
@@ -2196,6 +2214,8 @@ static K2N8<real> k2n8_params(const DevMesh& m, const void* F, void* Pidot, cons
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.flag = flag;
   for (int i = 0; i < 64; ++i) P.Gh[i] = (float)(0.5 * m.ops.G[i]);
+  P.ko = (const real*)rk.ko;
+  P.nko = rk.nko;
   return P;
 }
 
@@ -2307,8 +2327,7 @@ int launch_cons_fk_n8(const DevMesh& m, const DevCoef& c, const void* Fin, void*
     attr = true;
   }
   if (m.Ne <= 0) return 0;
-  k_cons_fk_n8<<<(unsigned)m.Ne, FK_THREADS, fk_smem(), s>>>(P);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return launch_dep(k_cons_fk_n8, (unsigned)m.Ne, FK_THREADS, fk_smem(), s, P);
 }
 
 int launch_cons_k2_n8(const DevMesh& m, const void* F, void* Pidot, const void* bbuf, const ConsBC& bc,
