@@ -1,54 +1,47 @@
-// wt_cons_n8.cu -- the n = 8 curvilinear hot path as persistent,
-// bulk-copy-pipelined, tensor-core kernels, in two precision forms.
+// wt_cons_n8.cu -- the n = 8 curvilinear hot path.
 //
 // Same arithmetic as k_cons_k1 / k_cons_k2 in wt_cons.cu (the split-form
 // gradient / flux / Phidot and the split-form divergence of
 // wave3d_curved_rhs!, src/wave3d_curved.jl:205-258, with the curvilinear
 // boundary pass of src/boundaries3d.jl:131-232 and the fused RK4 stage
-// update), organised for B200:
-//   * one CTA of 16 warps per SM loops over elements (persistent grid);
-//   * the fields the derivative contractions read at other nodes of an
-//     element (Phi and the nine metric terms in K1; the three flux components
-//     and the metric terms in K2) are staged into shared memory with 1D bulk
-//     copies (cp.async.bulk ... mbarrier::complete_tx), one copy per field
-//     block; the metric terms and the flux live in global memory in an
-//     element layout that makes the shared-memory accesses bank-conflict-free
-//     (FP64: an XOR swizzle of the node index; FP32: k-planes padded to 68
-//     words; see Lay below).  A ring of
-//     NSTAGE stages keeps NSTAGE - 1 elements in flight; one thread polls
-//     each stage's mbarrier, the rest wait at the CTA barrier; every wait is
-//     bounded and raises an error flag instead of spinning forever;
-//   * the fields used only at their own node (background coefficients, Pi,
-//     1/J, the RK4 state) are prefetched into registers one element ahead;
-//   * the 8x8 reference-derivative contractions run on tensor cores.  For
-//     axis al an element's 64 pencils form 8 tiles of 8 (the MMA N
-//     dimension); warp w owns tile w&7 and warps w and w+8 split the fields
-//     of a tile.  Every axis writes its own partial sums, so one barrier
-//     separates the contraction pass from the node pass.  The centred-flux
-//     SATs are added in the same pass: output row l = 0 or 7 of the MMA is
-//     the node row on face 2al or 2al+1.
-//       FP64 form: mma.sync.m8n8k4.f64, G the A operand in registers, the
-//       staged field -- or the split-form product Ja*u / Ja.F formed while
-//       loading -- the B operand.
-//       FP32 forms: split-precision BF16, mma.sync.m16n8k16 with FP32
-//       accumulation.  Three-term split (default): G and the operand v are
-//       split into bf16 terms hi + mid + lo (24 significant bits, as FP32);
-//       MMA 1 with A = [[G_hi, G_hi], [G_mid, G_mid]], B = [v_hi; v_mid] and
-//       MMA 2 with A = [[G_hi, G_lo], [G_mid, 0]], B = [v_lo; v_hi] sum every
-//       product down to relative size 2^-16 (rows 0-7 and 8-15 added in
-//       FP32).  Two-term split (hi + lo): one MMA with A = [[G_hi, G_hi],
-//       [G_lo, G_lo]], B = [v_hi; v_lo]; it carries ~16 significant bits and
-//       misses FP32 accuracy by a factor of ~30 on the n = 8 warped workload,
-//       so it is kept only for the precision study; there, because every row
-//       of G sums to zero, the operand is taken relative to its value at node
-//       3 of the pencil (D(v - c) = D v), so the split error scales with the
-//       variation of the field along the pencil, not with its size;
-//   * a node phase (one node per thread) forms flux, Phidot / divergence,
-//     boundary terms (boundary elements only) and the RK4 stage update and
-//     writes coalesced results (FP32 form: Kahan-compensated final sum);
-//   * per-element tables (SAT face mask, neighbour face sources) are loaded
-//     one element before the neighbour traces they address, so no load in
-//     the loop waits on another load.
+// update), in three families:
+//   * FP64 (k_cons_fk_n8): one element per CTA, contractions on the FP64 tensor
+//     cores (mma.sync.m8n8k4.f64, G the A operand in registers, the staged field
+//     -- or the split-form product Ja u / Ja.F formed while loading -- the B
+//     operand); the two halves alone or fused;
+//   * FP32 on CUDA cores, plain and compensated (k_cons_k1_n8c, k_cons_k2_n8c);
+//   * FP32 as split-precision BF16 on tensor cores (k_cons_k1_n8, k_cons_k2_n8).
+// The fields read at other nodes of an element (Phi and the nine metric terms in
+// K1; the three flux components and the metric terms in K2) are staged into
+// shared memory with 1D bulk copies (cp.async.bulk ... mbarrier::complete_tx), one
+// copy per field block; the metric terms and the flux live in global memory in
+// an element layout that makes the shared-memory accesses bank-conflict-free
+// (FP64: an XOR swizzle of the node index; BF16 forms: k-planes padded to 68
+// words; see Lay below).  One thread polls a stage's mbarrier, the rest wait at
+// the CTA barrier; every wait is bounded and raises an error flag instead of
+// spinning forever.
+//
+// The split-BF16 kernels are persistent: one CTA of 16 warps loops over elements,
+// a ring of NSTAGE stages keeps NSTAGE - 1 elements in flight, the fields used
+// only at their own node are prefetched into registers one element ahead, and the
+// per-element tables one element before the traces they address.  For axis al an
+// element's 64 pencils form 8 tiles of 8 (the MMA N dimension); warp w owns tile
+// w&7 and warps w and w+8 split the fields of a tile.  Every axis writes its own
+// partial sums, so one barrier separates the contraction pass from the node pass.
+// The centred-flux SATs are added in the same pass: output row l = 0 or 7 of the
+// MMA is the node row on face 2al or 2al+1.  mma.sync.m16n8k16 with FP32
+// accumulation.  Three-term split (default): G and the operand v are
+// split into bf16 terms hi + mid + lo (24 significant bits, as FP32);
+// MMA 1 with A = [[G_hi, G_hi], [G_mid, G_mid]], B = [v_hi; v_mid] and
+// MMA 2 with A = [[G_hi, G_lo], [G_mid, 0]], B = [v_lo; v_hi] sum every
+// product down to relative size 2^-16 (rows 0-7 and 8-15 added in
+// FP32).  Two-term split (hi + lo): one MMA with A = [[G_hi, G_hi],
+// [G_lo, G_lo]], B = [v_hi; v_lo]; it carries ~16 significant bits and
+// misses FP32 accuracy by a factor of ~30 on the n = 8 warped workload,
+// so it is kept only for the precision study; there, because every row
+// of G sums to zero, the operand is taken relative to its value at node
+// 3 of the pencil (D(v - c) = D v), so the split error scales with the
+// variation of the field along the pencil, not with its size.
 #include "wt_common.cuh"
 #include "wt_launch.cuh"
 #include "../../include/wavetoy_b200.h"
@@ -158,26 +151,6 @@ struct Lay<float> {
   static constexpr int FS = ::wt::n8::FS;
   __device__ __forceinline__ static int at(int n) { return pad(n & 7, (n >> 3) & 7, n >> 6); }
 };
-// K1's Phi (the caller's unpadded element block).  FP64: every thread loads
-// its node one element ahead (coalesced) and stores it into a double buffer in
-// the Lay<double> layout (REG = true, conflict-free like the other fields;
-// copying it by rows instead needs many small bulk copies, which the copy
-// engine serialises).  FP32: one bulk copy into the stage (unpadded).
-template <typename real>
-struct PhiLay;
-template <>
-struct PhiLay<double> {
-  static constexpr bool REG = true;
-  static constexpr int SZ = 0;  // words in the stage
-  __device__ __forceinline__ static int at(int n) { return Lay<double>::at(n); }
-};
-template <>
-struct PhiLay<float> {
-  static constexpr bool REG = false;
-  static constexpr int SZ = N3;
-  __device__ __forceinline__ static int at(int n) { return n; }
-};
-
 // Node of tile w for axis al at position p along al, pencil slot g.
 // Pencil orders: al=0 (j = w, k = slot); al=1 (i = slot, k = w); al=2 (i = slot, j = w).
 __device__ __forceinline__ int bn(int al, int w, int p, int g) {
@@ -193,9 +166,9 @@ __device__ __forceinline__ int opq(int al, int w, int b, int tig) {
   return al == 0 ? w + 8 * sl : sl + 8 * w;
 }
 
-// The partial sums of the contractions with their roundings written out, so that
-// the two-kernel stages and the fused stage kernel give the same bits however the
-// compiler would contract each: half_form = 0.5 d + 0.5 m e, half_pair = 0.5 m1 d1
+// The sums of the FP64 kernel with their roundings written out, so that the
+// two-kernel stages and the fused stages, instantiations of one template, give the
+// same bits however the compiler would contract each: half_form = 0.5 d + 0.5 m e, half_pair = 0.5 m1 d1
 // + 0.5 m2 d2, dot3 = a0 b0 + a1 b1 + a2 b2, madd = r + a b.
 template <typename real>
 __device__ __forceinline__ real half_form(real d, real m, real e) { return fma((real)0.5 * m, e, (real)0.5 * d); }
@@ -239,22 +212,7 @@ __device__ __forceinline__ void split_G(const double* G, int gq, int tig, int nt
   a2[3] = 0u;
 }
 
-// resident CTAs per SM
-template <typename real>
-struct Occ {
-  static constexpr int k1 = 1, k2 = 1;
-};
-template <>
-struct Occ<float> {
-  static constexpr int k1 = 2, k2 = 2;
-};
-// K1 stages the ten background coefficients with the copies instead of
-// prefetching them into registers (FP32: two CTAs then fit on an SM; FP64:
-// the registers go to the contraction pass)
-template <typename real>
-struct StageCoef {
-  static constexpr bool value = true;
-};
+constexpr int OCC = 2;  // resident CTAs per SM of the split-BF16 kernels
 
 }  // namespace n8
 
@@ -438,58 +396,51 @@ __device__ __forceinline__ void k1_boundary(const K1N8<real>& Q, long long e, in
   }
 }
 
-// K1 staged fields: Phi (PhiLay), Ja (9 fields in the Lay layout, one block
+// K1 staged fields: Phi (unpadded), Ja (9 fields in the Lay layout, one block
 // each from the global copy) and the ten coefficient fields (unpadded, read in
 // node order).  Register prefetch: Pi, invJ, y, acc, comp.
 template <typename real>
 __host__ __device__ constexpr size_t k1_stage() {
-  return (size_t)n8::PhiLay<real>::SZ + 9 * (size_t)n8::Lay<real>::FS +
-         (n8::StageCoef<real>::value ? 10 * (size_t)n8::N3 : 0);
+  return 9 * (size_t)n8::Lay<real>::FS + 11 * (size_t)n8::N3;
 }
 template <typename real>
 constexpr size_t k1_smem() {
-  return (n8::NSTAGE * k1_stage<real>() + 9 * n8::Lay<real>::FS + 2 * 6 * n8::N2 +
-          (n8::PhiLay<real>::REG ? 2 * n8::N3 : 0)) *
-             sizeof(real) +
+  return (n8::NSTAGE * k1_stage<real>() + 9 * n8::Lay<real>::FS + 2 * 6 * n8::N2) * sizeof(real) +
          n8::N2 * sizeof(double) + 64;
 }
 
-// NT: FP32 split terms (3 or 2); ignored by the FP64 form.  BATCH: the
+// NT: FP32 split terms (3 or 2).  BATCH: the
 // persistent loop runs over a work list of (solve, element) tiles and every
 // tile reads the parameter block of its solve (plist); P then only supplies
 // what is common to the launch (stage, operator, status word).
 // GR: gradient-only instantiation (the energy's apply_gradient3d!, src/wave3d_curved.jl:275-280):
 // no coefficients, Pi or RK state are read; the node phase writes the gradient to P.gout.
 template <typename real, int NT, bool BATCH, bool GR = false>
-__global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
+__global__ void __launch_bounds__(n8::THREADS, n8::OCC)
     k_cons_k1_n8(const K1N8<real> P, const K1N8<real>* __restrict__ plist, const int2* __restrict__ tiles,
                  long long ntiles) {
   using namespace n8;
-  constexpr bool F64 = std::is_same<real, double>::value;
-  constexpr bool SC = StageCoef<real>::value;
-  constexpr int NCOPY_C = SC && !GR ? 10 : 0;  // coefficient blocks copied per stage
+  constexpr int NCOPY_C = GR ? 0 : 10;  // coefficient blocks copied per stage
   constexpr size_t K1_STAGE = k1_stage<real>();
-  constexpr int FS = Lay<real>::FS, PSZ = PhiLay<real>::SZ;
+  constexpr int FS = Lay<real>::FS, PSZ = N3;  // Phi is staged unpadded
   extern __shared__ __align__(128) unsigned char smraw[];
   double* sG = reinterpret_cast<double*>(smraw);                // 64 (FP64 operator)
   real* stg = reinterpret_cast<real*>(sG + N2);                 // NSTAGE stages x 10 fields
   real* sg = stg + NSTAGE * K1_STAGE;                           // 9 padded partial gradients [al*3 + c]
   real* sface = sg + 9 * FS;                                    // 2 x 6 x 64
-  real* sphi = sface + 2 * 6 * N2;                              // PhiLay::REG: 2 x 512 (Lay)
-  constexpr bool PHIR = PhiLay<real>::REG;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sphi + (PHIR ? 2 * N3 : 0));  // NSTAGE
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sface + 2 * 6 * N2);  // NSTAGE
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tig = lane & 3, wt8 = warp & 7, half = warp >> 3;
   const real inv2H = (real)(1.0 / (2.0 * P.H[0]));
-  const bool comp_on = !F64 && P.epi && P.comp != nullptr;  // FP32 state only
+  const bool comp_on = P.epi && P.comp != nullptr;  // FP32 state only
   const bool need_y = P.epi && (P.stage == 1 || P.stage == 2 || (comp_on && P.stage == 3));
   const bool need_acc = P.epi && P.stage >= 1;
   const bool need_comp = comp_on && P.stage == 3;
-  const unsigned tx_bytes = (unsigned)((K1_STAGE - (SC ? 10 - NCOPY_C : 0) * (size_t)N3) * sizeof(real));
+  const unsigned tx_bytes = (unsigned)((K1_STAGE - (10 - NCOPY_C) * (size_t)N3) * sizeof(real));
   // node-phase coordinates of this thread
   const int ti = tid & 7, tj = (tid >> 3) & 7, tk = tid >> 6;
-  const int tpad = Lay<real>::at(tid), tphi = PhiLay<real>::at(tid);
+  const int tpad = Lay<real>::at(tid);
   const long long T = ntiles;
   const long long GS = gridDim.x;
   // tile t = (solve, element); (-1, -1) past the end
@@ -522,7 +473,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
     __syncwarp();
     real* d = stg + s * K1_STAGE;
     // copies: Phi (unless it goes through registers), 9 Ja, 10 coefficients
-    constexpr int NPHI = PHIR ? 0 : 1;
+    constexpr int NPHI = 1;
     for (int c = lane; c < NPHI + 9 + NCOPY_C; c += 32) {
       if (c < NPHI) {
         bulk_g2s(d, Q.Phi + e * N3, N3 * (unsigned)sizeof(real), &bar[s]);
@@ -548,19 +499,14 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
   auto emask_at = [&](int2 tl) -> int { return tl.x >= 0 ? prm(tl.x).emask[tl.y] : 0; };
   // pointwise fields of this thread's node
   struct PW {
-    real c[10], Pi, invJ, y, acc, comp, phi;
+    real Pi, invJ, y, acc, comp;
   };
   auto pw_load = [&](int2 tl, PW& w) {
     if (tl.x < 0) return;
     const K1N8<real>& Q = prm(tl.x);
     const long long n = (long long)tl.y * N3 + tid;
-    if constexpr (PHIR) w.phi = Q.Phi[n];
     w.invJ = Q.invdetJ[n];
     if constexpr (GR) return;
-    if constexpr (!SC) {
-#pragma unroll
-      for (int c = 0; c < 10; ++c) w.c[c] = Q.c10[c * Q.nn + n];
-    }
     w.Pi = Q.Pi[n];
     w.y = need_y ? Q.y[n] : (real)0;
     w.acc = need_acc ? Q.acc[n] : (real)0;
@@ -580,19 +526,13 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
     const real fv = face_load(src_load(t0), t0.x);
     if (tid < 6 * N2) sface[tid] = fv;
     pw_load(t0, cur);
-    if constexpr (PHIR) sphi[tphi] = cur.phi;
     src1 = src_load(t1);
   }
   __syncthreads();
   // A operand: FP64 G entries (rows gq, columns tig and 4 + tig); FP32 split pairs
   double aG0 = 0.0, aG1 = 0.0;
   uint32_t aS[4] = {0, 0, 0, 0}, aS2[4] = {0, 0, 0, 0};
-  if constexpr (F64) {
-    aG0 = sG[gq * 8 + tig];
-    aG1 = sG[gq * 8 + 4 + tig];
-  } else {
-    split_G(sG, gq, tig, NT, aS, aS2);
-  }
+  split_G(sG, gq, tig, NT, aS, aS2);
 
   int it = 0;
   for (long long t = blockIdx.x; t < T; t += GS, ++it) {
@@ -635,7 +575,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
     const K1N8<real>& Q = prm(t0.x);
     const long long e = t0.y;
     const real* d = stg + s * K1_STAGE;
-    const real* sPhi = PHIR ? sphi + fb * N3 : d;  // PhiLay
+    const real* sPhi = d;
     const real* sJa = d + PSZ;                      // 9 fields (Lay), index (al*3 + c)
     const real* sfc = sface + fb * 6 * N2;
     const int mask = emcur & 63;
@@ -650,52 +590,32 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
     // face 2 al, row 7: face 2 al + 1).
     auto grad_axis = [&](int al, int comps) {
       real cu[2], cm[3][2];
-      if constexpr (F64) {
-        double du[2] = {0, 0}, dm[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+      // the three-term split carries FP32's 24 bits, so only the two-term
+      // form takes the operand relative to its pencil value at node PREF
+      constexpr bool OFS = NT == 2;
+      const int nn0 = bn(al, wt8, 2 * tig, gq), nn1 = bn(al, wt8, 2 * tig + 1, gq);
+      const int nd0 = Lay<real>::at(nn0), nd1 = Lay<real>::at(nn1);
+      const float u0 = sPhi[nn0], u1 = sPhi[nn1];
+      const int nnr = OFS ? bn(al, wt8, PREF, gq) : 0, ndr = Lay<real>::at(nnr);
+      const float ur = OFS ? sPhi[nnr] : 0.f;
+      float fu[4] = {0, 0, 0, 0}, fm[3][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}};
+      mma_split<NT>(fu, aS, aS2, u0 - ur, u1 - ur);
 #pragma unroll
-        for (int kc = 0; kc < 2; ++kc) {
-          const int nn = bnode(al, wt8, kc, gq, tig), nd = Lay<real>::at(nn);
-          const double u = sPhi[PhiLay<real>::at(nn)];
-          const double a = kc ? aG1 : aG0;
-          dmma(du[0], du[1], a, u);
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            if ((comps >> c) & 1) dmma(dm[c][0], dm[c][1], a, sJa[(al * 3 + c) * FS + nd] * u);
-        }
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          cu[b] = du[b];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) cm[c][b] = dm[c][b];
-        }
-      } else {
-        // the three-term split carries FP32's 24 bits, so only the two-term
-        // form takes the operand relative to its pencil value at node PREF
-        constexpr bool OFS = NT == 2;
-        const int nn0 = bn(al, wt8, 2 * tig, gq), nn1 = bn(al, wt8, 2 * tig + 1, gq);
-        const int nd0 = Lay<real>::at(nn0), nd1 = Lay<real>::at(nn1);
-        const float u0 = sPhi[PhiLay<real>::at(nn0)], u1 = sPhi[PhiLay<real>::at(nn1)];
-        const int nnr = OFS ? bn(al, wt8, PREF, gq) : 0, ndr = Lay<real>::at(nnr);
-        const float ur = OFS ? sPhi[PhiLay<real>::at(nnr)] : 0.f;
-        float fu[4] = {0, 0, 0, 0}, fm[3][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}};
-        mma_split<NT>(fu, aS, aS2, u0 - ur, u1 - ur);
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-          if ((comps >> c) & 1) {
-            const real* mc = sJa + (al * 3 + c) * FS;
-            if constexpr (OFS) {
-              const float pr = mc[ndr] * ur;
-              mma_split<NT>(fm[c], aS, aS2, fmaf(mc[nd0], u0, -pr), fmaf(mc[nd1], u1, -pr));
-            } else {
-              mma_split<NT>(fm[c], aS, aS2, mc[nd0] * u0, mc[nd1] * u1);
-            }
+      for (int c = 0; c < 3; ++c)
+        if ((comps >> c) & 1) {
+          const real* mc = sJa + (al * 3 + c) * FS;
+          if constexpr (OFS) {
+            const float pr = mc[ndr] * ur;
+            mma_split<NT>(fm[c], aS, aS2, fmaf(mc[nd0], u0, -pr), fmaf(mc[nd1], u1, -pr));
+          } else {
+            mma_split<NT>(fm[c], aS, aS2, mc[nd0] * u0, mc[nd1] * u1);
           }
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          cu[b] = fu[b] + fu[b + 2];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) cm[c][b] = fm[c][b] + fm[c][b + 2];
         }
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        cu[b] = fu[b] + fu[b + 2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) cm[c][b] = fm[c][b] + fm[c][b + 2];
       }
       const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
       const bool sat = sface_f >= 0 && ((mask >> sface_f) & 1);
@@ -703,7 +623,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
       for (int b = 0; b < 2; ++b) {
         const int nno = onode(al, wt8, b, gq, tig), no = Lay<real>::at(nno);
         real jump = 0;
-        if (sat) jump = (gq ? inv2H : -inv2H) * (sfc[sface_f * N2 + opq(al, wt8, b, tig)] - sPhi[PhiLay<real>::at(nno)]);
+        if (sat) jump = (gq ? inv2H : -inv2H) * (sfc[sface_f * N2 + opq(al, wt8, b, tig)] - sPhi[nno]);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
           if ((comps >> c) & 1) {
@@ -725,9 +645,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
     // ---- node phase: one node per thread ----
     {
       const long long n = e * N3 + tid;
-      real u;
-      if constexpr (PHIR) u = cur.phi;
-      else u = sPhi[tphi];
+      const real u = sPhi[tid];
       real g0 = (sg[tpad] + sg[3 * FS + tpad]) + sg[6 * FS + tpad];
       real g1 = (sg[FS + tpad] + sg[4 * FS + tpad]) + sg[7 * FS + tpad];
       real g2 = (sg[2 * FS + tpad] + sg[5 * FS + tpad]) + sg[8 * FS + tpad];
@@ -739,7 +657,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
       } else {
       real cc[10];
 #pragma unroll
-      for (int c = 0; c < 10; ++c) cc[c] = SC ? d[PSZ + 9 * FS + c * N3 + tid] : cur.c[c];
+      for (int c = 0; c < 10; ++c) cc[c] = d[PSZ + 9 * FS + c * N3 + tid];
       const real a = cc[0];
       const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
       const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
@@ -755,7 +673,6 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
         Q.F[fstr + fo] = F1;
         Q.F[2 * fstr + fo] = F2;
       }
-      for (int c = 0; c < Q.nko; ++c) phid += Q.ko[c * Q.nn + n];
       if (P.epi)
         n8_rk<real>(P.stage, Q.dt, phid, u, cur.y, cur.acc, cur.comp, n, Q.y, Q.acc, Q.out, comp_on ? Q.comp : nullptr,
                     P.flag);
@@ -764,8 +681,6 @@ __global__ void __launch_bounds__(n8::THREADS, n8::Occ<real>::k1)
       }  // !GR
     }
     if (has_next && tid < 6 * N2) sface[(fb ^ 1) * 6 * N2 + tid] = fnext;
-    if constexpr (PHIR)
-      if (has_next) sphi[(fb ^ 1) * N3 + tphi] = nxt.phi;
     cur = nxt;
     emcur = emnext;
     src1 = src2;
@@ -811,40 +726,30 @@ struct K2N8 {
 };
 
 // K2 staged fields: 0..2 F, 3..11 Ja.  Register prefetch: invJ, y, acc, comp.
-// Two shapes (K2Shape): 512 threads (one node per thread, warps w and w + 8
-// split the fields of pencil tile w & 7, a ring of NSTAGE stages) or 256
-// threads (two nodes per thread, each warp does both halves of its tile, one
-// stage whose next copy is issued as soon as the contraction pass has read
-// it) -- the 256-thread shape fits two CTAs on an SM for FP64.  Partial
-// divergences: one field per (axis, half) in the 512-thread shape; one per axis
-// in the 256-thread shape, whose threads add the two halves in registers.
+// 512 threads: one node per thread, warps w and w + 8 split the fields of pencil
+// tile w & 7, a ring of NSTAGE stages; partial divergences one field per (axis, half).
 constexpr int K2_NF = 12;
 template <typename real>
 struct K2Shape {
-  static constexpr int THR = std::is_same<real, double>::value ? 256 : 512;
-  static constexpr int NS = THR == 512 ? n8::NSTAGE : 1;          // stages
-  static constexpr int OCC = std::is_same<real, double>::value ? 2 : n8::Occ<real>::k2;
-  static constexpr int NSD = THR == 512 ? 6 : 3;                  // partial-divergence fields
+  static constexpr int NSD = 6;  // partial-divergence fields
   static constexpr size_t STAGE = (size_t)K2_NF * n8::Lay<real>::FS;
 };
 template <typename real>
 constexpr size_t k2_smem() {
-  return (K2Shape<real>::NS * K2Shape<real>::STAGE + K2Shape<real>::NSD * n8::Lay<real>::FS + 2 * 6 * 3 * n8::N2) *
+  return (n8::NSTAGE * K2Shape<real>::STAGE + K2Shape<real>::NSD * n8::Lay<real>::FS + 2 * 6 * 3 * n8::N2) *
              sizeof(real) +
          n8::N2 * sizeof(double) + 64;
 }
 
 template <typename real, int NT, bool BATCH>
-__global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
+__global__ void __launch_bounds__(n8::THREADS, n8::OCC)
     k_cons_k2_n8(const K2N8<real> P, const K2N8<real>* __restrict__ plist, const int2* __restrict__ tiles,
                  long long ntiles) {
   using namespace n8;
-  constexpr bool F64 = std::is_same<real, double>::value;
-  constexpr int THR = K2Shape<real>::THR, NS = K2Shape<real>::NS;
+  constexpr int THR = THREADS, NS = NSTAGE;
   constexpr int NPT = N3 / THR;                 // nodes per thread in the node pass
   constexpr int NFACE = 6 * 3 * N2;             // 1152 neighbour face values
   constexpr int NFR = (NFACE + THR - 1) / THR;  // face values per thread
-  constexpr int NHALF = THR == 512 ? 1 : 2;     // halves of its tile a warp does
   constexpr int FS = Lay<real>::FS, NSD = K2Shape<real>::NSD;
   constexpr size_t K2_STAGE = K2Shape<real>::STAGE;
   extern __shared__ __align__(128) unsigned char smraw[];
@@ -857,7 +762,7 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tig = lane & 3, wt8 = warp & 7;
   const real inv2H = (real)(1.0 / (2.0 * P.H[0]));
-  const bool comp_on = !F64 && P.epi && P.comp != nullptr;  // FP32 state only
+  const bool comp_on = P.epi && P.comp != nullptr;  // FP32 state only
   const bool need_y = P.epi && (P.stage <= 2 || (comp_on && P.stage == 3));
   const bool need_acc = P.epi && P.stage >= 1;
   const bool need_comp = comp_on && P.stage == 3;
@@ -962,12 +867,7 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
   __syncthreads();
   double aG0 = 0.0, aG1 = 0.0;
   uint32_t aS[4] = {0, 0, 0, 0}, aS2[4] = {0, 0, 0, 0};
-  if constexpr (F64) {
-    aG0 = sG[gq * 8 + tig];
-    aG1 = sG[gq * 8 + 4 + tig];
-  } else {
-    split_G(sG, gq, tig, NT, aS, aS2);
-  }
+  split_G(sG, gq, tig, NT, aS, aS2);
 
   int it = 0;
   for (long long t = blockIdx.x; t < T; t += GS, ++it) {
@@ -1002,10 +902,8 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
           if (tile_at(t + k * GS).x >= 0) wait_phase(&bar[(it + k) % NS], ((it + k) / NS) & 1, nullptr);
       return;
     }
-    if constexpr (NS > 1) {
-      const int2 ti_ = NS == 2 ? t1 : tile_at(t + (NS - 1) * GS);
-      if (warp == 0 && ti_.x >= 0) issue(ti_, (it + NS - 1) % NS);
-    }
+    const int2 ti_ = NS == 2 ? t1 : tile_at(t + (NS - 1) * GS);
+    if (warp == 0 && ti_.x >= 0) issue(ti_, (it + NS - 1) % NS);
     const K2N8<real>& Q = prm(t0.x);
     const long long e = t0.y;
     const real* d = stg + s * K2_STAGE;
@@ -1021,78 +919,49 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
       const real* m0 = sJa + (al * 3 + 0) * FS;
       const real* m1 = sJa + (al * 3 + 1) * FS;
       const real* m2 = sJa + (al * 3 + 2) * FS;
-      real rsum[2] = {0, 0};
+      const int half = warp >> 3;
+      real cx[2], cy[2];
+      constexpr bool OFS = NT == 2;  // operand offset only for the two-term split (see K1)
+      constexpr int NQ = OFS ? 3 : 2;
+      const int nd[3] = {Lay<real>::at(bn(al, wt8, 2 * tig, gq)), Lay<real>::at(bn(al, wt8, 2 * tig + 1, gq)),
+                         Lay<real>::at(bn(al, wt8, PREF, gq))};
+      float vx[3] = {0, 0, 0}, vy[3] = {0, 0, 0};
 #pragma unroll
-      for (int hh = 0; hh < NHALF; ++hh) {
-        const int half = THR == 512 ? (warp >> 3) : hh;
-        real cx[2], cy[2];
-        if constexpr (F64) {
-          double dx[2] = {0, 0}, dy[2] = {0, 0};
-#pragma unroll
-          for (int kc = 0; kc < 2; ++kc) {
-            const int nd = Lay<real>::at(bnode(al, wt8, kc, gq, tig));
-            const double a = kc ? aG1 : aG0;
-            if (half == 0) {
-              // contravariant flux Ja^al . F and F_0
-              const double f0 = sF[nd];
-              const double ft = dot3<double>(m0[nd], f0, m1[nd], sF[FS + nd], m2[nd], sF[2 * FS + nd]);
-              dmma(dx[0], dx[1], a, ft);
-              dmma(dy[0], dy[1], a, f0);
-            } else {
-              dmma(dx[0], dx[1], a, sF[FS + nd]);
-              dmma(dy[0], dy[1], a, sF[2 * FS + nd]);
-            }
-          }
-          cx[0] = dx[0]; cx[1] = dx[1]; cy[0] = dy[0]; cy[1] = dy[1];
+      for (int q = 0; q < NQ; ++q) {
+        if (half == 0) {
+          const float f0 = sF[nd[q]];
+          vx[q] = m0[nd[q]] * f0 + m1[nd[q]] * sF[FS + nd[q]] + m2[nd[q]] * sF[2 * FS + nd[q]];
+          vy[q] = f0;
         } else {
-          constexpr bool OFS = NT == 2;  // operand offset only for the two-term split (see K1)
-          constexpr int NQ = OFS ? 3 : 2;
-          const int nd[3] = {Lay<real>::at(bn(al, wt8, 2 * tig, gq)), Lay<real>::at(bn(al, wt8, 2 * tig + 1, gq)),
-                             Lay<real>::at(bn(al, wt8, PREF, gq))};
-          float vx[3] = {0, 0, 0}, vy[3] = {0, 0, 0};
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) {
-            if (half == 0) {
-              const float f0 = sF[nd[q]];
-              vx[q] = m0[nd[q]] * f0 + m1[nd[q]] * sF[FS + nd[q]] + m2[nd[q]] * sF[2 * FS + nd[q]];
-              vy[q] = f0;
-            } else {
-              vx[q] = sF[FS + nd[q]];
-              vy[q] = sF[2 * FS + nd[q]];
-            }
-          }
-          float fx[4] = {0, 0, 0, 0}, fy[4] = {0, 0, 0, 0};
-          mma_split<NT>(fx, aS, aS2, vx[0] - vx[2], vx[1] - vx[2]);
-          mma_split<NT>(fy, aS, aS2, vy[0] - vy[2], vy[1] - vy[2]);
-          cx[0] = fx[0] + fx[2]; cx[1] = fx[1] + fx[3];
-          cy[0] = fy[0] + fy[2]; cy[1] = fy[1] + fy[3];
-        }
-        // half 1 adds the centred-flux SAT of an interior al-face on its rows
-        const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
-        const bool sat = half == 1 && sface_f >= 0 && ((mask >> sface_f) & 1);
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int no = Lay<real>::at(onode(al, wt8, b, gq, tig));
-          real r;
-          if (half == 0) {
-            r = half_form<real>(cx[b], m0[no], cy[b]);
-          } else {
-            r = half_pair<real>(m1[no], cx[b], m2[no], cy[b]);
-          }
-          if (sat) {
-            const int pq = opq(al, wt8, b, tig);
-            const real sacc = dot3<real>(m0[no], sfc[(sface_f * 3 + 0) * N2 + pq] - sF[no],
-                                         m1[no], sfc[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no],
-                                         m2[no], sfc[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
-            r = madd(r, gq ? inv2H : -inv2H, sacc);
-          }
-          if constexpr (NHALF == 2) rsum[b] = hh ? rsum[b] + r : r;
-          else sdiv[(al * 2 + half) * FS + no] = r;
+          vx[q] = sF[FS + nd[q]];
+          vy[q] = sF[2 * FS + nd[q]];
         }
       }
-      if constexpr (NHALF == 2) {
+      float fx[4] = {0, 0, 0, 0}, fy[4] = {0, 0, 0, 0};
+      mma_split<NT>(fx, aS, aS2, vx[0] - vx[2], vx[1] - vx[2]);
+      mma_split<NT>(fy, aS, aS2, vy[0] - vy[2], vy[1] - vy[2]);
+      cx[0] = fx[0] + fx[2]; cx[1] = fx[1] + fx[3];
+      cy[0] = fy[0] + fy[2]; cy[1] = fy[1] + fy[3];
+      // half 1 adds the centred-flux SAT of an interior al-face on its rows
+      const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
+      const bool sat = half == 1 && sface_f >= 0 && ((mask >> sface_f) & 1);
 #pragma unroll
-        for (int b = 0; b < 2; ++b) sdiv[al * FS + Lay<real>::at(onode(al, wt8, b, gq, tig))] = rsum[b];
+      for (int b = 0; b < 2; ++b) {
+        const int no = Lay<real>::at(onode(al, wt8, b, gq, tig));
+        real r;
+        if (half == 0) {
+          r = half_form<real>(cx[b], m0[no], cy[b]);
+        } else {
+          r = half_pair<real>(m1[no], cx[b], m2[no], cy[b]);
+        }
+        if (sat) {
+          const int pq = opq(al, wt8, b, tig);
+          const real sacc = dot3<real>(m0[no], sfc[(sface_f * 3 + 0) * N2 + pq] - sF[no],
+                                       m1[no], sfc[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no],
+                                       m2[no], sfc[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
+          r = madd(r, gq ? inv2H : -inv2H, sacc);
+        }
+        sdiv[(al * 2 + half) * FS + no] = r;
       }
     }
     __syncthreads();
@@ -1107,11 +976,8 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
       const int tpad = Lay<real>::at(node);
       const long long n = e * N3 + node;
       real dv;
-      if constexpr (NSD == 3)
-        dv = (sdiv[tpad] + sdiv[FS + tpad]) + sdiv[2 * FS + tpad];
-      else
-        dv = ((sdiv[tpad] + sdiv[2 * FS + tpad]) + sdiv[4 * FS + tpad]) +
-             ((sdiv[FS + tpad] + sdiv[3 * FS + tpad]) + sdiv[5 * FS + tpad]);
+      dv = ((sdiv[tpad] + sdiv[2 * FS + tpad]) + sdiv[4 * FS + tpad]) +
+           ((sdiv[FS + tpad] + sdiv[3 * FS + tpad]) + sdiv[5 * FS + tpad]);
       dv *= cur[r].invJ;
       if (bnd && Q.bc_on) {
         const int idx3[3] = {ti, tj, tk};
@@ -1123,7 +989,6 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
           dv += Q.bbuf[(long long)::wt::bc_slot(Q.bslot[f + 6 * e], Q.nbf) * N2 + p + 8 * q];
         }
       }
-      for (int c = 0; c < Q.nko; ++c) dv += Q.ko[c * Q.nn + n];
       if (P.epi)
         n8_rk<real>(P.stage, Q.dt, dv, cur[r].y, cur[r].y, cur[r].acc, cur[r].comp, n, Q.y, Q.acc, Q.out,
                     comp_on ? Q.comp : nullptr, P.flag);
@@ -1177,22 +1042,27 @@ __global__ void __launch_bounds__(K2Shape<real>::THR, K2Shape<real>::OCC)
 // place; the divergence partials wait in registers until every warp is done with
 // F and then replace it; the node pass reads its coefficients and RK words
 // directly (asking L2 for them when the CTA starts gained nothing, and asking for
-// the element 222 or 444 CTAs ahead cost 5-20 %).  Each partial sum is formed by
-// the instructions k_cons_k2_n8<double> and k_cons_k1_n8<double> use and added in
-// their order, so the fused step equals the two-kernel step bit for bit.
-// Measured (B200, 40^3 elements): 1.90 ms a launch, 4.5 TB/s of its 33 words (70 %
-// of the measured copy rate), before 2.36 ms; 41 % -> 63 % of DRAM throughput at
-// 24^3 elements.  What is left: waits on global loads (a third of the stalls),
+// the element 222 or 444 CTAs ahead cost 5-20 %).  K1, K2 and the energy's gradient
+// are instantiations of the same template, so the fused step equals the two-kernel
+// step bit for bit.
+// Measured (B200, 40^3 elements, one launch alone): fused 1.69 ms, 5.1 TB/s of its 33
+// words (78 % of the measured copy rate), before 2.36; K1 1.13 (28 words, 6.5 TB/s),
+// before 1.34; K2 0.96 (16 words, 4.4 TB/s), before 1.01.  In a running step the
+// sum is 9 % longer.  What is left: waits on global loads (a third of the stalls),
 // fixed-latency tensor and FP64 chains, and the shared-memory pipe (61 % busy).
 struct FKN8 {
   K2N8<double> a;  // stage s: F_s in (a.F0..F2), the Pi stage update
   K1N8<double> b;  // stage s + 1: Phi_{s+1} in (b.Phi), F_{s+1} out (b.F), the Phi stage update
 };
 constexpr int FK_THREADS = 256;
-constexpr int FK_NA = 12;  // F (3) + Ja (9) blocks
 constexpr int FK_NFF = 6 * 3 * 64, FK_NFP = 6 * 64;  // flux / Phi face values
-constexpr size_t fk_smem() { return (FK_NA * 512 + 512 + FK_NFF + FK_NFP) * sizeof(double) + 16; }
-static_assert(3 * (fk_smem() + 64 + 1024) <= 233472, "three CTAs of the fused stage kernel must fit an SM");
+// which halves a launch runs: K2 (divergence of F_s, Pi stage), K1 (gradient of Phi, flux, Phi
+// stage), both (the fused stage), or K1's gradient alone (the energy)
+enum { N8_K1 = 1, N8_K2 = 2, N8_FK = 3, N8_GRAD = 4 };
+constexpr size_t fk_smem(int half) {
+  return ((half & N8_K2 ? 3 * 512 + FK_NFF : 0) + 9 * 512 + (half & ~N8_K2 ? 512 + FK_NFP : 0)) * sizeof(double) + 16;
+}
+static_assert(3 * (fk_smem(N8_FK) + 64 + 1024) <= 233472, "three CTAs of the fused stage kernel must fit an SM");
 
 namespace n8 {
 // per-thread 8-byte asynchronous copy global -> shared, zero-filled when !valid
@@ -1228,57 +1098,75 @@ __device__ __forceinline__ double n8_rk_out(int stage, double dt, double k, doub
   return o;
 }
 
-__global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_constant__ FKN8 P) {
+// BATCH: tile blockIdx.x of a work list, each tile reading its solve's parameter
+// blocks (plA, plB); otherwise element e0 + blockIdx.x of the single solve P0.
+template <int HALF, bool BATCH>
+__global__ void __launch_bounds__(FK_THREADS, 3)
+    k_cons_fk_n8(const __grid_constant__ FKN8 P0, const K2N8<double>* plA, const K1N8<double>* plB, const int2* tiles) {
   using namespace n8;
   using real = double;
   constexpr int FS = Lay<double>::FS;
-  const K2N8<double>& A = P.a;
-  const K1N8<double>& B = P.b;
+  constexpr bool DIV = (HALF & N8_K2) != 0, GRAD = (HALF & ~N8_K2) != 0, FUSED = HALF == N8_FK;
   extern __shared__ __align__(128) unsigned char smraw[];
   double* sF = reinterpret_cast<double*>(smraw);  // 3 flux blocks, then the divergence partials [al] (Lay)
-  double* sJa = sF + 3 * FS;                      // 9 metric blocks, then the gradient partials [al * 3 + c] (Lay)
-  double* sphi = sJa + 9 * FS;                    // Phi_{s+1} (Lay)
-  double* sfF = sphi + N3;                        // flux face traces [f][c][pq]
-  double* sfP = sfF + FK_NFF;                     // Phi face traces [f][pq]
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sfP + FK_NFP);
+  double* sJa = sF + (DIV ? 3 * FS : 0);          // 9 metric blocks, then the gradient partials [al * 3 + c] (Lay)
+  double* sphi = sJa + 9 * FS;                    // the Phi the gradient reads (Lay)
+  double* sfP = sphi + (GRAD ? N3 : 0);           // Phi face traces [f][pq]
+  double* sfF = sfP + (GRAD ? FK_NFP : 0);        // flux face traces [f][c][pq]
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sfF + (DIV ? FK_NFF : 0));
   __shared__ int abort_flag;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tig = lane & 3;
-  const real inv2H = (real)(1.0 / (2.0 * A.H[0]));
-  const int sa = A.stage, sb = B.stage;  // sb = sa + 1
-  const bool needQacc = sa >= 1, needPy = sb == 1 || sb == 2;
-  const long long e = blockIdx.x;
+  int sid = 0;
+  long long e;
+  if constexpr (BATCH) {
+    const int2 tl = tiles[blockIdx.x];
+    sid = tl.x;
+    e = tl.y;
+  } else {
+    e = (DIV ? P0.a.e0 : P0.b.e0) + blockIdx.x;
+  }
+  const K2N8<double>& A = BATCH && DIV ? plA[sid] : P0.a;
+  const K1N8<double>& B = BATCH && GRAD ? plB[sid] : P0.b;
+  const long long Ne = DIV ? A.Ne : B.Ne;
+  const double* Ja = DIV ? A.Ja : B.Ja;
+  const int32_t* fsrcs = DIV ? A.fsrc : B.fsrc;
+  const double* Gm = DIV ? A.G : B.G;
+  const real inv2H = (real)(1.0 / (2.0 * (DIV ? A.H : B.H)[0]));
 
-  if (warp == 0) {  // F_s and Ja of the element
+  if (warp == 0) {  // the copies of F (after dep_wait) and Ja
     if (lane == 0) {
       abort_flag = 0;
       mbar_init(bar, 1);
       fence_barrier_init();
       fence_proxy_async();
-      mbar_expect_tx(bar, (unsigned)(FK_NA * FS * sizeof(real)));
+      mbar_expect_tx(bar, (unsigned)((DIV ? 12 : 9) * FS * sizeof(real)));
     }
     __syncwarp();
-    if (lane >= 3 && lane < FK_NA)
-      bulk_g2s(sF + lane * FS, A.Ja + ((long long)(lane - 3) * A.Ne + e) * FS, FS * (unsigned)sizeof(real), bar);
+    if (lane < 9) bulk_g2s(sJa + lane * FS, Ja + ((long long)lane * Ne + e) * FS, FS * (unsigned)sizeof(real), bar);
   }
   int fsrc[2];
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int idx = tid + r * FK_THREADS;
-    fsrc[r] = idx < FK_NFP ? ::wt::bc_src(A.fsrc[(idx >> 6) + 6 * e], A.Ne) : -1;
+    fsrc[r] = idx < FK_NFP ? ::wt::bc_src(fsrcs[(idx >> 6) + 6 * e], Ne) : -1;
   }
-  const int em = A.emask[e], mask = em & 63, bnd = em >> 6;
-  const double aG0 = A.G[gq * 8 + tig], aG1 = A.G[gq * 8 + 4 + tig];
+  const int em = (DIV ? A.emask : B.emask)[e], mask = em & 63, bnd = em >> 6;
+  const double aG0 = Gm[gq * 8 + tig], aG1 = Gm[gq * 8 + 4 + tig];
   dep_wait();  // above: mesh tables and metric terms, which no launch of a step writes
-  if (warp == 0 && lane < 3)
-    bulk_g2s(sF + lane * FS, (lane == 0 ? A.F0 : lane == 1 ? A.F1 : A.F2) + e * FS, FS * (unsigned)sizeof(real), bar);
+  if constexpr (DIV) {
+    if (warp == 0 && lane < 3)
+      bulk_g2s(sF + lane * FS, (lane == 0 ? A.F0 : lane == 1 ? A.F1 : A.F2) + e * FS, FS * (unsigned)sizeof(real), bar);
+  }
+  if constexpr (GRAD) {
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int w = tid + r * FK_THREADS;
-    cp_async8z(sphi + Lay<real>::at(w), B.Phi + e * N3 + w, true);
+    for (int r = 0; r < 2; ++r) {
+      const int w = tid + r * FK_THREADS;
+      cp_async8z(sphi + Lay<real>::at(w), B.Phi + e * N3 + w, true);
+    }
   }
   // neighbour face traces (zero-filled where a face has no neighbour); one thread
-  // per face node, so the four fields share one address
+  // per face node, so the fields share one address
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int idx = tid + r * FK_THREADS;
@@ -1286,24 +1174,26 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
       const int f = idx >> 6, pq = idx & 63, src = fsrc[r];
       const int nd = src >= 0 ? nbr_face_node(src, pq & 7, pq >> 3, N) : 0;
       const long long b = src >= 0 ? (long long)(src >> 6) * N3 : 0;
-      const long long at = b + Lay<real>::at(nd);
-      double* d = sfF + f * 3 * N2 + pq;
-      cp_async8z(d, A.F0 + at, src >= 0);
-      cp_async8z(d + N2, A.F1 + at, src >= 0);
-      cp_async8z(d + 2 * N2, A.F2 + at, src >= 0);
-      cp_async8z(sfP + idx, B.Phi + b + nd, src >= 0);
+      if constexpr (DIV) {
+        const long long at = b + Lay<real>::at(nd);
+        double* d = sfF + f * 3 * N2 + pq;
+        cp_async8z(d, A.F0 + at, src >= 0);
+        cp_async8z(d + N2, A.F1 + at, src >= 0);
+        cp_async8z(d + 2 * N2, A.F2 + at, src >= 0);
+      }
+      if constexpr (GRAD) cp_async8z(sfP + idx, B.Phi + b + nd, src >= 0);
     }
   }
   cp_async_wait_all();
-  if (tid == 0 && !wait_phase(bar, 0, A.flag)) abort_flag = 1;
+  if (tid == 0 && !wait_phase(bar, 0, DIV ? A.flag : B.flag)) abort_flag = 1;
   __syncthreads();
   if (abort_flag) {  // wait (bounded) for the copies in flight, then leave
     if (tid == 0) wait_phase(bar, 0, nullptr);
     return;
   }
 
-  // ---- contractions of tile `warp`: per axis the divergence of F_s (K2 half,
-  // kept in rs) and the split-form gradient of Phi_{s+1} (K1 half, in place) ----
+  // ---- contractions of tile `warp`: per axis the divergence of F (kept in rs) and
+  // the split-form gradient of Phi (in place) ----
   real rs[3][2];
 #pragma unroll
   for (int al = 0; al < 3; ++al) {
@@ -1317,16 +1207,21 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
       const int nd = Lay<real>::at(bnode(al, warp, kc, gq, tig));
       const double a = kc ? aG1 : aG0;
       const double j0 = m0[nd], j1 = m1[nd], j2 = m2[nd];
-      const double f0 = sF[nd], f1 = sF[FS + nd], f2 = sF[2 * FS + nd], u = sphi[nd];
-      const double ft = dot3(j0, f0, j1, f1, j2, f2);
-      dmma(dt[0], dt[1], a, ft);
-      dmma(d0[0], d0[1], a, f0);
-      dmma(d1[0], d1[1], a, f1);
-      dmma(d2[0], d2[1], a, f2);
-      dmma(du[0], du[1], a, u);
-      dmma(dm[0][0], dm[0][1], a, j0 * u);
-      dmma(dm[1][0], dm[1][1], a, j1 * u);
-      dmma(dm[2][0], dm[2][1], a, j2 * u);
+      if constexpr (DIV) {
+        const double f0 = sF[nd], f1 = sF[FS + nd], f2 = sF[2 * FS + nd];
+        const double ft = dot3(j0, f0, j1, f1, j2, f2);
+        dmma(dt[0], dt[1], a, ft);
+        dmma(d0[0], d0[1], a, f0);
+        dmma(d1[0], d1[1], a, f1);
+        dmma(d2[0], d2[1], a, f2);
+      }
+      if constexpr (GRAD) {
+        const double u = sphi[nd];
+        dmma(du[0], du[1], a, u);
+        dmma(dm[0][0], dm[0][1], a, j0 * u);
+        dmma(dm[1][0], dm[1][1], a, j1 * u);
+        dmma(dm[2][0], dm[2][1], a, j2 * u);
+      }
     }
     const int sface_f = gq == 0 ? 2 * al : gq == 7 ? 2 * al + 1 : -1;
     const bool sat = sface_f >= 0 && ((mask >> sface_f) & 1);
@@ -1342,82 +1237,114 @@ __global__ void __launch_bounds__(FK_THREADS, 3) k_cons_fk_n8(const __grid_const
       real g2 = half_form(dm[2][b], j2, du[b]);
       if (sat) {
         const int pq = opq(al, warp, b, tig);
-        const real sacc = dot3(j0, sfF[(sface_f * 3 + 0) * N2 + pq] - sF[no],
-                               j1, sfF[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no],
-                               j2, sfF[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
-        r1 = madd(r1, gq ? inv2H : -inv2H, sacc);
-        const real jump = (gq ? inv2H : -inv2H) * (sfP[sface_f * N2 + pq] - sphi[no]);
-        g0 = madd(g0, j0, jump);
-        g1 = madd(g1, j1, jump);
-        g2 = madd(g2, j2, jump);
+        if constexpr (DIV) {
+          const real sacc = dot3(j0, sfF[(sface_f * 3 + 0) * N2 + pq] - sF[no],
+                                 j1, sfF[(sface_f * 3 + 1) * N2 + pq] - sF[FS + no],
+                                 j2, sfF[(sface_f * 3 + 2) * N2 + pq] - sF[2 * FS + no]);
+          r1 = madd(r1, gq ? inv2H : -inv2H, sacc);
+        }
+        if constexpr (GRAD) {
+          const real jump = (gq ? inv2H : -inv2H) * (sfP[sface_f * N2 + pq] - sphi[no]);
+          g0 = madd(g0, j0, jump);
+          g1 = madd(g1, j1, jump);
+          g2 = madd(g2, j2, jump);
+        }
       }
       rs[al][b] = r0 + r1;
       gr[0][b] = g0;
       gr[1][b] = g1;
       gr[2][b] = g2;
     }
-    __syncwarp();  // every lane has read this (axis, tile)'s metric terms
+    if constexpr (GRAD) {
+      __syncwarp();  // every lane has read this (axis, tile)'s metric terms
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      const int no = Lay<real>::at(onode(al, warp, b, gq, tig));
-      m0[no] = gr[0][b];
-      m1[no] = gr[1][b];
-      m2[no] = gr[2][b];
+      for (int b = 0; b < 2; ++b) {
+        const int no = Lay<real>::at(onode(al, warp, b, gq, tig));
+        m0[no] = gr[0][b];
+        m1[no] = gr[1][b];
+        m2[no] = gr[2][b];
+      }
     }
   }
-  __syncthreads();  // every warp is done with F
+  if constexpr (DIV) {
+    __syncthreads();  // every warp is done with F
 #pragma unroll
-  for (int al = 0; al < 3; ++al)
+    for (int al = 0; al < 3; ++al)
 #pragma unroll
-    for (int b = 0; b < 2; ++b) sF[al * FS + Lay<real>::at(onode(al, warp, b, gq, tig))] = rs[al][b];
+      for (int b = 0; b < 2; ++b) sF[al * FS + Lay<real>::at(onode(al, warp, b, gq, tig))] = rs[al][b];
+  }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int w = tid + r * FK_THREADS, tp = Lay<real>::at(w);
     const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
     const long long n = e * N3 + w;
-    real cc[10];
-#pragma unroll
-    for (int c = 0; c < 10; ++c) cc[c] = B.c10[c * B.nn + n];
-    const real invJ = A.invdetJ[n], Qy = A.y[n], Qacc = needQacc ? A.acc[n] : (real)0;
-    const real Py = needPy ? B.y[n] : (real)0, Pacc = B.acc[n];  // stage s + 1 >= 1 reads the accumulator
-    // ---- divergence node pass: boundary terms, Pi stage update (K2 half) ----
-    real dv = (sF[tp] + sF[FS + tp]) + sF[2 * FS + tp];
-    dv *= invJ;
-    if (bnd && A.bc_on) {
-      const int idx3[3] = {ti, tj, tk};
-      for (int f = 0; f < 6; ++f) {
-        if (A.bdry[f + 6 * e] == 0) continue;
-        const int ax = f >> 1;
-        if (idx3[ax] != ((f & 1) ? 7 : 0)) continue;
-        const int p = ax == 0 ? tj : ti, q = ax == 2 ? tj : tk;
-        dv += A.bbuf[(long long)::wt::bc_slot(A.bslot[f + 6 * e], A.nbf) * N2 + p + 8 * q];
+    const real invJ = (DIV ? A.invdetJ : B.invdetJ)[n];
+    real Pi = 0;
+    if constexpr (DIV) {
+      // ---- divergence node pass: boundary terms, Pi stage update (K2 half) ----
+      const bool need_y = A.epi && A.stage <= 2, need_acc = A.epi && A.stage >= 1;
+      const real Qy = need_y ? A.y[n] : (real)0, Qacc = need_acc ? A.acc[n] : (real)0;
+      real dv = (sF[tp] + sF[FS + tp]) + sF[2 * FS + tp];
+      dv *= invJ;
+      if (bnd && A.bc_on) {
+        const int idx3[3] = {ti, tj, tk};
+        for (int f = 0; f < 6; ++f) {
+          if (A.bdry[f + 6 * e] == 0) continue;
+          const int ax = f >> 1;
+          if (idx3[ax] != ((f & 1) ? 7 : 0)) continue;
+          const int p = ax == 0 ? tj : ti, q = ax == 2 ? tj : tk;
+          dv += A.bbuf[(long long)::wt::bc_slot(A.bslot[f + 6 * e], A.nbf) * N2 + p + 8 * q];
+        }
+      }
+      for (int c = 0; c < A.nko; ++c) dv += A.ko[c * A.nn + n];
+      if constexpr (FUSED) {
+        Pi = n8_rk_out(A.stage, A.dt, dv, Qy, Qacc, n, A.acc, A.out);  // Pi_{s+1}
+      } else {
+        if (A.epi)
+          n8_rk<real>(A.stage, A.dt, dv, Qy, Qy, Qacc, (real)0, n, A.y, A.acc, A.out, nullptr, A.flag);
+        else
+          A.Pidot[n] = dv;
       }
     }
-    for (int c = 0; c < A.nko; ++c) dv += A.ko[c * A.nn + n];
-    const real Pi = n8_rk_out(sa, A.dt, dv, Qy, Qacc, n, A.acc, A.out);  // Pi_{s+1}
-    // ---- gradient node pass: flux F_{s+1}, Phidot, boundary terms, Phi stage update (K1 half) ----
-    const real u = sphi[tp];
-    real g0 = (sJa[tp] + sJa[3 * FS + tp]) + sJa[6 * FS + tp];
-    real g1 = (sJa[FS + tp] + sJa[4 * FS + tp]) + sJa[7 * FS + tp];
-    real g2 = (sJa[2 * FS + tp] + sJa[5 * FS + tp]) + sJa[8 * FS + tp];
-    g0 *= invJ; g1 *= invJ; g2 *= invJ;
-    const real a = cc[0];
-    const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
-    const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
-    const real F0 = b0 * Pi + (K0 * g0 + K1v * g1 + K2 * g2);
-    const real F1 = b1 * Pi + (K1v * g0 + K3 * g1 + K4 * g2);
-    const real F2 = b2 * Pi + (K2 * g0 + K4 * g1 + K5 * g2);
-    real phid = b0 * g0 + b1 * g1 + b2 * g2 + a * Pi;
-    if (bnd && B.bc_on) k1_boundary<real>(B, e, ti, tj, tk, n, u, Pi, g0, g1, g2, cc, phid);
-    {
-      const long long fo = e * FS + tp, fstr = B.Ne * FS;
-      B.F[fo] = F0;
-      B.F[fstr + fo] = F1;
-      B.F[2 * fstr + fo] = F2;
+    if constexpr (GRAD) {
+      // ---- gradient node pass: flux, Phidot, boundary terms, Phi stage update (K1 half) ----
+      const real u = sphi[tp];
+      real g0 = (sJa[tp] + sJa[3 * FS + tp]) + sJa[6 * FS + tp];
+      real g1 = (sJa[FS + tp] + sJa[4 * FS + tp]) + sJa[7 * FS + tp];
+      real g2 = (sJa[2 * FS + tp] + sJa[5 * FS + tp]) + sJa[8 * FS + tp];
+      g0 *= invJ; g1 *= invJ; g2 *= invJ;
+      if constexpr (HALF == N8_GRAD) {
+        B.gout[n] = g0;
+        B.gout[B.nn + n] = g1;
+        B.gout[2 * B.nn + n] = g2;
+      } else {
+        real cc[10];
+#pragma unroll
+        for (int c = 0; c < 10; ++c) cc[c] = B.c10[c * B.nn + n];
+        if constexpr (!FUSED) Pi = B.Pi[n];
+        const bool need_y = B.epi && (B.stage == 1 || B.stage == 2), need_acc = B.epi && B.stage >= 1;
+        const real Py = need_y ? B.y[n] : (real)0, Pacc = need_acc ? B.acc[n] : (real)0;
+        const real a = cc[0];
+        const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
+        const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
+        // the roundings written out: the same bits in every instantiation
+        const real F0 = fma(b0, Pi, dot3(K0, g0, K1v, g1, K2, g2));
+        const real F1 = fma(b1, Pi, dot3(K1v, g0, K3, g1, K4, g2));
+        const real F2 = fma(b2, Pi, dot3(K2, g0, K4, g1, K5, g2));
+        real phid = fma(a, Pi, dot3(b0, g0, b1, g1, b2, g2));
+        if (bnd && B.bc_on) k1_boundary<real>(B, e, ti, tj, tk, n, u, Pi, g0, g1, g2, cc, phid);
+        const long long fo = e * FS + tp, fstr = B.Ne * FS;
+        B.F[fo] = F0;
+        B.F[fstr + fo] = F1;
+        B.F[2 * fstr + fo] = F2;
+        for (int c = 0; c < B.nko; ++c) phid += B.ko[c * B.nn + n];
+        if (FUSED || B.epi)
+          n8_rk<real>(B.stage, B.dt, phid, u, Py, Pacc, (real)0, n, B.y, B.acc, B.out, nullptr, B.flag);
+        else
+          B.Phidot[n] = phid;
+      }
     }
-    for (int c = 0; c < B.nko; ++c) phid += B.ko[c * B.nn + n];
-    n8_rk<real>(sb, B.dt, phid, u, Py, Pacc, (real)0, n, B.y, B.acc, B.out, nullptr, B.flag);
   }
 }
 
@@ -2219,6 +2146,22 @@ static K2N8<real> k2n8_params(const DevMesh& m, const void* F, void* Pidot, cons
   return P;
 }
 
+// the FP64 kernels: HALF of the elements of P (plA, plB NULL) or of a work list
+template <int HALF, bool BATCH>
+static int n8d_launch(const FKN8& P, const void* plA, const void* plB, const int2* tiles, long long ntiles,
+                      cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(k_cons_fk_n8<HALF, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)fk_smem(HALF)) != cudaSuccess)
+      return -2;
+    attr = true;
+  }
+  if (ntiles <= 0) return 0;
+  return launch_dep(k_cons_fk_n8<HALF, BATCH>, (unsigned)ntiles, FK_THREADS, fk_smem(HALF), s, P,
+                    (const K2N8<double>*)plA, (const K1N8<double>*)plB, tiles);
+}
+
 // Launch K1 (which = 1) or K2 (which = 2) of one instantiation: a single solve
 // (plist == nullptr, ntiles = P.Ne) or a work list over the solves of plist.
 template <typename real, int NT, bool BATCH>
@@ -2231,7 +2174,7 @@ static int n8_launch(int which, const void* hP, const void* plist, const int2* t
         return -2;
       attr1 = true;
     }
-    const long long cap = (long long)sm_count() * n8::Occ<real>::k1;
+    const long long cap = (long long)sm_count() * n8::OCC;
     const long long grid = ntiles < cap ? ntiles : cap;
     if (grid <= 0) return 0;
     k_cons_k1_n8<real, NT, BATCH><<<(unsigned)grid, n8::THREADS, k1_smem<real>(), s>>>(
@@ -2243,10 +2186,10 @@ static int n8_launch(int which, const void* hP, const void* plist, const int2* t
         return -2;
       attr2 = true;
     }
-    const long long cap = (long long)sm_count() * K2Shape<real>::OCC;
+    const long long cap = (long long)sm_count() * n8::OCC;
     const long long grid = ntiles < cap ? ntiles : cap;
     if (grid <= 0) return 0;
-    k_cons_k2_n8<real, NT, BATCH><<<(unsigned)grid, K2Shape<real>::THR, k2_smem<real>(), s>>>(
+    k_cons_k2_n8<real, NT, BATCH><<<(unsigned)grid, n8::THREADS, k2_smem<real>(), s>>>(
         *(const K2N8<real>*)hP, (const K2N8<real>*)plist, tiles, ntiles);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -2292,7 +2235,15 @@ static int n8c_launch(int which, const void* hP, const void* plist, const int2* 
 template <bool BATCH>
 static int n8_dispatch(int which, int precision, int fp32_form, const void* hP, const void* plist, const int2* tiles,
                        long long ntiles, cudaStream_t s) {
-  if (precision == 0) return n8_launch<double, 0, BATCH>(which, hP, plist, tiles, ntiles, s);
+  if (precision == 0) {
+    FKN8 P;
+    if (which == 1) {
+      P.b = *(const K1N8<double>*)hP;
+      return n8d_launch<N8_K1, BATCH>(P, nullptr, plist, tiles, ntiles, s);
+    }
+    P.a = *(const K2N8<double>*)hP;
+    return n8d_launch<N8_K2, BATCH>(P, plist, nullptr, tiles, ntiles, s);
+  }
   if (fp32_form == WT_FP32_COMPENSATED) return n8c_launch<BATCH, true>(which, hP, plist, tiles, ntiles, s);
   if (fp32_form == WT_FP32_CUDA_CORES) return n8c_launch<BATCH, false>(which, hP, plist, tiles, ntiles, s);
   if (fp32_form == WT_FP32_BF16X2) return n8_launch<float, 2, BATCH>(which, hP, plist, tiles, ntiles, s);
@@ -2320,14 +2271,7 @@ int launch_cons_fk_n8(const DevMesh& m, const DevCoef& c, const void* Fin, void*
   FKN8 P;
   P.a = k2n8_params<double>(m, Fin, nullptr, bbuf, bc, rkQ, m.errflag);
   P.b = k1n8_params<double>(m, c, Phi, nullptr, Fout, nullptr, bbuf, bc, rkP, m.errflag);
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_cons_fk_n8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fk_smem()) != cudaSuccess)
-      return -2;
-    attr = true;
-  }
-  if (m.Ne <= 0) return 0;
-  return launch_dep(k_cons_fk_n8, (unsigned)m.Ne, FK_THREADS, fk_smem(), s, P);
+  return n8d_launch<N8_FK, false>(P, nullptr, nullptr, nullptr, m.Ne, s);
 }
 
 int launch_cons_k2_n8(const DevMesh& m, const void* F, void* Pidot, const void* bbuf, const ConsBC& bc,
@@ -2370,7 +2314,7 @@ static int launch_grad_n8_t(const K1N8<real>& P, bool cuda_core, cudaStream_t s)
       return -2;
     attr = true;
   }
-  const long long cap = (long long)sm_count() * n8::Occ<real>::k1, grid = P.Ne < cap ? P.Ne : cap;
+  const long long cap = (long long)sm_count() * n8::OCC, grid = P.Ne < cap ? P.Ne : cap;
   k_cons_k1_n8<real, NT, false, true><<<(unsigned)grid, n8::THREADS, k1_smem<real>(), s>>>(P, nullptr, nullptr, P.Ne);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -2382,7 +2326,9 @@ int launch_grad_n8(const DevMesh& m, const void* Phi, void* grad, unsigned* flag
   if (m.precision == 0) {
     K1N8<double> P = k1n8_params<double>(m, none, Phi, nullptr, nullptr, nullptr, nullptr, bc, rk, flag);
     P.gout = (double*)grad;
-    return launch_grad_n8_t<double, 0>(P, false, s);
+    FKN8 Q;
+    Q.b = P;
+    return n8d_launch<N8_GRAD, false>(Q, nullptr, nullptr, nullptr, m.Ne, s);
   }
   K1N8<float> P = k1n8_params<float>(m, none, Phi, nullptr, nullptr, nullptr, nullptr, bc, rk, flag);
   P.gout = (float*)grad;
