@@ -127,7 +127,7 @@ int wt_ctx_nonfinite(wt_ctx* ctx, int* flag);
 int wt_ctx_selftest_wait(wt_ctx* ctx, int arrive, long long polls);
 /* Per-kernel timing for measurement: while enabled, the fused RK4 step records
  * CUDA events around each launch of its kernels (gradient/flux K1, divergence
- * K2, and the fused stage kernel of FP64 n = 8 solves) on the launching
+ * K2, and the fused stage kernel of n = 8 solves) on the launching
  * stream; wt_ctx_profile_read synchronises and returns the summed milliseconds
  * and launch counts {K1, K2, fused stage}, then clears. */
 int wt_ctx_profile(wt_ctx* ctx, int enable);
@@ -327,13 +327,16 @@ int wt_workspace_mu(wt_ws* ws, double* mu);
  * own estimate differs from it. */
 int wt_workspace_set_mu(wt_ws* ws, double mu);
 /* Fused RK4 stages (the integrator-in-RHS idea of the reference's IDEAS.md:48-50;
- * no entry point of its own there): with on = 1 (the default) an FP64 n = 8
- * solve without Kreiss-Oliger dissipation steps through the fused stage kernel,
- * which runs the divergence half of stage s and the gradient half of stage
- * s + 1 in one launch (five launches per RK4 step instead of eight, 28 % fewer
- * DRAM bytes).  The results equal the two-kernel stages' bit for bit; on = 0
- * selects the two-kernel stages.  Takes effect at the next step call; the
- * second flux buffer (3 x 8 bytes per node) is allocated then. */
+ * no entry point of its own there): with on = 1 (the default) an n = 8 solve in
+ * FP64, or in compensated FP32 without Kreiss-Oliger dissipation, steps through
+ * the fused stage kernel, which runs the divergence half of stage s and the
+ * gradient half of stage s + 1 in one launch (five launches per RK4 step instead
+ * of eight, 28 % fewer DRAM bytes).  The results equal the two-kernel stages' bit
+ * for bit; on = 0 selects the two-kernel stages.  Takes effect at the next step
+ * call.  The second flux buffer is allocated with FP64's first such step (3 x 8
+ * bytes per node) or FP32's step buffers (2 x 4 bytes per node more than without;
+ * where that would leave less than an eighth of the device's memory free, the
+ * two-kernel stages run). */
 int wt_workspace_set_fused(wt_ws* ws, int on);
 
 /* ---- right-hand sides (device pointers, async) ------------------------------*/

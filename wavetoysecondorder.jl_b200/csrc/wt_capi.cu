@@ -75,7 +75,7 @@ struct wt_ws {
   double mu = 0.0, inv_mu5 = 0.0;
   bool mu_done = false;  // mu is computed on first use (Kreiss-Oliger or wt_workspace_mu)
   void* F = nullptr;      // 3 nn
-  void* F2 = nullptr;     // FP64 n = 8 fused stages: the second flux buffer (F ping-pongs between launches)
+  void* F2 = nullptr;     // n = 8 fused stages: the second flux buffer (F ping-pongs between launches)
   int fused = 1;          // FP64 n = 8 RK4 steps through the fused stage kernel (wt_workspace_set_fused)
   void* bbuf = nullptr;   // nbf N^2
   void* grad = nullptr;   // 3 nn
@@ -333,13 +333,32 @@ int ws_buffers(wt_ws* ws) {
   return 0;
 }
 
+// Whether the fused stages of this mesh run the compensated FP32 form: the
+// default FP32 form, through the kernels that implement it.
+bool compensated(const wt::DevMesh& m, bool n8) {
+  return m.precision == WT_F32 && m.fp32_form == WT_FP32_COMPENSATED && (n8 || wt::cons_gen_cp_supported(m));
+}
+
+// Whether whole RK4 steps of this workspace have a fused stage kernel (see step_curved_fused)
+bool ko_fused(const wt::DevMesh& m);
+bool fused_form(const wt_ws* ws, double eps_ko) {
+  const wt::DevMesh& m = ws->mesh->m;
+  if (!ws->fused || m.N != 8) return false;
+  if (m.precision == WT_F64) return eps_ko == 0.0 || ko_fused(m);
+  return eps_ko == 0.0 && compensated(m, true);
+}
+// the fused stages' second flux buffer
+int fused_buffer(wt_ws* ws) {
+  const wt::DevMesh& m = ws->mesh->m;
+  return ensure(ws, &ws->F2, 3 * (size_t)wt::n8_padded_field_size(m.Ne) * rsize(m.precision));
+}
+
 int ws_step_buffers(wt_ws* ws) {
   const wt::DevMesh& m = ws->mesh->m;
   const size_t nb = (size_t)m.nn * rsize(m.precision);
   WT_TRY(ws_buffers(ws));
   WT_TRY(ensure(ws, &ws->S0, nb));
   WT_TRY(ensure(ws, &ws->S1, nb));
-  WT_TRY(ensure(ws, &ws->SQ, nb));
   WT_TRY(ensure(ws, &ws->accP, nb));
   WT_TRY(ensure(ws, &ws->accQ, nb));
   if (m.precision == WT_F32) {
@@ -347,6 +366,19 @@ int ws_step_buffers(wt_ws* ws) {
     WT_TRY(ensure(ws, &ws->compQ, nb));
     WT_TRY(ensure(ws, &ws->kP, nb));  // the compensated form's copy of Phi's high part (stage 2 -> 3)
   }
+  // Last, as the fused FP32 stages' second flux buffer is not a must: where it would
+  // leave less than an eighth of the device free, the two-kernel stages run.  Their
+  // Pi, SQ, which the fused stages do not use, takes its first field.
+  if (m.precision == WT_F32 && !ws->SQ && !ws->F2 && fused_form(ws, 0.0)) {
+    size_t avail = 0, total = 0;
+    const size_t need = 3 * (size_t)wt::n8_padded_field_size(m.Ne) * sizeof(float);
+    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) cudaGetLastError();
+    if (avail >= need + total / 8) {
+      WT_TRY(fused_buffer(ws));
+      ws->SQ = ws->F2;
+    }
+  }
+  WT_TRY(ensure(ws, &ws->SQ, nb));
   return 0;
 }
 
@@ -1228,6 +1260,7 @@ int wt_workspace_create(wt_ctx* ctx, wt_mesh* mesh, wt_ws** out) {
 int wt_workspace_destroy(wt_ws* ws) {
   if (!ws) return WT_EINVAL;
   cudaStreamSynchronize(ws->ctx->stream);
+  if (ws->SQ == ws->F2) ws->SQ = nullptr;
   void* bufs[] = {ws->F, ws->F2, ws->bbuf, ws->grad, ws->kP, ws->kQ, ws->S0, ws->S1, ws->SQ, ws->accP, ws->accQ,
                   ws->trace, ws->trace2, ws->ko, ws->zero, ws->Lu, ws->compP, ws->compQ, ws->erk, ws->evo[0], ws->evo[1],
                   ws->evo[2], ws->evo[3], ws->evoE};
@@ -1584,12 +1617,6 @@ static PhiStage phi_stage(const wt_ws* ws, void* Phi, int st, bool cp) {
   return {st == 3 ? ws->kP : Phi, st == 0 ? ws->compP : SP[(st - 1) % 2], st == 2 ? ws->kP : nullptr};
 }
 
-// Whether the fused stages of this mesh run the compensated FP32 form: the
-// default FP32 form, through the kernels that implement it.
-static bool compensated(const wt::DevMesh& m, bool n8) {
-  return m.precision == WT_F32 && m.fp32_form == WT_FP32_COMPENSATED && (n8 || wt::cons_gen_cp_supported(m));
-}
-
 // One half of fused RK4 stage st (eps_ko = 0): part 1 launches K1 (flux, boundary
 // terms, the Phi stage update), part 2 K2 (divergence, the Pi stage update).
 static int rk4_stage_part(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, void* Pi, double dt, int st,
@@ -1635,7 +1662,8 @@ static int rk4_stage_part(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi
   return 0;
 }
 
-// The RK4 step of an FP64 n = 8 solve through the fused stage kernel: K1_0,
+// The RK4 step of an n = 8 solve (FP64, or FP32 in the compensated form without
+// dissipation) through the fused stage kernel: K1_0,
 // FK_0, FK_1, FK_2 (each the K2 half of stage s and the K1 half of stage s + 1),
 // K2_3 -- five launches instead of eight, the flux ping-ponging between ws->F
 // and ws->F2.  Time-dependent backgrounds are re-sampled before the launch
@@ -1644,8 +1672,7 @@ static int rk4_stage_part(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi
 static bool fused_path(const wt_ws* ws, const wt_coef* coef, void* Phi, void* Pi, double eps_ko,
                        const wt::ConsBC& b, int use_metric) {
   const wt::DevMesh& m = ws->mesh->m;
-  if (!ws->fused || m.precision != WT_F64 || m.N != 8 || !ws->F2) return false;
-  if (eps_ko != 0.0 && !wt::ko_all_lines(m)) return false;
+  if (!fused_form(ws, eps_ko) || !ws->F2) return false;
   wt::RKStage r;
   r.on = 1;
   r.y = Phi; r.acc = ws->accP; r.out = ws->S0;
@@ -1661,20 +1688,22 @@ static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* 
   void* SP[2] = {ws->S0, ws->S1};
   void* FB[2] = {ws->F, ws->F2};
   const double toff[4] = {0.0, 0.5 * dt, 0.5 * dt, dt};  // RK4 stage times
-  const bool ko = eps_ko != 0.0;
+  const bool ko = eps_ko != 0.0, cp = compensated(m, true);
   const void *koP = nullptr, *koQ = nullptr;  // the increments the next launch adds
   int nko = 0;
   auto rkP = [&](int st) {
     wt::RKStage r;
     r.on = 1; r.stage = st; r.dt = dt;
-    r.y = Phi; r.acc = ws->accP; r.out = SP[st % 2];
+    r.y = Phi; r.acc = ws->accP; r.out = SP[st % 2]; r.comp = ws->compP;
     r.ko = koP; r.nko = nko;
+    const PhiStage ps = phi_stage(ws, Phi, st, cp);
+    r.phit = ps.phit; r.hcopy = ps.hcopy;
     return r;
   };
   auto rkQ = [&](int st) {
     wt::RKStage r;
     r.on = 1; r.stage = st; r.dt = dt;
-    r.y = Pi; r.acc = ws->accQ;
+    r.y = Pi; r.acc = ws->accQ; r.comp = ws->compQ;
     r.out = ko && st < 3 ? ws->SQ : nullptr;  // without dissipation Pi's stage value stays in the fused kernel
     r.ko = koQ; r.nko = nko;
     return r;
@@ -1685,7 +1714,7 @@ static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* 
   auto increments = [&](const void* P, const void* Q) -> int {
     return ko ? ko_increments(ctx, ws, P, Q, eps_ko, &koP, &koQ, &nko) : 0;
   };
-  ws->halo_cp = 0;
+  ws->halo_cp = cp ? 1 : 0;
   ws->flux_block = wt::n8_flux_block(m);
   ws->flux_lay = wt::n8_flux_layout(m);
   if (coef->td) WT_TRY(coef_resample(ctx, coef, toff[0], s));
@@ -1693,7 +1722,7 @@ static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* 
   {
     wt::NvtxRange nv("rk4 stage 0 K1");
     prof_mark(ctx, 0);
-    WT_TRY(lrc(ctx, wt::launch_cons_k1(m, coef->c, Phi, Pi, FB[0], nullptr, ws->bbuf, nullptr, use_metric, b, rkP(0),
+    WT_TRY(lrc(ctx, wt::launch_cons_k1(m, coef->c, phi_stage(ws, Phi, 0, cp).in, Pi, FB[0], nullptr, ws->bbuf, nullptr, use_metric, b, rkP(0),
                                        s, true), "rk4 K1"));
     prof_mark(ctx, 0);
   }
@@ -1704,8 +1733,8 @@ static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* 
     WT_TRY(increments(SP[st % 2], st == 0 ? nullptr : ws->SQ));
     wt::NvtxRange nv(kNames[st]);
     prof_mark(ctx, 2);
-    WT_TRY(lrc(ctx, wt::launch_cons_fk_n8(m, coef->c, FB[st % 2], FB[(st + 1) % 2], SP[st % 2], ws->bbuf, b, rkQ(st),
-                                          rkP(st + 1), s), "rk4 fused stage"));
+    WT_TRY(lrc(ctx, wt::launch_cons_fk_n8(m, coef->c, FB[st % 2], FB[(st + 1) % 2],
+                                          phi_stage(ws, Phi, st + 1, cp).in, ws->bbuf, b, rkQ(st), rkP(st + 1), s), "rk4 fused stage"));
     prof_mark(ctx, 2);
     ctx->launches += 1;
   }
@@ -1894,11 +1923,7 @@ int wt_step_rk4_curved(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, v
   wt::ConsBC b;
   WT_TRY(make_bc(ctx, bc, use_metric, b));
   WT_TRY(ws_step_buffers(ws));
-  {  // the fused stages' second flux buffer (FP64 n = 8 whole-step calls only)
-    const wt::DevMesh& m = ws->mesh->m;
-    if (m.precision == WT_F64 && m.N == 8 && ws->fused && (eps_ko == 0.0 || ko_fused(m)))
-      WT_TRY(ensure(ws, &ws->F2, 3 * (size_t)wt::n8_padded_field_size(m.Ne) * sizeof(double)));
-  }
+  if (fused_form(ws, eps_ko) && ws->mesh->m.precision == WT_F64) WT_TRY(fused_buffer(ws));
   if (eps_ko != 0.0 && ko_fused(ws->mesh->m)) WT_TRY(ko_buffers(ws));
   if (eps_ko != 0.0) WT_TRY(ensure_mu(ws));
   if (coef->td) WT_TRY(need_setup_geometry(coef->mesh, "wt_step_rk4_curved (time-dependent background)"));

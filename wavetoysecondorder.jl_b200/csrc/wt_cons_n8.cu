@@ -9,7 +9,8 @@
 //     cores (mma.sync.m8n8k4.f64, G the A operand in registers, the staged field
 //     -- or the split-form product Ja u / Ja.F formed while loading -- the B
 //     operand); the two halves alone or fused;
-//   * FP32 on CUDA cores, plain and compensated (k_cons_k1_n8c, k_cons_k2_n8c);
+//   * FP32 on CUDA cores: compensated (k_cons_cc_n8, the halves alone or fused) and
+//     plain (k_cons_k1_n8c, k_cons_k2_n8c);
 //   * FP32 as split-precision BF16 on tensor cores (k_cons_k1_n8, k_cons_k2_n8).
 // The fields read at other nodes of an element (Phi and the nine metric terms in
 // K1; the three flux components and the metric terms in K2) are staged into
@@ -259,35 +260,6 @@ __device__ __forceinline__ void n8_rk(int stage, double dt, real k, real yin, re
   }
 }
 
-// RK4 stage update of the compensated FP32 form (Phi in K1, CP): the state is
-// the pair (y, lo) = (high, low part); the stage the next K1 reads is y + out
-// with out = lo + c dt k, so the stage value keeps the state's low part and
-// rounds only the small increment; acc holds the step increment; the step's
-// final sum is formed in FP64 and split again into y and lo.  Stage 2 also
-// copies y into hcopy, which stage 3 reads in place of y.  hi, accv, lov:
-// this node's y, acc and lo.
-__device__ __forceinline__ void n8_rk_cp(int stage, double dt, float k, float hi, float accv, float lov, long long n,
-                                         float* y, float* acc, float* out, float* lo, float* hcopy, unsigned* flag) {
-  if (stage == 0) {
-    out[n] = lov + (float)(0.5 * dt) * k;
-    acc[n] = (float)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = lov + (float)(0.5 * dt) * k;
-    acc[n] = accv + (float)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = lov + (float)dt * k;
-    acc[n] = accv + (float)(dt / 3.0) * k;
-    hcopy[n] = hi;
-  } else {
-    const float inc = accv + (float)(dt / 6.0) * k;
-    const double v = (double)hi + ((double)lov + (double)inc);
-    const float h = (float)v;
-    y[n] = h;
-    lo[n] = (float)(v - (double)h);
-    if (flag && !isfinite(h)) atomicOr(flag, 1u);
-  }
-}
-
 // ---------------------------------------------------------------------------
 template <typename real>
 struct K1N8 {
@@ -306,6 +278,7 @@ struct K1N8 {
   const int32_t* fsrc;
   const double* G;
   const double* H;
+  double inv2H;  // 1 / (2 H[0])
   real* F;
   real* Phidot;
   real* bbuf;
@@ -324,16 +297,16 @@ struct K1N8 {
   real* out;
   real* comp;
   unsigned* flag;
+  float2 Ge[16];  // 0.5 G in the sum/difference basis (cc_contract)
   float Gh[64];  // 0.5 G in FP32 (the CUDA-core form reads it from the constant bank)
   real* gout;    // gradient-only launches (GR): the three components of the split-form gradient
-  // Compensated FP32 form (cp = 1, CUDA-core kernels): the Phi the stage reads is
+  // Compensated FP32 form (k_cons_cc_n8): the Phi the stage reads is
   // Phi + Phit, with Phit the low part of the state at stage 0 and the previous
   // stage's small output after it (NULL: zero); the split-form gradient of it is
   // evaluated in FP64 with the metric terms split into an element-constant FP64
   // part Ja0 [9e + al*3 + c] and an FP32 deviation dJa (LayC blocks).
   // Stage 3 reads a copy of the state's high part that stage 2 writes (hcopy),
   // so that stage 3 may overwrite the state while neighbours still read it.
-  int cp;
   const real* Phit;
   const real* dJa;
   const double* Ja0;
@@ -344,17 +317,63 @@ struct K1N8 {
   int nko;
 };
 
-// Boundary terms of K1 at a node on an outer face (the curvilinear boundary
+// entry k of element e's boundary tags (k < 6) and slots
+__device__ __forceinline__ int face_entry(const int32_t* bdry, const int32_t* bslot, long long e, int k) {
+  return k < 6 ? bdry[6 * e + k] : bslot[6 * e + k - 6];
+}
+// the faces of an n = 8 element that node (ti, tj, tk) lies on
+__device__ __forceinline__ int node_faces(int ti, int tj, int tk) {
+  return (ti == 0 ? 1 : 0) | (ti == 7 ? 2 : 0) | (tj == 0 ? 4 : 0) | (tj == 7 ? 8 : 0) | (tk == 0 ? 16 : 0) |
+         (tk == 7 ? 32 : 0);
+}
+
+// Boundary terms of K1 at point (p, q) of an outer face (the curvilinear boundary
 // pass of src/boundaries3d.jl:131-232): characteristic SAT into phid and the
 // Pi boundary contribution into bbuf (read by K2).  cc: the ten coefficients.
 template <typename real>
-__device__ __forceinline__ void k1_boundary(const K1N8<real>& Q, long long e, int ti, int tj, int tk, long long n,
-                                            real u, real Pi, real g0, real g1, real g2, const real cc[10],
-                                            real& phid) {
+__device__ __forceinline__ void k1_boundary_face(const K1N8<real>& Q, int tag, int slot, int p, int q, long long n,
+                                                 real u, real Pi, real g0, real g1, real g2, const real cc[10],
+                                                 real& phid) {
   using n8::N2;
   const real a = cc[0];
   const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
   const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
+  real dF = 0, dP = 0;
+  if (tag != Q.exc_tag) {
+    const long long nb = (long long)Q.nbf * N2;
+    const long long bi = (long long)slot * N2 + p + 8 * q;
+    const real nx = Q.bnorm[bi], ny = Q.bnorm[nb + bi], nz = Q.bnorm[2 * nb + bi], wt = Q.bnorm[3 * nb + bi];
+    const real Kn =
+        K0 * nx * nx + K3 * ny * ny + K5 * nz * nz + (real)2 * (K1v * nx * ny + K2 * nx * nz + K4 * ny * nz);
+    const real a_n = sqrt(a * Kn);
+    const real bn_ = b0 * nx + b1 * ny + b2 * nz;
+    const real sigma = (real)Q.sigma;
+    if (Q.kind == 4) {
+      const real tau = sigma * (fabs(a_n - bn_) + fabs(a_n + bn_)) * wt;
+      const real gp = Q.gPhi ? Q.gPhi[n] : (real)0, gqv = Q.gPi ? Q.gPi[n] : (real)0;
+      dF = -tau * (u - gp);
+      dP = -tau * (Pi - gqv);
+    } else {
+      const real qv = nx * g0 + ny * g1 + nz * g2;
+      const real rr = Pi + ((bn_ + a_n) / a) * qv;
+      real gv = 0;
+      if (Q.kind != 2) {
+        const real gqv = Q.gPi ? Q.gPi[n] : (real)0;
+        const real gx = Q.gDx ? Q.gDx[n] : (real)0, gy = Q.gDy ? Q.gDy[n] : (real)0,
+                   gz = Q.gDz ? Q.gDz[n] : (real)0;
+        gv = gqv + ((bn_ + a_n) / a) * (nx * gx + ny * gy + nz * gz);
+      }
+      dP = -sigma * fabs(a_n + bn_) * wt * (rr - gv);
+    }
+  }
+  phid += dF;
+  Q.bbuf[(long long)slot * N2 + p + 8 * q] = dP;
+}
+// the same over the outer faces that node (ti, tj, tk) lies on
+template <typename real>
+__device__ __forceinline__ void k1_boundary(const K1N8<real>& Q, long long e, int ti, int tj, int tk, long long n,
+                                            real u, real Pi, real g0, real g1, real g2, const real cc[10],
+                                            real& phid) {
   const int idx3[3] = {ti, tj, tk};
   for (int f = 0; f < 6; ++f) {
     const int tag = Q.bdry[f + 6 * e];
@@ -362,37 +381,7 @@ __device__ __forceinline__ void k1_boundary(const K1N8<real>& Q, long long e, in
     const int ax = f >> 1;
     if (idx3[ax] != ((f & 1) ? 7 : 0)) continue;
     const int p = ax == 0 ? tj : ti, q = ax == 2 ? tj : tk;
-    const int slot = ::wt::bc_slot(Q.bslot[f + 6 * e], Q.nbf);
-    real dF = 0, dP = 0;
-    if (tag != Q.exc_tag) {
-      const long long nb = (long long)Q.nbf * N2;
-      const long long bi = (long long)slot * N2 + p + 8 * q;
-      const real nx = Q.bnorm[bi], ny = Q.bnorm[nb + bi], nz = Q.bnorm[2 * nb + bi], wt = Q.bnorm[3 * nb + bi];
-      const real Kn =
-          K0 * nx * nx + K3 * ny * ny + K5 * nz * nz + (real)2 * (K1v * nx * ny + K2 * nx * nz + K4 * ny * nz);
-      const real a_n = sqrt(a * Kn);
-      const real bn_ = b0 * nx + b1 * ny + b2 * nz;
-      const real sigma = (real)Q.sigma;
-      if (Q.kind == 4) {
-        const real tau = sigma * (fabs(a_n - bn_) + fabs(a_n + bn_)) * wt;
-        const real gp = Q.gPhi ? Q.gPhi[n] : (real)0, gqv = Q.gPi ? Q.gPi[n] : (real)0;
-        dF = -tau * (u - gp);
-        dP = -tau * (Pi - gqv);
-      } else {
-        const real qv = nx * g0 + ny * g1 + nz * g2;
-        const real rr = Pi + ((bn_ + a_n) / a) * qv;
-        real gv = 0;
-        if (Q.kind != 2) {
-          const real gqv = Q.gPi ? Q.gPi[n] : (real)0;
-          const real gx = Q.gDx ? Q.gDx[n] : (real)0, gy = Q.gDy ? Q.gDy[n] : (real)0,
-                     gz = Q.gDz ? Q.gDz[n] : (real)0;
-          gv = gqv + ((bn_ + a_n) / a) * (nx * gx + ny * gy + nz * gz);
-        }
-        dP = -sigma * fabs(a_n + bn_) * wt * (rr - gv);
-      }
-    }
-    phid += dF;
-    Q.bbuf[(long long)slot * N2 + p + 8 * q] = dP;
+    k1_boundary_face(Q, tag, ::wt::bc_slot(Q.bslot[f + 6 * e], Q.nbf), p, q, n, u, Pi, g0, g1, g2, cc, phid);
   }
 }
 
@@ -710,6 +699,7 @@ struct K2N8 {
   const int32_t* fsrc;
   const double* G;
   const double* H;
+  double inv2H;  // 1 / (2 H[0])
   const real* bbuf;
   int bc_on, nbf;
   real* Pidot;
@@ -720,8 +710,11 @@ struct K2N8 {
   real* out;
   real* comp;
   unsigned* flag;
+  const real* dJa;    // compensated FP32 form: Ja = Ja0 + dJa (see K1N8)
+  const double* Ja0;
   const real* ko;  // dissipation increments of Pidot (see K1N8)
   int nko;
+  float2 Ge[16];  // 0.5 G in the sum/difference basis (cc_contract)
   float Gh[64];
 };
 
@@ -1050,10 +1043,12 @@ __global__ void __launch_bounds__(n8::THREADS, n8::OCC)
 // before 1.34; K2 0.96 (16 words, 4.4 TB/s), before 1.01.  In a running step the
 // sum is 9 % longer.  What is left: waits on global loads (a third of the stalls),
 // fixed-latency tensor and FP64 chains, and the shared-memory pipe (61 % busy).
-struct FKN8 {
-  K2N8<double> a;  // stage s: F_s in (a.F0..F2), the Pi stage update
-  K1N8<double> b;  // stage s + 1: Phi_{s+1} in (b.Phi), F_{s+1} out (b.F), the Phi stage update
+template <typename real>
+struct FKT {
+  K2N8<real> a;  // stage s: F_s in (a.F0..F2), the Pi stage update
+  K1N8<real> b;  // stage s + 1: Phi_{s+1} in (b.Phi), F_{s+1} out (b.F), the Phi stage update
 };
+using FKN8 = FKT<double>;
 constexpr int FK_THREADS = 256;
 constexpr int FK_NFF = 6 * 3 * 64, FK_NFP = 6 * 64;  // flux / Phi face values
 // which halves a launch runs: K2 (divergence of F_s, Pi stage), K1 (gradient of Phi, flux, Phi
@@ -1374,9 +1369,6 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 4 : 0)
                : "memory");
 }
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 // index into a per-CTA table of the 6 x 64 face nodes for face source fs and
 // this face's point pq: the neighbour face's point after the orientation
 __device__ __forceinline__ int face_slot(int fs, int pq) {
@@ -1407,30 +1399,444 @@ __device__ __forceinline__ void contract8(const float* G, const float v[8], floa
 // each single-buffered and bulk-copied as soon as the pass that reads it is done,
 // so that three CTAs fit on an SM.
 constexpr size_t K1C_STAGE = 9 * (size_t)n8::LayC::FS;
-// node-pass buffer: c10 (10), Pi, invJ, [y], acc, comp -- the compensated form
-// reads the state's high part from the Phi pencils and holds no y
-template <bool CP>
-constexpr size_t k1c_b() { return (CP ? 14 : 15) * (size_t)n8::N3; }
+// node-pass buffer: c10 (10), Pi, invJ, y, acc, comp
+constexpr size_t K1C_B = 15 * (size_t)n8::N3;
 constexpr size_t K2C_STAGE = (size_t)K2_NF * n8::LayC::FS;
 constexpr int K1C_OCC = 3, K2C_OCC = 3;
 constexpr int K2C_NS = 2;  // K2c flux + Ja stages (one stage at four CTAs per SM leaves 80 registers: spills)
-template <bool CP = false>
 constexpr size_t k1c_smem() {
-  // CP adds one (single-buffered) copy of the small parts Phit: pencils and face traces
-  return (K1C_STAGE + k1c_b<CP>() + 9 * n8::LayC::FS + 2 * 6 * n8::N2 + 2 * n8::N3 +
-          (CP ? 6 * n8::N2 + n8::N3 : 0)) * sizeof(float) + 64;
+  return (K1C_STAGE + K1C_B + 9 * n8::LayC::FS + 2 * 6 * n8::N2 + 2 * n8::N3) * sizeof(float) + 64;
 }
 // per CTA: dynamic + static (a few words) + the 1 KB the SM reserves; 228 KB per SM
-static_assert(3 * (k1c_smem<true>() + 64 + 1024) <= 233472, "three compensated K1c CTAs must fit an SM");
+static_assert(3 * (k1c_smem() + 64 + 1024) <= 233472, "three K1c CTAs must fit an SM");
 // K2c node-pass fields (1/J and the RK state: invJ, y, acc, comp), one bulk-copied buffer
 constexpr size_t K2C_B = 4 * (size_t)n8::N3;
 constexpr size_t k2c_smem() {
   return (K2C_NS * K2C_STAGE + 3 * n8::LayC::FS + 2 * 6 * 3 * n8::N2 + K2C_B) * sizeof(float) + 64;
 }
 
-// CP: the compensated FP32 form (see K1N8::cp): Phi + Phit in FP64 through the
-// contractions, the RK4 epilogue of n8_rk_cp.
-template <bool BATCH, bool GR = false, bool CP = false>  // GR: gradient only (see k_cons_k1_n8)
+// ---------------------------------------------------------------------------
+// The compensated FP32 form (WT_FP32_COMPENSATED), n = 8: gradient
+// half, divergence half or both fused, as k_cons_fk_n8 does for FP64 (one launch
+// FK_s runs K2 of stage s and K1 of stage s + 1 of every element).
+//
+// The state u = Phi + Phit enters the derivative in FP64: FP32 rounding of it, or of
+// the contraction of it, would be amplified by the second derivative in Pi-dot.
+// With Ja = Ja0 + dJa (Ja0 element-constant, FP64):
+//   0.5 D(Ja u) + 0.5 Ja D u = (2 Ja0 + dJa) (0.5 D u) + 0.5 D(dJa u),
+// so the only contraction of u in FP32 acts on dJa u, which is as small as the
+// metric terms' variation over the element.  Once 0.5 D u has been formed in FP64
+// it is a gradient-sized value, and FP32 suffices for the rest.  The divergence
+// takes Ja = Ja0 + dJa, rounded to FP32 once.
+//
+// CTA: one element, 192 threads, one per (axis, pencil), CC_OCC CTAs per SM.  u is
+// formed once in shared memory in FP64 and 0.5 D u comes from the FP64 tensor cores
+// (a DFMA takes no constant operand); the FP32 contractions are packed FMAs in the
+// sum/difference basis (cc_contract).  As in the FP64 kernel an (axis, pencil) owns
+// its metric terms, so the gradient partials replace them in place, and the
+// divergence partials wait in registers until F is free.  Neighbour traces go
+// straight to the thread whose pencil ends on them; the node pass takes two nodes a
+// thread, and only a node on an outer face looks at the boundary tables.
+// Bound by issue (56%) and by the latency of the node words: 1950 instructions a
+// warp in the fused launch, which moves 35 words a node, 0.70 ms at 40^3 elements.
+// Measured (B200, 40^3 elements): RK4 step 6.44 -> 4.86 ms (two-kernel stages of this
+// template 5.36 ms), one right-hand side 1.39 -> 1.17 ms; 16^3: step 525 -> 374 us.
+// Four CTAs of 80 registers instead of five of 64: 5.33 against 5.04 ms; scalar FMAs
+// in this basis 4.97, in the plain basis 5.04, packed 4.92 ms, with a smaller error
+// of Pi against 64 bits (4.9-6.1e-7 after three steps, 5.7-6.3e-7 before); the loops
+// over the components unrolled (instruction cache) 5.17 ms.
+constexpr int CC_OCC = 5;
+constexpr size_t cc_smem(int half) {
+  return ((half & N8_K2 ? 3 * 512 + 6 * n8::CTHR : 0) + 9 * 512 + (half & N8_K1 ? 4 * 512 : 0)) * sizeof(float) +
+         (half & N8_K1 ? 512 * sizeof(double) : 0) + 16;
+}
+static_assert(CC_OCC * (cc_smem(N8_FK) + 128 + 1024) <= 233472, "CC_OCC fused CTAs must fit an SM");
+
+// out = 0.5 D v in the sum/difference basis: the operator is antisymmetric about its
+// centre (G[7-l][7-m] = -G[l][m]), so with e_m = v_m + v_{7-m}, d_m = v_m - v_{7-m}
+// (m < 4), p_l = sum_m A e, q_l = sum_m B d: out_l = q_l + p_l, out_{7-l} = q_l - p_l.
+// (p, q) is one packed FP32 pair: 16 packed FMAs and 16 additions instead of 64 FMAs.
+__device__ __forceinline__ void cc_contract(const float2* G, const float v[8], float out[8]) {
+  unsigned long long ed[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    const float e = v[m] + v[7 - m], d = v[m] - v[7 - m];
+    asm("mov.b64 %0, {%1, %2};" : "=l"(ed[m]) : "f"(e), "f"(d));
+  }
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    unsigned long long a;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(*reinterpret_cast<const unsigned long long*>(G + 4 * l)), "l"(ed[0]));
+#pragma unroll
+    for (int m = 1; m < 4; ++m)
+      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(*reinterpret_cast<const unsigned long long*>(G + 4 * l + m)), "l"(ed[m]));
+    float p, q;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(p), "=f"(q) : "l"(a));
+    out[l] = q + p;
+    out[7 - l] = q - p;
+  }
+}
+
+// RK4 weights of a stage: the increment to the next stage's value, and to the step's
+struct CCW {
+  float h, w;
+};
+__device__ __forceinline__ CCW cc_weights(int stage, double dt) {
+  return {(float)(stage == 2 ? dt : 0.5 * dt), (float)(stage == 0 || stage == 3 ? dt / 6.0 : dt / 3.0)};
+}
+__device__ __forceinline__ float2 cc_ld(const float* p, unsigned q) { return reinterpret_cast<const float2*>(p)[q]; }
+__device__ __forceinline__ void cc_st(float* p, unsigned q, float a, float b) {
+  reinterpret_cast<float2*>(p)[q] = make_float2(a, b);
+}
+
+template <int HALF, bool BATCH>
+__global__ void __launch_bounds__(n8::CTHR, CC_OCC)
+    k_cons_cc_n8(const __grid_constant__ FKT<float> P0, const K2N8<float>* plA, const K1N8<float>* plB,
+                 const int2* tiles) {
+  using namespace n8;
+  using LD = Lay<double>;
+  constexpr int FS = LayC::FS;
+  constexpr bool DIV = (HALF & N8_K2) != 0, GRAD = (HALF & N8_K1) != 0, FUSED = HALF == N8_FK;
+  extern __shared__ __align__(128) unsigned char smraw[];
+  float* sJa = reinterpret_cast<float*>(smraw);  // dJa, then the gradient partials [al * 3 + c] (LayC)
+  float* sF = sJa + 9 * FS;                      // F, then the divergence partials [al] (LayC)
+  float* sfn = sF + (DIV ? 3 * FS : 0);          // the flux across each thread's pencil ends [end * 3 + c][thread]
+  float* scu = sfn + (DIV ? 6 * CTHR : 0);       // 0.5 D_al u (LayC)
+  float* suf = scu + (GRAD ? 3 * FS : 0);        // u in FP32 (LayC)
+  double* su = reinterpret_cast<double*>(suf + (GRAD ? FS : 0));  // u (LD)
+  uint64_t* bar = reinterpret_cast<uint64_t*>(su + (GRAD ? N3 : 0));
+  __shared__ int abort_flag;
+  __shared__ float2 sm0[9];  // Ja0 = x + y
+  __shared__ int sbd[12];    // the faces' boundary tags and slots
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int al = tid >> 6, pc = tid & 63;  // axis (warp-uniform) and pencil
+  int sid = 0;
+  long long e;
+  if constexpr (BATCH) {
+    const int2 tl = tiles[blockIdx.x];
+    sid = tl.x;
+    e = tl.y;
+  } else {
+    e = (DIV ? P0.a.e0 : P0.b.e0) + blockIdx.x;
+  }
+  const K2N8<float>& A = BATCH && DIV ? plA[sid] : P0.a;
+  const K1N8<float>& B = BATCH && GRAD ? plB[sid] : P0.b;
+  const long long Ne = DIV ? A.Ne : B.Ne;
+  const long long eo = e * N3;  // this element's first node (and word of a LayC block)
+
+  if (warp == 0) {  // the copies of F (after dep_wait) and dJa
+    if (lane == 0) {
+      abort_flag = 0;
+      mbar_init(bar, 1);
+      fence_barrier_init();
+      fence_proxy_async();
+      mbar_expect_tx(bar, (unsigned)((DIV ? 12 : 9) * FS * sizeof(float)));
+    }
+    __syncwarp();
+    if (lane < 9)
+      bulk_g2s(sJa + lane * FS, (DIV ? A.dJa : B.dJa) + ((long long)lane * Ne + e) * FS, FS * (unsigned)sizeof(float),
+               bar);
+  } else if (warp == 5 && lane < 9) {
+    const double j = (DIV ? A.Ja0 : B.Ja0)[9 * e + lane];
+    sm0[lane] = make_float2((float)j, (float)(j - (double)(float)j));
+  }
+  if (tid >= 32 && tid < 44) sbd[tid - 32] = face_entry(DIV ? A.bdry : B.bdry, DIV ? A.bslot : B.bslot, e, tid - 32);
+  // the neighbours' nodes across this pencil's ends
+  long long nbo[2];  // their elements' first node
+  int nbn[2];        // the node; -1: no neighbour
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int src = ::wt::bc_src((DIV ? A.fsrc : B.fsrc)[2 * al + h + 6 * e], Ne);
+    nbo[h] = (long long)(src >> 6) * N3;
+    const int ax = (src & 7) >> 1;
+    const int a = (src & 32 ? pc >> 3 : pc & 7) ^ (src & 8 ? 7 : 0), b = (src & 32 ? pc & 7 : pc >> 3) ^ (src & 16 ? 7 : 0);
+    nbn[h] = src < 0 ? -1 : (a << (ax == 0 ? 3 : 0)) | (b << (ax == 2 ? 3 : 6)) | ((src & 1 ? 7 : 0) << (3 * ax));
+  }
+  const int em = (DIV ? A.emask : B.emask)[e];
+  const double inv2H = DIV ? A.inv2H : B.inv2H;
+  dep_wait();  // above: mesh tables and metric terms, which no launch of a step writes
+  if constexpr (DIV) {
+    if (warp == 0 && lane < 3)
+      bulk_g2s(sF + lane * FS, (lane == 0 ? A.F0 : lane == 1 ? A.F1 : A.F2) + eo, FS * (unsigned)sizeof(float), bar);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool ok = nbn[h] >= 0;
+      const long long at = ok ? nbo[h] + LayC::at(nbn[h]) : 0;
+      cp_async4(sfn + (3 * h + 0) * CTHR + tid, A.F0 + at, ok);
+      cp_async4(sfn + (3 * h + 1) * CTHR + tid, A.F1 + at, ok);
+      cp_async4(sfn + (3 * h + 2) * CTHR + tid, A.F2 + at, ok);
+    }
+  }
+  // threads < 128: nodes 2 q, 2 q + 1 for q = tid, tid + 128 (here and in the node pass)
+  float2 hi[2];  // the state's high part
+  double un[2] = {0, 0};
+  if constexpr (GRAD) {
+    if (tid < 128) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const unsigned q = tid + 128 * r;
+        hi[r] = cc_ld(B.Phi + eo, q);
+        const float2 lo = B.Phit ? cc_ld(B.Phit + eo, q) : make_float2(0.f, 0.f);
+        const double u0 = (double)hi[r].x + (double)lo.x, u1 = (double)hi[r].y + (double)lo.y;
+        const int d = LD::at(2 * q), s = LayC::at(2 * q);
+        su[d] = u0;
+        su[d ^ 1] = u1;
+        suf[s] = (float)u0;
+        suf[s ^ 1] = (float)u1;
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (nbn[h] >= 0) {
+        const long long n = nbo[h] + nbn[h];
+        un[h] = (double)B.Phi[n] + (B.Phit ? (double)B.Phit[n] : 0.0);
+      }
+  }
+  if constexpr (DIV) cp_async_wait_all();
+  if (tid == 0 && !wait_phase(bar, 0, DIV ? A.flag : B.flag)) abort_flag = 1;
+  __syncthreads();
+  if (abort_flag) {  // wait (bounded) for the copies in flight, then leave
+    if (tid == 0) wait_phase(bar, 0, nullptr);
+    return;
+  }
+
+  // Both layouts are linear over XOR (at(a + b) = at(a) ^ at(b) for a, b without
+  // common bits), so an address costs one or two XORs.
+  // ---- 0.5 D u on the FP64 tensor cores: four (axis, tile)s a warp ----
+  float j0 = 0, j1 = 0;
+  if constexpr (GRAD) {
+    const int gq = lane >> 2, tig = lane & 3, ax = warp >> 1;
+    const int sp = 3 * ax, sg = ax == 0 ? 6 : 0, sw = ax == 1 ? 6 : 3;  // bits: along the axis, pencil slot, tile
+    const double a0 = P0.b.Gd[gq * 8 + tig], a1 = P0.b.Gd[gq * 8 + 4 + tig];
+    const int t0 = (4 * (warp & 1)) << sw;
+    const int bi = LD::at((tig << sp) | (gq << sg) | t0), ik = LD::at(4 << sp), i1 = LD::at(1 << sw), i2 = LD::at(2 << sw);
+    const int bo = LayC::at((gq << sp) | ((2 * tig) << sg) | t0), ob = LayC::at(1 << sg), o1 = LayC::at(1 << sw),
+              o2 = LayC::at(2 << sw);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int in = bi ^ (q & 1 ? i1 : 0) ^ (q & 2 ? i2 : 0), on = bo ^ (q & 1 ? o1 : 0) ^ (q & 2 ? o2 : 0);
+      double d0 = 0, d1 = 0;
+      dmma(d0, d1, a0, su[in]);
+      dmma(d0, d1, a1, su[in ^ ik]);
+      scu[ax * FS + on] = (float)d0;
+      scu[ax * FS + (on ^ ob)] = (float)d1;
+    }
+    // centred-flux SAT of an interior al-face: jump on the face row (formed in FP64)
+    const int pd = LD::at(pnode(al, pc, 0)), p7 = LD::at(7 << (3 * al));
+    if (nbn[0] >= 0) j0 = (float)(-inv2H * (un[0] - su[pd]));
+    if (nbn[1] >= 0) j1 = (float)(inv2H * (un[1] - su[pd ^ p7]));
+  }
+  int addr[8];
+  {
+    const int s1 = LayC::at(1 << (3 * al)), s2 = LayC::at(2 << (3 * al)), s4 = LayC::at(4 << (3 * al));
+    addr[0] = LayC::at(pnode(al, pc, 0));
+    addr[1] = addr[0] ^ s1;
+    addr[2] = addr[0] ^ s2;
+    addr[3] = addr[1] ^ s2;
+#pragma unroll
+    for (int pos = 4; pos < 8; ++pos) addr[pos] = addr[pos - 4] ^ s4;
+  }
+  // ---- divergence of F along this pencil (K2 half) ----
+  float rs[8];
+  if constexpr (DIV) {
+    float w[8];
+    float s0 = 0, s1 = 0;
+#pragma unroll
+    for (int l = 0; l < 8; ++l) w[l] = rs[l] = 0;
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      const float* mc = sJa + (al * 3 + c) * FS;
+      const float2 m0 = sm0[al * 3 + c];
+      float F[8], m[8];
+#pragma unroll
+      for (int pos = 0; pos < 8; ++pos) {
+        F[pos] = sF[c * FS + addr[pos]];
+        m[pos] = m0.x + (m0.y + mc[addr[pos]]);
+        w[pos] = fmaf(m[pos], F[pos], w[pos]);
+      }
+      s0 = fmaf(m[0], sfn[c * CTHR + tid] - F[0], s0);
+      s1 = fmaf(m[7], sfn[(3 + c) * CTHR + tid] - F[7], s1);
+      float o[8];
+      cc_contract(P0.a.Ge, F, o);
+#pragma unroll
+      for (int l = 0; l < 8; ++l) rs[l] = fmaf(m[l], o[l], rs[l]);
+    }
+    {
+      float o[8];
+      cc_contract(P0.a.Ge, w, o);
+#pragma unroll
+      for (int l = 0; l < 8; ++l) rs[l] += o[l];
+    }
+    if (nbn[0] >= 0) rs[0] = fmaf(-(float)inv2H, s0, rs[0]);
+    if (nbn[1] >= 0) rs[7] = fmaf((float)inv2H, s1, rs[7]);
+  }
+  __syncthreads();  // 0.5 D u is complete, every thread is done with F
+  if constexpr (DIV) {
+#pragma unroll
+    for (int l = 0; l < 8; ++l) sF[al * FS + addr[l]] = rs[l];
+  }
+  // ---- split-form gradient of u along this pencil (K1 half), in place ----
+  if constexpr (GRAD) {
+    float cu[8], uf[8];
+#pragma unroll
+    for (int pos = 0; pos < 8; ++pos) {
+      cu[pos] = scu[al * FS + addr[pos]];
+      uf[pos] = suf[addr[pos]];
+    }
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+      float* mc = sJa + (al * 3 + c) * FS;
+      const float m0 = sm0[al * 3 + c].x;
+      float m[8], w[8];
+#pragma unroll
+      for (int pos = 0; pos < 8; ++pos) {
+        m[pos] = mc[addr[pos]];
+        w[pos] = m[pos] * uf[pos];
+      }
+      float o[8];
+      cc_contract(P0.b.Ge, w, o);  // 0.5 D(dJa u)
+#pragma unroll
+      for (int l = 0; l < 8; ++l) {
+        float r = fmaf(fmaf(2.f, m0, m[l]), cu[l], o[l]);
+        if (l == 0) r = fmaf(m0 + m[0], j0, r);
+        if (l == 7) r = fmaf(m0 + m[7], j1, r);
+        mc[addr[l]] = r;
+      }
+    }
+  }
+  __syncthreads();
+  // ---- node pass: two neighbouring nodes a thread, twice ----
+  if (tid >= 128) return;
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r) {
+    const unsigned q = tid + 128 * r;
+    const int w = 2 * q, at = LayC::at(w) & ~1;
+    const bool swp = (w >> 6) & 1;  // LayC exchanges the two
+    const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
+    auto pair = [&](const float* p) {  // p: three partials FS words apart from one another
+      const float2 a = *reinterpret_cast<const float2*>(p + at);
+      return a;
+    };
+    auto nat = [&](float2 v) { return swp ? make_float2(v.y, v.x) : v; };
+    // outer faces that nodes w and w + 1 lie on
+    const int out0 = (em >> 6) ? node_faces(ti, tj, tk) & ~em : 0, out1 = (em >> 6) ? node_faces(ti + 1, tj, tk) & ~em : 0;
+    const float2 iJ = cc_ld((DIV ? A.invdetJ : B.invdetJ) + eo, q);
+    float Pi[2] = {0, 0};
+    if constexpr (DIV) {
+      const float2 y = A.epi ? cc_ld(A.y + eo, q) : make_float2(0.f, 0.f);
+      const float2 ac = A.epi && A.stage >= 1 ? cc_ld(A.acc + eo, q) : make_float2(0.f, 0.f);
+      const float2 p0 = pair(sF), p1 = pair(sF + FS), p2 = pair(sF + 2 * FS);
+      const float2 sd = nat(make_float2((p0.x + p1.x) + p2.x, (p0.y + p1.y) + p2.y));
+      float dv[2] = {__fmul_rn(sd.x, iJ.x), __fmul_rn(sd.y, iJ.y)};  // the halves and the fused form round alike
+      if (A.bc_on) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          for (int b = x ? out1 : out0; b; b &= b - 1) {
+            const int f = __ffs(b) - 1, ax = f >> 1;
+            if (sbd[f] == 0) continue;
+            const int p = ax == 0 ? tj : ti + x, qq = ax == 2 ? tj : tk;
+            dv[x] += A.bbuf[(long long)::wt::bc_slot(sbd[6 + f], A.nbf) * N2 + p + 8 * qq];
+          }
+        }
+      }
+      if (FUSED || A.epi) {
+        // Kahan-compensated FP32 (as n8_rk): acc holds the step's increment
+        const CCW k = cc_weights(A.stage, A.dt);
+        const float a0 = fmaf(k.w, dv[0], ac.x), a1 = fmaf(k.w, dv[1], ac.y);
+        if (!FUSED && A.stage == 3) {
+          const float2 c = cc_ld(A.comp + eo, q);
+          const float t0 = a0 + c.x, t1 = a1 + c.y;
+          const float v0 = y.x + t0, v1 = y.y + t1;
+          cc_st(A.comp + eo, q, t0 - (v0 - y.x), t1 - (v1 - y.y));
+          cc_st(A.y + eo, q, v0, v1);
+          if (A.flag && !(isfinite(v0) && isfinite(v1))) atomicOr(A.flag, 1u);
+        } else {
+          cc_st(A.acc + eo, q, a0, a1);
+          Pi[0] = fmaf(k.h, dv[0], y.x);
+          Pi[1] = fmaf(k.h, dv[1], y.y);
+          if (!FUSED) cc_st(A.out + eo, q, Pi[0], Pi[1]);
+        }
+      } else {
+        cc_st(A.Pidot + eo, q, dv[0], dv[1]);
+      }
+    }
+    if constexpr (GRAD) {
+      if constexpr (!FUSED) {
+        const float2 v = cc_ld(B.Pi + eo, q);
+        Pi[0] = v.x;
+        Pi[1] = v.y;
+      }
+      float2 g[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float2 p0 = pair(sJa + c * FS), p1 = pair(sJa + (3 + c) * FS), p2 = pair(sJa + (6 + c) * FS);
+        g[c] = nat(make_float2((p0.x + p1.x) + p2.x, (p0.y + p1.y) + p2.y));
+        g[c].x *= iJ.x;
+        g[c].y *= iJ.y;
+      }
+      float2 cc[10];
+#pragma unroll
+      for (int c = 0; c < 10; ++c) cc[c] = cc_ld(B.c10 + c * B.nn + eo, q);
+      const float2 Pacc = B.epi && B.stage >= 1 ? cc_ld(B.acc + eo, q) : make_float2(0.f, 0.f);
+      const float2 Plo = B.epi ? cc_ld(B.comp + eo, q) : make_float2(0.f, 0.f);
+      float ph[2], F[3][2];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        auto el = [&](const float2& v) { return x ? v.y : v.x; };
+        const float g0 = el(g[0]), g1 = el(g[1]), g2 = el(g[2]);
+        const float b0 = el(cc[1]), b1 = el(cc[2]), b2 = el(cc[3]);
+        const float K1v = el(cc[5]), K2 = el(cc[6]), K4 = el(cc[8]);
+        F[0][x] = fmaf(b0, Pi[x], dot3(el(cc[4]), g0, K1v, g1, K2, g2));
+        F[1][x] = fmaf(b1, Pi[x], dot3(K1v, g0, el(cc[7]), g1, K4, g2));
+        F[2][x] = fmaf(b2, Pi[x], dot3(K2, g0, K4, g1, el(cc[9]), g2));
+        ph[x] = fmaf(el(cc[0]), Pi[x], dot3(b0, g0, b1, g1, b2, g2));
+        if (B.bc_on && (x ? out1 : out0)) {
+          float ce[10];
+#pragma unroll
+          for (int c = 0; c < 10; ++c) ce[c] = el(cc[c]);
+          // the whole stage value where a boundary term reads Phi itself
+          const float u = B.Phit ? el(hi[r]) + B.Phit[eo + w + x] : el(hi[r]);
+          for (int b = x ? out1 : out0; b; b &= b - 1) {
+            const int f = __ffs(b) - 1, ax = f >> 1;
+            if (sbd[f] == 0) continue;
+            const int p = ax == 0 ? tj : ti + x, qq = ax == 2 ? tj : tk;
+            k1_boundary_face<float>(B, sbd[f], ::wt::bc_slot(sbd[6 + f], B.nbf), p, qq, eo + w + x, u, Pi[x], g0, g1,
+                                    g2, ce, ph[x]);
+          }
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        *reinterpret_cast<float2*>(B.F + c * B.Ne * FS + eo + at) = nat(make_float2(F[c][0], F[c][1]));
+      if (FUSED || B.epi) {
+        // The state is the pair (y, lo) = (high, low part); the stage the next K1
+        // reads is y + out with out = lo + c dt k, so the stage value keeps the
+        // state's low part and rounds only the small increment; acc holds the step's
+        // increment; its final sum is formed in FP64 and split again into y and lo.
+        // Stage 2 also copies y into hcopy, which stage 3 reads in place of y.
+        const CCW k = cc_weights(B.stage, B.dt);
+        const float a0 = fmaf(k.w, ph[0], Pacc.x), a1 = fmaf(k.w, ph[1], Pacc.y);
+        if (B.stage == 3) {
+          const double v0 = (double)hi[r].x + ((double)Plo.x + (double)a0);
+          const double v1 = (double)hi[r].y + ((double)Plo.y + (double)a1);
+          const float h0 = (float)v0, h1 = (float)v1;
+          cc_st(B.y + eo, q, h0, h1);
+          cc_st(B.comp + eo, q, (float)(v0 - (double)h0), (float)(v1 - (double)h1));
+          if (B.flag && !(isfinite(h0) && isfinite(h1))) atomicOr(B.flag, 1u);
+        } else {
+          cc_st(B.acc + eo, q, a0, a1);
+          cc_st(B.out + eo, q, fmaf(k.h, ph[0], Plo.x), fmaf(k.h, ph[1], Plo.y));
+          if (B.stage == 2) cc_st(B.hcopy + eo, q, hi[r].x, hi[r].y);
+        }
+      } else {
+        cc_st(B.Phidot + eo, q, ph[0], ph[1]);
+      }
+    }
+  }
+}
+
+// The plain form of the gradient half (the compensated form: k_cons_cc_n8 above).
+template <bool BATCH, bool GR = false>  // GR: gradient only (see k_cons_k1_n8)
 __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
     k_cons_k1_n8c(const __grid_constant__ K1N8<float> P, const K1N8<float>* __restrict__ plist,
                   const int2* __restrict__ tiles, long long ntiles) {
@@ -1441,22 +1847,19 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
   constexpr int NFT = 6 * N2;                 // 384 neighbour Phi face values
   constexpr int NFR = (NFT + THR - 1) / THR;  // 2 per thread
   // node-pass buffer fields (sB)
-  constexpr int IY = 12, IACC = CP ? 12 : 13, ICOMP = CP ? 13 : 14;
+  constexpr int IY = 12, IACC = 13, ICOMP = 14;
   extern __shared__ __align__(128) unsigned char smraw[];
   real* sJa = reinterpret_cast<real*>(smraw);  // 9 fields (LayC), index al*3 + c
   real* sB = sJa + K1C_STAGE;                  // node order: c10 (10), Pi, invJ, [y], acc, comp
-  real* sg = sB + k1c_b<CP>();                 // 9 partial gradients [al*3 + c] (LayC)
+  real* sg = sB + K1C_B;                       // 9 partial gradients [al*3 + c] (LayC)
   real* sface = sg + 9 * FSC;                  // 2 x 384
   real* sphi = sface + 2 * NFT;                // 2 x 512 (LayC)
-  real* sfaceT = sphi + 2 * N3;                // CP: 384 small parts of the face traces
-  real* sphiT = sfaceT + (CP ? NFT : 0);       // CP: 512 small parts (LayC)
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sphiT + (CP ? N3 : 0));  // [0] Ja stage, [1] sB
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sphi + 2 * N3);  // [0] Ja stage, [1] sB
   __shared__ int abort_flag;
-  __shared__ __align__(16) double sJa0[2][9];  // CP: the element-constant metric part, double-buffered
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int al = tid >> 6, pc = tid & 63;  // contraction: axis (warp-uniform) and pencil
   // node of the neighbour's face-trace point for face source fs and this face's point pq
-  // (computed, not tabled: three compensated CTAs need the table's shared memory)
+  // (computed, not tabled: three CTAs need the table's shared memory)
   auto fnode = [](int fs, int pq) -> int {
     const int slot = face_slot(fs, pq);
     const int fn = slot >> 6;
@@ -1464,13 +1867,11 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
   };
   const real inv2H = (real)(1.0 / (2.0 * P.H[0]));
   const bool comp_on = P.epi && P.comp != nullptr;
-  // the compensated form reads the state's high part from the Phi pencils and the low part at every stage
-  const bool need_y = !CP && P.epi && (P.stage == 1 || P.stage == 2 || (comp_on && P.stage == 3));
+  const bool need_y = P.epi && (P.stage == 1 || P.stage == 2 || (comp_on && P.stage == 3));
   const bool need_acc = P.epi && P.stage >= 1;
-  const bool need_comp = comp_on && (CP || P.stage == 3);
+  const bool need_comp = comp_on && P.stage == 3;
   const unsigned txA = (unsigned)(K1C_STAGE * sizeof(real));
   const unsigned txB = (unsigned)((GR ? 1 : 12 + need_y + need_acc + need_comp) * N3 * sizeof(real));
-  const double inv2Hd = 1.0 / (2.0 * P.H[0]);
   const long long T = ntiles;
   const long long GS = gridDim.x;
   auto tile_at = [&](long long t) -> int2 {
@@ -1502,9 +1903,8 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
       mbar_expect_tx(&bar[0], txA);
     }
     __syncwarp();
-    const real* ja = CP ? Q.dJa : Q.Ja;
     if (lane < 9)
-      bulk_g2s(sJa + lane * FSC, ja + ((long long)lane * Q.Ne + tl.y) * FSC, FSC * (unsigned)sizeof(real), &bar[0]);
+      bulk_g2s(sJa + lane * FSC, Q.Ja + ((long long)lane * Q.Ne + tl.y) * FSC, FSC * (unsigned)sizeof(real), &bar[0]);
   };
   auto issueB = [&](int2 tl) {
     const K1N8<real>& Q = prm(tl.x);
@@ -1521,7 +1921,7 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
     } else if (lane < 10) src = Q.c10 + lane * Q.nn + o;
     else if (lane == 10) src = Q.Pi + o;
     else if (lane == 11) src = Q.invdetJ + o;
-    else if (lane == IY && !CP && need_y) src = Q.y + o;
+    else if (lane == IY && need_y) src = Q.y + o;
     else if (lane == IACC && need_acc) src = Q.acc + o;
     else if (lane == ICOMP && need_comp) src = Q.comp + o;
     if (src) bulk_g2s(sB + lane * N3, src, nb, &bar[1]);
@@ -1552,30 +1952,6 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
       const int node = tid + r * THR;
       if (node < N3) cp_async4(sphi + b * N3 + LayC::at(node), Q.Phi + (long long)tl.y * N3 + node, true);
     }
-    if constexpr (CP) {
-      if (tid < 9) cp_async8(&sJa0[b][tid], Q.Ja0 + 9 * (long long)tl.y + tid);
-    }
-  };
-  // CP: the small parts Phit of the same values into the single buffers sfaceT, sphiT
-  // (zero-filled where there is no neighbour or no Phit)
-  auto async_loadT = [&](int2 tl, const int src[NFR]) {
-    const K1N8<real>& Q = prm(tl.x);
-    const bool have = Q.Phit != nullptr;
-    const real* base = have ? Q.Phit : Q.Phi;
-#pragma unroll
-    for (int r = 0; r < NFR; ++r) {
-      const int idx = tid + r * THR;
-      if (idx < NFT) {
-        const bool ok = have && src[r] >= 0;
-        const real* g = ok ? base + (long long)(src[r] >> 6) * N3 + fnode(src[r], idx & 63) : base;
-        cp_async4(sfaceT + idx, g, ok);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < NPT; ++r) {
-      const int node = tid + r * THR;
-      if (node < N3) cp_async4(sphiT + LayC::at(node), base + (long long)tl.y * N3 + node, have);
-    }
   };
   auto emask_at = [&](int2 tl) -> int { return tl.x >= 0 ? prm(tl.x).emask[tl.y] : 0; };
 
@@ -1589,7 +1965,6 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
     int src0[NFR];
     src_load(t0, src0);
     async_load(t0, src0, 0);
-    if constexpr (CP) async_loadT(t0, src0);
     src_load(t1, src1);
     cp_async_wait_all();
   }
@@ -1624,57 +1999,7 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
     const int bnd = emcur >> 6;
     // ---- contractions: thread (al, pc); the operator in the constant bank is
     // 0.5 G (scaling by 1/2 is exact) ----
-    if constexpr (CP) {
-      // The state u = Phi + Phit enters the derivative in FP64: FP32 rounding of
-      // it, or of the contraction of it, would be amplified by the second
-      // derivative in Pi-dot.  With Ja = Ja0 + dJa (Ja0 element-constant, FP64):
-      //   0.5 D(Ja u) + 0.5 Ja D u = (2 Ja0 + dJa) (0.5 D u) + 0.5 D(dJa u),
-      // so the only contraction left in FP32 acts on dJa u, which is as small as
-      // the metric terms' variation over the element; its rounding error is that
-      // much smaller than the one of 0.5 D(Ja u) in FP32.  Once 0.5 D u has been
-      // formed in FP64 it is a gradient-sized value, and FP32 suffices for the rest.
-      const real* sPhiT = sphiT;
-      float cu[8], uf[8], jmp0, jmp1;
-      {
-        double u[8];
-#pragma unroll
-        for (int pos = 0; pos < 8; ++pos) u[pos] = (double)sPhi[addr[pos]] + (double)sPhiT[addr[pos]];
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-          double acc = P.Gd[l * 8] * u[0];
-#pragma unroll
-          for (int m = 1; m < 8; ++m) acc = fma(P.Gd[l * 8 + m], u[m], acc);
-          cu[l] = (float)acc;  // 0.5 D u
-        }
-        // centred-flux SAT of an interior al-face: jump on the face row (formed in FP64)
-        const bool sat0 = (mask >> (2 * al)) & 1, sat1 = (mask >> (2 * al + 1)) & 1;
-        const int f0 = (2 * al) * N2 + pc, f1 = (2 * al + 1) * N2 + pc;
-        jmp0 = sat0 ? (float)(-inv2Hd * (((double)sfc[f0] + (double)sfaceT[f0]) - u[0])) : 0.f;
-        jmp1 = sat1 ? (float)(inv2Hd * (((double)sfc[f1] + (double)sfaceT[f1]) - u[7])) : 0.f;
-#pragma unroll
-        for (int pos = 0; pos < 8; ++pos) uf[pos] = (float)u[pos];
-      }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const real* mc = sJa + (al * 3 + c) * FSC;
-        const float m0 = (float)sJa0[fb][al * 3 + c];
-        float w[8];
-#pragma unroll
-        for (int pos = 0; pos < 8; ++pos) w[pos] = mc[addr[pos]] * uf[pos];
-        real* gout = sg + (al * 3 + c) * FSC;
-#pragma unroll
-        for (int l = 0; l < 8; ++l) {
-          float o = P.Gh[l * 8] * w[0];
-#pragma unroll
-          for (int m = 1; m < 8; ++m) o = fmaf(P.Gh[l * 8 + m], w[m], o);  // 0.5 D(dJa u)
-          const float dl = mc[addr[l]];
-          float r = fmaf(2.f * m0 + dl, cu[l], o);
-          if (l == 0) r = fmaf(m0 + dl, jmp0, r);
-          if (l == 7) r = fmaf(m0 + dl, jmp1, r);
-          gout[addr[l]] = r;
-        }
-      }
-    } else {
+    {
       float u[8], cu[8], w[8], o[8];
 #pragma unroll
       for (int pos = 0; pos < 8; ++pos) u[pos] = sPhi[addr[pos]];
@@ -1707,9 +2032,6 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
     __syncthreads();  // partial gradients and sB complete; the Ja stage is free
     if (abort_flag) return;
     if (warp == 0 && has_next) issueA(t1);  // lands while the node pass runs
-    if constexpr (CP) {
-      if (has_next) async_loadT(t1, src1);  // the small parts are read by the contraction pass only
-    }
     // ---- node phase ----
 #pragma unroll
     for (int rr = 0; rr < NPT; ++rr) {
@@ -1718,7 +2040,7 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
       const int ti = node & 7, tj = (node >> 3) & 7, tk = node >> 6;
       const int at = LayC::at(node);
       const long long n = e * N3 + node;
-      const real u = sPhi[at];  // CP: the state's high part
+      const real u = sPhi[at];
       const real invJ = sB[11 * N3 + node];
       real g0 = (sg[at] + sg[3 * FSC + at]) + sg[6 * FSC + at];
       real g1 = (sg[FSC + at] + sg[4 * FSC + at]) + sg[7 * FSC + at];
@@ -1741,11 +2063,7 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
       const real F1 = b1 * Pi + (K1v * g0 + K3 * g1 + K4 * g2);
       const real F2 = b2 * Pi + (K2 * g0 + K4 * g1 + K5 * g2);
       real phid = b0 * g0 + b1 * g1 + b2 * g2 + a * Pi;
-      if (bnd && Q.bc_on) {
-        // the whole stage value where a boundary term reads Phi itself
-        const real uf = CP && Q.Phit ? u + Q.Phit[n] : u;
-        k1_boundary<real>(Q, e, ti, tj, tk, n, uf, Pi, g0, g1, g2, cc, phid);
-      }
+      if (bnd && Q.bc_on) k1_boundary<real>(Q, e, ti, tj, tk, n, u, Pi, g0, g1, g2, cc, phid);
       {  // flux in the LayC element-block layout read by K2
         const long long fo = e * FSC + at, fstr = Q.Ne * FSC;
         Q.F[fo] = F0;
@@ -1754,19 +2072,11 @@ __global__ void __launch_bounds__(n8::CTHR, K1C_OCC)
       }
       const real accv = need_acc ? sB[IACC * N3 + node] : (real)0;
       const real compv = need_comp ? sB[ICOMP * N3 + node] : (real)0;
-      if constexpr (CP) {
-        if (P.epi)
-          n8_rk_cp(P.stage, Q.dt, phid, u, accv, compv, n, Q.y, Q.acc, Q.out, Q.comp, Q.hcopy, P.flag);
-        else
-          Q.Phidot[n] = phid;
-      } else {
-        const real yv = need_y ? sB[IY * N3 + node] : (real)0;
-        if (P.epi)
-          n8_rk<real>(P.stage, Q.dt, phid, u, yv, accv, compv, n, Q.y, Q.acc, Q.out, comp_on ? Q.comp : nullptr,
-                      P.flag);
-        else
-          Q.Phidot[n] = phid;
-      }
+      const real yv = need_y ? sB[IY * N3 + node] : (real)0;
+      if (P.epi)
+        n8_rk<real>(P.stage, Q.dt, phid, u, yv, accv, compv, n, Q.y, Q.acc, Q.out, comp_on ? Q.comp : nullptr, P.flag);
+      else
+        Q.Phidot[n] = phid;
     }
     cp_async_wait_all();  // this thread's copies into buffers fb^1 (the barrier above the next element publishes them)
     emcur = emnext;
@@ -2105,6 +2415,7 @@ static K1N8<real> k1n8_params(const DevMesh& m, const DevCoef& c, const void* Ph
   P.Phi = (const real*)Phi; P.Pi = (const real*)Pi; P.c10 = (const real*)c.c10;
   P.Ja = (const real*)m.Ja_n8; P.invdetJ = (const real*)m.invdetJ_r;
   P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot; P.G = m.G; P.H = m.H;
+  P.inv2H = 1.0 / (2.0 * m.ops.H[0]);
   P.emask = m.emask; P.fsrc = m.fsrc;
   P.F = (real*)F; P.Phidot = (real*)Phidot; P.bbuf = (real*)bbuf;
   P.bc_on = bc.on; P.exc_tag = bc.exc_tag; P.nbf = m.nbf; P.kind = bc.kinds[0]; P.sigma = bc.sigma;
@@ -2114,8 +2425,12 @@ static K1N8<real> k1n8_params(const DevMesh& m, const DevCoef& c, const void* Ph
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.flag = flag;
   for (int i = 0; i < 64; ++i) P.Gh[i] = (float)(0.5 * m.ops.G[i]);
+  for (int l = 0; l < 4; ++l)
+    for (int q = 0; q < 4; ++q) {
+      const double a = m.ops.G[8 * l + q], b = m.ops.G[8 * l + 7 - q];
+      P.Ge[4 * l + q] = make_float2((float)(0.25 * (a + b)), (float)(0.25 * (a - b)));
+    }
   P.gout = nullptr;
-  P.cp = m.precision == WT_F32 && m.fp32_form == WT_FP32_COMPENSATED ? 1 : 0;
   P.Phit = (const real*)rk.phit;
   P.dJa = (const real*)m.dJa;
   P.Ja0 = m.Ja0;
@@ -2135,12 +2450,20 @@ static K2N8<real> k2n8_params(const DevMesh& m, const void* F, void* Pidot, cons
   P.F0 = (const real*)F; P.F1 = (const real*)F + fs; P.F2 = (const real*)F + 2 * fs;
   P.Ja = (const real*)m.Ja_n8; P.invdetJ = (const real*)m.invdetJ_r;
   P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot; P.G = m.G; P.H = m.H;
+  P.inv2H = 1.0 / (2.0 * m.ops.H[0]);
   P.emask = m.emask; P.fsrc = m.fsrc;
   P.bbuf = (const real*)bbuf; P.bc_on = bc.on; P.nbf = m.nbf;
   P.Pidot = (real*)Pidot;
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.flag = flag;
   for (int i = 0; i < 64; ++i) P.Gh[i] = (float)(0.5 * m.ops.G[i]);
+  for (int l = 0; l < 4; ++l)
+    for (int q = 0; q < 4; ++q) {
+      const double a = m.ops.G[8 * l + q], b = m.ops.G[8 * l + 7 - q];
+      P.Ge[4 * l + q] = make_float2((float)(0.25 * (a + b)), (float)(0.25 * (a - b)));
+    }
+  P.dJa = (const real*)m.dJa;
+  P.Ja0 = m.Ja0;
   P.ko = (const real*)rk.ko;
   P.nko = rk.nko;
   return P;
@@ -2195,7 +2518,7 @@ static int n8_launch(int which, const void* hP, const void* plist, const int2* t
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-template <bool BATCH, bool CP>
+template <bool BATCH>
 static int n8c_launch(int which, const void* hP, const void* plist, const int2* tiles, long long ntiles,
                       cudaStream_t s) {
   static bool attr1 = false, attr2 = false;
@@ -2203,18 +2526,18 @@ static int n8c_launch(int which, const void* hP, const void* plist, const int2* 
   const long long cap = (long long)sm_count() * occ;
   const long long grid = ntiles < cap ? ntiles : cap;
   if (which == 1) {
-    constexpr size_t smem = k1c_smem<CP>();
+    constexpr size_t smem = k1c_smem();
     if (!attr1) {
       // three CTAs per SM need (nearly) all of the SM's shared memory
-      if (cudaFuncSetAttribute(k_cons_k1_n8c<BATCH, false, CP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if (cudaFuncSetAttribute(k_cons_k1_n8c<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)smem) != cudaSuccess ||
-          cudaFuncSetAttribute(k_cons_k1_n8c<BATCH, false, CP>, cudaFuncAttributePreferredSharedMemoryCarveout,
+          cudaFuncSetAttribute(k_cons_k1_n8c<BATCH>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
         return -2;
       attr1 = true;
     }
     if (grid <= 0) return 0;
-    k_cons_k1_n8c<BATCH, false, CP><<<(unsigned)grid, n8::CTHR, smem, s>>>(
+    k_cons_k1_n8c<BATCH><<<(unsigned)grid, n8::CTHR, smem, s>>>(
         *(const K1N8<float>*)hP, (const K1N8<float>*)plist, tiles, ntiles);
   } else {
     if (!attr2) {
@@ -2232,6 +2555,31 @@ static int n8c_launch(int which, const void* hP, const void* plist, const int2* 
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+// the compensated FP32 kernels (see n8d_launch); a batch's launches, parallel
+// branches of a graph, do not gain from overlapping their predecessor
+template <int HALF, bool BATCH>
+static int cc_launch(const FKT<float>& P, const void* plA, const void* plB, const int2* tiles, long long ntiles,
+                     cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    if (cudaFuncSetAttribute(k_cons_cc_n8<HALF, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)cc_smem(HALF)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_cons_cc_n8<HALF, BATCH>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+      return -2;
+    attr = true;
+  }
+  if (ntiles <= 0) return 0;
+  if constexpr (BATCH) {
+    k_cons_cc_n8<HALF, BATCH><<<(unsigned)ntiles, n8::CTHR, cc_smem(HALF), s>>>(P, (const K2N8<float>*)plA,
+                                                                                (const K1N8<float>*)plB, tiles);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  } else {
+    return launch_dep(k_cons_cc_n8<HALF, BATCH>, (unsigned)ntiles, n8::CTHR, cc_smem(HALF), s, P,
+                      (const K2N8<float>*)plA, (const K1N8<float>*)plB, tiles);
+  }
+}
+
 template <bool BATCH>
 static int n8_dispatch(int which, int precision, int fp32_form, const void* hP, const void* plist, const int2* tiles,
                        long long ntiles, cudaStream_t s) {
@@ -2244,8 +2592,16 @@ static int n8_dispatch(int which, int precision, int fp32_form, const void* hP, 
     P.a = *(const K2N8<double>*)hP;
     return n8d_launch<N8_K2, BATCH>(P, plist, nullptr, tiles, ntiles, s);
   }
-  if (fp32_form == WT_FP32_COMPENSATED) return n8c_launch<BATCH, true>(which, hP, plist, tiles, ntiles, s);
-  if (fp32_form == WT_FP32_CUDA_CORES) return n8c_launch<BATCH, false>(which, hP, plist, tiles, ntiles, s);
+  if (fp32_form == WT_FP32_COMPENSATED) {
+    FKT<float> P;
+    if (which == 1) {
+      P.b = *(const K1N8<float>*)hP;
+      return cc_launch<N8_K1, BATCH>(P, nullptr, plist, tiles, ntiles, s);
+    }
+    P.a = *(const K2N8<float>*)hP;
+    return cc_launch<N8_K2, BATCH>(P, plist, nullptr, tiles, ntiles, s);
+  }
+  if (fp32_form == WT_FP32_CUDA_CORES) return n8c_launch<BATCH>(which, hP, plist, tiles, ntiles, s);
   if (fp32_form == WT_FP32_BF16X2) return n8_launch<float, 2, BATCH>(which, hP, plist, tiles, ntiles, s);
   return n8_launch<float, 3, BATCH>(which, hP, plist, tiles, ntiles, s);
 }
@@ -2266,8 +2622,14 @@ int launch_cons_k1_n8(const DevMesh& m, const DevCoef& c, const void* Phi, const
 
 int launch_cons_fk_n8(const DevMesh& m, const DevCoef& c, const void* Fin, void* Fout, const void* Phi, void* bbuf,
                       const ConsBC& bc, const RKStage& rkQ, const RKStage& rkP, cudaStream_t s) {
-  if (m.precision != 0 || rkQ.stage < 0 || rkQ.stage > 2 || rkP.stage != rkQ.stage + 1 || !rkQ.on || !rkP.on)
-    return -4;
+  if (rkQ.stage < 0 || rkQ.stage > 2 || rkP.stage != rkQ.stage + 1 || !rkQ.on || !rkP.on) return -4;
+  if (m.precision == 1) {
+    if (m.fp32_form != WT_FP32_COMPENSATED) return -4;
+    FKT<float> P;
+    P.a = k2n8_params<float>(m, Fin, nullptr, bbuf, bc, rkQ, m.errflag);
+    P.b = k1n8_params<float>(m, c, Phi, nullptr, Fout, nullptr, bbuf, bc, rkP, m.errflag);
+    return cc_launch<N8_FK, false>(P, nullptr, nullptr, nullptr, m.Ne, s);
+  }
   FKN8 P;
   P.a = k2n8_params<double>(m, Fin, nullptr, bbuf, bc, rkQ, m.errflag);
   P.b = k1n8_params<double>(m, c, Phi, nullptr, Fout, nullptr, bbuf, bc, rkP, m.errflag);
