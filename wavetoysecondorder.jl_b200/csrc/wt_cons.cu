@@ -104,15 +104,85 @@ __device__ __forceinline__ real contract(const real* __restrict__ f, const real*
   return s;
 }
 
-// The node pass of K1 at node n (element ec, node (i, j, k)): flux, Phidot,
-// boundary terms (into bbuf) and the RK4 stage update or Phidot.  g: the
-// gradient; u: the stage input (CP: its high part), ug: the value the gradient
-// differentiated; sd: the affine axis scales; a, b, K, Pi: the node's
-// coefficients and Pi.
-template <int N, typename real, bool CP, typename gt>
-__device__ __forceinline__ void k1_finish(const K1P<real>& P, long long ec, long long n, int i, int j, int k,
-                                          int emask, const real g[3], real u, gt ug, const real sd[3], real Hend,
-                                          real a, const real b[3], const real K[6], real Pi, real yv, real accv, real compv) {
+// the outer faces that node (i, j, k) lies on.  em: the element's emask
+template <int N>
+__device__ __forceinline__ int outer_faces(int em, int i, int j, int k) {
+  if (!(em >> 6)) return 0;
+  return ((i == 0 ? 1 : 0) | (i == N - 1 ? 2 : 0) | (j == 0 ? 4 : 0) | (j == N - 1 ? 8 : 0) | (k == 0 ? 16 : 0) |
+          (k == N - 1 ? 32 : 0)) & ~em;
+}
+
+// Boundary terms of K1 at point pq = p + N q (node n) of the element's outer face f:
+// the Pi part goes to the face's slot (read by K2), the Phi part is returned.  g: the
+// gradient; ug: the stage's Phi; sd: the face axis's affine scale; a, b, K, Pi: the
+// node's coefficients and Pi.
+template <int N, typename real, typename gt>
+__device__ __forceinline__ real k1_face(const K1P<real>& P, long long n, int f, int tag, int slot, int pq,
+                                        const real g[3], gt ug, real sd, real Hend, real a, const real b[3],
+                                        const real K[6], real Pi) {
+  constexpr int N2 = Ep<N>::N2;
+  const int ax = f >> 1;
+  real dF = 0, dP = 0;
+  if (!P.bc_curv) {
+    const int kind = P.kinds[f];
+    if (kind != 3) {
+      const real nh = (f & 1) ? (real)1 : (real)-1;
+      const real Kdd = ax == 0 ? K[0] : ax == 1 ? K[3] : K[5];
+      const real a_n = sqrt(a * Kdd);
+      const real bax = b[ax];
+      const real bn = nh * bax;
+      const real wt = sd / Hend;
+      if (kind == 4) {
+        const real tau = P.sigma * (fabs(a_n - bax) + fabs(a_n + bax)) * wt;
+        const real gp = P.gPhi ? P.gPhi[n] : (real)0, gq = P.gPi ? P.gPi[n] : (real)0;
+        dF = -tau * ((real)ug - gp);
+        dP = -tau * (Pi - gq);
+      } else {
+        const real qv = nh * g[ax];
+        const real r = Pi + ((bn + a_n) / a) * qv;
+        const real gv = kind == 2 ? (real)0 : (P.gPhi ? P.gPhi[n] : (real)0);
+        dP = -P.sigma * fabs(a_n + bn) * wt * (r - gv);
+      }
+    }
+  } else if (tag != P.exc_tag) {
+    const int kind = P.kinds[0];
+    const long long nb = (long long)P.nbf * N2;
+    const long long bi = (long long)slot * N2 + pq;
+    const real nx = P.bnorm[bi], ny = P.bnorm[nb + bi], nz = P.bnorm[2 * nb + bi], wt = P.bnorm[3 * nb + bi];
+    const real Kn = K[0] * nx * nx + K[3] * ny * ny + K[5] * nz * nz +
+                    (real)2 * (K[1] * nx * ny + K[2] * nx * nz + K[4] * ny * nz);
+    const real a_n = sqrt(a * Kn);
+    const real bn = b[0] * nx + b[1] * ny + b[2] * nz;
+    if (kind == 4) {
+      const real tau = P.sigma * (fabs(a_n - bn) + fabs(a_n + bn)) * wt;
+      const real gp = P.gPhi ? P.gPhi[n] : (real)0, gq = P.gPi ? P.gPi[n] : (real)0;
+      dF = -tau * ((real)ug - gp);
+      dP = -tau * (Pi - gq);
+    } else {
+      const real qv = nx * g[0] + ny * g[1] + nz * g[2];
+      const real r = Pi + ((bn + a_n) / a) * qv;
+      real gv = 0;
+      if (kind != 2) {
+        const real gq = P.gPi ? P.gPi[n] : (real)0;
+        const real gx = P.gDx ? P.gDx[n] : (real)0, gy = P.gDy ? P.gDy[n] : (real)0,
+                   gz = P.gDz ? P.gDz[n] : (real)0;
+        gv = gq + ((bn + a_n) / a) * (nx * gx + ny * gy + nz * gz);
+      }
+      dP = -P.sigma * fabs(a_n + bn) * wt * (r - gv);
+    }
+  }
+  P.bbuf[(long long)slot * N2 + pq] = dP;
+  return dF;
+}
+
+// The node pass of K1 at node n: flux, Phidot with its boundary increments (faces,
+// sdf: the outer faces it lies on and where their increments are; NULL: none) and the
+// RK4 stage update or Phidot.  g: the gradient; u: the stage input (CP: its high
+// part); a, b, K, Pi: the node's coefficients and Pi.
+template <int N, typename real, bool CP>
+__device__ __forceinline__ void k1_finish(const K1P<real>& P, long long n, int i, int j, int k, int emask,
+                                          const real* sdf, const real g[3], real u, real a, const real b[3],
+                                          const real K[6], real Pi, real yv, real accv, real compv) {
   constexpr int N2 = Ep<N>::N2;
   const long long nn = P.nn;
   // flux and Phidot
@@ -120,69 +190,11 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long ec, long
   const real F1 = b[1] * Pi + (K[1] * g[0] + K[3] * g[1] + K[4] * g[2]);
   const real F2 = b[2] * Pi + (K[2] * g[0] + K[4] * g[1] + K[5] * g[2]);
   real phid = b[0] * g[0] + b[1] * g[1] + b[2] * g[2] + a * Pi;
-  // boundary increments (per boundary face of the node; Pi parts go to the face slot)
-  if (P.bc_on && (emask >> 6)) {
-    const int idx3[3] = {i, j, k};
-    for (int f = 0; f < 6; ++f) {
-      const int tag = P.bdry[f + 6 * ec];
-      if (tag == 0) continue;
-      const int ax = f >> 1;
-      if (idx3[ax] != frow(f, N)) continue;
-      const int p = ax == 0 ? j : i, q = ax == 2 ? j : k;
-      const int slot = ::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf);
-      real dF = 0, dP = 0;
-      if (!P.bc_curv) {
-        const int kind = P.kinds[f];
-        if (kind != 3) {
-          const real nh = (f & 1) ? (real)1 : (real)-1;
-          const real Kdd = ax == 0 ? K[0] : ax == 1 ? K[3] : K[5];
-          const real a_n = sqrt(a * Kdd);
-          const real bax = b[ax];
-          const real bn = nh * bax;
-          const real wt = sd[ax] / Hend;
-          if (kind == 4) {
-            const real tau = P.sigma * (fabs(a_n - bax) + fabs(a_n + bax)) * wt;
-            const real gp = P.gPhi ? P.gPhi[n] : (real)0, gq = P.gPi ? P.gPi[n] : (real)0;
-            dF = -tau * ((real)ug - gp);
-            dP = -tau * (Pi - gq);
-          } else {
-            const real qv = nh * g[ax];
-            const real r = Pi + ((bn + a_n) / a) * qv;
-            const real gv = kind == 2 ? (real)0 : (P.gPhi ? P.gPhi[n] : (real)0);
-            dP = -P.sigma * fabs(a_n + bn) * wt * (r - gv);
-          }
-        }
-      } else if (tag != P.exc_tag) {
-        const int kind = P.kinds[0];
-        const long long nb = (long long)P.nbf * N2;
-        const long long bi = (long long)slot * N2 + p + N * q;
-        const real nx = P.bnorm[bi], ny = P.bnorm[nb + bi], nz = P.bnorm[2 * nb + bi], wt = P.bnorm[3 * nb + bi];
-        const real Kn = K[0] * nx * nx + K[3] * ny * ny + K[5] * nz * nz +
-                        (real)2 * (K[1] * nx * ny + K[2] * nx * nz + K[4] * ny * nz);
-        const real a_n = sqrt(a * Kn);
-        const real bn = b[0] * nx + b[1] * ny + b[2] * nz;
-        if (kind == 4) {
-          const real tau = P.sigma * (fabs(a_n - bn) + fabs(a_n + bn)) * wt;
-          const real gp = P.gPhi ? P.gPhi[n] : (real)0, gq = P.gPi ? P.gPi[n] : (real)0;
-          dF = -tau * ((real)ug - gp);
-          dP = -tau * (Pi - gq);
-        } else {
-          const real qv = nx * g[0] + ny * g[1] + nz * g[2];
-          const real r = Pi + ((bn + a_n) / a) * qv;
-          real gv = 0;
-          if (kind != 2) {
-            const real gq = P.gPi ? P.gPi[n] : (real)0;
-            const real gx = P.gDx ? P.gDx[n] : (real)0, gy = P.gDy ? P.gDy[n] : (real)0,
-                       gz = P.gDz ? P.gDz[n] : (real)0;
-            gv = gq + ((bn + a_n) / a) * (nx * gx + ny * gy + nz * gz);
-          }
-          dP = -P.sigma * fabs(a_n + bn) * wt * (r - gv);
-        }
-      }
-      phid += dF;
-      P.bbuf[(long long)slot * N2 + p + N * q] = dP;
+  if (sdf)
+    for (int fs = outer_faces<N>(emask, i, j, k); fs; fs &= fs - 1) {
+      const int f = __ffs(fs) - 1, fa = f >> 1;
+      phid += sdf[f * N2 + (fa == 0 ? j : i) + N * (fa == 2 ? j : k)];
     }
-  }
   for (int c = 0; c < P.nko; ++c) phid += P.ko[c * nn + n];
   P.F[n] = F0;
   P.F[nn + n] = F1;
@@ -213,7 +225,13 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long ec, long
 // 601; N = 7, 20^3 1581 -> 1003 / 1118 -> 579.  Fields that are read along pencils (Phi and the metric terms in
 // K1, F and the metric terms in K2) arrive by cp.async in a padded layout; axis
 // al's results replace its own metric terms there, pencil by pencil, and after one
-// barrier a node pass sums the three axes, in node order.
+// barrier a node pass sums the three axes, in node order.  Boundary terms are
+// evaluated by the threads whose pencils end on an outer face, all faces at once;
+// in the node pass the faces of a warp's nodes came one after another (a square root
+// and a division each), 2.5 us a launch.  Measured (B200), one RK4 step with the
+// terms in the node pass / by the pencil ends: N = 4, 8^3 elements FP64 52.7 -> 39.8
+// us, N = 7, 4^3 57.0 -> 42.3, N = 6, 8^3 61 -> 51; FP32 N = 4, 8^3 41.3 -> 33.1;
+// N = 7, 20^3 FP64 1045 -> 992, N = 5, 28^3 FP32 585 -> 544.
 //
 // BATCH: the CTA's elements come from a work list of (solve, element) tiles
 // and each tile reads the parameter block of its solve (plist); otherwise
@@ -280,17 +298,18 @@ constexpr int k1_words() {
 template <int N, typename real, bool CURV, bool BATCH, bool CP>
 __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
     k_cons_k1(const __grid_constant__ K1P<real> P0, const __grid_constant__ OpP<N, real> O,
-              const K1P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles, int epb) {
+              const K1P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles, int epb, int dfw) {
   using L = Pen<N>;
   using gt = typename std::conditional<CP, double, real>::type;  // precision of u and D u
   constexpr int N2 = L::N2, N3 = L::N3, TE = L::TE, NS = L::NS, P1 = L::P1;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int tid = threadIdx.x, le = tid / TE, t = tid - le * TE, ax = t / N2, pq = t - ax * N2, p = pq % N, q = pq / N;
-  real* sphi = reinterpret_cast<real*>(smraw) + (size_t)le * k1_words<N, real, CURV, CP>();
+  real* sphi = reinterpret_cast<real*>(smraw) + (size_t)le * (k1_words<N, real, CURV, CP>() + dfw);
   real* sphit = sphi + NS;               // CP
   real* sr = sphi + (CP ? 2 : 1) * NS;   // metric terms, then the axes' results
   constexpr bool PF = L::template pf1<real>();
   real* sw = sr + (CURV ? 9 : 3) * NS;   // the node pass's own words (PF)
+  real* sdf = sw + (PF ? 15 * N3 : 0);   // boundary increments of Phidot [face][pq] (dfw words)
   int sid;
   long long e;
   const bool valid = tile_element<BATCH>(P0, tiles, ntiles, epb, le, sid, e);
@@ -301,7 +320,7 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
   const bool pf_comp = P.epi && P.comp && (CP || P.stage == 3);
   real jh[2] = {0, 0};  // n jump / (2 H) at the two ends
   gt un[2] = {0, 0};
-  int src[2] = {-1, -1};
+  int src[2] = {-1, -1}, tag[2] = {0, 0}, emask = 0;
   real m0[3] = {0, 0, 0}, sd = 0;
   if (valid) {  // what no launch of a step writes: metric terms and tables
     if constexpr (CURV) {
@@ -315,7 +334,11 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
       }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+    for (int h = 0; h < 2; ++h) {
+      src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+      tag[h] = P.bdry[2 * ax + h + 6 * ec];
+    }
+    emask = P.emask[ec];
   }
   dep_wait();
   if (valid) {
@@ -420,16 +443,39 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
     }
   }
   __syncthreads();
+  const bool grad_only = P.c10 == nullptr;
+  // boundary terms, each thread those of its pencil's ends
+  if (valid && P.bc_on && (emask >> 6) && !grad_only) {
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      const int f = 2 * ax + h, l = h ? N - 1 : 0;
+      real dF = 0;
+      if ((h ? tag[1] : tag[0]) != 0) {
+        const int w = ax == 0 ? l + N * pq : ax == 1 ? p + N * (l + N * q) : pq + N2 * l, at = L::place(w);
+        const long long n = ec * N3 + w;
+        real b[3], K[6], g[3];
+        const real a = P.c10[n], Pi = P.Pi[n];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) b[c] = P.c10[(1 + c) * nn + n];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) K[c] = P.c10[(4 + c) * nn + n];
+        const real invJ = CURV ? P.invdetJ[n] : (real)1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          g[c] = CURV ? (sr[c * NS + at] + sr[(3 + c) * NS + at] + sr[(6 + c) * NS + at]) * invJ : sr[c * NS + at];
+        gt ug = sphi[at];
+        if constexpr (CP) {
+          if (P.Phit) ug += (gt)sphit[at];
+        }
+        dF = k1_face<N, real>(P, n, f, h ? tag[1] : tag[0], ::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf), pq, g, ug, sd,
+                              (real)P.H[0], a, b, K, Pi);
+      }
+      if (dfw) sdf[f * N2 + pq] = dF;
+    }
+  }
+  if (dfw) __syncthreads();
   if (!valid) return;
   cp_async_wait_own();
-  const bool grad_only = P.c10 == nullptr;
-  const int emask = P.emask[ec];
-  real sda[3] = {0, 0, 0};
-  if constexpr (!CURV) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) sda[d] = P.sdiag[3 * ec + d];
-  }
-  const real Hend = (real)P.H[0];
 #pragma unroll
   for (int it = 0; it < L::NI; ++it) {
     const int w = t + it * TE;
@@ -465,11 +511,8 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
     }
     if (grad_only) continue;
     const real u = sphi[at];  // CP: the high part
-    gt ug = u;
-    if constexpr (CP) {
-      if (P.Phit) ug += (gt)sphit[at];
-    }
-    k1_finish<N, real, CP>(P, ec, n, w % N, (w / N) % N, w / N2, emask, g, u, ug, sda, Hend, a, b, K, Pi, yv, accv, compv);
+    k1_finish<N, real, CP>(P, n, w % N, (w / N) % N, w / N2, emask, P.bc_on && dfw ? sdf : nullptr, g, u, a, b, K, Pi, yv,
+                           accv, compv);
   }
 }
 
@@ -508,7 +551,7 @@ struct K2P {
 // shared words of one element in K2: F and the nine metric terms / axis results
 template <int N, bool CURV>
 constexpr int k2_words() {
-  return Pen<N>::NS * (CURV ? 12 : 3) + 4 * Pen<N>::N3;
+  return Pen<N>::NS * (CURV ? 12 : 3) + 4 * Pen<N>::N3 + 6 * Pen<N>::N2;
 }
 
 template <int N, typename real, bool CURV, bool BATCH>
@@ -528,10 +571,11 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
   const long long ec = valid ? e : 0, nn = P.nn;
   const real* const Fp[3] = {P.F0, P.F1, P.F2};
   real* sw = sF + (CURV ? 12 : 3) * NS;  // the node pass's own words
+  real* sbb = sw + 4 * N3;               // the outer faces' boundary terms [face][pq]
   const bool pf_y = P.epi && (P.stage <= 2 || P.comp);
   const bool pf_acc = P.epi && P.stage >= 1;
   const bool pf_comp = P.epi && P.comp && P.stage == 3;
-  int src[2] = {-1, -1};
+  int src[2] = {-1, -1}, slot[2] = {-1, -1}, emask = 0;
   real fn[2][CURV ? 3 : 1] = {}, sd = 0;
   if (valid) {  // what no launch of a step writes: metric terms and tables
     if constexpr (CURV) {
@@ -544,7 +588,11 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
       }
     }
 #pragma unroll
-    for (int h = 0; h < 2; ++h) src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+    for (int h = 0; h < 2; ++h) {
+      src[h] = ::wt::bc_src(P.fsrc[2 * ax + h + 6 * ec], P.Ne);
+      if (P.bc_on && P.bdry[2 * ax + h + 6 * ec] != 0) slot[h] = ::wt::bc_slot(P.bslot[2 * ax + h + 6 * ec], P.nbf);
+    }
+    if (P.bc_on) emask = P.emask[ec];
   }
   dep_wait();
   if (valid) {
@@ -554,6 +602,13 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
       if (N3 % TE != 0 && w >= N3) break;
 #pragma unroll
       for (int c = 0; c < 3; ++c) cp_async_word(sF + c * NS + L::place(w), Fp[c] + ec * N3 + w);
+    }
+    if (emask >> 6) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (slot[h] >= 0) cp_async_word(sbb + (2 * ax + h) * N2 + pq, P.bbuf + (long long)slot[h] * N2 + pq);
+        else sbb[(2 * ax + h) * N2 + pq] = 0;
+      }
     }
     cp_async_commit();
 #pragma unroll
@@ -640,7 +695,6 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
   __syncthreads();
   if (!valid) return;
   cp_async_wait_own();
-  const int emask = P.emask[ec];
 #pragma unroll
   for (int it = 0; it < L::NI; ++it) {
     const int w = t + it * TE;
@@ -650,14 +704,11 @@ __global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
     real dv;
     if constexpr (CURV) dv = (sJ[at] + sJ[3 * NS + at] + sJ[6 * NS + at]) * sw[w];
     else dv = sF[at] + sF[NS + at] + sF[2 * NS + at];
-    if (P.bc_on && (emask >> 6)) {
-      const int idx3[3] = {w % N, (w / N) % N, w / N2};
-      for (int f = 0; f < 6; ++f) {
-        if (P.bdry[f + 6 * ec] == 0) continue;
-        const int fa = f >> 1;
-        if (idx3[fa] != frow(f, N)) continue;
-        const int fp = fa == 0 ? idx3[1] : idx3[0], fq = fa == 2 ? idx3[1] : idx3[2];
-        dv += P.bbuf[(long long)::wt::bc_slot(P.bslot[f + 6 * ec], P.nbf) * N2 + fp + N * fq];
+    if (emask >> 6) {
+      const int i = w % N, j = (w / N) % N, k = w / N2;
+      for (int fs = outer_faces<N>(emask, i, j, k); fs; fs &= fs - 1) {
+        const int f = __ffs(fs) - 1, fa = f >> 1;
+        dv += sbb[f * N2 + (fa == 0 ? j : i) + N * (fa == 2 ? j : k)];
       }
     }
     for (int c = 0; c < P.nko; ++c) dv += P.ko[c * nn + n];
@@ -795,15 +846,25 @@ static int gen_smem(K kernel, size_t smem) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess ? 0 : -2;
 }
 
+// whether boundary terms of K1 reach Phidot
+template <typename real>
+static bool k1_phi_increments(const K1P<real>& P) {
+  for (int f = 0; f < 6; ++f)
+    if (P.kinds[f] == 4) return true;
+  return false;
+}
+
 template <int N, typename real, bool CURV, bool BATCH, bool CP>
 static int k1_run(const K1P<real>& P, const OpP<N, real>& O, const void* plist, const int2* tiles, long long ne,
                   int variant, cudaStream_t s) {
   if (ne <= 0) return 0;
   const int epb = elements_per_cta<N>(ne, variant);
-  const size_t smem = (size_t)epb * k1_words<N, real, CURV, CP>() * sizeof(real);
+  // room for the boundary increments of Phidot where there can be any (full-Dirichlet faces)
+  const int dfw = BATCH || (P.bc_on && k1_phi_increments(P)) ? 6 * Pen<N>::N2 : 0;
+  const size_t smem = (size_t)epb * (k1_words<N, real, CURV, CP>() + dfw) * sizeof(real);
   if (gen_smem(k_cons_k1<N, real, CURV, BATCH, CP>, smem)) return -2;
   return launch_dep(k_cons_k1<N, real, CURV, BATCH, CP>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P,
-                    O, (const K1P<real>*)plist, tiles, ne, epb);
+                    O, (const K1P<real>*)plist, tiles, ne, epb, dfw);
 }
 
 template <int N, typename real, bool CURV, bool BATCH>
