@@ -863,7 +863,7 @@ static int k1_run(const K1P<real>& P, const OpP<N, real>& O, const void* plist, 
   const int dfw = BATCH || (P.bc_on && k1_phi_increments(P)) ? 6 * Pen<N>::N2 : 0;
   const size_t smem = (size_t)epb * (k1_words<N, real, CURV, CP>() + dfw) * sizeof(real);
   if (gen_smem(k_cons_k1<N, real, CURV, BATCH, CP>, smem)) return -2;
-  return launch_dep(k_cons_k1<N, real, CURV, BATCH, CP>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P,
+  return launch_dep<!BATCH>(k_cons_k1<N, real, CURV, BATCH, CP>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P,
                     O, (const K1P<real>*)plist, tiles, ne, epb, dfw);
 }
 
@@ -874,7 +874,7 @@ static int k2_run(const K2P<real>& P, const OpP<N, real>& O, const void* plist, 
   const int epb = elements_per_cta<N>(ne, variant);
   const size_t smem = (size_t)epb * k2_words<N, CURV>() * sizeof(real);
   if (gen_smem(k_cons_k2<N, real, CURV, BATCH>, smem)) return -2;
-  return launch_dep(k_cons_k2<N, real, CURV, BATCH>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P, O,
+  return launch_dep<!BATCH>(k_cons_k2<N, real, CURV, BATCH>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P, O,
                     (const K2P<real>*)plist, tiles, ne, epb);
 }
 

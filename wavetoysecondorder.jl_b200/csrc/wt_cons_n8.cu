@@ -2481,7 +2481,7 @@ static int n8d_launch(const FKN8& P, const void* plA, const void* plB, const int
     attr = true;
   }
   if (ntiles <= 0) return 0;
-  return launch_dep(k_cons_fk_n8<HALF, BATCH>, (unsigned)ntiles, FK_THREADS, fk_smem(HALF), s, P,
+  return launch_dep<!BATCH>(k_cons_fk_n8<HALF, BATCH>, (unsigned)ntiles, FK_THREADS, fk_smem(HALF), s, P,
                     (const K2N8<double>*)plA, (const K1N8<double>*)plB, tiles);
 }
 
@@ -2555,8 +2555,7 @@ static int n8c_launch(int which, const void* hP, const void* plist, const int2* 
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// the compensated FP32 kernels (see n8d_launch); a batch's launches, parallel
-// branches of a graph, do not gain from overlapping their predecessor
+// the compensated FP32 kernels (see n8d_launch)
 template <int HALF, bool BATCH>
 static int cc_launch(const FKT<float>& P, const void* plA, const void* plB, const int2* tiles, long long ntiles,
                      cudaStream_t s) {
@@ -2570,14 +2569,8 @@ static int cc_launch(const FKT<float>& P, const void* plA, const void* plB, cons
     attr = true;
   }
   if (ntiles <= 0) return 0;
-  if constexpr (BATCH) {
-    k_cons_cc_n8<HALF, BATCH><<<(unsigned)ntiles, n8::CTHR, cc_smem(HALF), s>>>(P, (const K2N8<float>*)plA,
-                                                                                (const K1N8<float>*)plB, tiles);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  } else {
-    return launch_dep(k_cons_cc_n8<HALF, BATCH>, (unsigned)ntiles, n8::CTHR, cc_smem(HALF), s, P,
-                      (const K2N8<float>*)plA, (const K1N8<float>*)plB, tiles);
-  }
+  return launch_dep<!BATCH>(k_cons_cc_n8<HALF, BATCH>, (unsigned)ntiles, n8::CTHR, cc_smem(HALF), s, P,
+                            (const K2N8<float>*)plA, (const K1N8<float>*)plB, tiles);
 }
 
 template <bool BATCH>

@@ -25,7 +25,10 @@ __device__ __forceinline__ void dep_wait() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-template <typename... P, typename... A>
+// The launches of a batch, parallel branches of one graph, gain nothing from it (an
+// FP32 batch of 24 small solves 748 us a call so, 703 us with ordinary launches): DEP
+// = false launches the ordinary way.
+template <bool DEP = true, typename... P, typename... A>
 int launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... a) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -36,7 +39,7 @@ int launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStr
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = DEP ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, P(a)...) == cudaSuccess ? 0 : -2;
 }
 
