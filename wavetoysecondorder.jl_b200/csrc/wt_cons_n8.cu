@@ -157,6 +157,12 @@ struct Lay<float> {
 __device__ __forceinline__ int bn(int al, int w, int p, int g) {
   return al == 0 ? p + 8 * w + 64 * g : al == 1 ? g + 8 * p + 64 * w : g + 8 * w + 64 * p;
 }
+// node at position pos of pencil pc along axis al; pc = a + 8 b numbers the
+// other two axes in increasing order, so it is also the pencil's face index
+__device__ __forceinline__ int pnode(int al, int pc, int pos) {
+  const int a = pc & 7, b = pc >> 3;
+  return al == 0 ? pos + 8 * a + 64 * b : al == 1 ? a + 8 * pos + 64 * b : a + 8 * b + 64 * pos;
+}
 // FP64 B operand: position p = 4 kc + tig along al, pencil slot g
 __device__ __forceinline__ int bnode(int al, int w, int kc, int g, int tig) { return bn(al, w, 4 * kc + tig, g); }
 // outputs (both forms): row l = g along al, pencil slot 2 tig + b
@@ -317,10 +323,6 @@ struct K1N8 {
   int nko;
 };
 
-// entry k of element e's boundary tags (k < 6) and slots
-__device__ __forceinline__ int face_entry(const int32_t* bdry, const int32_t* bslot, long long e, int k) {
-  return k < 6 ? bdry[6 * e + k] : bslot[6 * e + k - 6];
-}
 // the faces of an n = 8 element that node (ti, tj, tk) lies on
 __device__ __forceinline__ int node_faces(int ti, int tj, int tk) {
   return (ti == 0 ? 1 : 0) | (ti == 7 ? 2 : 0) | (tj == 0 ? 4 : 0) | (tj == 7 ? 8 : 0) | (tk == 0 ? 16 : 0) |
@@ -1140,11 +1142,15 @@ __global__ void __launch_bounds__(FK_THREADS, 3)
     __syncwarp();
     if (lane < 9) bulk_g2s(sJa + lane * FS, Ja + ((long long)lane * Ne + e) * FS, FS * (unsigned)sizeof(real), bar);
   }
-  int fsrc[2];
+  int fsrc[2], slot[2] = {-1, -1};
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const int idx = tid + r * FK_THREADS;
     fsrc[r] = idx < FK_NFP ? ::wt::bc_src(fsrcs[(idx >> 6) + 6 * e], Ne) : -1;
+    if constexpr (DIV) {
+      if (idx < FK_NFP && A.bc_on && A.bdry[(idx >> 6) + 6 * e] != 0)
+        slot[r] = ::wt::bc_slot(A.bslot[(idx >> 6) + 6 * e], A.nbf);
+    }
   }
   const int em = (DIV ? A.emask : B.emask)[e], mask = em & 63, bnd = em >> 6;
   const double aG0 = Gm[gq * 8 + tig], aG1 = Gm[gq * 8 + 4 + tig];
@@ -1172,7 +1178,9 @@ __global__ void __launch_bounds__(FK_THREADS, 3)
       if constexpr (DIV) {
         const long long at = b + Lay<real>::at(nd);
         double* d = sfF + f * 3 * N2 + pq;
-        cp_async8z(d, A.F0 + at, src >= 0);
+        // an outer face, without a trace, has its boundary terms in the first component's place
+        const double* d0 = slot[r] >= 0 ? A.bbuf + (long long)slot[r] * N2 + pq : A.F0 + at;
+        cp_async8z(d, d0, src >= 0 || slot[r] >= 0);
         cp_async8z(d + N2, A.F1 + at, src >= 0);
         cp_async8z(d + 2 * N2, A.F2 + at, src >= 0);
       }
@@ -1269,32 +1277,27 @@ __global__ void __launch_bounds__(FK_THREADS, 3)
       for (int b = 0; b < 2; ++b) sF[al * FS + Lay<real>::at(onode(al, warp, b, gq, tig))] = rs[al][b];
   }
   __syncthreads();
+  real Pi[2] = {0, 0};
+  if constexpr (DIV) {
+    // ---- divergence node pass: boundary terms, Pi stage update (K2 half) ----
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int w = tid + r * FK_THREADS, tp = Lay<real>::at(w);
-    const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
-    const long long n = e * N3 + w;
-    const real invJ = (DIV ? A.invdetJ : B.invdetJ)[n];
-    real Pi = 0;
-    if constexpr (DIV) {
-      // ---- divergence node pass: boundary terms, Pi stage update (K2 half) ----
+    for (int r = 0; r < 2; ++r) {
+      const int w = tid + r * FK_THREADS, tp = Lay<real>::at(w);
+      const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
+      const long long n = e * N3 + w;
       const bool need_y = A.epi && A.stage <= 2, need_acc = A.epi && A.stage >= 1;
       const real Qy = need_y ? A.y[n] : (real)0, Qacc = need_acc ? A.acc[n] : (real)0;
       real dv = (sF[tp] + sF[FS + tp]) + sF[2 * FS + tp];
-      dv *= invJ;
-      if (bnd && A.bc_on) {
-        const int idx3[3] = {ti, tj, tk};
-        for (int f = 0; f < 6; ++f) {
-          if (A.bdry[f + 6 * e] == 0) continue;
-          const int ax = f >> 1;
-          if (idx3[ax] != ((f & 1) ? 7 : 0)) continue;
-          const int p = ax == 0 ? tj : ti, q = ax == 2 ? tj : tk;
-          dv += A.bbuf[(long long)::wt::bc_slot(A.bslot[f + 6 * e], A.nbf) * N2 + p + 8 * q];
+      dv *= A.invdetJ[n];
+      if (bnd && A.bc_on)
+        for (int b = node_faces(ti, tj, tk) & ~mask; b; b &= b - 1) {
+          const int f = __ffs(b) - 1, ax = f >> 1;
+          dv += sfF[f * 3 * N2 + (ax == 0 ? tj : ti) + 8 * (ax == 2 ? tj : tk)];
         }
-      }
       for (int c = 0; c < A.nko; ++c) dv += A.ko[c * A.nn + n];
       if constexpr (FUSED) {
-        Pi = n8_rk_out(A.stage, A.dt, dv, Qy, Qacc, n, A.acc, A.out);  // Pi_{s+1}
+        Pi[r] = n8_rk_out(A.stage, A.dt, dv, Qy, Qacc, n, A.acc, A.out);  // Pi_{s+1}
+        if (bnd && B.bc_on) sF[tp] = Pi[r];
       } else {
         if (A.epi)
           n8_rk<real>(A.stage, A.dt, dv, Qy, Qy, Qacc, (real)0, n, A.y, A.acc, A.out, nullptr, A.flag);
@@ -1302,8 +1305,42 @@ __global__ void __launch_bounds__(FK_THREADS, 3)
           A.Pidot[n] = dv;
       }
     }
-    if constexpr (GRAD) {
-      // ---- gradient node pass: flux, Phidot, boundary terms, Phi stage update (K1 half) ----
+  }
+  // ---- boundary terms of the gradient half, a thread per point of an outer face: all
+  // faces at once (see k_cons_k1 in wt_cons.cu); increments of Phidot into sfP ----
+  if constexpr (GRAD && HALF != N8_GRAD) {
+    if (bnd && B.bc_on) {  // the same for the whole CTA
+      if constexpr (FUSED) __syncthreads();  // Pi is complete, every thread has read its boundary terms
+#pragma unroll 1
+      for (int idx = tid; idx < FK_NFP; idx += FK_THREADS) {
+        const int f = idx >> 6, tag = B.bdry[f + 6 * e];
+        real dF = 0;
+        if (tag != 0) {
+          const int ax = f >> 1, w = pnode(ax, idx & 63, f & 1 ? 7 : 0), tp = Lay<real>::at(w);
+          const long long n = e * N3 + w;
+          real cc[10];
+#pragma unroll
+          for (int c = 0; c < 10; ++c) cc[c] = B.c10[c * B.nn + n];
+          const real P1 = FUSED ? sF[tp] : B.Pi[n], invJ = B.invdetJ[n];
+          const real g0 = ((sJa[tp] + sJa[3 * FS + tp]) + sJa[6 * FS + tp]) * invJ;
+          const real g1 = ((sJa[FS + tp] + sJa[4 * FS + tp]) + sJa[7 * FS + tp]) * invJ;
+          const real g2 = ((sJa[2 * FS + tp] + sJa[5 * FS + tp]) + sJa[8 * FS + tp]) * invJ;
+          k1_boundary_face<real>(B, tag, ::wt::bc_slot(B.bslot[f + 6 * e], B.nbf), idx & 7, (idx >> 3) & 7, n, sphi[tp],
+                                 P1, g0, g1, g2, cc, dF);
+        }
+        sfP[idx] = dF;
+      }
+      __syncthreads();
+    }
+  }
+  if constexpr (GRAD) {
+    // ---- gradient node pass: flux, Phidot, Phi stage update (K1 half) ----
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int w = tid + r * FK_THREADS, tp = Lay<real>::at(w);
+      const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
+      const long long n = e * N3 + w;
+      const real invJ = B.invdetJ[n];
       const real u = sphi[tp];
       real g0 = (sJa[tp] + sJa[3 * FS + tp]) + sJa[6 * FS + tp];
       real g1 = (sJa[FS + tp] + sJa[4 * FS + tp]) + sJa[7 * FS + tp];
@@ -1317,18 +1354,22 @@ __global__ void __launch_bounds__(FK_THREADS, 3)
         real cc[10];
 #pragma unroll
         for (int c = 0; c < 10; ++c) cc[c] = B.c10[c * B.nn + n];
-        if constexpr (!FUSED) Pi = B.Pi[n];
+        if constexpr (!FUSED) Pi[r] = B.Pi[n];
         const bool need_y = B.epi && (B.stage == 1 || B.stage == 2), need_acc = B.epi && B.stage >= 1;
         const real Py = need_y ? B.y[n] : (real)0, Pacc = need_acc ? B.acc[n] : (real)0;
         const real a = cc[0];
         const real b0 = cc[1], b1 = cc[2], b2 = cc[3];
         const real K0 = cc[4], K1v = cc[5], K2 = cc[6], K3 = cc[7], K4 = cc[8], K5 = cc[9];
         // the roundings written out: the same bits in every instantiation
-        const real F0 = fma(b0, Pi, dot3(K0, g0, K1v, g1, K2, g2));
-        const real F1 = fma(b1, Pi, dot3(K1v, g0, K3, g1, K4, g2));
-        const real F2 = fma(b2, Pi, dot3(K2, g0, K4, g1, K5, g2));
-        real phid = fma(a, Pi, dot3(b0, g0, b1, g1, b2, g2));
-        if (bnd && B.bc_on) k1_boundary<real>(B, e, ti, tj, tk, n, u, Pi, g0, g1, g2, cc, phid);
+        const real F0 = fma(b0, Pi[r], dot3(K0, g0, K1v, g1, K2, g2));
+        const real F1 = fma(b1, Pi[r], dot3(K1v, g0, K3, g1, K4, g2));
+        const real F2 = fma(b2, Pi[r], dot3(K2, g0, K4, g1, K5, g2));
+        real phid = fma(a, Pi[r], dot3(b0, g0, b1, g1, b2, g2));
+        if (bnd && B.bc_on)
+          for (int b = node_faces(ti, tj, tk) & ~mask; b; b &= b - 1) {
+            const int f = __ffs(b) - 1, ax = f >> 1;
+            phid += sfP[f * N2 + (ax == 0 ? tj : ti) + 8 * (ax == 2 ? tj : tk)];
+          }
         const long long fo = e * FS + tp, fstr = B.Ne * FS;
         B.F[fo] = F0;
         B.F[fstr + fo] = F1;
@@ -1375,12 +1416,6 @@ __device__ __forceinline__ int face_slot(int fs, int pq) {
   int pn, qn;
   face_perm((fs >> 3) & 7, pq & 7, pq >> 3, N, pn, qn);
   return ((fs & 7) << 6) + pn + 8 * qn;
-}
-// node at position pos of pencil pc along axis al; pc = a + 8 b numbers the
-// other two axes in increasing order, so it is also the pencil's face index
-__device__ __forceinline__ int pnode(int al, int pc, int pos) {
-  const int a = pc & 7, b = pc >> 3;
-  return al == 0 ? pos + 8 * a + 64 * b : al == 1 ? a + 8 * pos + 64 * b : a + 8 * b + 64 * pos;
 }
 // out[l] = sum_m G[l][m] v[m]
 __device__ __forceinline__ void contract8(const float* G, const float v[8], float out[8]) {
@@ -1435,12 +1470,14 @@ constexpr size_t k2c_smem() {
 // sum/difference basis (cc_contract).  As in the FP64 kernel an (axis, pencil) owns
 // its metric terms, so the gradient partials replace them in place, and the
 // divergence partials wait in registers until F is free.  Neighbour traces go
-// straight to the thread whose pencil ends on them; the node pass takes two nodes a
-// thread, and only a node on an outer face looks at the boundary tables.
+// straight to the thread whose pencil ends on them, which also evaluates the boundary
+// terms there; the node pass takes two nodes a thread.
 // Bound by issue (56%) and by the latency of the node words: 1950 instructions a
 // warp in the fused launch, which moves 35 words a node, 0.70 ms at 40^3 elements.
-// Measured (B200, 40^3 elements): RK4 step 6.44 -> 4.86 ms (two-kernel stages of this
-// template 5.36 ms), one right-hand side 1.39 -> 1.17 ms; 16^3: step 525 -> 374 us.
+// Measured (B200, 40^3 elements): RK4 step 6.44 -> 4.70 ms (two-kernel stages of this
+// template 5.36 ms before the last change), one right-hand side 1.39 -> 1.18 ms; 16^3:
+// step 525 -> 359 us; 6^3: 74 -> 41 us.  Boundary terms in the node pass instead: 4.73
+// ms, 373 us, 57.5 us.
 // Four CTAs of 80 registers instead of five of 64: 5.33 against 5.04 ms; scalar FMAs
 // in this basis 4.97, in the plain basis 5.04, packed 4.92 ms, with a smaller error
 // of Pi against 64 bits (4.9-6.1e-7 after three steps, 5.7-6.3e-7 before); the loops
@@ -1507,7 +1544,6 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
   uint64_t* bar = reinterpret_cast<uint64_t*>(su + (GRAD ? N3 : 0));
   __shared__ int abort_flag;
   __shared__ float2 sm0[9];  // Ja0 = x + y
-  __shared__ int sbd[12];    // the faces' boundary tags and slots
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int al = tid >> 6, pc = tid & 63;  // axis (warp-uniform) and pencil
   int sid = 0;
@@ -1540,14 +1576,17 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
     const double j = (DIV ? A.Ja0 : B.Ja0)[9 * e + lane];
     sm0[lane] = make_float2((float)j, (float)(j - (double)(float)j));
   }
-  if (tid >= 32 && tid < 44) sbd[tid - 32] = face_entry(DIV ? A.bdry : B.bdry, DIV ? A.bslot : B.bslot, e, tid - 32);
   // the neighbours' nodes across this pencil's ends
   long long nbo[2];  // their elements' first node
   int nbn[2];        // the node; -1: no neighbour
+  int slot[2] = {-1, -1};  // the outer faces' slots
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int src = ::wt::bc_src((DIV ? A.fsrc : B.fsrc)[2 * al + h + 6 * e], Ne);
     nbo[h] = (long long)(src >> 6) * N3;
+    if constexpr (DIV) {
+      if (A.bc_on && A.bdry[2 * al + h + 6 * e] != 0) slot[h] = ::wt::bc_slot(A.bslot[2 * al + h + 6 * e], A.nbf);
+    }
     const int ax = (src & 7) >> 1;
     const int a = (src & 32 ? pc >> 3 : pc & 7) ^ (src & 8 ? 7 : 0), b = (src & 32 ? pc & 7 : pc >> 3) ^ (src & 16 ? 7 : 0);
     nbn[h] = src < 0 ? -1 : (a << (ax == 0 ? 3 : 0)) | (b << (ax == 2 ? 3 : 6)) | ((src & 1 ? 7 : 0) << (3 * ax));
@@ -1562,7 +1601,9 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
     for (int h = 0; h < 2; ++h) {
       const bool ok = nbn[h] >= 0;
       const long long at = ok ? nbo[h] + LayC::at(nbn[h]) : 0;
-      cp_async4(sfn + (3 * h + 0) * CTHR + tid, A.F0 + at, ok);
+      // an outer face, without a trace, has its boundary terms in the first component's place
+      cp_async4(sfn + (3 * h + 0) * CTHR + tid, slot[h] >= 0 ? A.bbuf + (long long)slot[h] * N2 + pc : A.F0 + at,
+                ok || slot[h] >= 0);
       cp_async4(sfn + (3 * h + 1) * CTHR + tid, A.F1 + at, ok);
       cp_async4(sfn + (3 * h + 2) * CTHR + tid, A.F2 + at, ok);
     }
@@ -1705,74 +1746,98 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
     }
   }
   __syncthreads();
-  // ---- node pass: two neighbouring nodes a thread, twice ----
-  if (tid >= 128) return;
+  // ---- node pass: threads < 128, two neighbouring nodes each, twice ----
+  const bool outer = (em >> 6) != 0;  // the element has outer faces
+  auto nat = [](float2 v, bool swp) { return swp ? make_float2(v.y, v.x) : v; };  // LayC exchanges the two
+  auto sum3 = [](const float* p, int at, int st) {
+    const float2 a = *reinterpret_cast<const float2*>(p + at), b = *reinterpret_cast<const float2*>(p + st + at),
+                 c = *reinterpret_cast<const float2*>(p + 2 * st + at);
+    return make_float2((a.x + b.x) + c.x, (a.y + b.y) + c.y);
+  };
+  if constexpr (DIV) {
+    if (tid < 128) {
 #pragma unroll 1
-  for (int r = 0; r < 2; ++r) {
-    const unsigned q = tid + 128 * r;
-    const int w = 2 * q, at = LayC::at(w) & ~1;
-    const bool swp = (w >> 6) & 1;  // LayC exchanges the two
-    const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
-    auto pair = [&](const float* p) {  // p: three partials FS words apart from one another
-      const float2 a = *reinterpret_cast<const float2*>(p + at);
-      return a;
-    };
-    auto nat = [&](float2 v) { return swp ? make_float2(v.y, v.x) : v; };
-    // outer faces that nodes w and w + 1 lie on
-    const int out0 = (em >> 6) ? node_faces(ti, tj, tk) & ~em : 0, out1 = (em >> 6) ? node_faces(ti + 1, tj, tk) & ~em : 0;
-    const float2 iJ = cc_ld((DIV ? A.invdetJ : B.invdetJ) + eo, q);
-    float Pi[2] = {0, 0};
-    if constexpr (DIV) {
-      const float2 y = A.epi ? cc_ld(A.y + eo, q) : make_float2(0.f, 0.f);
-      const float2 ac = A.epi && A.stage >= 1 ? cc_ld(A.acc + eo, q) : make_float2(0.f, 0.f);
-      const float2 p0 = pair(sF), p1 = pair(sF + FS), p2 = pair(sF + 2 * FS);
-      const float2 sd = nat(make_float2((p0.x + p1.x) + p2.x, (p0.y + p1.y) + p2.y));
-      float dv[2] = {__fmul_rn(sd.x, iJ.x), __fmul_rn(sd.y, iJ.y)};  // the halves and the fused form round alike
-      if (A.bc_on) {
+      for (int r = 0; r < 2; ++r) {
+        const unsigned q = tid + 128 * r;
+        const int w = 2 * q, at = LayC::at(w) & ~1;
+        const bool swp = (w >> 6) & 1;
+        const float2 y = A.epi ? cc_ld(A.y + eo, q) : make_float2(0.f, 0.f);
+        const float2 ac = A.epi && A.stage >= 1 ? cc_ld(A.acc + eo, q) : make_float2(0.f, 0.f);
+        const float2 iJ = cc_ld(A.invdetJ + eo, q), sd = nat(sum3(sF, at, FS), swp);
+        float dv[2] = {__fmul_rn(sd.x, iJ.x), __fmul_rn(sd.y, iJ.y)};  // the halves and the fused form round alike
+        if (outer && A.bc_on) {
+          const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          for (int b = x ? out1 : out0; b; b &= b - 1) {
-            const int f = __ffs(b) - 1, ax = f >> 1;
-            if (sbd[f] == 0) continue;
-            const int p = ax == 0 ? tj : ti + x, qq = ax == 2 ? tj : tk;
-            dv[x] += A.bbuf[(long long)::wt::bc_slot(sbd[6 + f], A.nbf) * N2 + p + 8 * qq];
+          for (int x = 0; x < 2; ++x)
+            for (int b = node_faces(ti + x, tj, tk) & ~em; b; b &= b - 1) {
+              const int f = __ffs(b) - 1, ax = f >> 1;
+              dv[x] += sfn[3 * (f & 1) * CTHR + 64 * ax + (ax == 0 ? tj : ti + x) + 8 * (ax == 2 ? tj : tk)];
+            }
+        }
+        if (FUSED || A.epi) {
+          // Kahan-compensated FP32 (as n8_rk): acc holds the step's increment
+          const CCW k = cc_weights(A.stage, A.dt);
+          const float a0 = fmaf(k.w, dv[0], ac.x), a1 = fmaf(k.w, dv[1], ac.y);
+          if (!FUSED && A.stage == 3) {
+            const float2 c = cc_ld(A.comp + eo, q);
+            const float t0 = a0 + c.x, t1 = a1 + c.y;
+            const float v0 = y.x + t0, v1 = y.y + t1;
+            cc_st(A.comp + eo, q, t0 - (v0 - y.x), t1 - (v1 - y.y));
+            cc_st(A.y + eo, q, v0, v1);
+            if (A.flag && !(isfinite(v0) && isfinite(v1))) atomicOr(A.flag, 1u);
+          } else {
+            cc_st(A.acc + eo, q, a0, a1);
+            const float2 o = make_float2(fmaf(k.h, dv[0], y.x), fmaf(k.h, dv[1], y.y));
+            if (!FUSED) cc_st(A.out + eo, q, o.x, o.y);
+            else *reinterpret_cast<float2*>(sF + at) = nat(o, swp);  // Pi of stage s + 1, in its nodes' first partials
           }
-        }
-      }
-      if (FUSED || A.epi) {
-        // Kahan-compensated FP32 (as n8_rk): acc holds the step's increment
-        const CCW k = cc_weights(A.stage, A.dt);
-        const float a0 = fmaf(k.w, dv[0], ac.x), a1 = fmaf(k.w, dv[1], ac.y);
-        if (!FUSED && A.stage == 3) {
-          const float2 c = cc_ld(A.comp + eo, q);
-          const float t0 = a0 + c.x, t1 = a1 + c.y;
-          const float v0 = y.x + t0, v1 = y.y + t1;
-          cc_st(A.comp + eo, q, t0 - (v0 - y.x), t1 - (v1 - y.y));
-          cc_st(A.y + eo, q, v0, v1);
-          if (A.flag && !(isfinite(v0) && isfinite(v1))) atomicOr(A.flag, 1u);
         } else {
-          cc_st(A.acc + eo, q, a0, a1);
-          Pi[0] = fmaf(k.h, dv[0], y.x);
-          Pi[1] = fmaf(k.h, dv[1], y.y);
-          if (!FUSED) cc_st(A.out + eo, q, Pi[0], Pi[1]);
+          cc_st(A.Pidot + eo, q, dv[0], dv[1]);
         }
-      } else {
-        cc_st(A.Pidot + eo, q, dv[0], dv[1]);
       }
     }
-    if constexpr (GRAD) {
-      if constexpr (!FUSED) {
-        const float2 v = cc_ld(B.Pi + eo, q);
-        Pi[0] = v.x;
-        Pi[1] = v.y;
+  }
+  if constexpr (GRAD) {
+    // boundary terms, each thread those of its pencil's ends: all faces at once (see
+    // k_cons_k1 in wt_cons.cu); increments of Phidot into scu
+    if (outer && B.bc_on) {  // the same for the whole CTA
+      if constexpr (FUSED) __syncthreads();  // Pi is complete, every thread has read its boundary terms
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        const int f = 2 * al + h, tag = B.bdry[f + 6 * e];
+        float dF = 0;
+        if (tag != 0) {
+          const int w = pnode(al, pc, h ? 7 : 0), at = LayC::at(w);
+          float cc[10], g[3];
+#pragma unroll
+          for (int c = 0; c < 10; ++c) cc[c] = B.c10[c * B.nn + eo + w];
+          const float P1 = FUSED ? sF[at] : B.Pi[eo + w], iJ = B.invdetJ[eo + w];
+#pragma unroll
+          for (int c = 0; c < 3; ++c)
+            g[c] = __fmul_rn((sJa[c * FS + at] + sJa[(3 + c) * FS + at]) + sJa[(6 + c) * FS + at], iJ);
+          // the whole stage value where a boundary term reads Phi itself
+          const float u = B.Phit ? B.Phi[eo + w] + B.Phit[eo + w] : B.Phi[eo + w];
+          k1_boundary_face<float>(B, tag, ::wt::bc_slot(B.bslot[f + 6 * e], B.nbf), pc & 7, pc >> 3, eo + w, u, P1, g[0],
+                                  g[1], g[2], cc, dF);
+        }
+        scu[h * CTHR + tid] = dF;
       }
+      __syncthreads();
+    }
+    if (tid >= 128) return;
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {
+      const unsigned q = tid + 128 * r;
+      const int w = 2 * q, at = LayC::at(w) & ~1;
+      const bool swp = (w >> 6) & 1;
+      const float2 iJ = cc_ld(B.invdetJ + eo, q);
+      const float2 Pi = FUSED ? nat(*reinterpret_cast<const float2*>(sF + at), swp) : cc_ld(B.Pi + eo, q);
       float2 g[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float2 p0 = pair(sJa + c * FS), p1 = pair(sJa + (3 + c) * FS), p2 = pair(sJa + (6 + c) * FS);
-        g[c] = nat(make_float2((p0.x + p1.x) + p2.x, (p0.y + p1.y) + p2.y));
-        g[c].x *= iJ.x;
-        g[c].y *= iJ.y;
+        g[c] = nat(sum3(sJa + c * FS, at, 3 * FS), swp);
+        g[c].x = __fmul_rn(g[c].x, iJ.x);
+        g[c].y = __fmul_rn(g[c].y, iJ.y);
       }
       float2 cc[10];
 #pragma unroll
@@ -1783,31 +1848,26 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         auto el = [&](const float2& v) { return x ? v.y : v.x; };
-        const float g0 = el(g[0]), g1 = el(g[1]), g2 = el(g[2]);
+        const float g0 = el(g[0]), g1 = el(g[1]), g2 = el(g[2]), P = el(Pi);
         const float b0 = el(cc[1]), b1 = el(cc[2]), b2 = el(cc[3]);
         const float K1v = el(cc[5]), K2 = el(cc[6]), K4 = el(cc[8]);
-        F[0][x] = fmaf(b0, Pi[x], dot3(el(cc[4]), g0, K1v, g1, K2, g2));
-        F[1][x] = fmaf(b1, Pi[x], dot3(K1v, g0, el(cc[7]), g1, K4, g2));
-        F[2][x] = fmaf(b2, Pi[x], dot3(K2, g0, K4, g1, el(cc[9]), g2));
-        ph[x] = fmaf(el(cc[0]), Pi[x], dot3(b0, g0, b1, g1, b2, g2));
-        if (B.bc_on && (x ? out1 : out0)) {
-          float ce[10];
+        F[0][x] = fmaf(b0, P, dot3(el(cc[4]), g0, K1v, g1, K2, g2));
+        F[1][x] = fmaf(b1, P, dot3(K1v, g0, el(cc[7]), g1, K4, g2));
+        F[2][x] = fmaf(b2, P, dot3(K2, g0, K4, g1, el(cc[9]), g2));
+        ph[x] = fmaf(el(cc[0]), P, dot3(b0, g0, b1, g1, b2, g2));
+      }
+      if (outer && B.bc_on) {
+        const int ti = w & 7, tj = (w >> 3) & 7, tk = w >> 6;
 #pragma unroll
-          for (int c = 0; c < 10; ++c) ce[c] = el(cc[c]);
-          // the whole stage value where a boundary term reads Phi itself
-          const float u = B.Phit ? el(hi[r]) + B.Phit[eo + w + x] : el(hi[r]);
-          for (int b = x ? out1 : out0; b; b &= b - 1) {
+        for (int x = 0; x < 2; ++x)
+          for (int b = node_faces(ti + x, tj, tk) & ~em; b; b &= b - 1) {
             const int f = __ffs(b) - 1, ax = f >> 1;
-            if (sbd[f] == 0) continue;
-            const int p = ax == 0 ? tj : ti + x, qq = ax == 2 ? tj : tk;
-            k1_boundary_face<float>(B, sbd[f], ::wt::bc_slot(sbd[6 + f], B.nbf), p, qq, eo + w + x, u, Pi[x], g0, g1,
-                                    g2, ce, ph[x]);
+            ph[x] += scu[(f & 1) * CTHR + 64 * ax + (ax == 0 ? tj : ti + x) + 8 * (ax == 2 ? tj : tk)];
           }
-        }
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c)
-        *reinterpret_cast<float2*>(B.F + c * B.Ne * FS + eo + at) = nat(make_float2(F[c][0], F[c][1]));
+        *reinterpret_cast<float2*>(B.F + c * B.Ne * FS + eo + at) = nat(make_float2(F[c][0], F[c][1]), swp);
       if (FUSED || B.epi) {
         // The state is the pair (y, lo) = (high, low part); the stage the next K1
         // reads is y + out with out = lo + c dt k, so the stage value keeps the
