@@ -1461,8 +1461,8 @@ constexpr size_t k2c_smem() {
 //   0.5 D(Ja u) + 0.5 Ja D u = (2 Ja0 + dJa) (0.5 D u) + 0.5 D(dJa u),
 // so the only contraction of u in FP32 acts on dJa u, which is as small as the
 // metric terms' variation over the element.  Once 0.5 D u has been formed in FP64
-// it is a gradient-sized value, and FP32 suffices for the rest.  The divergence
-// takes Ja = Ja0 + dJa, rounded to FP32 once.
+// it is a gradient-sized value, and FP32 suffices for the rest.  The divergence of F
+// takes the same split, all in FP32: 0.5 D(dJa F) rounds less than 0.5 D(Ja F).
 //
 // CTA: one element, 192 threads, one per (axis, pencil), CC_OCC CTAs per SM.  u is
 // formed once in shared memory in FP64 and 0.5 D u comes from the FP64 tensor cores
@@ -1479,9 +1479,10 @@ constexpr size_t k2c_smem() {
 // step 525 -> 359 us; 6^3: 74 -> 41 us.  Boundary terms in the node pass instead: 4.73
 // ms, 373 us, 57.5 us.
 // Four CTAs of 80 registers instead of five of 64: 5.33 against 5.04 ms; scalar FMAs
-// in this basis 4.97, in the plain basis 5.04, packed 4.92 ms, with a smaller error
-// of Pi against 64 bits (4.9-6.1e-7 after three steps, 5.7-6.3e-7 before); the loops
-// over the components unrolled (instruction cache) 5.17 ms.
+// in this basis 4.97, in the plain basis 5.04, packed 4.92 ms; the loops over the
+// components unrolled (instruction cache) 5.17 ms.  Error of Pi against 64 bits,
+// geometric mean over 16 inputs, relative to the kernels before: 0.96 on 2^3
+// elements, 0.84 on 3^3, 1.003 on 4^3, 0.97 on 6^3, 0.96 on 8^3; of Phi the same.
 constexpr int CC_OCC = 5;
 constexpr size_t cc_smem(int half) {
   return ((half & N8_K2 ? 3 * 512 + 6 * n8::CTHR : 0) + 9 * 512 + (half & N8_K1 ? 4 * 512 : 0)) * sizeof(float) +
@@ -1692,15 +1693,15 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
 #pragma unroll
       for (int pos = 0; pos < 8; ++pos) {
         F[pos] = sF[c * FS + addr[pos]];
-        m[pos] = m0.x + (m0.y + mc[addr[pos]]);
+        m[pos] = mc[addr[pos]];
         w[pos] = fmaf(m[pos], F[pos], w[pos]);
       }
-      s0 = fmaf(m[0], sfn[c * CTHR + tid] - F[0], s0);
-      s1 = fmaf(m[7], sfn[(3 + c) * CTHR + tid] - F[7], s1);
+      s0 = fmaf(m0.x + (m0.y + m[0]), sfn[c * CTHR + tid] - F[0], s0);
+      s1 = fmaf(m0.x + (m0.y + m[7]), sfn[(3 + c) * CTHR + tid] - F[7], s1);
       float o[8];
       cc_contract(P0.a.Ge, F, o);
 #pragma unroll
-      for (int l = 0; l < 8; ++l) rs[l] = fmaf(m[l], o[l], rs[l]);
+      for (int l = 0; l < 8; ++l) rs[l] = fmaf(fmaf(2.f, m0.x, m[l]), o[l], rs[l]);
     }
     {
       float o[8];
