@@ -90,14 +90,19 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
   dep_wait();
   const real* const fp = blockIdx.y ? P.f[1] : P.f[0];
   real* const op = (blockIdx.y ? P.out[1] : P.out[0]) + a * P.ostride;
-  real ev[M], od[HH];
+  real ev[M], od[HH], vl, vh;  // vl, vh: the pencil's end values
+  // The sums are taken relative to the centre (G's rows sum to zero): D of a smooth
+  // field then rounds at its variation's size, not at its own, and the end values of
+  // the first pass are the field's, so that a continuous field has no jumps.
   auto fold = [&](const real v[N]) {
 #pragma unroll
     for (int i = 0; i < HH; ++i) {
-      ev[i] = v[i] + v[N - 1 - i];
+      ev[i] = (v[i] - v[N & 1 ? HH : HH - 1]) + (v[N - 1 - i] - v[HH]);
       od[i] = v[i] - v[N - 1 - i];
     }
-    if (N & 1) ev[M - 1] = v[HH];
+    if (N & 1) ev[M - 1] = 0;
+    vl = v[0];
+    vh = v[N - 1];
   };
   auto load = [&](auto st) {
     constexpr int stride = decltype(st)::value;
@@ -135,7 +140,6 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
 #pragma unroll 2
   for (int it = 0; it < 6; ++it) {
     real* eb = ends + (it & 1) * 2 * T;
-    const real vl = (real)0.5 * (ev[0] + od[0]), vh = (real)0.5 * (ev[0] - od[0]);
     eb[tid] = vl;
     eb[T + tid] = vh;
     __syncthreads();
@@ -161,6 +165,8 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
     for (int i = 0; i < M; ++i) ev[i] = ne[i];
 #pragma unroll
     for (int i = 0; i < HH; ++i) od[i] = no[i];
+    vl = (real)0.5 * (ev[0] + od[0]);
+    vh = (real)0.5 * (ev[0] - od[0]);
   }
   auto unfold = [&](real v[N]) {
 #pragma unroll
