@@ -220,9 +220,9 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long n, int i
 // 24 N words a node).  What bounds the kernels now is the latency of their global
 // loads at the occupancy the pencils' registers leave: N = 6 FP64, 24^3 elements,
 // K1 reaches 4.7 TB/s (26 words a node), K2 3.1 TB/s (14 words).  Measured, one RK4
-// step (B200, FP64 / compensated FP32): N = 4, 36^3 elements 1184 -> 1026 / 876 ->
-// 687 us; N = 5, 28^3 1280 -> 845 / 765 -> 611; N = 6, 24^3 1336 -> 971 / 942 ->
-// 601; N = 7, 20^3 1581 -> 1003 / 1118 -> 579.  Fields that are read along pencils (Phi and the metric terms in
+// step (B200, FP64 / compensated FP32; thread per node -> now): N = 4, 36^3 elements
+// 1184 -> 963 / 876 -> 648 us; N = 5, 28^3 1280 -> 802 / 765 -> 544; N = 6, 24^3 1336 ->
+// 950 / 942 -> 579; N = 7, 20^3 1581 -> 992 / 1118 -> 545.  Fields that are read along pencils (Phi and the metric terms in
 // K1, F and the metric terms in K2) arrive by cp.async in a padded layout; axis
 // al's results replace its own metric terms there, pencil by pencil, and after one
 // barrier a node pass sums the three axes, in node order.  Boundary terms are

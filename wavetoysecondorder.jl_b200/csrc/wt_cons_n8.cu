@@ -1043,7 +1043,8 @@ __global__ void __launch_bounds__(n8::THREADS, n8::OCC)
 // Measured (B200, 40^3 elements, one launch alone): fused 1.69 ms, 5.1 TB/s of its 33
 // words (78 % of the measured copy rate), before 2.36; K1 1.13 (28 words, 6.5 TB/s),
 // before 1.34; K2 0.96 (16 words, 4.4 TB/s), before 1.01.  In a running step the
-// sum is 9 % longer.  What is left: waits on global loads (a third of the stalls),
+// sum is 9 % longer.  Boundary terms by face points between the halves of the
+// node pass, not in it: 16^3 elements, one step 517 -> 508 us, 6^3 61 -> 57.  What is left: waits on global loads (a third of the stalls),
 // fixed-latency tensor and FP64 chains, and the shared-memory pipe (61 % busy).
 template <typename real>
 struct FKT {
@@ -1494,11 +1495,15 @@ static_assert(CC_OCC * (cc_smem(N8_FK) + 128 + 1024) <= 233472, "CC_OCC fused CT
 // centre (G[7-l][7-m] = -G[l][m]), so with e_m = v_m + v_{7-m}, d_m = v_m - v_{7-m}
 // (m < 4), p_l = sum_m A e, q_l = sum_m B d: out_l = q_l + p_l, out_{7-l} = q_l - p_l.
 // (p, q) is one packed FP32 pair: 16 packed FMAs and 16 additions instead of 64 FMAs.
+// The sums are relative to the centre pair's (G's rows sum to zero): D of a smooth v
+// then rounds at its variation's size, and the rounding of A does not turn a constant
+// into a derivative (without it the error of Phi after 200 steps was 1.7 times the
+// plain basis's on 24^3 elements; 1 % of the step).
 __device__ __forceinline__ void cc_contract(const float2* G, const float v[8], float out[8]) {
   unsigned long long ed[4];
 #pragma unroll
   for (int m = 0; m < 4; ++m) {
-    const float e = v[m] + v[7 - m], d = v[m] - v[7 - m];
+    const float e = (v[m] - v[3]) + (v[7 - m] - v[4]), d = v[m] - v[7 - m];
     asm("mov.b64 %0, {%1, %2};" : "=l"(ed[m]) : "f"(e), "f"(d));
   }
 #pragma unroll
@@ -1701,7 +1706,7 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
       float o[8];
       cc_contract(P0.a.Ge, F, o);
 #pragma unroll
-      for (int l = 0; l < 8; ++l) rs[l] = fmaf(fmaf(2.f, m0.x, m[l]), o[l], rs[l]);
+      for (int l = 0; l < 8; ++l) rs[l] = fmaf(fmaf(2.f, m0.x, fmaf(2.f, m0.y, m[l])), o[l], rs[l]);
     }
     {
       float o[8];
@@ -1728,7 +1733,7 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
       float* mc = sJa + (al * 3 + c) * FS;
-      const float m0 = sm0[al * 3 + c].x;
+      const float2 m0 = sm0[al * 3 + c];
       float m[8], w[8];
 #pragma unroll
       for (int pos = 0; pos < 8; ++pos) {
@@ -1739,9 +1744,9 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
       cc_contract(P0.b.Ge, w, o);  // 0.5 D(dJa u)
 #pragma unroll
       for (int l = 0; l < 8; ++l) {
-        float r = fmaf(fmaf(2.f, m0, m[l]), cu[l], o[l]);
-        if (l == 0) r = fmaf(m0 + m[0], j0, r);
-        if (l == 7) r = fmaf(m0 + m[7], j1, r);
+        float r = fmaf(fmaf(2.f, m0.x, fmaf(2.f, m0.y, m[l])), cu[l], o[l]);
+        if (l == 0) r = fmaf(m0.x + (m0.y + m[0]), j0, r);
+        if (l == 7) r = fmaf(m0.x + (m0.y + m[7]), j1, r);
         mc[addr[l]] = r;
       }
     }
