@@ -434,9 +434,9 @@ def run_ours(args):
     # K2_3 reads acc and writes the state: 2)
     k2_words = 3 + 10 + (2 if fused else 3)
     if fused:
-        traffic_pn = profiled_traffic("fk_curv_f64")
+        traffic_pn = profiled_traffic(f"fk_curv_{args.precision}")
         rl_kernel, rl_words, rl_achieved, rl_avg_s = (
-            "k_cons_fk_n8 (fused stage: divergence + Pi stage s, gradient + flux + Phi stage s + 1)", fk_words,
+            "k_cons_fk_n8 / k_cons_cc_n8 (fused stage: divergence + Pi stage s, gradient + flux + Phi stage s + 1)", fk_words,
             fk_achieved, fk_avg_s)
     else:
         traffic_pn = profiled_traffic(f"k1_curv_{args.precision}" if args.precision == "f64" or args.fp32_form == "cuda"
@@ -535,7 +535,7 @@ def precision_study(wt, ctx, args, seed, p, ic, dt64, ref, E64_0, value64, hbm):
         e1.record(stream)
         torch.cuda.synchronize()
         ctx.profile(False)
-        (k1_ms, k1_n), (k2_ms, k2_n), _ = ctx.profile_read()
+        (k1_ms, k1_n), (k2_ms, k2_n), (fk_ms, fk_n) = ctx.profile_read()
         t_s = e0.elapsed_time(e1) / 1000.0
         v = 2.0 * nn * args.steps / t_s
         extra = max(0, args.study_steps - args.warmup - args.steps)   # untimed, up to the study's step count
@@ -550,7 +550,8 @@ def precision_study(wt, ctx, args, seed, p, ic, dt64, ref, E64_0, value64, hbm):
             "speedup_vs_f64": v / value64,
             "step_roofline": {"algorithmic_bytes_per_step": step_bytes,
                               "frac": step_bytes / (t_s / args.steps) / 1e9 / hbm},
-            "kernels_ms_per_launch": {"k1": k1_ms / max(k1_n, 1), "k2": k2_ms / max(k2_n, 1)},
+            "kernels_ms_per_launch": {"k1": k1_ms / max(k1_n, 1), "k2": k2_ms / max(k2_n, 1),
+                                      "fk": fk_ms / max(fk_n, 1)},
             "rel_l2_vs_f64": float(torch.linalg.norm(d) / torch.linalg.norm(refv)),
             "max_err_vs_f64": float(d.abs().max() / refv.abs().max()),
             "energy_drift": E / E0 - 1.0, "steps_compared": max(args.study_steps, args.warmup + args.steps),
