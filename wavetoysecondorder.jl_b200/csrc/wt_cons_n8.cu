@@ -1475,15 +1475,14 @@ constexpr size_t k2c_smem() {
 // terms there; the node pass takes two nodes a thread.
 // Bound by issue (56%) and by the latency of the node words: 1950 instructions a
 // warp in the fused launch, which moves 35 words a node, 0.70 ms at 40^3 elements.
-// Measured (B200, 40^3 elements): RK4 step 6.44 -> 4.70 ms (two-kernel stages of this
-// template 5.36 ms before the last change), one right-hand side 1.39 -> 1.18 ms; 16^3:
-// step 525 -> 359 us; 6^3: 74 -> 41 us.  Boundary terms in the node pass instead: 4.73
-// ms, 373 us, 57.5 us.
-// Four CTAs of 80 registers instead of five of 64: 5.33 against 5.04 ms; scalar FMAs
-// in this basis 4.97, in the plain basis 5.04, packed 4.92 ms; the loops over the
-// components unrolled (instruction cache) 5.17 ms.  Error of Pi against 64 bits,
-// geometric mean over 16 inputs, relative to the kernels before: 0.96 on 2^3
-// elements, 0.84 on 3^3, 1.003 on 4^3, 0.97 on 6^3, 0.96 on 8^3; of Phi the same.
+// Measured (B200, 40^3 elements): RK4 step 6.44 -> 4.80 ms (two-kernel stages of this
+// template, an earlier form of it: 5.36 against 4.87 fused), one right-hand side 1.39 ->
+// 1.21 ms; 16^3: step 525 -> 366 us; 6^3: 74 -> 41 us.  Boundary terms in the node pass
+// instead, other things equal: 4.73 for 4.70 ms, 373 for 359 us, 57.5 for 41.3 us.
+// On the way there: four CTAs of 80 registers instead of five of 64: 5.33 against 5.04
+// ms; scalar FMAs in this basis 4.97, in the plain basis 5.04, packed 4.92 ms; the loops
+// over the components unrolled (instruction cache) 5.17 ms.  After 200 steps on 24^3
+// elements the state is 4.4e-7 from FP64 in Pi and 4.3e-8 in Phi, before 4.4e-7 and 4.0e-8.
 constexpr int CC_OCC = 5;
 constexpr size_t cc_smem(int half) {
   return ((half & N8_K2 ? 3 * 512 + 6 * n8::CTHR : 0) + 9 * 512 + (half & N8_K1 ? 4 * 512 : 0)) * sizeof(float) +
