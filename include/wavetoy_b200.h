@@ -522,7 +522,8 @@ int wt_step_erk_curved_tableau(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void
 /* The method's Butcher tableau (host only): stages, c[s], A[s*s] (row major), b[s]. */
 int wt_erk_tableau(int method, int* stages, double* c, double* A, double* b);
 /* RK4 of the SIPG system as first-order (u, ut):
- * u' = ut + eps mu^-5 sum_d D_d^6 u,  ut' = rhs_wave3d!(u, ut) + eps mu^-5 sum_d D_d^6 ut. */
+ * u' = ut + eps mu^-5 sum_d D_d^6 u,  ut' = rhs_wave3d!(u, ut) + eps mu^-5 sum_d D_d^6 ut.
+ * The state is u, ut alone, in FP32 too: a call keeps nothing for the next. */
 int wt_step_rk4_sipg(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, int nsteps,
                      const double bdry_values[6], double tau, double sommerfeld_R, double eps_ko);
 /* End-to-end evolve with host buffers, the shape of evolve3d(formulation =

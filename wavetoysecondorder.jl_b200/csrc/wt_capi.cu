@@ -2231,8 +2231,8 @@ static int step_sipg_once(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, 
     S.rkU.on = S.rkV.on = 1;
     S.rkU.stage = S.rkV.stage = st;
     S.rkU.dt = S.rkV.dt = dt;
-    S.rkU.y = u; S.rkU.acc = ws->accP; S.rkU.out = SP[st % 2]; S.rkU.comp = ws->compP;
-    S.rkV.y = ut; S.rkV.acc = ws->accQ; S.rkV.out = ws->SQ; S.rkV.comp = ws->compQ;
+    S.rkU.y = u; S.rkU.acc = ws->accP; S.rkU.out = SP[st % 2];
+    S.rkV.y = ut; S.rkV.acc = ws->accQ; S.rkV.out = ws->SQ;
     wt::NvtxRange nv("rk4 sipg stage");
     WT_TRY(lrc(ctx, wt::launch_sipg(m, S, false, s), "rk4 sipg"));
     ctx->launches += 1;
@@ -2248,7 +2248,6 @@ int wt_step_rk4_sipg(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, int n
   if (nsteps < 0 || !(dt > 0)) return fail(ctx, WT_EINVAL, "bad nsteps/dt");
   if (!ws->mesh->m.affine) return fail(ctx, WT_ENOTSUP, "SIPG stepping supports affine meshes only");
   WT_TRY(ws_step_buffers(ws));
-  comp_track(ws, u, ut);
   if (eps_ko != 0.0) {  // buffers and mu before any graph capture
     WT_TRY(ko_buffers(ws));
     WT_TRY(ensure_mu(ws));

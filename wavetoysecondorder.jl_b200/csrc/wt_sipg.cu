@@ -59,7 +59,7 @@ struct SipgP {
   int nko;               // dissipation increments per field (0, 1 or 3 fields of nn words)
   const real* koU;
   const real* koV;
-  real *yU, *accU, *outU, *compU, *yV, *accV, *outV, *compV;
+  real *yU, *accU, *outU, *yV, *accV, *outV;
 };
 
 // elements per CTA: about 200 threads
@@ -124,8 +124,7 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
   // contractions (each thread reads back only its own): ut, dissipation
   // increments, RK states and accumulators
   real* sw = reinterpret_cast<real*>(smraw) + (size_t)4 * epb * NS + (size_t)le * (5 + 2 * P.nko) * N3;
-  const bool fin = P.compU && P.stage == 3;
-  const bool ld_y = P.stage == 1 || P.stage == 2 || fin, ld_acc = P.stage >= 1;
+  const bool ld_y = P.stage == 1 || P.stage == 2, ld_acc = P.stage >= 1;
   if (!TRACE && P.epi) {
 #pragma unroll
     for (int it = 0; it < NI; ++it) {
@@ -238,9 +237,9 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
         }
         const real yU = ld_y ? sw[N3 + wn] : (real)0, yV = ld_y ? sw[2 * N3 + wn] : (real)0;
         const real aU = ld_acc ? sw[3 * N3 + wn] : (real)0, aV = ld_acc ? sw[4 * N3 + wn] : (real)0;
-        const real cU = fin ? P.compU[n] : (real)0, cV = fin ? P.compV[n] : (real)0;
-        su[at] = rk_epilogue_v<real>(P.stage, P.dt, kU, uin, yU, aU, cU, P.yU, P.accU, P.outU, P.compU, n, nullptr);
-        rk_epilogue_v<real>(P.stage, P.dt, kV, vin, yV, aV, cV, P.yV, P.accV, P.outV, P.compV, n, nullptr);
+        // FP32 too without low parts: a step depends on (u, ut) alone, nothing stays behind in the workspace
+        su[at] = rk_epilogue_v<real>(P.stage, P.dt, kU, uin, yU, aU, (real)0, P.yU, P.accU, P.outU, nullptr, n, nullptr);
+        rk_epilogue_v<real>(P.stage, P.dt, kV, vin, yV, aV, (real)0, P.yV, P.accV, P.outV, nullptr, n, nullptr);
       }
     }
     if (!P.epi) return;
@@ -268,8 +267,8 @@ static SipgP<N, real> sipg_params(const DevMesh& m, const SipgStage& S) {
   P.tau = (real)S.tau; P.inv_R = (real)S.inv_R;
   P.epi = S.rkU.on; P.stage = S.rkU.stage; P.dt = S.rkU.dt;
   P.nko = S.nko; P.koU = (const real*)S.koU; P.koV = (const real*)S.koV;
-  P.yU = (real*)S.rkU.y; P.accU = (real*)S.rkU.acc; P.outU = (real*)S.rkU.out; P.compU = (real*)S.rkU.comp;
-  P.yV = (real*)S.rkV.y; P.accV = (real*)S.rkV.acc; P.outV = (real*)S.rkV.out; P.compV = (real*)S.rkV.comp;
+  P.yU = (real*)S.rkU.y; P.accU = (real*)S.rkU.acc; P.outU = (real*)S.rkU.out;
+  P.yV = (real*)S.rkV.y; P.accV = (real*)S.rkV.acc; P.outV = (real*)S.rkV.out;
   return P;
 }
 
