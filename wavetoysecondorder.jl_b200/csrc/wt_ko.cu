@@ -7,22 +7,29 @@
 // six times needs, per pass, only the two end values of the pencils next to it.
 //
 // What bounds it: per axis and field 3 words of DRAM traffic per node (the
-// field in, the destination in and out) against 6 N multiply-adds, which FP64
-// at N = 8 would make the longer of the two.  The derivative matrix is
-// antisymmetric about its centre (G[N-1-i][N-1-p] = -G[i][p]), so in the basis
-// of sums and differences of mirrored values a pass is two half-size products,
-// N^2/2 multiply-adds per pencil, and the six passes stay in that basis.  The
-// half-size matrices are kernel parameters (constant bank: no shared-memory
-// operand loads).  Only the end values go through shared memory, double
-// buffered, one barrier per pass.  Axis 0 pencils are contiguous in memory:
-// each warp transposes its 32 pencils through a padded shared buffer of its
-// own; along axes 1 and 2 consecutive threads hold consecutive nodes and load
-// directly.
+// field in, the destination in and out) against 6 N multiply-adds.  The operator
+// is kernel parameters (constant bank: no shared-memory operand loads), of which
+// half the rows suffice: G is antisymmetric about its centre, G[N-1-i][N-1-p] =
+// -G[i][p], exactly as stored, so an entry serves both mirrored rows (with all rows
+// as operands the 64 registers spill and n = 8 takes four times as long).  Only the end values go through shared memory, double buffered, one barrier
+// per pass.  Axis 0 pencils are contiguous in memory: each warp transposes its 32
+// pencils through a padded shared buffer of its own; along axes 1 and 2 consecutive
+// threads hold consecutive nodes and load directly.
 //
-// Measured (FP64, one axis of two fields, B200): 24^3 elements of n = 8, 66 us
-// (5.2 TB/s; the whole pencils through shared memory on every pass, two
-// barriers each and the matrix read from shared memory: 212 us); 40^3 of n = 6,
-// 150 us (before: 450 us).
+// Rounding.  Sums and differences of mirrored values would halve the multiply-adds,
+// but their own rounding, amplified by six passes, is 1.3 to 4.7 times the plain sums'
+// error on a field that oscillates within an element (n = 8, one wavelength an element,
+// FP64: 3.3e-14 -> 1.5e-13; white noise 2.4e-16 -> 3.1e-16), so the passes take the plain
+// sums.  Where a pencil varies by less than half its size, the first pass takes the
+// values relative to the pencil's centre (G's rows sum to zero), which then loses
+// nothing on the way: the error of a resolved field falls (pulses of width 0.1 on 24
+// elements, n = 8: FP64 0.62, FP32 0.06 of the plain sums'), and no other field's
+// grows (within 3 %).
+//
+// Measured (FP64, three axes of one field, B200): 24^3 elements of n = 8, 114 us, 40^3 of
+// n = 6, 260 us (in sums and differences 96 and 247).  The whole pencils
+// through shared memory on every pass, two barriers each and the matrix read from there:
+// 315 and 680 us.
 #include "wt_common.cuh"
 #include "wt_launch.cuh"
 
@@ -34,9 +41,7 @@ namespace wt {
 
 template <int N, typename real>
 struct KoP {
-  static constexpr int M = (N + 1) / 2, HH = N / 2;
-  real A[M * HH];  // even part of D v from the differences: A[i][p] = G[i][p] - G[i][N-1-p]; centre row G[c][p]
-  real B[HH * M];  // odd part of D v from the sums: G[i][p] + G[i][N-1-p]; centre column 2 G[i][c]
+  real G[(N + 1) / 2 * N];  // the upper half's rows
   const real* f[2];
   real* out[2];
   long long ostride;  // words between the outputs of consecutive axes (0: one output)
@@ -59,7 +64,7 @@ struct KoP {
 // 3 % slower at 40^3 n = 6, 13 % on a 4^3 step.)
 template <int N, typename real, int TMAX>
 __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant__ KoP<N, real> P) {
-  constexpr int N2 = N * N, N3 = N * N * N, M = KoP<N, real>::M, HH = KoP<N, real>::HH;
+  constexpr int N2 = N * N, N3 = N * N * N, HH = N / 2;
   constexpr int NP = N | 1;  // odd pitch of a staged pencil: no bank conflicts
   extern __shared__ __align__(16) unsigned char smraw[];
   real* ends = reinterpret_cast<real*>(smraw);  // [2 buffers][low, high end][thread]
@@ -90,30 +95,14 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
   dep_wait();
   const real* const fp = blockIdx.y ? P.f[1] : P.f[0];
   real* const op = (blockIdx.y ? P.out[1] : P.out[0]) + a * P.ostride;
-  real ev[M], od[HH], vl, vh;  // vl, vh: the pencil's end values
-  // The sums are taken relative to the centre (G's rows sum to zero): D of a smooth
-  // field then rounds at its variation's size, not at its own, and the end values of
-  // the first pass are the field's, so that a continuous field has no jumps.
-  auto fold = [&](const real v[N]) {
-#pragma unroll
-    for (int i = 0; i < HH; ++i) {
-      ev[i] = (v[i] - v[N & 1 ? HH : HH - 1]) + (v[N - 1 - i] - v[HH]);
-      od[i] = v[i] - v[N - 1 - i];
-    }
-    if (N & 1) ev[M - 1] = 0;
-    vl = v[0];
-    vh = v[N - 1];
-  };
+  real v[N];
   auto load = [&](auto st) {
     constexpr int stride = decltype(st)::value;
     const real* f = fp + (act ? base : 0);
-    real v[N];
 #pragma unroll
     for (int l = 0; l < N; ++l) v[l] = act ? f[l * stride] : (real)0;
-    fold(v);
   };
   if (d == 0) {
-    real v[N];
 #pragma unroll
     for (int it = 0; it < N; ++it) {
       const int w = it * 32 + lane, pr = w / N;
@@ -129,7 +118,6 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
 #pragma unroll
     for (int l = 0; l < N; ++l) v[l] = stage[lane * NP + l];
     __syncwarp();
-    fold(v);
   } else if (d == 1) {
     load(std::integral_constant<int, N>());
   } else {
@@ -137,51 +125,56 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
   }
   const bool has_prev = act && (closed || sg > 0), has_next = act && (closed || sg < len - 1);
   const int tp = pb + PB * (sg == 0 ? len - 1 : sg - 1), tn = pb + PB * (sg == len - 1 ? 0 : sg + 1);
-#pragma unroll 2
-  for (int it = 0; it < 6; ++it) {
-    real* eb = ends + (it & 1) * 2 * T;
-    eb[tid] = vl;
-    eb[T + tid] = vh;
-    __syncthreads();
-    // the centred-flux SAT of the two end nodes, in the sum / difference basis
-    const real lo = has_prev ? P.cH * (vl - eb[T + tp]) : (real)0;
-    const real hi = has_next ? P.cH * (eb[tn] - vh) : (real)0;
-    real ne[M], no[HH];
-#pragma unroll
-    for (int i = 0; i < M; ++i) {
-      real acc = i == 0 ? lo + hi : (real)0;
-#pragma unroll
-      for (int p = 0; p < HH; ++p) acc += P.A[i * HH + p] * od[p];
-      ne[i] = s * acc;
-    }
-#pragma unroll
-    for (int i = 0; i < HH; ++i) {
-      real acc = i == 0 ? lo - hi : (real)0;
-#pragma unroll
-      for (int p = 0; p < M; ++p) acc += P.B[i * M + p] * ev[p];
-      no[i] = s * acc;
-    }
-#pragma unroll
-    for (int i = 0; i < M; ++i) ev[i] = ne[i];
-#pragma unroll
-    for (int i = 0; i < HH; ++i) od[i] = no[i];
-    vl = (real)0.5 * (ev[0] + od[0]);
-    vh = (real)0.5 * (ev[0] - od[0]);
-  }
-  auto unfold = [&](real v[N]) {
-#pragma unroll
-    for (int i = 0; i < HH; ++i) {
-      v[i] = P.koT * ((real)0.5 * (ev[i] + od[i]));
-      v[N - 1 - i] = P.koT * ((real)0.5 * (ev[i] - od[i]));
-    }
-    if (N & 1) v[HH] = P.koT * ev[M - 1];
+  // the centre that the first pass takes the pencil relative to, or 0 (see above):
+  // magnitudes by their leading bits, half of one a step of the exponent
+  auto mag = [](real a) {
+    if constexpr (sizeof(real) == 8) return __double2hiint(a) & 0x7fffffff;
+    else return __float_as_int(a) & 0x7fffffff;
   };
+  constexpr int HALF = sizeof(real) == 8 ? 1 << 20 : 1 << 23;
+  real c = v[HH];
+  int mv = 0, mc = 0;
+#pragma unroll
+  for (int l = 0; l < N; ++l) {
+    mv = max(mv, mag(v[l]));
+    mc = max(mc, mag(v[l] - c));
+  }
+  if (mc >= mv - HALF) c = 0;
+  // v <- D v; the sums over x, the jumps to the neighbours' ends over v
+  auto pass = [&](int it, auto x) {
+    real* eb = ends + (it & 1) * 2 * T;
+    eb[tid] = v[0];
+    eb[T + tid] = v[N - 1];
+    __syncthreads();
+    // the centred-flux SAT of the two end nodes
+    const real lo = has_prev ? v[0] - eb[T + tp] : (real)0;
+    const real hi = has_next ? eb[tn] - v[N - 1] : (real)0;
+    real w[N];
+#pragma unroll
+    for (int p = 0; p < N; ++p) {
+      const real xp = x(p), xm = x(N - 1 - p);
+#pragma unroll
+      for (int i = 0; i < HH; ++i) {
+        const real g = P.G[i * N + p];
+        w[i] = p ? w[i] + g * xp : g * xp;
+        w[N - 1 - i] = p ? w[N - 1 - i] - g * xm : -(g * xm);
+      }
+      if (N & 1) w[HH] = p ? w[HH] + P.G[HH * N + p] * xp : P.G[HH * N] * xp;
+    }
+    w[0] += P.cH * lo;
+    w[N - 1] += P.cH * hi;
+#pragma unroll
+    for (int l = 0; l < N; ++l) v[l] = s * w[l];
+  };
+  pass(0, [&](int p) { return v[p] - c; });
+#pragma unroll 1
+  for (int it = 1; it < 6; ++it) pass(it, [&](int p) { return v[p]; });
+#pragma unroll
+  for (int l = 0; l < N; ++l) v[l] *= P.koT;
   auto store = [&](auto st) {
     constexpr int stride = decltype(st)::value;
     if (!act) return;
     real* o = op + base;
-    real v[N];
-    unfold(v);
     if (P.rmw) {
 #pragma unroll
       for (int l = 0; l < N; ++l) v[l] += o[l * stride];
@@ -190,8 +183,6 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
     for (int l = 0; l < N; ++l) o[l * stride] = v[l];
   };
   if (d == 0) {
-    real v[N];
-    unfold(v);
 #pragma unroll
     for (int l = 0; l < N; ++l) stage[lane * NP + l] = v[l];
     __syncwarp();
@@ -231,14 +222,7 @@ template <int N, typename real>
 static int ko_lines_n(const DevMesh& m, const int* axes, int nax, int nf, void* const* out, long long ostride, int rmw,
                       const void* const* f, double koT, cudaStream_t s) {
   KoP<N, real> P;
-  constexpr int M = KoP<N, real>::M, HH = KoP<N, real>::HH;
-  const std::vector<double>& G = m.ops.G;
-  for (int i = 0; i < M; ++i)
-    for (int p = 0; p < HH; ++p)
-      P.A[i * HH + p] = (real)((N & 1) && i == M - 1 ? G[i * N + p] : G[i * N + p] - G[i * N + N - 1 - p]);
-  for (int i = 0; i < HH; ++i)
-    for (int p = 0; p < M; ++p)
-      P.B[i * M + p] = (real)((N & 1) && p == M - 1 ? 2.0 * G[i * N + p] : G[i * N + p] + G[i * N + N - 1 - p]);
+  for (int q = 0; q < (N + 1) / 2 * N; ++q) P.G[q] = (real)m.ops.G[q];
   for (int q = 0; q < 2; ++q) {
     P.f[q] = (const real*)f[q < nf ? q : 0];
     P.out[q] = (real*)out[q < nf ? q : 0];
