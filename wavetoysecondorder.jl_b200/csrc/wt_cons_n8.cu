@@ -303,7 +303,7 @@ struct K1N8 {
   real* out;
   real* comp;
   unsigned* flag;
-  float2 Ge[16];  // 0.5 G in the sum/difference basis (cc_contract)
+  float2 Gp[32];  // 0.5 G, column by column, two rows a pair (cc_contract)
   float Gh[64];  // 0.5 G in FP32 (the CUDA-core form reads it from the constant bank)
   real* gout;    // gradient-only launches (GR): the three components of the split-form gradient
   // Compensated FP32 form (k_cons_cc_n8): the Phi the stage reads is
@@ -716,7 +716,7 @@ struct K2N8 {
   const double* Ja0;
   const real* ko;  // dissipation increments of Pidot (see K1N8)
   int nko;
-  float2 Ge[16];  // 0.5 G in the sum/difference basis (cc_contract)
+  float2 Gp[32];  // 0.5 G, column by column, two rows a pair (cc_contract)
   float Gh[64];
 };
 
@@ -1467,22 +1467,24 @@ constexpr size_t k2c_smem() {
 //
 // CTA: one element, 192 threads, one per (axis, pencil), CC_OCC CTAs per SM.  u is
 // formed once in shared memory in FP64 and 0.5 D u comes from the FP64 tensor cores
-// (a DFMA takes no constant operand); the FP32 contractions are packed FMAs in the
-// sum/difference basis (cc_contract).  As in the FP64 kernel an (axis, pencil) owns
+// (a DFMA takes no constant operand); the FP32 contractions are packed FMAs
+// (cc_contract).  As in the FP64 kernel an (axis, pencil) owns
 // its metric terms, so the gradient partials replace them in place, and the
 // divergence partials wait in registers until F is free.  Neighbour traces go
 // straight to the thread whose pencil ends on them, which also evaluates the boundary
 // terms there; the node pass takes two nodes a thread.
-// Bound by issue (56%) and by the latency of the node words: 1950 instructions a
-// warp in the fused launch, which moves 35 words a node, 0.70 ms at 40^3 elements.
-// Measured (B200, 40^3 elements): RK4 step 6.44 -> 4.80 ms (two-kernel stages of this
-// template, an earlier form of it: 5.36 against 4.87 fused), one right-hand side 1.39 ->
-// 1.21 ms; 16^3: step 525 -> 366 us; 6^3: 74 -> 41 us.  Boundary terms in the node pass
-// instead, other things equal: 4.73 for 4.70 ms, 373 for 359 us, 57.5 for 41.3 us.
-// On the way there: four CTAs of 80 registers instead of five of 64: 5.33 against 5.04
-// ms; scalar FMAs in this basis 4.97, in the plain basis 5.04, packed 4.92 ms; the loops
-// over the components unrolled (instruction cache) 5.17 ms.  After 200 steps on 24^3
-// elements the state is 4.4e-7 from FP64 in Pi and 4.3e-8 in Phi, before 4.4e-7 and 4.0e-8.
+// Bound by issue and by the latency of the node words (see the profile of small cases);
+// the fused launch moves 35 words a node.
+// Measured (B200, 40^3 elements): RK4 step 4.9 ms, before this template 6.44; 16^3: step 365 us (525); 6^3: 43 us (74).  In sums and differences of
+// mirrored values, which round worse (see cc_contract), 1 % faster.  Of an earlier form: two-kernel stages
+// 5.36 ms against 4.87 fused; boundary terms in the node pass 4.73 for 4.70 ms, 373 for
+// 359 us, 57.5 for 41.3 us; four CTAs of 80 registers instead of five of 64 5.33 against
+// 5.04 ms; the loops over the components unrolled (instruction cache) 5.17 ms.
+// Error against FP64 (relative, pulses): Pi after one step on 24^3 elements 4.1e-7 (the
+// kernels before this template 4.7e-7), Phi 2.5e-8 (2.5e-8: its rounding to FP32).  After
+// 200 steps Pi 4.4e-7 (4.4e-7), Phi 4.6e-8 (4.0e-8); Phi is then within 0.4 and 1.7 times
+// the earlier kernels' on seven meshes, 0.6 to 1.3 with the operator in twice 24 bits: the
+// rounding of the operator's entries to FP32, a bias that the steps add up.
 constexpr int CC_OCC = 5;
 constexpr size_t cc_smem(int half) {
   return ((half & N8_K2 ? 3 * 512 + 6 * n8::CTHR : 0) + 9 * 512 + (half & N8_K1 ? 4 * 512 : 0)) * sizeof(float) +
@@ -1490,33 +1492,33 @@ constexpr size_t cc_smem(int half) {
 }
 static_assert(CC_OCC * (cc_smem(N8_FK) + 128 + 1024) <= 233472, "CC_OCC fused CTAs must fit an SM");
 
-// out = 0.5 D v in the sum/difference basis: the operator is antisymmetric about its
-// centre (G[7-l][7-m] = -G[l][m]), so with e_m = v_m + v_{7-m}, d_m = v_m - v_{7-m}
-// (m < 4), p_l = sum_m A e, q_l = sum_m B d: out_l = q_l + p_l, out_{7-l} = q_l - p_l.
-// (p, q) is one packed FP32 pair: 16 packed FMAs and 16 additions instead of 64 FMAs.
-// The sums are relative to the centre pair's (G's rows sum to zero): D of a smooth v
-// then rounds at its variation's size, and the rounding of A does not turn a constant
-// into a derivative (without it the error of Phi after 200 steps was 1.7 times the
-// plain basis's on 24^3 elements; 1 % of the step).
+// out = 0.5 D v, two rows of a column a packed FMA, summed in the columns' order.  Where
+// the pencil varies by less than three quarters of its size (at four of its nodes: all
+// eight decide alike and cost 1 % of the step), v is taken relative to its centre (G's rows sum to zero; their rounding to FP32 then makes no derivative of a
+// constant).  Rounding against 64 bits, FP32 values, plain sums / so / in sums and
+// differences of mirrored values (which take half the multiply-adds): a sixth of a
+// wavelength an element 9.1e-7 / 4.4e-7 / 4.9e-7, a half 3.0 / 3.0 / 4.3e-7, one 1.4 / 1.4 /
+// 2.9e-7, white noise 5.9 / 5.9 / 7.1e-8.
 __device__ __forceinline__ void cc_contract(const float2* G, const float v[8], float out[8]) {
-  unsigned long long ed[4];
+  float c = v[3];
+  const float mv = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[2])), fmaxf(fabsf(v[5]), fabsf(v[7])));
+  const float mc = fmaxf(fmaxf(fabsf(v[0] - c), fabsf(v[2] - c)), fmaxf(fabsf(v[5] - c), fabsf(v[7] - c)));
+  if (!(mc < 0.75f * mv)) c = 0;
+  unsigned long long a[4];
 #pragma unroll
-  for (int m = 0; m < 4; ++m) {
-    const float e = (v[m] - v[3]) + (v[7 - m] - v[4]), d = v[m] - v[7 - m];
-    asm("mov.b64 %0, {%1, %2};" : "=l"(ed[m]) : "f"(e), "f"(d));
+  for (int m = 0; m < 8; ++m) {
+    const float x = v[m] - c;
+    unsigned long long xx;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(xx) : "f"(x));
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const unsigned long long g = *reinterpret_cast<const unsigned long long*>(G + 4 * m + l);
+      if (m == 0) asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(a[l]) : "l"(g), "l"(xx));
+      else asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a[l]) : "l"(g), "l"(xx));
+    }
   }
 #pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    unsigned long long a;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(*reinterpret_cast<const unsigned long long*>(G + 4 * l)), "l"(ed[0]));
-#pragma unroll
-    for (int m = 1; m < 4; ++m)
-      asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(*reinterpret_cast<const unsigned long long*>(G + 4 * l + m)), "l"(ed[m]));
-    float p, q;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(p), "=f"(q) : "l"(a));
-    out[l] = q + p;
-    out[7 - l] = q - p;
-  }
+  for (int l = 0; l < 4; ++l) asm("mov.b64 {%0, %1}, %2;" : "=f"(out[2 * l]), "=f"(out[2 * l + 1]) : "l"(a[l]));
 }
 
 // RK4 weights of a stage: the increment to the next stage's value, and to the step's
@@ -1703,13 +1705,13 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
       s0 = fmaf(m0.x + (m0.y + m[0]), sfn[c * CTHR + tid] - F[0], s0);
       s1 = fmaf(m0.x + (m0.y + m[7]), sfn[(3 + c) * CTHR + tid] - F[7], s1);
       float o[8];
-      cc_contract(P0.a.Ge, F, o);
+      cc_contract(P0.a.Gp, F, o);
 #pragma unroll
       for (int l = 0; l < 8; ++l) rs[l] = fmaf(fmaf(2.f, m0.x, fmaf(2.f, m0.y, m[l])), o[l], rs[l]);
     }
     {
       float o[8];
-      cc_contract(P0.a.Ge, w, o);
+      cc_contract(P0.a.Gp, w, o);
 #pragma unroll
       for (int l = 0; l < 8; ++l) rs[l] += o[l];
     }
@@ -1740,7 +1742,7 @@ __global__ void __launch_bounds__(n8::CTHR, CC_OCC)
         w[pos] = m[pos] * uf[pos];
       }
       float o[8];
-      cc_contract(P0.b.Ge, w, o);  // 0.5 D(dJa u)
+      cc_contract(P0.b.Gp, w, o);  // 0.5 D(dJa u)
 #pragma unroll
       for (int l = 0; l < 8; ++l) {
         float r = fmaf(fmaf(2.f, m0.x, fmaf(2.f, m0.y, m[l])), cu[l], o[l]);
@@ -2490,11 +2492,7 @@ static K1N8<real> k1n8_params(const DevMesh& m, const DevCoef& c, const void* Ph
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.flag = flag;
   for (int i = 0; i < 64; ++i) P.Gh[i] = (float)(0.5 * m.ops.G[i]);
-  for (int l = 0; l < 4; ++l)
-    for (int q = 0; q < 4; ++q) {
-      const double a = m.ops.G[8 * l + q], b = m.ops.G[8 * l + 7 - q];
-      P.Ge[4 * l + q] = make_float2((float)(0.25 * (a + b)), (float)(0.25 * (a - b)));
-    }
+  for (int i = 0; i < 32; ++i) P.Gp[i] = make_float2(P.Gh[i % 4 * 16 + i / 4], P.Gh[i % 4 * 16 + 8 + i / 4]);
   P.gout = nullptr;
   P.Phit = (const real*)rk.phit;
   P.dJa = (const real*)m.dJa;
@@ -2522,11 +2520,7 @@ static K2N8<real> k2n8_params(const DevMesh& m, const void* F, void* Pidot, cons
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.flag = flag;
   for (int i = 0; i < 64; ++i) P.Gh[i] = (float)(0.5 * m.ops.G[i]);
-  for (int l = 0; l < 4; ++l)
-    for (int q = 0; q < 4; ++q) {
-      const double a = m.ops.G[8 * l + q], b = m.ops.G[8 * l + 7 - q];
-      P.Ge[4 * l + q] = make_float2((float)(0.25 * (a + b)), (float)(0.25 * (a - b)));
-    }
+  for (int i = 0; i < 32; ++i) P.Gp[i] = make_float2(P.Gh[i % 4 * 16 + i / 4], P.Gh[i % 4 * 16 + 8 + i / 4]);
   P.dJa = (const real*)m.dJa;
   P.Ja0 = m.Ja0;
   P.ko = (const real*)rk.ko;
