@@ -333,10 +333,10 @@ int wt_workspace_set_mu(wt_ws* ws, double mu);
  * gradient half of stage s + 1 in one launch (five launches per RK4 step instead
  * of eight, 28 % fewer DRAM bytes).  The results equal the two-kernel stages' bit
  * for bit; on = 0 selects the two-kernel stages.  Takes effect at the next step
- * call.  The second flux buffer is allocated with FP64's first such step (3 x 8
- * bytes per node) or FP32's step buffers (2 x 4 bytes per node more than without;
- * where that would leave less than an eighth of the device's memory free, the
- * two-kernel stages run). */
+ * call.  The second flux buffer (three fields) is allocated with the first such
+ * step.  In FP32, and in FP64 with dissipation, only where that leaves an eighth
+ * of the device's memory free; otherwise the two-kernel stages run, until a call
+ * of this function has the next step look again. */
 int wt_workspace_set_fused(wt_ws* ws, int on);
 
 /* ---- right-hand sides (device pointers, async) ------------------------------*/

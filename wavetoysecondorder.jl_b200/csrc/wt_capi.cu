@@ -76,7 +76,8 @@ struct wt_ws {
   bool mu_done = false;  // mu is computed on first use (Kreiss-Oliger or wt_workspace_mu)
   void* F = nullptr;      // 3 nn
   void* F2 = nullptr;     // n = 8 fused stages: the second flux buffer (F ping-pongs between launches)
-  int fused = 1;          // FP64 n = 8 RK4 steps through the fused stage kernel (wt_workspace_set_fused)
+  int fused = 1;          // n = 8 RK4 steps through the fused stage kernel (wt_workspace_set_fused)
+  int f2_short = 0, ko_short = 0;  // F2, ko: there was no room for it (see room)
   void* bbuf = nullptr;   // nbf N^2
   void* grad = nullptr;   // 3 nn
   void* kP = nullptr;     // nn (Phidot / u_t slope)
@@ -347,10 +348,32 @@ bool fused_form(const wt_ws* ws, double eps_ko) {
   if (m.precision == WT_F64) return eps_ko == 0.0 || ko_fused(m);
   return eps_ko == 0.0 && compensated(m, true);
 }
-// the fused stages' second flux buffer
-int fused_buffer(wt_ws* ws) {
+
+// Whether a buffer that only makes steps faster leaves an eighth of the device's memory
+// free (and may be allocated at all: not while the caller captures the stream).  Where it
+// does not, the step runs without it, and the workspace does not ask again on every call.
+bool room(wt_ctx* ctx, size_t bytes) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  size_t avail = 0, total = 0;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+      cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return avail >= bytes + total / 8;
+}
+
+// The fused stages' second flux buffer.  FP64 steps without dissipation always have it;
+// the others where there is room, else they run the two-kernel stages.
+int fused_buffer(wt_ws* ws, double eps_ko) {
   const wt::DevMesh& m = ws->mesh->m;
-  return ensure(ws, &ws->F2, 3 * (size_t)wt::n8_padded_field_size(m.Ne) * rsize(m.precision));
+  const size_t bytes = 3 * (size_t)wt::n8_padded_field_size(m.Ne) * rsize(m.precision);
+  if (ws->F2) return 0;
+  if (m.precision == WT_F32 || eps_ko != 0.0) {
+    if (!ws->f2_short && !room(ws->ctx, bytes)) ws->f2_short = 1;
+    if (ws->f2_short) return 0;
+  }
+  return ensure(ws, &ws->F2, bytes);
 }
 
 int ws_step_buffers(wt_ws* ws) {
@@ -359,6 +382,7 @@ int ws_step_buffers(wt_ws* ws) {
   WT_TRY(ws_buffers(ws));
   WT_TRY(ensure(ws, &ws->S0, nb));
   WT_TRY(ensure(ws, &ws->S1, nb));
+  WT_TRY(ensure(ws, &ws->SQ, nb));
   WT_TRY(ensure(ws, &ws->accP, nb));
   WT_TRY(ensure(ws, &ws->accQ, nb));
   if (m.precision == WT_F32) {
@@ -366,19 +390,6 @@ int ws_step_buffers(wt_ws* ws) {
     WT_TRY(ensure(ws, &ws->compQ, nb));
     WT_TRY(ensure(ws, &ws->kP, nb));  // the compensated form's copy of Phi's high part (stage 2 -> 3)
   }
-  // Last, as the fused FP32 stages' second flux buffer is not a must: where it would
-  // leave less than an eighth of the device free, the two-kernel stages run.  Their
-  // Pi, SQ, which the fused stages do not use, takes its first field.
-  if (m.precision == WT_F32 && !ws->SQ && !ws->F2 && fused_form(ws, 0.0)) {
-    size_t avail = 0, total = 0;
-    const size_t need = 3 * (size_t)wt::n8_padded_field_size(m.Ne) * sizeof(float);
-    if (cudaMemGetInfo(&avail, &total) != cudaSuccess) cudaGetLastError();
-    if (avail >= need + total / 8) {
-      WT_TRY(fused_buffer(ws));
-      ws->SQ = ws->F2;
-    }
-  }
-  WT_TRY(ensure(ws, &ws->SQ, nb));
   return 0;
 }
 
@@ -506,8 +517,11 @@ bool ko_fused(const wt::DevMesh& m) { return m.precision == WT_F64 && wt::ko_all
 int ko_buffers(wt_ws* ws) {
   const wt::DevMesh& m = ws->mesh->m;
   const size_t nb = (size_t)m.nn * rsize(m.precision);
-  if (ko_split(m)) return ensure(ws, &ws->ko, 6 * nb);
-  WT_TRY(ws_buffers(ws));  // F: the scratch of meshes without straight lines
+  if (ws->ko) return 0;
+  if (ko_split(m) && !ws->ko_short) {
+    if (room(ws->ctx, 6 * nb)) return ensure(ws, &ws->ko, 6 * nb);
+    ws->ko_short = 1;
+  }
   return ws_k_buffers(ws);
 }
 
@@ -518,7 +532,7 @@ int ko_increments(wt_ctx* ctx, wt_ws* ws, const void* P, const void* Q, double e
   const wt::DevMesh& m = ws->mesh->m;
   const size_t nb = (size_t)m.nn * rsize(m.precision);
   const double koT = eps_ko * ws->inv_mu5;
-  const bool split = ko_split(m);
+  const bool split = ws->ko != nullptr;
   void* bufP = split ? ws->ko : ws->kP;
   void* bufQ = split ? (void*)((char*)ws->ko + 3 * nb) : ws->kQ;
   *koP = bufP;
@@ -1260,7 +1274,6 @@ int wt_workspace_create(wt_ctx* ctx, wt_mesh* mesh, wt_ws** out) {
 int wt_workspace_destroy(wt_ws* ws) {
   if (!ws) return WT_EINVAL;
   cudaStreamSynchronize(ws->ctx->stream);
-  if (ws->SQ == ws->F2) ws->SQ = nullptr;
   void* bufs[] = {ws->F, ws->F2, ws->bbuf, ws->grad, ws->kP, ws->kQ, ws->S0, ws->S1, ws->SQ, ws->accP, ws->accQ,
                   ws->trace, ws->trace2, ws->ko, ws->zero, ws->Lu, ws->compP, ws->compQ, ws->erk, ws->evo[0], ws->evo[1],
                   ws->evo[2], ws->evo[3], ws->evoE};
@@ -1272,6 +1285,7 @@ int wt_workspace_destroy(wt_ws* ws) {
 int wt_workspace_set_fused(wt_ws* ws, int on) {
   if (!ws) return WT_EINVAL;
   ws->fused = on ? 1 : 0;
+  ws->f2_short = 0;
   return 0;
 }
 
@@ -1662,6 +1676,20 @@ static int rk4_stage_part(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi
   return 0;
 }
 
+// Whether a step of these arguments has fused stages (step_curved_fused), given the
+// second flux buffer.
+static bool fused_path(const wt_ws* ws, const wt_coef* coef, void* Phi, void* Pi, double eps_ko,
+                       const wt::ConsBC& b, int use_metric) {
+  const wt::DevMesh& m = ws->mesh->m;
+  if (!fused_form(ws, eps_ko)) return false;
+  wt::RKStage r;
+  r.on = 1;
+  r.y = Phi; r.acc = ws->accP; r.out = ws->S0;
+  wt::RKStage q = r;
+  q.y = Pi; q.acc = ws->accQ; q.out = ws->SQ;
+  return wt::cons_n8_path(m, coef->c, use_metric, b, r, q, {Phi, Pi, ws->F, ws->S1});
+}
+
 // The RK4 step of an n = 8 solve (FP64, or FP32 in the compensated form without
 // dissipation) through the fused stage kernel: K1_0,
 // FK_0, FK_1, FK_2 (each the K2 half of stage s and the K1 half of stage s + 1),
@@ -1669,18 +1697,6 @@ static int rk4_stage_part(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi
 // and ws->F2.  Time-dependent backgrounds are re-sampled before the launch
 // whose K1 half reads them (the K2 halves read no coefficients).  The results
 // equal those of the two-kernel stages bit for bit.
-static bool fused_path(const wt_ws* ws, const wt_coef* coef, void* Phi, void* Pi, double eps_ko,
-                       const wt::ConsBC& b, int use_metric) {
-  const wt::DevMesh& m = ws->mesh->m;
-  if (!fused_form(ws, eps_ko) || !ws->F2) return false;
-  wt::RKStage r;
-  r.on = 1;
-  r.y = Phi; r.acc = ws->accP; r.out = ws->S0;
-  wt::RKStage q = r;
-  q.y = Pi; q.acc = ws->accQ; q.out = ws->SQ;
-  return wt::cons_n8_path(m, coef->c, use_metric, b, r, q, {Phi, Pi, ws->F, ws->F2, ws->S1});
-}
-
 static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, void* Pi, double dt,
                              double eps_ko, const wt::ConsBC& b, int use_metric) {
   const wt::DevMesh& m = ws->mesh->m;
@@ -1756,7 +1772,7 @@ static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* 
 
 static int step_curved_once(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, void* Pi, double dt,
                             double eps_ko, const wt::ConsBC& b, int use_metric) {
-  if (fused_path(ws, coef, Phi, Pi, eps_ko, b, use_metric))
+  if (ws->F2 && fused_path(ws, coef, Phi, Pi, eps_ko, b, use_metric))
     return step_curved_fused(ctx, ws, coef, Phi, Pi, dt, eps_ko, b, use_metric);
   const wt::DevMesh& m = ws->mesh->m;
   cudaStream_t s = ctx->stream;
@@ -1923,8 +1939,8 @@ int wt_step_rk4_curved(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, v
   wt::ConsBC b;
   WT_TRY(make_bc(ctx, bc, use_metric, b));
   WT_TRY(ws_step_buffers(ws));
-  if (fused_form(ws, eps_ko) && ws->mesh->m.precision == WT_F64) WT_TRY(fused_buffer(ws));
   if (eps_ko != 0.0 && ko_fused(ws->mesh->m)) WT_TRY(ko_buffers(ws));
+  if (fused_path(ws, coef, Phi, Pi, eps_ko, b, use_metric)) WT_TRY(fused_buffer(ws, eps_ko));
   if (eps_ko != 0.0) WT_TRY(ensure_mu(ws));
   if (coef->td) WT_TRY(need_setup_geometry(coef->mesh, "wt_step_rk4_curved (time-dependent background)"));
   comp_track(ws, Phi, Pi);
