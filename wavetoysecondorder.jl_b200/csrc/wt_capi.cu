@@ -2658,8 +2658,8 @@ int batch_one_step(wt_batch* b, cudaStream_t s) {
 }
 
 // Time K1 and K2 of stage 0 of a generic group in each launch variant
-// (elements per CTA) and keep the fastest of each (stage 0 writes only stage
-// scratch, never the solution state).  epb_variant: bits 0-1 K1's choice, bits
+// of its own CTA shape and keep the fastest of each (stage 0 writes only stage
+// scratch, never the solution state; orders with one shape: nothing to time).  epb_variant: bits 0-1 K1's choice, bits
 // 2-3 K2's.  A variant fixed by wt_batch_set_variant is kept untimed.
 int batch_tune_group(wt_batch* b, wt_batch::Group& g) {
   cudaStream_t s = b->ctx->own_stream;
@@ -2667,7 +2667,7 @@ int batch_tune_group(wt_batch* b, wt_batch::Group& g) {
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   int choice = 0, rc = 0;
-  const int nvar = wt::cons_gen_third_variant(g.N) ? 3 : 2;
+  const int nvar = wt::cons_gen_variants(g.N), shapes = wt::cons_gen_shapes(g.N);
   for (int which = 1; which <= 2 && !rc; ++which) {
     const int sh = 2 * (which - 1);
     if (b->force_var[which - 1] >= 0) {
@@ -2676,7 +2676,7 @@ int batch_tune_group(wt_batch* b, wt_batch::Group& g) {
     }
     float best = 1e30f;
     int best_v = 0;
-    for (int v = 0; v < nvar && !rc; ++v) {
+    for (int v = 0; v < shapes && shapes > 1 && !rc; ++v) {
       g.epb_variant = (choice & ~(3 << sh)) | (v << sh);
       for (int rep = 0; rep < 2 && !rc; ++rep) rc = batch_launch(b, g, which, 0, s);  // warm up
       cudaEventRecord(e0, s);
@@ -2761,7 +2761,7 @@ int batch_rebuild(wt_batch* b) {
       if (!g.n8) WT_TRY(batch_tune_group(b, g));
   } else {
     for (auto& g : b->groups) {  // untuned: the fixed variants, else the default one
-      const int nvar = wt::cons_gen_third_variant(g.N) ? 3 : 2;
+      const int nvar = wt::cons_gen_variants(g.N);
       int v[2];
       for (int w = 0; w < 2; ++w) v[w] = b->force_var[w] >= 0 && b->force_var[w] < nvar ? b->force_var[w] : 0;
       g.epb_variant = g.n8 ? 0 : v[0] | (v[1] << 2);

@@ -919,8 +919,14 @@ static int gen_batch(int which, bool cp, int variant, const void* plist, const i
   return k2_run<N, real, true, true>(K2P<real>(), O, plist, tiles, ntiles, variant, s);
 }
 
-// orders with a third CTA shape (variant 2)
-bool cons_gen_third_variant(int N) { return N == 4 || N == 6; }
+// The launch variants a batch may be given (variant 2: n = 4 and 6), and how many of them
+// are different CTA shapes: n = 4 three, two or one element a CTA, n = 5 two or one; from
+// n = 6 a CTA holds one element whichever is asked for.
+int cons_gen_variants(int N) { return N == 4 || N == 6 ? 3 : 2; }
+template <int N>
+static int gen_shapes() {
+  return Pen<N>::EPB == 1 ? 1 : cons_gen_variants(N) == 3 && (Pen<N>::EPB + 1) / 2 > 1 ? 3 : 2;
+}
 
 size_t cons_gen_param_size(int precision, int which) {
   if (precision == 0) return which == 1 ? sizeof(K1P<double>) : sizeof(K2P<double>);
@@ -969,6 +975,8 @@ bool cons_n8_path(const DevMesh& m, const DevCoef& c, int use_metric, const Cons
     if (!a16(p)) return false;
   return a16(c.c10) && a16(m.invdetJ_r);
 }
+
+int cons_gen_shapes(int N) { WT_DISPATCH_N(N, (gen_shapes<NN>())); }
 
 bool cons_gen_cp_supported(const DevMesh& m) { return gen_cp(m, nullptr); }
 

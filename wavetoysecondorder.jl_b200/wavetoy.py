@@ -626,7 +626,8 @@ class Batch(_Child):
 
     def set_variant(self, k1: int = -1, k2: int = -1):
         """Fix the launch variants of the generic groups' K1 and K2 (wt_batch_set_variant): 0 the default
-        elements per CTA, 1 half of it, 2 one (n = 4, 6); -1 leaves the choice to the autotuner."""
+        elements per CTA, 1 half of it, 2 one (n = 4, 6); the same launch from n = 6, where a CTA holds
+        one element; -1 leaves the choice to the autotuner."""
         self.ctx.check(library().wt_batch_set_variant(self.h, int(k1), int(k2)), "wt_batch_set_variant")
 
     def step(self, nsteps: int = 1):
