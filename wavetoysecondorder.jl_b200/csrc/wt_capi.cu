@@ -501,11 +501,12 @@ int ko_add2(wt_ctx* ctx, const wt::DevMesh& m, void* dstP, const void* fP, void*
 // Where the dissipation increments of a fused RK4 stage go.  Split: one launch
 // writes the three axes' parts of both fields (6 nn words, added where they are
 // consumed); otherwise three launches sum them into kP, kQ.  Both move 9 words per
-// node and field.  Split up to kKoSplitNodes nodes, where two launches a stage
-// count and the extra 4 nn words of memory do not: ten SIPG steps on 4^3 elements,
-// n = 6, 623 us against 815 us; one step on 40^3 (13.8M nodes) 4.04 ms split
-// against 3.69 ms summed, the destination then staying in L2 from axis to axis.
-constexpr long long kKoSplitNodes = 4 << 20;
+// node and field.  Split where two launches a stage weigh more than the destination's
+// staying in L2 from axis to axis (and its 4 nn words less of memory).  Four steps
+// (B200, FP64), split / summed: SIPG n = 6, 46,656 nodes 185 / 213 us, 216,000 274 / 379,
+// 373,248 409 / 468, 592,704 599 / 607, 884,736 950 / 838, 13.8 million 15.1 / 13.4 ms; RK4
+// n = 8, 512,000 nodes 1.13 / 1.21 ms, 884,736 1.72 / 1.69; n = 4 and 6 turn at 330,000.
+constexpr long long kKoSplitNodes = 1 << 19;
 bool ko_split(const wt::DevMesh& m) { return wt::ko_all_lines(m) && m.nn <= kKoSplitNodes; }
 
 // Whether the RK4 stages of a dissipative solve add the increments inside K1 and K2
