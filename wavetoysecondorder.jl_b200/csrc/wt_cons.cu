@@ -239,7 +239,7 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long n, int i
 template <int N>
 struct Pen {
   static constexpr int N2 = N * N, N3 = N * N * N, TE = 3 * N2;
-  static constexpr int EPB = TE >= 96 ? 1 : 160 / TE;  // the most elements a CTA holds
+  static constexpr int EPB = TE >= 96 ? 1 : N == 2 ? 8 : 160 / TE;  // the most elements a CTA holds (n = 2: 13 are 5-8 % slower)
   static constexpr int T = TE * EPB;
   static constexpr int P1 = N | 1;       // odd row pitch: x pencils without bank conflicts
   static constexpr int NS = N * N * P1;  // words of one padded field of an element
@@ -248,8 +248,16 @@ struct Pen {
   // registers, a few spills; 576 without spills took 15-30 % longer), N = 6: 640
   // with the node pass's words prefetched (pf1), N = 7: 600, N = 8: 448 (at 768 the pencils
   // spill: N = 7 33 % slower); FP32: 1024.
-  template <typename real>
-  static constexpr int occ() { return (sizeof(real) == 4 ? 1024 : N == 8 ? 448 : N == 7 ? 600 : N == 6 ? 640 : 768) / T; }
+  // The affine form (CURV false) at N = 2 and 4, where the node pass is most of the work,
+  // waits on its loads and takes more threads: one right-hand side of 1.5 million nodes, FP64
+  // N = 4 96.0 -> 83.5 us, N = 2 112 -> 93.5; FP32 N = 4 69.0 -> 67.0, N = 2 83 -> 72 (a
+  // thread per node: 88.5, 102.8, 66.0, 72.2).
+  template <typename real, bool CURV>
+  static constexpr int occ() {
+    constexpr bool F32 = sizeof(real) == 4;
+    if (!CURV && (N == 2 || N == 4)) return (F32 && N == 2 ? 1536 : 1280) / T;
+    return (F32 ? 1024 : N == 8 ? 448 : N == 7 ? 600 : N == 6 ? 640 : 768) / T;
+  }
   // Whether K1 copies the node pass's words (coefficients, Pi, 1/J, RK words) to
   // shared memory at kernel start: it hides their latency and costs resident
   // CTAs.  24^3 elements, one step (B200): N = 6 FP64 971 us with, 1044 without;
@@ -296,7 +304,7 @@ constexpr int k1_words() {
 //   0.5 D(Ja u) + 0.5 Ja D u = (Ja0 + 0.5 dJa) D u + 0.5 D(dJa u),
 // and only the last contraction, of the small dJa u, runs in FP32.
 template <int N, typename real, bool CURV, bool BATCH, bool CP>
-__global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
+__global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real, CURV>())
     k_cons_k1(const __grid_constant__ K1P<real> P0, const __grid_constant__ OpP<N, real> O,
               const K1P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles, int epb, int dfw) {
   using L = Pen<N>;
@@ -555,7 +563,7 @@ constexpr int k2_words() {
 }
 
 template <int N, typename real, bool CURV, bool BATCH>
-__global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real>())
+__global__ void __launch_bounds__(Pen<N>::T, Pen<N>::template occ<real, CURV>())
     k_cons_k2(const __grid_constant__ K2P<real> P0, const __grid_constant__ OpP<N, real> O,
               const K2P<real>* __restrict__ plist, const int2* __restrict__ tiles, long long ntiles, int epb) {
   using L = Pen<N>;
