@@ -2532,14 +2532,8 @@ static K2N8<real> k2n8_params(const DevMesh& m, const void* F, void* Pidot, cons
 template <int HALF, bool BATCH>
 static int n8d_launch(const FKN8& P, const void* plA, const void* plB, const int2* tiles, long long ntiles,
                       cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_cons_fk_n8<HALF, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)fk_smem(HALF)) != cudaSuccess)
-      return -2;
-    attr = true;
-  }
   if (ntiles <= 0) return 0;
+  if (allow_smem(k_cons_fk_n8<HALF, BATCH>, fk_smem(HALF))) return -2;
   return launch_dep<!BATCH>(k_cons_fk_n8<HALF, BATCH>, (unsigned)ntiles, FK_THREADS, fk_smem(HALF), s, P,
                     (const K2N8<double>*)plA, (const K1N8<double>*)plB, tiles);
 }
@@ -2548,26 +2542,15 @@ static int n8d_launch(const FKN8& P, const void* plA, const void* plB, const int
 // (plist == nullptr, ntiles = P.Ne) or a work list over the solves of plist.
 template <typename real, int NT, bool BATCH>
 static int n8_launch(int which, const void* hP, const void* plist, const int2* tiles, long long ntiles, cudaStream_t s) {
-  static bool attr1 = false, attr2 = false;
   if (which == 1) {
-    if (!attr1) {
-      if (cudaFuncSetAttribute(k_cons_k1_n8<real, NT, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)k1_smem<real>()) != cudaSuccess)
-        return -2;
-      attr1 = true;
-    }
+    if (allow_smem(k_cons_k1_n8<real, NT, BATCH>, k1_smem<real>())) return -2;
     const long long cap = (long long)sm_count() * n8::OCC;
     const long long grid = ntiles < cap ? ntiles : cap;
     if (grid <= 0) return 0;
     k_cons_k1_n8<real, NT, BATCH><<<(unsigned)grid, n8::THREADS, k1_smem<real>(), s>>>(
         *(const K1N8<real>*)hP, (const K1N8<real>*)plist, tiles, ntiles);
   } else {
-    if (!attr2) {
-      if (cudaFuncSetAttribute(k_cons_k2_n8<real, NT, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)k2_smem<real>()) != cudaSuccess)
-        return -2;
-      attr2 = true;
-    }
+    if (allow_smem(k_cons_k2_n8<real, NT, BATCH>, k2_smem<real>())) return -2;
     const long long cap = (long long)sm_count() * n8::OCC;
     const long long grid = ntiles < cap ? ntiles : cap;
     if (grid <= 0) return 0;
@@ -2580,33 +2563,18 @@ static int n8_launch(int which, const void* hP, const void* plist, const int2* t
 template <bool BATCH>
 static int n8c_launch(int which, const void* hP, const void* plist, const int2* tiles, long long ntiles,
                       cudaStream_t s) {
-  static bool attr1 = false, attr2 = false;
   const int occ = which == 1 ? K1C_OCC : K2C_OCC;
   const long long cap = (long long)sm_count() * occ;
   const long long grid = ntiles < cap ? ntiles : cap;
   if (which == 1) {
     constexpr size_t smem = k1c_smem();
-    if (!attr1) {
-      // three CTAs per SM need (nearly) all of the SM's shared memory
-      if (cudaFuncSetAttribute(k_cons_k1_n8c<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem) != cudaSuccess ||
-          cudaFuncSetAttribute(k_cons_k1_n8c<BATCH>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-        return -2;
-      attr1 = true;
-    }
+    // three CTAs per SM need (nearly) all of the SM's shared memory
+    if (allow_smem(k_cons_k1_n8c<BATCH>, smem, true)) return -2;
     if (grid <= 0) return 0;
     k_cons_k1_n8c<BATCH><<<(unsigned)grid, n8::CTHR, smem, s>>>(
         *(const K1N8<float>*)hP, (const K1N8<float>*)plist, tiles, ntiles);
   } else {
-    if (!attr2) {
-      if (cudaFuncSetAttribute(k_cons_k2_n8c<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k2c_smem()) !=
-              cudaSuccess ||
-          cudaFuncSetAttribute(k_cons_k2_n8c<BATCH>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-        return -2;
-      attr2 = true;
-    }
+    if (allow_smem(k_cons_k2_n8c<BATCH>, k2c_smem(), true)) return -2;
     if (grid <= 0) return 0;
     k_cons_k2_n8c<BATCH><<<(unsigned)grid, n8::CTHR, k2c_smem(), s>>>(*(const K2N8<float>*)hP,
                                                                        (const K2N8<float>*)plist, tiles, ntiles);
@@ -2618,16 +2586,8 @@ static int n8c_launch(int which, const void* hP, const void* plist, const int2* 
 template <int HALF, bool BATCH>
 static int cc_launch(const FKT<float>& P, const void* plA, const void* plB, const int2* tiles, long long ntiles,
                      cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_cons_cc_n8<HALF, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)cc_smem(HALF)) != cudaSuccess ||
-        cudaFuncSetAttribute(k_cons_cc_n8<HALF, BATCH>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-      return -2;
-    attr = true;
-  }
   if (ntiles <= 0) return 0;
+  if (allow_smem(k_cons_cc_n8<HALF, BATCH>, cc_smem(HALF), true)) return -2;
   return launch_dep<!BATCH>(k_cons_cc_n8<HALF, BATCH>, (unsigned)ntiles, n8::CTHR, cc_smem(HALF), s, P,
                             (const K2N8<float>*)plA, (const K1N8<float>*)plB, tiles);
 }
@@ -2707,27 +2667,13 @@ template <typename real, int NT>
 static int launch_grad_n8_t(const K1N8<real>& P, bool cuda_core, cudaStream_t s) {
   if constexpr (std::is_same<real, float>::value) {
     if (cuda_core) {
-      static bool attr = false;
-      if (!attr) {
-        if (cudaFuncSetAttribute(k_cons_k1_n8c<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)k1c_smem()) != cudaSuccess ||
-            cudaFuncSetAttribute(k_cons_k1_n8c<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-          return -2;
-        attr = true;
-      }
+      if (allow_smem(k_cons_k1_n8c<false, true>, k1c_smem(), true)) return -2;
       const long long cap = (long long)sm_count() * K1C_OCC, grid = P.Ne < cap ? P.Ne : cap;
       k_cons_k1_n8c<false, true><<<(unsigned)grid, n8::CTHR, k1c_smem(), s>>>(P, nullptr, nullptr, P.Ne);
       return cudaGetLastError() == cudaSuccess ? 0 : -2;
     }
   }
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_cons_k1_n8<real, NT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)k1_smem<real>()) != cudaSuccess)
-      return -2;
-    attr = true;
-  }
+  if (allow_smem(k_cons_k1_n8<real, NT, false, true>, k1_smem<real>())) return -2;
   const long long cap = (long long)sm_count() * n8::OCC, grid = P.Ne < cap ? P.Ne : cap;
   k_cons_k1_n8<real, NT, false, true><<<(unsigned)grid, n8::THREADS, k1_smem<real>(), s>>>(P, nullptr, nullptr, P.Ne);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

@@ -43,4 +43,17 @@ int launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStr
   return cudaLaunchKernelEx(&cfg, kernel, P(a)...) == cudaSuccess ? 0 : -2;
 }
 
+// Let a kernel have `bytes` of dynamic shared memory, and (carveout) the SM give shared
+// memory all it can, where the kernel's CTAs need it to be resident as planned.  Called
+// before each launch: the attributes belong to the current device, and a process may
+// have contexts on several, or reset one (under 1 us a call; steps replay a graph).
+template <typename K>
+int allow_smem(K kernel, size_t bytes, bool carveout = false) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return -2;
+  if (carveout && cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+    return -2;
+  return 0;
+}
+
 }  // namespace wt
