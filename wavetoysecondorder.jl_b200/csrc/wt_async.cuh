@@ -23,14 +23,4 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int n>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(n) : "memory"); }
 
-// 4- or 8-byte cp.async, zero-filled (src not read) when !valid
-template <typename T>
-__device__ __forceinline__ void cp_async_word_z(T* dst, const T* src, bool valid) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 8)
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(valid ? 8 : 0) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(valid ? 4 : 0) : "memory");
-}
-
 }  // namespace wt

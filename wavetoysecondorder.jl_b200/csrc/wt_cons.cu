@@ -45,13 +45,10 @@ struct K1P {
   const real* Ja;
   const real* invdetJ;
   const real* sdiag;
-  const int32_t* nbr;
-  const int32_t* nbrf;
   const int32_t* bdry;
   const int32_t* bslot;
   const int32_t* emask;  // per element: SAT face mask (bits 0-5), outer face (bit 6)
   const int32_t* fsrc;   // per (f,e): 8 * neighbour + neighbour face, -1 without SAT
-  const double* G;
   const double* H;
   real* F;
   real* Phidot;
@@ -534,14 +531,10 @@ struct K2P {
   const real* Ja;
   const real* invdetJ;
   const real* sdiag;
-  const int32_t* nbr;
-  const int32_t* nbrf;
   const int32_t* bdry;
   const int32_t* bslot;
   const int32_t* emask;
   const int32_t* fsrc;
-  const double* G;
-  const double* H;
   const real* bbuf;
   int bc_on, nbf;
   real* Pidot;
@@ -781,9 +774,9 @@ static K1P<real> k1p_params(const DevMesh& m, const DevCoef& c, const void* Phi,
   P.Phi = (const real*)Phi; P.Pi = (const real*)Pi;
   P.c10 = (const real*)c.c10;
   P.Ja = (const real*)m.Ja_r; P.invdetJ = (const real*)m.invdetJ_r; P.sdiag = (const real*)m.sdiag;
-  P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot;
+  P.bdry = m.bdry; P.bslot = m.bslot;
   P.emask = m.emask; P.fsrc = m.fsrc;
-  P.G = m.G; P.H = m.H;
+  P.H = m.H;
   P.F = (real*)F; P.Phidot = (real*)Phidot; P.bbuf = (real*)bbuf; P.grad_out = (real*)grad_out;
   P.bc_on = bc.on; P.bc_curv = bc.curv; P.exc_tag = bc.exc_tag; P.nbf = m.nbf;
   for (int f = 0; f < 6; ++f) P.kinds[f] = bc.kinds[f];
@@ -813,9 +806,8 @@ static K2P<real> k2p_params(const DevMesh& m, const void* F, void* Pidot, const 
   P.F1 = F1 ? (const real*)F1 : (const real*)F + m.nn;
   P.F2 = F2 ? (const real*)F2 : (const real*)F + 2 * m.nn;
   P.Ja = (const real*)m.Ja_r; P.invdetJ = (const real*)m.invdetJ_r; P.sdiag = (const real*)m.sdiag;
-  P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot;
+  P.bdry = m.bdry; P.bslot = m.bslot;
   P.emask = m.emask; P.fsrc = m.fsrc;
-  P.G = m.G; P.H = m.H;
   P.bbuf = (const real*)bbuf; P.bc_on = bc.on; P.nbf = m.nbf;
   P.Pidot = (real*)Pidot;
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;

@@ -223,7 +223,7 @@ constexpr int OCC = 2;  // resident CTAs per SM of the split-BF16 kernels
 
 }  // namespace n8
 
-// RK4 stage update shared by both kernels (see rk_epilogue in wt_cons.cu):
+// RK4 stage update shared by both kernels (see rk_epilogue_v in wt_rk.cuh):
 // with comp (FP32 state) acc holds the step increment and the final sum is
 // Kahan-compensated, comp holding the low part the FP32 state lost (the state
 // is y + comp); yv, accv, compv are this node's prefetched values.
@@ -276,8 +276,6 @@ struct K1N8 {
   const real* c10;
   const real* Ja;
   const real* invdetJ;
-  const int32_t* nbr;
-  const int32_t* nbrf;
   const int32_t* bdry;
   const int32_t* bslot;
   const int32_t* emask;
@@ -520,8 +518,7 @@ __global__ void __launch_bounds__(n8::THREADS, n8::OCC)
     src1 = src_load(t1);
   }
   __syncthreads();
-  // A operand: FP64 G entries (rows gq, columns tig and 4 + tig); FP32 split pairs
-  double aG0 = 0.0, aG1 = 0.0;
+  // A operand: split pairs of G
   uint32_t aS[4] = {0, 0, 0, 0}, aS2[4] = {0, 0, 0, 0};
   split_G(sG, gq, tig, NT, aS, aS2);
 
@@ -693,8 +690,6 @@ struct K2N8 {
   const real* F2;
   const real* Ja;
   const real* invdetJ;
-  const int32_t* nbr;
-  const int32_t* nbrf;
   const int32_t* bdry;
   const int32_t* bslot;
   const int32_t* emask;
@@ -860,7 +855,6 @@ __global__ void __launch_bounds__(n8::THREADS, n8::OCC)
     src_load(t1, src1);
   }
   __syncthreads();
-  double aG0 = 0.0, aG1 = 0.0;
   uint32_t aS[4] = {0, 0, 0, 0}, aS2[4] = {0, 0, 0, 0};
   split_G(sG, gq, tig, NT, aS, aS2);
 
@@ -1064,14 +1058,11 @@ static_assert(3 * (fk_smem(N8_FK) + 64 + 1024) <= 233472, "three CTAs of the fus
 
 namespace n8 {
 // per-thread 8-byte asynchronous copy global -> shared, zero-filled when !valid
-// (src must still be a valid address); commit / wait for all groups but the
-// newest / wait for all (cp_async_wait_all)
+// (src must still be a valid address); wait for all of them
 __device__ __forceinline__ void cp_async8z(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 8 : 0)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_prior() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 }  // namespace n8
 
@@ -2481,7 +2472,7 @@ static K1N8<real> k1n8_params(const DevMesh& m, const DevCoef& c, const void* Ph
   P.Ne = m.Ne; P.nn = m.nn; P.e0 = 0;
   P.Phi = (const real*)Phi; P.Pi = (const real*)Pi; P.c10 = (const real*)c.c10;
   P.Ja = (const real*)m.Ja_n8; P.invdetJ = (const real*)m.invdetJ_r;
-  P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot; P.G = m.G; P.H = m.H;
+  P.bdry = m.bdry; P.bslot = m.bslot; P.G = m.G; P.H = m.H;
   P.inv2H = 1.0 / (2.0 * m.ops.H[0]);
   P.emask = m.emask; P.fsrc = m.fsrc;
   P.F = (real*)F; P.Phidot = (real*)Phidot; P.bbuf = (real*)bbuf;
@@ -2512,7 +2503,7 @@ static K2N8<real> k2n8_params(const DevMesh& m, const void* F, void* Pidot, cons
   const long long fs = m.Ne * n8_fs(m);
   P.F0 = (const real*)F; P.F1 = (const real*)F + fs; P.F2 = (const real*)F + 2 * fs;
   P.Ja = (const real*)m.Ja_n8; P.invdetJ = (const real*)m.invdetJ_r;
-  P.nbr = m.nbr; P.nbrf = m.nbrf; P.bdry = m.bdry; P.bslot = m.bslot; P.G = m.G; P.H = m.H;
+  P.bdry = m.bdry; P.bslot = m.bslot; P.G = m.G; P.H = m.H;
   P.inv2H = 1.0 / (2.0 * m.ops.H[0]);
   P.emask = m.emask; P.fsrc = m.fsrc;
   P.bbuf = (const real*)bbuf; P.bc_on = bc.on; P.nbf = m.nbf;

@@ -124,7 +124,7 @@ __global__ void k_rk_update(long long n, int stage, double dt, real* __restrict_
                             real* __restrict__ out, const real* __restrict__ k, real* __restrict__ comp) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const real kv = k[i];
-    if (comp) {  // increment form with a Kahan-compensated final sum (see rk_epilogue)
+    if (comp) {  // increment form with a Kahan-compensated final sum (see rk_epilogue_v)
       if (stage == 0) {
         out[i] = y[i] + (real)(0.5 * dt) * kv;
         acc[i] = (real)(dt / 6.0) * kv;

@@ -4,83 +4,13 @@
 
 namespace wt {
 
-// Low-storage classic RK4 stage update.  Without compensation acc holds
-// y + partial increments.  With compensation (FP32 state) acc holds the
-// increment of the step alone and the final y + increment is a Kahan sum; comp
-// holds the low part the FP32 y lost (the state is y + comp), so that small
-// increments are not lost to the rounding of y over many steps.
-template <typename real>
-__device__ __forceinline__ void rk_epilogue(int stage, double dt, real k, real yin, real* y, real* acc, real* out,
-                                            real* comp, long long n, unsigned int* nonfinite) {
-  if (comp) {
-    if (stage == 0) {
-      out[n] = yin + (real)(0.5 * dt) * k;
-      acc[n] = (real)(dt / 6.0) * k;
-    } else if (stage == 1) {
-      out[n] = y[n] + (real)(0.5 * dt) * k;
-      acc[n] = acc[n] + (real)(dt / 3.0) * k;
-    } else if (stage == 2) {
-      out[n] = y[n] + (real)dt * k;
-      acc[n] = acc[n] + (real)(dt / 3.0) * k;
-    } else {
-      const real inc = acc[n] + (real)(dt / 6.0) * k;
-      const real yv = y[n];
-      const real t = inc + comp[n];
-      const real v = yv + t;
-      comp[n] = t - (v - yv);
-      y[n] = v;
-      if (nonfinite && !isfinite((double)v)) atomicOr(nonfinite, 1u);
-    }
-    return;
-  }
-  if (stage == 0) {
-    out[n] = yin + (real)(0.5 * dt) * k;
-    acc[n] = yin + (real)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = y[n] + (real)(0.5 * dt) * k;
-    acc[n] = acc[n] + (real)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = y[n] + (real)dt * k;
-    acc[n] = acc[n] + (real)(dt / 3.0) * k;
-  } else {
-    real v = acc[n] + (real)(dt / 6.0) * k;
-    y[n] = v;
-    if (nonfinite && !isfinite((double)v)) atomicOr(nonfinite, 1u);
-  }
-}
-
-// RK4 stage update of the compensated FP32 form (the Phi side, K1): the state
-// is (y, comp) = (high, low part) and the stage the next K1 reads is its high
-// part plus out = low part + c dt k; the step's final sum is formed in FP64 and
-// split again.  hi: this node's high part of the state (the K1 input).
-__device__ __forceinline__ void rk_epilogue_cp(int stage, double dt, float k, float hi, float* y, float* acc,
-                                               float* out, float* comp, float* hcopy, long long n,
-                                               unsigned int* nonfinite) {
-  const float lo = comp[n];
-  if (stage == 0) {
-    out[n] = lo + (float)(0.5 * dt) * k;
-    acc[n] = (float)(dt / 6.0) * k;
-  } else if (stage == 1) {
-    out[n] = lo + (float)(0.5 * dt) * k;
-    acc[n] = acc[n] + (float)(dt / 3.0) * k;
-  } else if (stage == 2) {
-    out[n] = lo + (float)dt * k;
-    acc[n] = acc[n] + (float)(dt / 3.0) * k;
-    hcopy[n] = hi;
-  } else {
-    const float inc = acc[n] + (float)(dt / 6.0) * k;
-    const double v = (double)hi + ((double)lo + (double)inc);
-    const float h = (float)v;
-    y[n] = h;
-    comp[n] = (float)(v - (double)h);
-    if (nonfinite && !isfinite(h)) atomicOr(nonfinite, 1u);
-  }
-}
-
-// The RK4 stage updates above with the words they read at node n passed in
-// (yv = y[n], accv = acc[n], compv = comp[n]; only those the stage reads need
-// to be valid): the same arithmetic in the same order.  Returns the value the
-// stage wrote (the next stage's input, or the new state).
+// Low-storage classic RK4 stage update of node n, with the words it reads passed in
+// (yv = y[n], accv = acc[n], compv = comp[n]; only those the stage reads need to be
+// valid).  Without compensation acc holds y + partial increments.  With it (comp, FP32
+// state) acc holds the increment of the step alone and the final y + increment is a
+// Kahan sum; comp holds the low part the FP32 y lost (the state is y + comp), so that
+// small increments are not lost to the rounding of y over many steps.  Returns the
+// value the stage wrote (the next stage's input, or the new state).
 template <typename real>
 __device__ __forceinline__ real rk_epilogue_v(int stage, double dt, real k, real yin, real yv, real accv, real compv,
                                               real* y, real* acc, real* out, real* comp, long long n,
@@ -129,11 +59,13 @@ __device__ __forceinline__ real rk_epilogue_v(int stage, double dt, real k, real
   return v;
 }
 
-// rk_epilogue_cp with lov = comp[n] and accv = acc[n] passed in
-__device__ __forceinline__ void rk_epilogue_cp_v(int stage, double dt, float k, float hi, float lov, float accv,
+// The same of the compensated FP32 form (the Phi side, K1): the state is (y, comp) =
+// (high, low part) and the stage the next K1 reads is its high part plus out = low part +
+// c dt k; the step's final sum is formed in FP64 and split again.  hi: this node's high
+// part of the state (the K1 input); stage 2 copies it into hcopy, which stage 3 reads.
+__device__ __forceinline__ void rk_epilogue_cp_v(int stage, double dt, float k, float hi, float lo, float accv,
                                                  float* y, float* acc, float* out, float* comp, float* hcopy,
                                                  long long n, unsigned int* nonfinite) {
-  const float lo = lov;
   if (stage == 0) {
     out[n] = lo + (float)(0.5 * dt) * k;
     acc[n] = (float)(dt / 6.0) * k;
