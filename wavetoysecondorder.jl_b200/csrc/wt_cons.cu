@@ -785,7 +785,6 @@ static K1P<real> k1p_params(const DevMesh& m, const DevCoef& c, const void* Phi,
   P.gDx = (const real*)bc.gDx; P.gDy = (const real*)bc.gDy; P.gDz = (const real*)bc.gDz;
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.nonfinite = rk.nonfinite;
-  if (!rk.on) P.y = P.acc = (real*)Phi;  // not read, but never a null address to form a load from
   P.Phit = (const real*)rk.phit; P.dJa = (const real*)m.dJa; P.Ja0 = m.Ja0; P.hcopy = (real*)rk.hcopy;
   P.ko = (const real*)rk.ko; P.nko = rk.nko;
   return P;
@@ -812,7 +811,6 @@ static K2P<real> k2p_params(const DevMesh& m, const void* F, void* Pidot, const 
   P.Pidot = (real*)Pidot;
   P.epi = rk.on; P.stage = rk.stage; P.dt = rk.dt;
   P.y = (real*)rk.y; P.acc = (real*)rk.acc; P.out = (real*)rk.out; P.comp = (real*)rk.comp; P.nonfinite = nonfinite;
-  if (!rk.on) P.y = P.acc = (real*)P.F0;  // not read (see k1p_params)
   P.ko = (const real*)rk.ko; P.nko = rk.nko;
   return P;
 }
