@@ -331,11 +331,11 @@ int wt_workspace_set_mu(wt_ws* ws, double mu);
  * FP64, or in compensated FP32 without Kreiss-Oliger dissipation, steps through
  * the fused stage kernel, which runs the divergence half of stage s and the
  * gradient half of stage s + 1 in one launch (five launches per RK4 step instead
- * of eight, 28 % fewer DRAM bytes).  The results equal the two-kernel stages' bit
+ * of eight, 20 % fewer DRAM bytes).  The results equal the two-kernel stages' bit
  * for bit; on = 0 selects the two-kernel stages.  Takes effect at the next step
  * call.  The second flux buffer (three fields) is allocated with the first such
- * step.  In FP32, and in FP64 with dissipation, only where that leaves an eighth
- * of the device's memory free; otherwise the two-kernel stages run, until a call
+ * step.  In FP32, and in FP64 with dissipation, only where that leaves 1/32 of
+ * the device's memory free; otherwise the two-kernel stages run, until a call
  * of this function has the next step look again. */
 int wt_workspace_set_fused(wt_ws* ws, int on);
 

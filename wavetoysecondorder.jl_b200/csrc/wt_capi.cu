@@ -349,9 +349,10 @@ bool fused_form(const wt_ws* ws, double eps_ko) {
   return eps_ko == 0.0 && compensated(m, true);
 }
 
-// Whether a buffer that only makes steps faster leaves an eighth of the device's memory
-// free (and may be allocated at all: not while the caller captures the stream).  Where it
-// does not, the step runs without it, and the workspace does not ask again on every call.
+// Whether a buffer that only makes steps faster leaves 1/32 of the device's memory free
+// (and may be allocated at all: not while the caller captures the stream).  Where it does
+// not, the step runs without it, and the workspace does not ask again on every call.  No
+// more than that: a caller's own pool may hold most of the memory for good.
 bool room(wt_ctx* ctx, size_t bytes) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   size_t avail = 0, total = 0;
@@ -360,7 +361,7 @@ bool room(wt_ctx* ctx, size_t bytes) {
     cudaGetLastError();
     return false;
   }
-  return avail >= bytes + total / 8;
+  return avail >= bytes + total / 32;
 }
 
 // The fused stages' second flux buffer.  FP64 steps without dissipation always have it;
@@ -502,12 +503,17 @@ int ko_add2(wt_ctx* ctx, const wt::DevMesh& m, void* dstP, const void* fP, void*
 // writes the three axes' parts of both fields (6 nn words, added where they are
 // consumed); otherwise three launches sum them into kP, kQ.  Both move 9 words per
 // node and field.  Split where two launches a stage weigh more than the destination's
-// staying in L2 from axis to axis (and its 4 nn words less of memory).  Four steps
-// (B200, FP64), split / summed: SIPG n = 6, 46,656 nodes 185 / 213 us, 216,000 274 / 379,
-// 373,248 409 / 468, 592,704 599 / 607, 884,736 950 / 838, 13.8 million 15.1 / 13.4 ms; RK4
-// n = 8, 512,000 nodes 1.13 / 1.21 ms, 884,736 1.72 / 1.69; n = 4 and 6 turn at 330,000.
-constexpr long long kKoSplitNodes = 1 << 19;
-bool ko_split(const wt::DevMesh& m) { return wt::ko_all_lines(m) && m.nn <= kKoSplitNodes; }
+// staying in L2 from axis to axis.  Where that is, by the consumer, type and order (time
+// summed over time split, four steps of 0.2 / 0.35 / 0.6 / 1 / 2.6 / 8 million nodes, B200):
+// k_sipg FP32 n = 6 1.50 1.27 1.11 1.09 1.10 1.13 (n = 2 to 8 the like), FP64 n = 4 1.28 1.14
+// 1.06 0.98 1.02 1.05 (n = 2, 3, 5 the like), n = 6 1.36 1.15 0.99 0.85 0.85 0.85 (n = 7, 8 the
+// like); RK4 stages (FP64) n = 4 1.06 0.95 0.91 0.90 0.92 0.94 (n = 2 to 7 the like), n = 8
+// 1.27 1.16 1.01 0.98 0.93 0.93.  Above 4 million nodes always summed: four fields less of
+// memory.
+bool ko_split(const wt::DevMesh& m, bool sipg) {
+  const long long most = sipg ? (m.precision == WT_F32 || m.N <= 5 ? 4 << 20 : 1 << 19) : m.N == 8 ? 1 << 19 : 1 << 18;
+  return wt::ko_all_lines(m) && m.nn <= most;
+}
 
 // Whether the RK4 stages of a dissipative solve add the increments inside K1 and K2
 // (24^3 x 8^3 FP64 step: 3.43 ms with separate update kernels, 2.86 ms so).
@@ -515,25 +521,24 @@ bool ko_split(const wt::DevMesh& m) { return wt::ko_all_lines(m) && m.nn <= kKoS
 // compensated form and updates the state in the plain one.
 bool ko_fused(const wt::DevMesh& m) { return m.precision == WT_F64 && wt::ko_all_lines(m); }
 
-int ko_buffers(wt_ws* ws) {
+int ko_buffers(wt_ws* ws, bool sipg) {
   const wt::DevMesh& m = ws->mesh->m;
   const size_t nb = (size_t)m.nn * rsize(m.precision);
-  if (ws->ko) return 0;
-  if (ko_split(m) && !ws->ko_short) {
-    if (room(ws->ctx, 6 * nb)) return ensure(ws, &ws->ko, 6 * nb);
-    ws->ko_short = 1;
+  if (ko_split(m, sipg)) {
+    if (!ws->ko && !ws->ko_short && !room(ws->ctx, 6 * nb)) ws->ko_short = 1;
+    if (!ws->ko_short) return ensure(ws, &ws->ko, 6 * nb);
   }
   return ws_k_buffers(ws);
 }
 
 // The increments eps mu^-5 sum_d D_d^6 of P and Q (either may be NULL) for a fused
 // stage: nko fields each, nn words apart.
-int ko_increments(wt_ctx* ctx, wt_ws* ws, const void* P, const void* Q, double eps_ko, const void** koP,
+int ko_increments(wt_ctx* ctx, wt_ws* ws, const void* P, const void* Q, double eps_ko, bool sipg, const void** koP,
                   const void** koQ, int* nko) {
   const wt::DevMesh& m = ws->mesh->m;
   const size_t nb = (size_t)m.nn * rsize(m.precision);
   const double koT = eps_ko * ws->inv_mu5;
-  const bool split = ws->ko != nullptr;
+  const bool split = ws->ko && ko_split(m, sipg);
   void* bufP = split ? ws->ko : ws->kP;
   void* bufQ = split ? (void*)((char*)ws->ko + 3 * nb) : ws->kQ;
   *koP = bufP;
@@ -1729,7 +1734,7 @@ static int step_curved_fused(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* 
   // K2_s and K1_{s+1}, so before it come the increments of Phi_{s+1} and, except
   // for s = 0 (computed with Phi_0's), of the Pi_s that the launch before stored
   auto increments = [&](const void* P, const void* Q) -> int {
-    return ko ? ko_increments(ctx, ws, P, Q, eps_ko, &koP, &koQ, &nko) : 0;
+    return ko ? ko_increments(ctx, ws, P, Q, eps_ko, false, &koP, &koQ, &nko) : 0;
   };
   ws->halo_cp = cp ? 1 : 0;
   ws->flux_block = wt::n8_flux_block(m);
@@ -1786,7 +1791,7 @@ static int step_curved_once(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* P
     if (eps_ko == 0.0 || ko_fused(m)) {
       const void *koP = nullptr, *koQ = nullptr;
       int nko = 0;
-      if (eps_ko != 0.0) WT_TRY(ko_increments(ctx, ws, inP, inQ, eps_ko, &koP, &koQ, &nko));
+      if (eps_ko != 0.0) WT_TRY(ko_increments(ctx, ws, inP, inQ, eps_ko, false, &koP, &koQ, &nko));
       WT_TRY(rk4_stage_part(ctx, ws, coef, Phi, Pi, dt, st, 1, b, use_metric, 0, -1, koP, nko));
       WT_TRY(rk4_stage_part(ctx, ws, coef, Phi, Pi, dt, st, 2, b, use_metric, 0, -1, koQ, nko));
     } else {
@@ -1940,7 +1945,7 @@ int wt_step_rk4_curved(wt_ctx* ctx, wt_ws* ws, const wt_coef* coef, void* Phi, v
   wt::ConsBC b;
   WT_TRY(make_bc(ctx, bc, use_metric, b));
   WT_TRY(ws_step_buffers(ws));
-  if (eps_ko != 0.0 && ko_fused(ws->mesh->m)) WT_TRY(ko_buffers(ws));
+  if (eps_ko != 0.0 && ko_fused(ws->mesh->m)) WT_TRY(ko_buffers(ws, false));
   if (fused_path(ws, coef, Phi, Pi, eps_ko, b, use_metric)) WT_TRY(fused_buffer(ws, eps_ko));
   if (eps_ko != 0.0) WT_TRY(ensure_mu(ws));
   if (coef->td) WT_TRY(need_setup_geometry(coef->mesh, "wt_step_rk4_curved (time-dependent background)"));
@@ -2244,7 +2249,7 @@ static int step_sipg_once(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, 
     S.tau = tau;
     S.inv_R = (std::isfinite(R) && R > 0) ? 1.0 / R : 0.0;
     if (eps_ko != 0.0)
-      WT_TRY(ko_increments(ctx, ws, S.u, S.ut, eps_ko, &S.koU, &S.koV, &S.nko));
+      WT_TRY(ko_increments(ctx, ws, S.u, S.ut, eps_ko, true, &S.koU, &S.koV, &S.nko));
     S.rkU.on = S.rkV.on = 1;
     S.rkU.stage = S.rkV.stage = st;
     S.rkU.dt = S.rkV.dt = dt;
@@ -2266,7 +2271,7 @@ int wt_step_rk4_sipg(wt_ctx* ctx, wt_ws* ws, void* u, void* ut, double dt, int n
   if (!ws->mesh->m.affine) return fail(ctx, WT_ENOTSUP, "SIPG stepping supports affine meshes only");
   WT_TRY(ws_step_buffers(ws));
   if (eps_ko != 0.0) {  // buffers and mu before any graph capture
-    WT_TRY(ko_buffers(ws));
+    WT_TRY(ko_buffers(ws, true));
     WT_TRY(ensure_mu(ws));
   }
   const wt::DevMesh& m = ws->mesh->m;

@@ -236,15 +236,17 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long n, int i
 template <int N>
 struct Pen {
   static constexpr int N2 = N * N, N3 = N * N * N, TE = 3 * N2;
-  static constexpr int EPB = TE >= 96 ? 1 : N == 2 ? 8 : 160 / TE;  // the most elements a CTA holds (n = 2: 13 are 5-8 % slower)
+  // The most elements a CTA holds: 160 threads' worth (N = 2, where that is 13: 8, 5-8 % faster).
+  static constexpr int EPB = TE >= 96 ? 1 : N == 2 ? 8 : 160 / TE;
   static constexpr int T = TE * EPB;
   static constexpr int P1 = N | 1;       // odd row pitch: x pencils without bank conflicts
   static constexpr int NS = N * N * P1;  // words of one padded field of an element
   static constexpr int NI = (N3 + TE - 1) / TE;  // nodes per thread of the node pass
   // Threads per SM the registers are sized for.  FP64 up to N = 5: 768 (72
-  // registers, a few spills; 576 without spills took 15-30 % longer), N = 6: 640
-  // with the node pass's words prefetched (pf1), N = 7: 600, N = 8: 448 (at 768 the pencils
-  // spill: N = 7 33 % slower); FP32: 1024.
+  // registers; 576 without spills took 15-30 % longer), N = 6: 640 with the node pass's
+  // words prefetched (pf1), N = 7: 600, N = 8: 448 (N = 7 at 768: 33 % slower); FP32: 1024.
+  // A thread spills up to 60 bytes at most orders; K1 at N = 4 24 to 250 (affine), at N = 2
+  // 112 (affine), K1 and K2 at N = 7 FP64 140.
   // The affine form (CURV false) at N = 2 and 4, where the node pass is most of the work,
   // waits on its loads and takes more threads: one right-hand side of 1.5 million nodes, FP64
   // N = 4 96.0 -> 83.5 us, N = 2 112 -> 93.5; FP32 N = 4 69.0 -> 67.0, N = 2 83 -> 72 (a

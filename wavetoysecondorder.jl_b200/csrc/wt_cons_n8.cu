@@ -1464,13 +1464,15 @@ constexpr size_t k2c_smem() {
 // divergence partials wait in registers until F is free.  Neighbour traces go
 // straight to the thread whose pencil ends on them, which also evaluates the boundary
 // terms there; the node pass takes two nodes a thread.
-// Bound by issue and by the latency of the node words (see the profile of small cases);
-// the fused launch moves 35 words a node.
-// Measured (B200, 40^3 elements): RK4 step 4.9 ms, before this template 6.44; 16^3: step 365 us (525); 6^3: 43 us (74).  In sums and differences of
-// mirrored values, which round worse (see cc_contract), 1 % faster.  Of an earlier form: two-kernel stages
-// 5.36 ms against 4.87 fused; boundary terms in the node pass 4.73 for 4.70 ms, 373 for
-// 359 us, 57.5 for 41.3 us; four CTAs of 80 registers instead of five of 64 5.33 against
-// 5.04 ms; the loops over the components unrolled (instruction cache) 5.17 ms.
+// Bound by issue (58 %) and by the latency of the node words: 2090 instructions a warp in
+// the fused launch, which moves 35 words a node.
+// Measured (B200): RK4 step at 40^3 elements 4.9 ms, before this template 6.44; 16^3 365 us
+// (525); 6^3 43 us (74); one right-hand side at 40^3 1.24 ms (1.39).  In sums and
+// differences of mirrored values, which round worse (see cc_contract), 1 % faster.  Of an
+// earlier form: two-kernel stages 5.36 ms against 4.87 fused; boundary terms in the node
+// pass 4.73 for 4.70 ms, 373 for 359 us, 57.5 for 41.3 us; four CTAs of 80 registers
+// instead of five of 64 5.33 against 5.04 ms; the loops over the components unrolled
+// (instruction cache) 5.17 ms.
 // Error against FP64 (relative, pulses): Pi after one step on 24^3 elements 4.1e-7 (the
 // kernels before this template 4.7e-7), Phi 2.5e-8 (2.5e-8: its rounding to FP32).  After
 // 200 steps Pi 4.4e-7 (4.4e-7), Phi 4.6e-8 (4.0e-8); Phi is then within 0.4 and 1.7 times

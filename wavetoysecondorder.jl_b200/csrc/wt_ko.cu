@@ -11,8 +11,8 @@
 // is kernel parameters (constant bank: no shared-memory operand loads), of which
 // half the rows suffice: G is antisymmetric about its centre, G[N-1-i][N-1-p] =
 // -G[i][p], exactly as stored, so an entry serves both mirrored rows (with all rows
-// as operands the 64 registers spill and n = 8 takes four times as long).  Only the end values go through shared memory, double buffered, one barrier
-// per pass.  Axis 0 pencils are contiguous in memory: each warp transposes its 32
+// as operands the 64 registers spill and n = 8 takes four times as long).  Only the
+// end values go through shared memory, double buffered, one barrier per pass.  Axis 0 pencils are contiguous in memory: each warp transposes its 32
 // pencils through a padded shared buffer of its own; along axes 1 and 2 consecutive
 // threads hold consecutive nodes and load directly.
 //
@@ -21,15 +21,15 @@
 // error on a field that oscillates within an element (n = 8, one wavelength an element,
 // FP64: 3.3e-14 -> 1.5e-13; white noise 2.4e-16 -> 3.1e-16), so the passes take the plain
 // sums.  Where a pencil varies by less than half its size, the first pass takes the
-// values relative to the pencil's centre (G's rows sum to zero), which then loses
-// nothing on the way: the error of a resolved field falls (pulses of width 0.1 on 24
+// values relative to the pencil's centre (G's rows sum to zero), a difference that then
+// hardly rounds: the error of a resolved field falls (pulses of width 0.1 on 24
 // elements, n = 8: FP64 0.62, FP32 0.06 of the plain sums'), and no other field's
 // grows (within 3 %).
 //
 // Measured (FP64, three axes of one field, B200): 24^3 elements of n = 8, 114 us, 40^3 of
-// n = 6, 260 us (in sums and differences 96 and 247).  The whole pencils
-// through shared memory on every pass, two barriers each and the matrix read from there:
-// 315 and 680 us.
+// n = 6, 260 us (in sums and differences 96 and 247).  With the whole pencils through
+// shared memory on every pass, two barriers each and the matrix read from there: 315 and
+// 680 us.
 #include "wt_common.cuh"
 #include "wt_launch.cuh"
 

@@ -48,7 +48,7 @@ __device__ __forceinline__ real ctr(const real* __restrict__ f, const real* __re
 // derivative each (dd_01 along y, dd_02 and dd_12 along z) and the boundary terms
 // of the pencil's two ends (in the node pass, where most warps hold nodes of all
 // faces, they took a third of the instructions), then a node pass in node order.  Measured (FP64, n = 5, 28^3 elements, B200): 80 us
-// (3.0 TB/s), before 255 us.
+// (3.0 TB/s), before 255 us.  (At N = 8 a thread spills 160 bytes.)
 template <int N, typename real>
 struct StrongP {
   double G[N * N];
