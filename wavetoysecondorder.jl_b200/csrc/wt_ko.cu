@@ -20,14 +20,15 @@
 // but their own rounding, amplified by six passes, is 1.3 to 4.7 times the plain sums'
 // error on a field that oscillates within an element (n = 8, one wavelength an element,
 // FP64: 3.3e-14 -> 1.5e-13; white noise 2.4e-16 -> 3.1e-16), so the passes take the plain
-// sums.  Where a pencil varies by less than half its size, the first pass takes the
-// values relative to the pencil's centre (G's rows sum to zero), a difference that then
-// hardly rounds: the error of a resolved field falls (pulses of width 0.1 on 24
-// elements, n = 8: FP64 0.62, FP32 0.06 of the plain sums'), and no other field's
-// grows (within 3 %).
+// sums.  Where a pencil varies by less than half its size (at four of its nodes: all
+// decide alike), the first pass takes the values relative to the pencil's centre (G's
+// rows sum to zero), a difference that then hardly rounds: the error of a resolved field
+// falls (pulses of width 0.1 on 24 elements, n = 8: FP64 0.62, FP32 0.06 of the plain
+// sums'), and no other field's grows (within 3 %; at n = 5 and 7 by up to a third against
+// a reference that counts the stored rows' sums, 1e-15, as the operator's).
 //
-// Measured (FP64, three axes of one field, B200): 24^3 elements of n = 8, 114 us, 40^3 of
-// n = 6, 260 us (in sums and differences 96 and 247).  With the whole pencils through
+// Measured (FP64, three axes of one field, B200): 24^3 elements of n = 8, 109 us, 40^3 of
+// n = 6, 263 us (in sums and differences 97 and 250).  With the whole pencils through
 // shared memory on every pass, two barriers each and the matrix read from there: 315 and
 // 680 us.
 #include "wt_common.cuh"
@@ -135,7 +136,8 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
   real c = v[HH];
   int mv = 0, mc = 0;
 #pragma unroll
-  for (int l = 0; l < N; ++l) {
+  for (int q = 0; q < 4; ++q) {
+    const int l = q == 0 ? 0 : q == 1 ? (N > 2 ? 2 : 1) : q == 2 ? (N > 3 ? N - 3 : 0) : N - 1;
     mv = max(mv, mag(v[l]));
     mc = max(mc, mag(v[l] - c));
   }
@@ -167,7 +169,8 @@ __global__ void __launch_bounds__(TMAX, 1024 / TMAX) k_ko(const __grid_constant_
     for (int l = 0; l < N; ++l) v[l] = s * w[l];
   };
   pass(0, [&](int p) { return v[p] - c; });
-#pragma unroll 1
+  constexpr int UN = N == 6 ? 1 : 5;  // (unrolled: 40^3 of n = 6 8 % slower, 24^3 of n = 8 4 % faster)
+#pragma unroll UN
   for (int it = 1; it < 6; ++it) pass(it, [&](int p) { return v[p]; });
 #pragma unroll
   for (int l = 0; l < N; ++l) v[l] *= P.koT;
