@@ -572,7 +572,7 @@ int wt_snapshot_load(wt_ctx* ctx, wt_mesh* mesh, void* Phi, void* Pi, double* t,
  * parallel branches of that graph.  The first step after a change also picks
  * the launch variant of the generic (n != 8) kernels, K1 and K2 separately, by
  * timing (autotuner, on by default): 0 the default elements per CTA, 1 half of
- * it, 2 (n = 4 and 6) one.  A CTA holds 8 elements of n = 2, 5 of n = 3, 3 of
+ * it, 2 (n = 4 and 6) one.  A CTA holds 13 elements of n = 2, 5 of n = 3, 3 of
  * n = 4, 2 of n = 5 and one from n = 6, where all variants are the same launch
  * and none is timed; every variant gives the same bits
  * (wt_batch_group_info's epb_variant: bits 0-1 K1's variant, bits 2-3 K2's).  A member with a time-dependent background is re-sampled at

@@ -236,8 +236,7 @@ __device__ __forceinline__ void k1_finish(const K1P<real>& P, long long n, int i
 template <int N>
 struct Pen {
   static constexpr int N2 = N * N, N3 = N * N * N, TE = 3 * N2;
-  // The most elements a CTA holds: 160 threads' worth (N = 2, where that is 13: 8, 5-8 % faster).
-  static constexpr int EPB = TE >= 96 ? 1 : N == 2 ? 8 : 160 / TE;
+  static constexpr int EPB = TE >= 96 ? 1 : 160 / TE;  // the most elements a CTA holds
   static constexpr int T = TE * EPB;
   static constexpr int P1 = N | 1;       // odd row pitch: x pencils without bank conflicts
   static constexpr int NS = N * N * P1;  // words of one padded field of an element
@@ -245,8 +244,8 @@ struct Pen {
   // Threads per SM the registers are sized for.  FP64 up to N = 5: 768 (72
   // registers; 576 without spills took 15-30 % longer), N = 6: 640 with the node pass's
   // words prefetched (pf1), N = 7: 600, N = 8: 448 (N = 7 at 768: 33 % slower); FP32: 1024.
-  // A thread spills up to 60 bytes at most orders; K1 at N = 4 24 to 250 (affine), at N = 2
-  // 112 (affine), K1 and K2 at N = 7 FP64 140.
+  // A thread spills up to 60 bytes at most orders; at N = 7 FP64 K2 80, batches 164; the
+  // affine form at N = 2 and 4 FP64 104 and 252.
   // The affine form (CURV false) at N = 2 and 4, where the node pass is most of the work,
   // waits on its loads and takes more threads: one right-hand side of 1.5 million nodes, FP64
   // N = 4 96.0 -> 83.5 us, N = 2 112 -> 93.5; FP32 N = 4 69.0 -> 67.0, N = 2 83 -> 72 (a
@@ -268,10 +267,10 @@ struct Pen {
 
 // the operator: G in FP64 (CP's gradient of Phi) and in the state's type, 1 / (2 H_end)
 template <int N, typename real>
-struct OpP {
+struct alignas(16) OpP {  // G off a 16-byte boundary: taken in pairs its entries spill (N = 7 FP64 K1 11 % slower)
+  real c2H;
   real G[N * N];
   double Gd[N * N];
-  real c2H;
 };
 
 // where a tile's element is: false if there is none
@@ -830,12 +829,13 @@ static OpP<N, real> op_params(const DevMesh* m) {
   return O;
 }
 
-// Elements per CTA.  Default (variant 0): Pen<N>::EPB, fewer where the work would
-// otherwise leave SMs without a CTA; variants 1 and 2 (batches): half and one.
-// (One CTA shape gives the same bits as another.)
-template <int N>
+// Elements per CTA.  Default (variant 0): Pen<N>::EPB (affine form at N = 2: 8 of its 13,
+// 5-8 % faster), fewer where the work would otherwise leave SMs without a CTA; variants 1
+// and 2 (batches): half and one.  (One CTA shape gives the same bits as another.)
+template <int N, bool CURV>
 static int elements_per_cta(long long ne, int variant) {
-  const int most = variant == 0 ? Pen<N>::EPB : variant == 1 ? (Pen<N>::EPB + 1) / 2 : 1;
+  const int all = N == 2 && !CURV ? 8 : Pen<N>::EPB;
+  const int most = variant == 0 ? all : variant == 1 ? (Pen<N>::EPB + 1) / 2 : 1;
   const long long fill = ne / (2 * 148);
   return (int)(fill < 1 ? 1 : fill < most ? fill : most);
 }
@@ -858,7 +858,7 @@ template <int N, typename real, bool CURV, bool BATCH, bool CP>
 static int k1_run(const K1P<real>& P, const OpP<N, real>& O, const void* plist, const int2* tiles, long long ne,
                   int variant, cudaStream_t s) {
   if (ne <= 0) return 0;
-  const int epb = elements_per_cta<N>(ne, variant);
+  const int epb = elements_per_cta<N, CURV>(ne, variant);
   // room for the boundary increments of Phidot where there can be any (full-Dirichlet faces)
   const int dfw = BATCH || (P.bc_on && k1_phi_increments(P)) ? 6 * Pen<N>::N2 : 0;
   const size_t smem = (size_t)epb * (k1_words<N, real, CURV, CP>() + dfw) * sizeof(real);
@@ -871,7 +871,7 @@ template <int N, typename real, bool CURV, bool BATCH>
 static int k2_run(const K2P<real>& P, const OpP<N, real>& O, const void* plist, const int2* tiles, long long ne,
                   int variant, cudaStream_t s) {
   if (ne <= 0) return 0;
-  const int epb = elements_per_cta<N>(ne, variant);
+  const int epb = elements_per_cta<N, CURV>(ne, variant);
   const size_t smem = (size_t)epb * k2_words<N, CURV>() * sizeof(real);
   if (gen_smem(k_cons_k2<N, real, CURV, BATCH>, smem)) return -2;
   return launch_dep<!BATCH>(k_cons_k2<N, real, CURV, BATCH>, (unsigned)((ne + epb - 1) / epb), Pen<N>::TE * epb, smem, s, P, O,

@@ -21,6 +21,10 @@
 // cp.async under the contractions: what bounds the kernel is the latency of its
 // loads (42 % of the warps resident, 38 % of DRAM bandwidth).
 //
+// One instantiation each for the right-hand side, the stage and the traces: a stage that
+// is switched off at run time costs the right-hand side up to 30 % (1.5 million nodes, FP64
+// n = 4 39 -> 31 us, n = 6 28.6 -> 22.8).
+//
 // Measured (FP64, n = 6, 40^3 elements, one stage, B200): 361 us, where the
 // trace, right-hand-side (thread per node, operands from shared memory), copy and
 // two update kernels took 1.1 ms; 4^3 elements: 4.5 us a launch in the replayed
@@ -54,7 +58,7 @@ struct SipgP {
   const real* bnorm;
   real bv[6];
   real tau, inv_R;
-  int epi, stage;        // fused RK4 stage of u_t = ut + koU, ut_t = L u + koV
+  int stage;             // fused RK4 stage of u_t = ut + koU, ut_t = L u + koV
   double dt;
   int nko;               // dissipation increments per field (0, 1 or 3 fields of nn words)
   const real* koU;
@@ -68,9 +72,13 @@ struct SipgEp {
   static constexpr int MAX = 3 * N * N >= 128 ? 1 : 224 / (3 * N * N);
 };
 
-template <int N, typename real, bool TRACE>
+// what a launch does: the right-hand side, the RK4 stage, the traces of u alone
+enum { SIPG_RHS = 0, SIPG_STAGE = 1, SIPG_TRACE = 2 };
+
+template <int N, typename real, int MODE>
 __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N * SipgEp<N>::MAX))
     k_sipg(const __grid_constant__ SipgP<N, real> P, int epb) {
+  constexpr bool TRACE = MODE == SIPG_TRACE, EPI = MODE == SIPG_STAGE;
   constexpr int N2 = N * N, N3 = N * N * N, TE = 3 * N2;
   constexpr int P1 = N | 1;        // odd row pitch: x pencils without bank conflicts
   constexpr int NS = N * N * P1;   // words of one field of an element
@@ -125,7 +133,7 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
   // increments, RK states and accumulators
   real* sw = reinterpret_cast<real*>(smraw) + (size_t)4 * epb * NS + (size_t)le * (5 + 2 * P.nko) * N3;
   const bool ld_y = P.stage == 1 || P.stage == 2, ld_acc = P.stage >= 1;
-  if (!TRACE && P.epi) {
+  if constexpr (EPI) {
 #pragma unroll
     for (int it = 0; it < NI; ++it) {
       const int w = t + it * TE;
@@ -225,7 +233,7 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
         const int at = place(wn);
         const long long n = ec * N3 + wn;
         real kV = sr[at] + sr[NS + at] + sr[2 * NS + at];
-        if (!P.epi) {
+        if constexpr (!EPI) {
           P.utt[n] = kV;
           continue;
         }
@@ -242,9 +250,10 @@ __global__ void __launch_bounds__(3 * N * N * SipgEp<N>::MAX, 900 / (3 * N * N *
         rk_epilogue_v<real>(P.stage, P.dt, kV, vin, yV, aV, (real)0, P.yV, P.accV, P.outV, nullptr, n, nullptr);
       }
     }
-    if (!P.epi) return;
-    __syncthreads();
-    if (valid) ends();  // traces of the new u for the next stage
+    if constexpr (EPI) {
+      __syncthreads();
+      if (valid) ends();  // traces of the new u for the next stage
+    }
   }
 }
 
@@ -265,32 +274,35 @@ static SipgP<N, real> sipg_params(const DevMesh& m, const SipgStage& S) {
   P.nbf = m.nbf; P.bnorm = (const real*)m.bnorm;
   for (int f = 0; f < 6; ++f) P.bv[f] = (real)S.bvals[f];
   P.tau = (real)S.tau; P.inv_R = (real)S.inv_R;
-  P.epi = S.rkU.on; P.stage = S.rkU.stage; P.dt = S.rkU.dt;
+  P.stage = S.rkU.stage; P.dt = S.rkU.dt;
   P.nko = S.nko; P.koU = (const real*)S.koU; P.koV = (const real*)S.koV;
   P.yU = (real*)S.rkU.y; P.accU = (real*)S.rkU.acc; P.outU = (real*)S.rkU.out;
   P.yV = (real*)S.rkV.y; P.accV = (real*)S.rkV.acc; P.outV = (real*)S.rkV.out;
   return P;
 }
 
-template <int N, typename real>
-static int sipg_run(const DevMesh& m, const SipgStage& S, bool trace_only, cudaStream_t s) {
+template <int N, typename real, int MODE>
+static int sipg_run(const DevMesh& m, const SipgStage& S, cudaStream_t s) {
   const SipgP<N, real> P = sipg_params<N, real>(m, S);
   // fewer elements per CTA when the mesh would not give every SM a CTA
   const int epb = (int)std::max<long long>(1, std::min<long long>(SipgEp<N>::MAX, m.Ne / 148));
   const unsigned blocks = (unsigned)((m.Ne + epb - 1) / epb);
-  size_t smem = (size_t)(trace_only ? 1 : 4) * epb * N * N * (N | 1) * sizeof(real);
-  if (P.epi) smem += (size_t)(5 + 2 * P.nko) * epb * N * N * N * sizeof(real);
-  if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k_sipg<N, real, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess)
-    return -2;
-  return launch_dep(trace_only ? k_sipg<N, real, true> : k_sipg<N, real, false>, blocks, 3 * N * N * epb, smem, s, P,
-                    epb);
+  size_t smem = (size_t)(MODE == SIPG_TRACE ? 1 : 4) * epb * N * N * (N | 1) * sizeof(real);
+  if (MODE == SIPG_STAGE) smem += (size_t)(5 + 2 * P.nko) * epb * N * N * N * sizeof(real);
+  if (smem > 48 * 1024 && allow_smem(k_sipg<N, real, MODE>, smem)) return -2;
+  return launch_dep(k_sipg<N, real, MODE>, blocks, 3 * N * N * epb, smem, s, P, epb);
+}
+
+template <int N, typename real>
+static int sipg_mode(const DevMesh& m, const SipgStage& S, bool trace_only, cudaStream_t s) {
+  return trace_only    ? sipg_run<N, real, SIPG_TRACE>(m, S, s)
+         : S.rkU.on    ? sipg_run<N, real, SIPG_STAGE>(m, S, s)
+                       : sipg_run<N, real, SIPG_RHS>(m, S, s);
 }
 
 int launch_sipg(const DevMesh& m, const SipgStage& S, bool trace_only, cudaStream_t s) {
 #define WT_SIPG_CASE(NN) \
-  case NN: return m.precision == 0 ? sipg_run<NN, double>(m, S, trace_only, s) : sipg_run<NN, float>(m, S, trace_only, s);
+  case NN: return m.precision == 0 ? sipg_mode<NN, double>(m, S, trace_only, s) : sipg_mode<NN, float>(m, S, trace_only, s);
   switch (m.N) {
     WT_SIPG_CASE(2) WT_SIPG_CASE(3) WT_SIPG_CASE(4) WT_SIPG_CASE(5) WT_SIPG_CASE(6) WT_SIPG_CASE(7) WT_SIPG_CASE(8)
     default: return -4;
