@@ -2663,10 +2663,10 @@ int batch_one_step(wt_batch* b, cudaStream_t s) {
   return 0;
 }
 
-// Time K1 and K2 of stage 0 of a generic group in each launch variant
-// of its own CTA shape and keep the fastest of each (stage 0 writes only stage
-// scratch, never the solution state; orders with one shape: nothing to time).  epb_variant: bits 0-1 K1's choice, bits
-// 2-3 K2's.  A variant fixed by wt_batch_set_variant is kept untimed.
+// Time K1 and K2 of stage 0 of a generic group in each launch variant of its own CTA
+// shape and keep the fastest of each (stage 0 writes only stage scratch, never the
+// solution state; orders with one shape: nothing to time).  epb_variant: bits 0-1 K1's
+// choice, bits 2-3 K2's.  A variant fixed by wt_batch_set_variant is kept untimed.
 int batch_tune_group(wt_batch* b, wt_batch::Group& g) {
   cudaStream_t s = b->ctx->own_stream;
   cudaEvent_t e0, e1;

@@ -1485,13 +1485,14 @@ constexpr size_t cc_smem(int half) {
 }
 static_assert(CC_OCC * (cc_smem(N8_FK) + 128 + 1024) <= 233472, "CC_OCC fused CTAs must fit an SM");
 
-// out = 0.5 D v, two rows of a column a packed FMA, summed in the columns' order.  Where
-// the pencil varies by less than three quarters of its size (at four of its nodes: all
-// eight decide alike and cost 1 % of the step), v is taken relative to its centre (G's rows sum to zero; their rounding to FP32 then makes no derivative of a
+// out = 0.5 D v, two rows of a column a packed FMA, summed in the columns' order.
+// Where the pencil varies by less than three quarters of its size (at four of its
+// nodes: all eight decide alike and cost 1 % of the step), v is taken relative to its
+// centre (G's rows sum to zero; their rounding to FP32 then makes no derivative of a
 // constant).  Rounding against 64 bits, FP32 values, plain sums / so / in sums and
 // differences of mirrored values (which take half the multiply-adds): a sixth of a
-// wavelength an element 9.1e-7 / 4.4e-7 / 4.9e-7, a half 3.0 / 3.0 / 4.3e-7, one 1.4 / 1.4 /
-// 2.9e-7, white noise 5.9 / 5.9 / 7.1e-8.
+// wavelength an element 9.1e-7 / 4.4e-7 / 4.9e-7, a half 3.0 / 3.0 / 4.3e-7, one 1.4 /
+// 1.4 / 2.9e-7, white noise 5.9 / 5.9 / 7.1e-8.
 __device__ __forceinline__ void cc_contract(const float2* G, const float v[8], float out[8]) {
   float c = v[3];
   const float mv = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[2])), fmaxf(fabsf(v[5]), fabsf(v[7])));

@@ -6,15 +6,15 @@
 // in registers and the threads of a CTA hold whole element lines: applying D_d
 // six times needs, per pass, only the two end values of the pencils next to it.
 //
-// What bounds it: per axis and field 3 words of DRAM traffic per node (the
-// field in, the destination in and out) against 6 N multiply-adds.  The operator
-// is kernel parameters (constant bank: no shared-memory operand loads), of which
-// half the rows suffice: G is antisymmetric about its centre, G[N-1-i][N-1-p] =
-// -G[i][p], exactly as stored, so an entry serves both mirrored rows (with all rows
-// as operands the 64 registers spill and n = 8 takes four times as long).  Only the
-// end values go through shared memory, double buffered, one barrier per pass.  Axis 0 pencils are contiguous in memory: each warp transposes its 32
-// pencils through a padded shared buffer of its own; along axes 1 and 2 consecutive
-// threads hold consecutive nodes and load directly.
+// What bounds it: per axis and field 3 words of DRAM traffic per node (the field in,
+// the destination in and out) against 6 N multiply-adds.  The operator is kernel
+// parameters (constant bank: no shared-memory operand loads), of which half the rows
+// suffice: G is antisymmetric about its centre, G[N-1-i][N-1-p] = -G[i][p], exactly as
+// stored, so an entry serves both mirrored rows (with all rows as operands the 64
+// registers spill and n = 8 takes four times as long).  Only the end values go through
+// shared memory, double buffered, one barrier per pass.  Axis 0 pencils are contiguous
+// in memory: each warp transposes its 32 pencils through a padded shared buffer of its
+// own; along axes 1 and 2 consecutive threads hold consecutive nodes and load directly.
 //
 // Rounding.  Sums and differences of mirrored values would halve the multiply-adds,
 // but their own rounding, amplified by six passes, is 1.3 to 4.7 times the plain sums'

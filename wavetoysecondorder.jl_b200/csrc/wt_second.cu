@@ -41,14 +41,14 @@ __device__ __forceinline__ real ctr(const real* __restrict__ f, const real* __re
 // s sum_b G^{ab} d_b / |n|, |n|^2 = G^{aa}, so the interior / Dirichlet SAT is
 //   -(s sum_b G^{ab} d_b + tau |n| (u - u_nbr)) / H_r.
 //
-// Bound by memory latency and bandwidth: 11 words a node (u, nine coefficients,
-// the result; the 9 inverse-Jacobian entries and their 27 derivatives, node-major,
-// were 36).  3 N^2 threads per element, one per (axis, pencil), operator in the
-// constant bank: first d_a and dd_aa along the own axis, then one mixed
-// derivative each (dd_01 along y, dd_02 and dd_12 along z) and the boundary terms
-// of the pencil's two ends (in the node pass, where most warps hold nodes of all
-// faces, they took a third of the instructions), then a node pass in node order.  Measured (FP64, n = 5, 28^3 elements, B200): 80 us
-// (3.0 TB/s), before 255 us.  (At N = 8 a thread spills 160 bytes.)
+// Bound by memory latency and bandwidth: 11 words a node (u, nine coefficients, the
+// result; the 9 inverse-Jacobian entries and their 27 derivatives, node-major, were
+// 36).  3 N^2 threads per element, one per (axis, pencil), operator in the constant
+// bank: first d_a and dd_aa along the own axis, then one mixed derivative each (dd_01
+// along y, dd_02 and dd_12 along z) and the boundary terms of the pencil's two ends (in
+// the node pass, where most warps hold nodes of all faces, they took a third of the
+// instructions), then a node pass in node order.  Measured (FP64, n = 5, 28^3 elements,
+// B200): 80 us (3.0 TB/s), before 255 us.  (At N = 8 a thread spills 160 bytes.)
 template <int N, typename real>
 struct StrongP {
   double G[N * N];

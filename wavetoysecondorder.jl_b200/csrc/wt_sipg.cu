@@ -19,13 +19,14 @@
 // normal-derivative traces that the next stage reads, so no separate trace,
 // copy or update pass over the fields is left.  The node pass's words arrive by
 // cp.async under the contractions: what bounds the kernel is the latency of its
-// loads (42 % of the warps resident, 38 % of DRAM bandwidth).
+// loads (41 % of the warps resident, 3.9 TB/s).
 //
 // One instantiation each for the right-hand side, the stage and the traces: a stage that
 // is switched off at run time costs the right-hand side up to 30 % (1.5 million nodes, FP64
 // n = 4 39 -> 31 us, n = 6 28.6 -> 22.8).
 //
-// Measured (FP64, n = 6, 40^3 elements, one stage, B200): 361 us, where the
+// Measured (FP64, n = 6, 40^3 elements, one stage, B200): 290 us, 355 with dissipation
+// increments, where the
 // trace, right-hand-side (thread per node, operands from shared memory), copy and
 // two update kernels took 1.1 ms; 4^3 elements: 4.5 us a launch in the replayed
 // graph, two launches a stage instead of eleven.
